@@ -20,6 +20,8 @@ OK, TRUNCATED, NO_CHAIN, CORRUPT_BLOCK, INFLATE, CRC, TOO_MANY, CAPACITY, CUDA, 
 #: launch parameters (cb_set_param / cb_get_param)
 (PARAM_CHAIN_TILE, PARAM_INFLATE_FORM, PARAM_DECODE_ROOT, PARAM_COPY_WARPS, PARAM_DECODE_STEPS, PARAM_DECODE_PREFETCH,
  PARAM_SPLIT_MIN_JOBS, PARAM_COPY_UNITS, PARAM_DECODE_PIPELINE) = range(1, 10)
+#: PARAM_SPLIT_MIN_JOBS by default: form 3 for any number of jobs
+SPLIT_MIN_JOBS_ANY = 8192
 
 
 class MemberJob(ctypes.Structure):

@@ -53,9 +53,9 @@ def _tag_arrays(k: int, nrec: int):
 
 
 def inflate_launches(form: int = 0, n_jobs: int | None = None) -> int:
-    """Kernels of one inflate call: init, the persistent grid, finish; form 3 adds the slot scan and
-    splits the grid into decode and copy."""
-    return 5 if inflate_form(form, n_jobs) == 3 else KERNELS["inflate"]
+    """Kernels of one inflate call: init, the persistent grid, finish; form 3 adds the slot scan, splits
+    the grid into decode, copy and CRC32, and launches the one-kernel form for members it leaves."""
+    return 7 if inflate_form(form, n_jobs) == 3 else KERNELS["inflate"]
 
 
 @dataclass
@@ -251,8 +251,8 @@ class BatchPlan:
     with one launch; :meth:`check` reads every device summary with one copy and raises on a
     status or on counts that differ from the plan.
 
-    ``form`` is the inflate form (1: a member per warp, 2: a member per lane, 3: decode per lane and
-    copy per warp); None lets :meth:`autotune` choose it, with the other launch parameters, by timing
+    ``form`` is the inflate form (1: a member per warp, 2: a member per lane, 3: decode, copy and CRC32
+    as kernels of their own); None lets :meth:`autotune` choose it, with the other launch parameters, by timing
     this batch (or from the tuning cache for a batch of the same shape on the same device).
     """
 

@@ -13,8 +13,9 @@ Same API and chunk semantics as cubam's ``src/cubam/bgzf.py`` read side
    inflate job per non-empty member is written with its output offset.  The
    compressed bytes of the incomplete last member stay on the GPU.
 3. **Inflate.** ``cb_inflate_form`` in the library's default form (form 3:
-   the Huffman decode with one member per lane into a token arena, then the
-   copy with one member per warp), with the CRC32 and ISIZE checks.
+   the Huffman decode into an arena of symbols, a warp per member whose lanes
+   decode 32 segments of it at once, then the copy and the CRC32, each with a
+   warp per member), with the CRC32 and ISIZE checks.
 
 Errors are the reference's ``ValueError`` messages; a CRC32 mismatch (which
 cubam does not check) is a ``ValueError`` too, unless ``check_crc=False``.
@@ -240,11 +241,12 @@ def scan_members(buf: torch.Tensor, eof: bool, out_base: int = 0, jobs_cap: int 
 def inflate_form(form: int = 0, n_jobs: int | None = None) -> int:
     """The inflate form a call of ``n_jobs`` jobs with ``form`` runs, as ``cb_inflate_form`` chooses it:
     0 is the library's default (``CB_PARAM_INFLATE_FORM``; form 1 in place of form 3 below
-    ``CB_PARAM_SPLIT_MIN_JOBS`` jobs)."""
+    ``CB_PARAM_SPLIT_MIN_JOBS`` jobs, when that was set)."""
     if form:
         return int(form)
     f = int(_lib.lib.cb_get_param(_lib.PARAM_INFLATE_FORM))
-    if f == 3 and n_jobs is not None and n_jobs < int(_lib.lib.cb_get_param(_lib.PARAM_SPLIT_MIN_JOBS)):
+    least = int(_lib.lib.cb_get_param(_lib.PARAM_SPLIT_MIN_JOBS))
+    if f == 3 and n_jobs is not None and least != _lib.SPLIT_MIN_JOBS_ANY and n_jobs < least:
         return 1
     return f
 
@@ -270,7 +272,7 @@ def inflate_jobs(jobs: torch.Tensor, n_jobs: int, out: torch.Tensor, check_crc: 
     """Launch ``cb_inflate_form`` of ``n_jobs`` jobs into ``out``; returns the device summary (no sync).
 
     ``form`` 0 lets the library choose (``CB_PARAM_INFLATE_FORM``), 1 is one member per warp, 2 one per
-    lane, 3 the two-kernel form (``cb_inflate_split``: decode one member per lane, copy one per warp).
+    lane, 3 the split form (``cb_inflate_split``: decode, copy and CRC32 as kernels of their own).
     ``job_status`` (device uint32/int32 of ``n_jobs``) receives a status code per job when given.
     """
     summ = torch.zeros(ctypes_sizeof(_lib.InflateSummary), dtype=torch.uint8, device="cuda")

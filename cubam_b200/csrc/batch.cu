@@ -127,9 +127,8 @@ int header_size(const uint8_t* dev, int64_t avail, cudaStream_t s, int64_t* size
 }
 
 int inflate_ws_for(cb_batch* b) {
-    int64_t form = cb_param(CB_PARAM_INFLATE_FORM);
-    if (form == 3 && b->total_jobs < cb_param(CB_PARAM_SPLIT_MIN_JOBS)) form = 1;
-    b->form = (int)form;
+    const int form = cb_default_form(b->total_jobs);
+    b->form = form;
     b->inflate_ws_bytes = form == 3 ? cb_inflate_split_workspace_bytes(b->total_jobs, b->total_out)
                                     : cb_inflate_workspace_bytes();
     if (b->inflate_ws_bytes < 512) b->inflate_ws_bytes = 512;

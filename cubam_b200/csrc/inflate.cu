@@ -12,12 +12,15 @@
 //  2. one member per lane (k_inflate_lanes): 8 lanes of each of 16 warps per SM each inflate a
 //     member of their own, 128 members per SM in flight.
 //
-// cb_inflate runs form 1 (the faster at every batch size measured); cb_inflate_form takes the form
-// from the caller.
+// cb_inflate runs form 3 (inflate_split.cu) unless its workspace is of these forms' size; then, and
+// for the members form 3 leaves (k_inflate_listed), form 1 runs.  cb_inflate_form takes the form from
+// the caller.
 //
 // Every loop is bounded by the member's sizes or a fixed count: output beyond ISIZE, a distance
 // before the member's start, bits read beyond the payload, bad code lengths and invalid symbols are
 // per-member errors.
+
+#include <atomic>
 
 #include "common.cuh"
 #include "crc.cuh"
@@ -1184,6 +1187,36 @@ __global__ void __launch_bounds__(wm::WARPS * 32, 4)
     }
 }
 
+// The jobs list[4 * k], k < *count: the members that the two-kernel form leaves (usually none).
+__global__ void __launch_bounds__(wm::WARPS * 32, 4)
+    k_inflate_listed(const cb_member_job* __restrict__ jobs, const uint32_t* __restrict__ list,
+                     const unsigned long long* __restrict__ count, uint8_t* out_base, int check_crc,
+                     uint32_t* job_status, cb_inflate_summary* summary, unsigned long long* queue) {
+    const unsigned long long n = *count;
+    if (n == 0) return;
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    wm::CtaSmem& S = *reinterpret_cast<wm::CtaSmem*>(smem_raw);
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+#pragma unroll
+        for (int b = 0; b < 4; b++) S.mulk[b][i] = gf_mul((uint32_t)i << (8 * b), kCrc.k992);
+    }
+    init_crc8(S.crc8);
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    wm::WarpSmem& W = S.w[threadIdx.x >> 5];
+    for (;;) {
+        unsigned long long k = 0;
+        if (lane == 0) k = atomicAdd(queue, 1ull);
+        k = __shfl_sync(FULL, k, 0);
+        if (k >= n) break;
+        const uint32_t j = list[4 * k];
+        const cb_member_job job = jobs[j];
+        const uint32_t st = inflate_member(job, out_base, check_crc != 0, W, S);
+        __syncwarp();
+        if (lane == 0) report(summary, job_status, (long long)j, st);
+    }
+}
+
 template <class C>
 __global__ void __launch_bounds__(C::WARPS * 32, 1)
     k_inflate_lanes(const cb_member_job* __restrict__ jobs, int64_t n_jobs, const int64_t* __restrict__ d_n_jobs,
@@ -1359,6 +1392,10 @@ __global__ void __launch_bounds__(C::WARPS * 32, 1)
 using namespace cb;
 
 int cb_set_error(cudaError_t e);  // abi.cu
+// inflate_split.cu: cb_inflate_split; with list_unfit the jobs that the workspace does not hold are inflated too
+int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base,
+                         int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
+                         size_t workspace_bytes, bool list_unfit, void* stream);
 
 namespace {
 
@@ -1410,19 +1447,40 @@ extern "C" int64_t cb_inflate_lane_slots(void) {
     return (int64_t)cb_device_sm_count() * b * Form2::WARPS * Form2::MLANES;
 }
 
+int cb_inflate_listed(const cb_member_job* jobs, const uint32_t* list, const unsigned long long* count,
+                      uint8_t* out_base, int check_crc, uint32_t* job_status, cb_inflate_summary* summary,
+                      unsigned long long* queue, cudaStream_t s) {
+    const size_t smem = sizeof(infl::wm::CtaSmem);
+    static std::atomic<bool> attr_set[MAX_DEVICES];
+    const int dev = cur_device();
+    if (dev < 0 || !attr_set[dev].load(std::memory_order_acquire)) {
+        const cudaError_t e = cudaFuncSetAttribute(infl::k_inflate_listed, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)smem);
+        if (e != cudaSuccess) return cb_set_error(e);
+        if (dev >= 0) attr_set[dev].store(true, std::memory_order_release);
+    }
+    infl::k_inflate_listed<<<cb_device_sm_count() * 2, infl::wm::WARPS * 32, smem, s>>>(
+        jobs, list, count, out_base, check_crc, job_status, summary, queue);
+    return cb_set_error(cudaGetLastError());
+}
+
 extern "C" int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base,
                                int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
                                size_t workspace_bytes, int form, void* stream) {
     if (!summary || !workspace || workspace_bytes < cb_inflate_workspace_bytes() || n_jobs < 0) return CB_ERR_ARG;
+    // A call of few jobs that leaves the form to the library takes any workspace: what of it form 3's arena
+    // does not hold is inflated by the one-kernel form.
+    bool any_workspace = false;
     if (form == 0) {
-        form = (int)cb_param(CB_PARAM_INFLATE_FORM);
-        if (form == 3 && n_jobs < cb_param(CB_PARAM_SPLIT_MIN_JOBS)) form = 1;
+        form = cb_default_form(n_jobs);
+        any_workspace = form == 3 && n_jobs < CB_SPLIT_MIN_JOBS_ANY;
+        if (any_workspace && workspace_bytes < cb_inflate_split_workspace_bytes(n_jobs, 0)) form = 1;
     }
     if (form == 3) {
-        // the split form needs its token arena: a workspace of the forms-1/2 size runs form 1 instead
+        // the split form needs its arena: a workspace of the forms-1/2 size runs form 1 instead
         if (workspace_bytes > cb_inflate_workspace_bytes())
-            return cb_inflate_split(jobs, n_jobs, d_n_jobs, out_base, check_crc, job_status, summary, workspace,
-                                    workspace_bytes, stream);
+            return cb_inflate_split_any(jobs, n_jobs, d_n_jobs, out_base, check_crc, job_status, summary, workspace,
+                                        workspace_bytes, any_workspace, stream);
         form = 1;
     }
     if (form != 1 && form != 2) return CB_ERR_ARG;

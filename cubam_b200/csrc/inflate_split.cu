@@ -4,36 +4,28 @@
 // (src/cubam/bgzf.py:587-611) with the CRC32 check added (cubam's reader does not check it,
 // docs/reading.md:48-51).  DEFLATE is RFC 1951.
 //
-// Why two kernels.  Huffman decoding is serial within a member, and the copy of a back-reference
-// needs the member's output up to 32 KiB back.  In BGZF files of BAM records most references reach
-// far (on the GEX-shaped workload the median distance is about 3 KB and only 7% are within 224
-// bytes), so a decoder that also copies either keeps 32 KiB per member on chip (few members in
-// flight, idle issue slots) or reads HBM at every match (long waits).  Here:
+//  1. k_decode: one member per WARP, its 32 lanes decoding 32 segments of the member's bits at once.
+//     A Huffman decoder that starts at a wrong bit falls in step with the true symbols soon (on BAM
+//     members after 64 bits in half of the cases, after 512 in 99.5%), so every lane starts OVERLAP
+//     bits before its segment and notes the first symbol that begins in it; that must be where the
+//     lane before stopped, and a lane for which it is not decodes its segment again from there.  The
+//     lanes share one set of code tables in shared memory.  Their symbols go to the member's slot of
+//     an arena in HBM as runs (one per lane): literal bytes, and 4-byte sequences of a literal count
+//     and a match.
+//  2. k_copy: one member per WARP.  The warp takes 64 sequences at a time, places them by a prefix sum
+//     of their lengths and writes the output 128 bytes per round, a 4-byte word per lane, to a ring
+//     in shared memory (the sources of matches) and to HBM.
+//  3. k_crc: the CRC32 of every member's output, a warp per member, in registers.
+//  4. Members whose symbols do not fit their slot (many tiny blocks) are inflated by the one-kernel
+//     form (cb_inflate_listed, inflate.cu).
 //
-//  1. k_decode: one member per LANE.  32 members per warp advance one symbol per step in lock step,
-//     each lane with its own tables in shared memory (16-bit entries, 2^LB literal/length and 2^DB
-//     distance root entries; longer codes by per-length limits kept in registers).  A step is one
-//     straight path for literals and matches alike (the warp pays for every path a lane takes, so
-//     they are merged and predicated), with a 64-bit bit buffer fed from two prefetched words, and
-//     writes the
-//     symbols as 16-bit units to a token arena in HBM: a literal is one unit, a match two (length and
-//     the high distance bits, then the low distance bits).  Block headers, code lengths and stored
-//     blocks are steps of the same lock-step loop; the code tables of one lane are built by the
-//     whole warp.  The output size, distances and the end of the payload are checked here.
-//  2. k_copy: one member per WARP.  The warp reads its member's units 32 at a time, places them by
-//     a prefix sum of their lengths, and writes the bytes 32 at a time into a 16 KiB ring in shared
-//     memory (sources up to about 16 KiB back; older ones, about one match in eight on the GEX-shaped
-//     workload, read the output already written to HBM); a byte finds its token from a bit mask of the
-//     tokens that start in its 32 bytes (one warp OR-reduction and a population count), and a byte
-//     whose source lies in the same 32 bytes takes it from another lane.  Completed 1 KiB windows go to HBM with 16-byte stores and into
-//     the CRC32 (32 lane columns joined in GF(2)).
+// Measured on 15,456 GEX members (398 MB to 1.01 GB; a member per lane in the decoder and a byte per lane in
+// the copy before): decode 3.05 ms (10.45), copy 4.04 (5.16, CRC32 included), CRC32 0.42.  39 members:
+// decode 0.5 ms, copy 0.5 (one kernel with one serial decoder per member: 4.2).
 //
-// Units are at most one per output byte, so a member's units take at most 2 ISIZE bytes: the arena
-// gives every member a slot of 2 ISIZE + 8 bytes at the prefix sum of the slots before it.
-//
-// Every loop is bounded: each decode step consumes input bits or produces output bytes, both
-// bounded per member; every shared-memory index is masked or checked; arena and output writes
-// stay within the member's slot and output range.
+// Every loop is bounded: a decode step consumes input bits, bounded per member, a repair round
+// confirms at least one more segment; every shared-memory index is masked or checked; arena and
+// output writes stay within the member's slot and output range.
 
 #include <mutex>
 
@@ -42,20 +34,6 @@
 
 namespace cb {
 namespace split {
-
-// ---------------------------------------------------------------- formats
-
-// 16-bit table entries (k_decode).
-//   bit 15 set: a length symbol: bits 12-14 extra bits, 8-11 code length, 0-7 base - 3.
-//   bit 15 clear: bits 12-14 kind, 8-11 code length, 0-7 value:
-//     0 literal (value: the byte), 1 end of block, 2 distance (value: symbol 0-29),
-//     3 special (value 0: a code longer than the root bits; 1: no such code), 4 code-length symbol.
-enum : uint32_t { E_LIT = 0, E_EOB = 1, E_DIST = 2, E_SPECIAL = 3, E_CL = 4 };
-constexpr uint16_t E_LONG = (uint16_t)(E_SPECIAL << 12);
-constexpr uint16_t E_BAD = (uint16_t)((E_SPECIAL << 12) | 1u);
-
-__device__ __forceinline__ uint32_t e_len(uint32_t e) { return (e >> 8) & 15u; }
-__device__ __forceinline__ uint32_t e_kind(uint32_t e) { return (e >> 12) & 7u; }
 
 // RFC 1951 3.2.5 in closed form: length symbol i = sym - 257 (0-28), distance symbol i (0-29).
 __device__ __forceinline__ void len_code(uint32_t i, uint32_t& base, uint32_t& ext) {
@@ -83,44 +61,24 @@ __device__ __forceinline__ void dist_code(uint32_t i, uint32_t& base, uint32_t& 
 // RFC 1951 3.2.7: order of the code length code lengths.
 __constant__ uint8_t kClOrder[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12, 3, 13, 2, 14, 1, 15};
 
-enum : int { T_CL = 0, T_LIT = 1, T_DIST = 2 };
+// ---------------------------------------------------------------- workspace
 
-__device__ __forceinline__ uint16_t sym_entry(int kind, uint32_t s, uint32_t L) {
-    if (kind == T_CL) return (uint16_t)((E_CL << 12) | (L << 8) | s);
-    if (kind == T_LIT) {
-        if (s < 256) return (uint16_t)((L << 8) | s);
-        if (s == 256) return (uint16_t)((E_EOB << 12) | (L << 8));
-        if (s < 286) {
-            uint32_t base, ext;
-            len_code(s - 257, base, ext);
-            return (uint16_t)(0x8000u | (ext << 12) | (L << 8) | (base - 3));
-        }
-        return E_BAD;
-    }
-    if (s < 30) return (uint16_t)((E_DIST << 12) | (L << 8) | s);
-    return E_BAD;
-}
-
-// 16-bit units (the token arena): a literal 0x00bb; a match head 0x8000 | (length - 3) << 6 |
-// (distance - 1) >> 9, followed by its tail 0xC000 | ((distance - 1) & 0x1FF).
-__device__ __forceinline__ uint32_t unit_match(uint32_t len, uint32_t dist) {
-    const uint32_t d = dist - 1;
-    return (0x8000u | ((len - 3) << 6) | (d >> 9)) | ((0xC000u | (d & 0x1FFu)) << 16);
-}
-
-// Workspace: [0, 256) queue counters; per job 16 bytes (units u32, status u32, arena slot u64); the
-// arena after that, 256-byte aligned.  Job j's slot is the prefix sum of slot_bytes over the jobs
-// before it (k_slots), so the arena holds 2 sum(ISIZE) + 16 n_jobs bytes at most, whatever the
-// jobs' output offsets are.
+// Workspace: [0, 256) queue counters; per job 16 bytes (u32 list of the members for the one-kernel
+// form, u32 status, u64 arena slot); the arena after that, 256-byte aligned.  Job j's slot is the
+// prefix sum of slot_bytes over the jobs before it (k_slots), so the arena holds
+// 2 sum(ISIZE) + 80 n_jobs bytes at most, whatever the jobs' output offsets are.
 constexpr size_t WS_HEAD = 256;
 constexpr size_t PER_JOB = 16;
+constexpr int Q_LISTED = 6;               // queue counter: members for the one-kernel form
+constexpr uint32_t ST_LISTED = 0x100;     // internal status: on that list
 __host__ __device__ __forceinline__ size_t arena_offset(long long n_jobs) {
     return (WS_HEAD + PER_JOB * (size_t)n_jobs + 255) & ~(size_t)255;
 }
-// A slot's bytes: 2 ISIZE for the units and room for the last word, rounded to 8 so that every slot
-// starts 8-byte aligned (k_decode stores the units as 4-byte words).
+// A slot's bytes, a multiple of 16 so that runs start 16-byte aligned.  Symbols take at most 4 bytes
+// per 3 output bytes (matches of length 3); the rest is room for the runs' heads and for lanes that
+// get more symbols than others.
 __host__ __device__ __forceinline__ unsigned long long slot_bytes(uint32_t isize) {
-    return (2ull * isize + 8ull + 7ull) & ~7ull;
+    return (2ull * isize + 64ull + 15ull) & ~15ull;
 }
 
 // The arena slot of every job: one CTA; thread t sums a contiguous run of jobs, a block scan joins
@@ -181,155 +139,16 @@ __global__ void __launch_bounds__(SLOT_NT) k_slots(const cb_member_job* __restri
     }
 }
 
-// ---------------------------------------------------------------- k_decode: one member per lane
-
-template <int LB_, int DB_, int WARPS_>
-struct DecCfg {
-    static constexpr int LB = LB_, DB = DB_, WARPS = WARPS_;
-    static constexpr int NLL = 15 - LB_, NLD = 15 - DB_;  // code lengths longer than the roots
-    static constexpr uint32_t LMASK = (1u << LB_) - 1, DMASK = (1u << DB_) - 1;
-    // One region per lane (bytes):
-    //   LIT   u16[2^LB]  literal/length root entries
-    //   DIST  u16[2^DB]  distance root entries
-    //   DSYM  u16[32]    entries of the distance codes longer than DB, canonical order
-    //   LSYM  u8[288]    low 8 bits of the symbols of literal/length codes longer than LB, canonical order
-    //   LHI   u32[9]     bit i: symbol i of LSYM is 256 or more
-    // While the lane reads a dynamic header: the code-length code's table (u16[128]) at 0, the
-    // code lengths (up to 286 + 30 bytes) at LSYM, where the 19 lengths of the code-length code
-    // wait first.
-    static constexpr int LIT = 0, DIST = LIT + (2 << LB_), DSYM = DIST + (2 << DB_);
-    static constexpr int LSYM = DSYM + 64 > 256 ? DSYM + 64 : 256;
-    static constexpr int LHI = LSYM + 288;
-    static constexpr int STRIDE = (LHI + 36 + 7) & ~7;
-    static_assert(LSYM + 320 <= STRIDE && NLL <= 9 && NLD <= 10 && LB_ >= 5 && DB_ >= 4, "table sizes");
-    struct WarpSmem {
-        alignas(16) uint8_t lane[32][STRIDE];
-        uint8_t lens[320];         // the code lengths of the lane whose tables the warp builds
-        uint32_t scratch[48];
-        uint32_t lim[20];          // limits computed for that lane: NLL literal/length, then NLD distance
-    };
-    struct CtaSmem {
-        WarpSmem w[WARPS_];
-    };
-};
-
-enum : int { S_IDLE = 0, S_HDR = 1, S_BUILD_CL = 2, S_CLENS = 3, S_BUILD = 4, S_RUN = 5, S_STORED = 6, S_FIN = 7,
-             S_DONE = 8 };
-
-// Canonical table of lens[0:nsym) for one lane, built by the whole warp: tab[2^lb] indexed by the
-// next lb bits (LSB first); codes longer than lb bits have their entries in sym[] in canonical
-// order and, for code length lb + 1 + i, lim[i] = (end of the length's codes, left-justified to 15
-// bits) | (index in sym[] of its first code minus that code) << 16.  Acceptance as zlib's inflate:
-// an over-subscribed code is an error; an incomplete one too, except a literal/length or distance
-// code whose longest code has length 1 (the code-length code must be complete).  Returns false on
-// error (the same in every lane).
-__device__ __noinline__ bool build_lane(const uint8_t* lens, int nsym, int lb, int kind, uint16_t* tab, uint32_t* lim,
-                                        uint16_t* sym, uint8_t* sym8, uint32_t* hi8, uint32_t* scratch) {
-    const int lane = threadIdx.x & 31;
-    if (lane < 16) scratch[lane] = 0;
-    if (hi8 && lane < 9) hi8[lane] = 0;
-    __syncwarp();
-    for (int s = lane; s < nsym; s += 32) {
-        const uint32_t L = lens[s];
-        if (L) atomicAdd(&scratch[L], 1u);
-    }
-    __syncwarp();
-    const uint32_t cnt = (lane >= 1 && lane < 16) ? scratch[lane] : 0u;
-    int left = 1, maxlen = 0;
-    uint32_t code = 0, index = 0, my_first = 0, my_index = 0;
-    for (int L = 1; L < 16; L++) {
-        const uint32_t c = __shfl_sync(FULL, cnt, L);
-        left = (left << 1) - (int)c;
-        if (c) maxlen = L;
-        if (lane == L) {
-            my_first = code;
-            my_index = index;
-        }
-        index += c;
-        code = (code + c) << 1;
-        if (left < 0) break;
-    }
-    __syncwarp();
-    if (left < 0) return false;
-    const bool incomplete = left > 0;
-    if (kind == T_CL && (incomplete || maxlen == 0)) return false;
-    if (incomplete && maxlen > 1) return false;
-    const uint32_t nshort = __shfl_sync(FULL, my_index, lb < 15 ? lb + 1 : 15);
-    if (lim && lane > lb && lane < 16) {
-        const uint32_t limit = (my_first + cnt) << (15 - lane);
-        const int base = (int)(my_index - nshort) - (int)my_first;
-        lim[lane - lb - 1] = (limit & 0xFFFFu) | ((uint32_t)(uint16_t)(int16_t)base << 16);
-    }
-    if (lane >= 1 && lane < 16) {
-        scratch[lane] = my_index;        // running insertion index of the length
-        scratch[16 + lane] = my_first;   // first code of the length
-        scratch[32 + lane] = my_index;   // first index of the length
-    }
-    // slots no code reaches (an incomplete code) decode as errors; complete codes cover every slot
-    if (incomplete || maxlen == 0)
-        for (int i = lane; i < (1 << lb); i += 32) tab[i] = E_BAD;
-    __syncwarp();
-    for (int base = 0; base < nsym; base += 32) {
-        const int s = base + lane;
-        const uint32_t L = s < nsym ? lens[s] : 0u;
-        const uint32_t peers = __match_any_sync(FULL, L);
-        const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-        const uint32_t pos = L ? scratch[L] : 0u;
-        __syncwarp();
-        if (L && lane == __ffs(peers) - 1) scratch[L] = pos + __popc(peers);
-        __syncwarp();
-        if (L) {
-            const uint32_t idx = pos + rank;
-            const uint32_t c = scratch[16 + L] + (idx - scratch[32 + L]);
-            const uint16_t e = sym_entry(kind, (uint32_t)s, L);
-            if ((int)L <= lb) {
-                const uint32_t r = __brev(c) >> (32 - L);
-                for (uint32_t x = r; x < (1u << lb); x += (1u << L)) tab[x] = e;
-            } else {
-                const uint32_t li = idx - nshort;
-                if (sym8) {  // literal/length: the symbol's low byte, and a bit for 256 and up
-                    sym8[li] = (uint8_t)s;
-                    if (s >= 256) atomicOr(&hi8[li >> 5], 1u << (li & 31));
-                } else {
-                    sym[li] = e;
-                }
-                tab[__brev(c >> (L - lb)) >> (32 - lb)] = E_LONG;
-            }
-        }
-        __syncwarp();
-    }
-    return true;
-}
-
-// The entry of a code longer than the root bits from the lane's limits: x holds the next 15+ bits.
-template <int N, int NSYM>
-__device__ __forceinline__ uint32_t long_entry(uint32_t x, const uint32_t (&lim)[N], const uint16_t* sym) {
-    const uint32_t c = __brev(x) >> 17;  // the next 15 bits, first bit highest
-    int idx = -1;
-#pragma unroll
-    for (int i = N - 1; i >= 0; i--)
-        if (c < (lim[i] & 0xFFFFu)) idx = (int)(int16_t)(lim[i] >> 16) + (int)(c >> (N - 1 - i));
-    return (idx >= 0 && idx < NSYM) ? (uint32_t)sym[idx] : (uint32_t)E_BAD;
-}
-
-// The same for literal/length codes, whose long-code symbols are kept as a low byte and a high bit.
-template <int N>
-__device__ __forceinline__ uint32_t long_lit_entry(uint32_t x, const uint32_t (&lim)[N], const uint8_t* sym8,
-                                                   const uint32_t* hi8) {
-    const uint32_t c = __brev(x) >> 17;  // the next 15 bits, first bit highest
-    int idx = -1;
-    uint32_t L = 0;
-#pragma unroll
-    for (int i = N - 1; i >= 0; i--) {
-        if (c < (lim[i] & 0xFFFFu)) {
-            idx = (int)(int16_t)(lim[i] >> 16) + (int)(c >> (N - 1 - i));
-            L = (uint32_t)(16 - N + i);
-        }
-    }
-    if (idx < 0 || idx >= 288) return E_BAD;
-    const uint32_t sym = (uint32_t)sym8[idx] | (((hi8[idx >> 5] >> (idx & 31)) & 1u) << 8);
-    return sym_entry(T_LIT, sym, L);
-}
+// ---------------------------------------------------------------- runs
+//
+// A run is what one lane decoded of a block (or a stored block): at its start, 16-byte aligned, a head
+// of four words (literal bytes, sequences, offset of the next run in the slot or RUN_END, end of the
+// run), then the literals, and from its end downwards the sequences, one word each:
+//   bits 24-31 literals before the match, 16-23 match length - 3, 15 set when there is a match,
+//   0-14 distance - 1.
+constexpr uint32_t RUN_END = 0xFFFFFFFFu;
+constexpr uint32_t SEQ_MATCH = 0x8000u;
+constexpr uint32_t SEQ_BAD = 1u;  // without SEQ_MATCH: the match has no valid distance
 
 __device__ __forceinline__ void report(cb_inflate_summary* summary, uint32_t* job_status, long long j, uint32_t st) {
     if (job_status) job_status[j] = st;
@@ -340,656 +159,1002 @@ __device__ __forceinline__ void report(cb_inflate_summary* summary, uint32_t* jo
     }
 }
 
+// ---------------------------------------------------------------- k_decode: one member per warp
+
+// Entries of the literal/length table: bits 0-5 the bits of the code and its extra bits (SLOW: a code
+// longer than the table resolves), 6-9 the code length, 16-23 the literal or the length base - 3, and
+// flags; a literal has none.
+constexpr uint32_t F_MATCH = 1u << 31, F_EOB = 1u << 30, F_BAD = 1u << 29;
+// Entries of the distance table: bits 0-9 as above, 16-30 the distance base - 1, 31 set for a distance
+// (so the upper half is SEQ_MATCH | base - 1); a symbol that is none has bits 16-31 SEQ_BAD.
+constexpr uint32_t SLOW = 32;
+constexpr int ROOT = 9, DROOT = 8;     // bits that index the root tables
+constexpr uint32_t LNG = 512;          // entries for the longer literal/length codes, after the root's
+constexpr uint32_t OVERLAP = 512;      // bits a lane decodes before its segment to fall in step
+constexpr uint32_t SEG_MIN = 128, SEG_MAX = 4096;  // bits of a segment
+constexpr int ROWS = 16;               // words of input kept per lane
+constexpr int STEPS = 5;               // decode steps between refills
+constexpr int LROWS = 8, SROWS = 8;    // words of staged literals and sequences per lane
+constexpr uint32_t LC_MAX = 240;       // literals before a match, about (one sequence holds up to 255)
+constexpr int DEC_WARPS = 2;
+static_assert(STEPS + 15 <= 4 * LROWS && STEPS + 3 <= SROWS, "staging holds a round and what is left of the last");
+
+// 10.3 KB per warp: 20 warps per SM.  The per-lane arrays (input, staging) are columns, word r of
+// lane l at r * 32 + l, so that their accesses never conflict.
+struct DecWarp {
+    uint32_t lit[(1 << ROOT) + LNG];
+    uint32_t dst[1 << DROOT];
+    uint32_t in[(ROWS + 2) * 32];   // rows ROWS, ROWS + 1 repeat rows 0, 1
+    uint32_t lst[LROWS * 32];       // while a header is read: the code lengths (bytes)
+    uint32_t sst[SROWS * 32];       // while a header is read: the code-length code's table (bytes)
+    uint32_t lfirst[17], lindex[17], dfirst[17], dindex[17];  // canonical codes by length, left-justified to 15 bits
+    uint32_t count[16];
+    uint16_t lsym[288];             // symbols in canonical order
+    uint16_t dsym[32];
+};
+
+__device__ __forceinline__ uint32_t lit_entry(uint32_t s, uint32_t L) {
+    if (s < 256) return L | (L << 6) | (s << 16);
+    if (s == 256) return F_EOB | L | (L << 6);
+    if (s >= 286) return F_BAD | L | (L << 6);
+    uint32_t base, ext;
+    len_code(s - 257, base, ext);
+    return F_MATCH | (L + ext) | (L << 6) | ((base - 3) << 16);
+}
+__device__ __forceinline__ uint32_t dist_entry(uint32_t s, uint32_t L) {
+    if (s >= 30) return L | (L << 6) | (SEQ_BAD << 16);
+    uint32_t base, ext;
+    dist_code(s, base, ext);
+    return (L + ext) | (L << 6) | ((SEQ_MATCH | (base - 1)) << 16);
+}
+
+// The lowest n bits set (n < 32).
+__device__ __forceinline__ uint32_t low_bits(uint32_t n) {
+#ifdef __CUDA_ARCH__
+    uint32_t m;
+    asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(m) : "r"(n));
+    return m;
+#else
+    return (1u << n) - 1u;
+#endif
+}
+
+// Spread entries written at the first slot of each code over the slots up to the next one (rows of 32).
+__device__ __forceinline__ void fill_forward(uint32_t* tab, int n) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t incl = 0xFFFFFFFFu >> (31 - lane);
+    uint32_t carry = 0;
+    for (int i = 0; i < n; i += 32) {
+        const uint32_t v = tab[i + lane];
+        const uint32_t below = __ballot_sync(FULL, v != 0) & incl;
+        const uint32_t f = __shfl_sync(FULL, v, below ? 31 - __clz(below) : 0);
+        const uint32_t x = below ? f : carry;
+        tab[i + lane] = x;
+        carry = __shfl_sync(FULL, x, 31);
+    }
+    __syncwarp();
+}
+
+// The decode tables of lens[0:nsym) (code lengths, at most 15; nsym <= 288, or 32 for distances), built
+// by the whole warp.  Tables are indexed by code bits first bit highest, so a code's slots are adjacent:
+// its entry is written at the first one and spread.  `limit` gets the first code longer than the root
+// (left-justified to 15 bits; past all codes when there is none); the LNG entries after the root's are
+// of 2^lsh codes each from there.  Acceptance as zlib's
+// inflate: an over-subscribed code is an error, an incomplete one too unless its longest code has
+// length 1.  Returns false on error (the same in every lane).
+template <bool LIT>
+__device__ __noinline__ bool build_tables(DecWarp& W, const uint8_t* lens, int nsym, uint32_t& limit, uint32_t& lsh) {
+    constexpr int NB = LIT ? 9 : 1, RB = LIT ? ROOT : DROOT;
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t* root = LIT ? W.lit : W.dst;
+    uint32_t* first = LIT ? W.lfirst : W.dfirst;
+    uint32_t* index = LIT ? W.lindex : W.dindex;
+    if (lane < 16) W.count[lane] = 0;
+    __syncwarp();
+    uint32_t lr[NB];  // each symbol's code length, and its rank within the length
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+        const int s = b * 32 + lane;
+        const uint32_t L = s < nsym ? lens[s] : 0u;
+        const uint32_t peers = __match_any_sync(FULL, L);
+        const uint32_t at = W.count[L];
+        __syncwarp();
+        if ((peers & lt) == 0) W.count[L] = at + __popc(peers);
+        __syncwarp();
+        lr[b] = L | ((at + __popc(peers & lt)) << 4);
+    }
+    const uint32_t cnt = lane >= 1 && lane < 16 ? W.count[lane] : 0u;
+    uint32_t tot;
+    // codes up to each length, left-justified (at most 288 << 14 < 2^23), and their number, in one sum
+    const uint32_t before = warp_exclusive_scan(((lane < 16 ? cnt << (15 - lane) : 0u) << 9) | cnt, tot);
+    const uint32_t total = tot >> 9;
+    const int maxlen = 31 - __clz(__ballot_sync(FULL, cnt != 0) | 1u);
+    if (total > 32768u || (total < 32768u && maxlen > 1)) return false;
+    if (lane < 17) {
+        first[lane] = lane < 16 ? before >> 9 : total;
+        index[lane] = before & 511u;
+    }
+    const uint32_t lim = __shfl_sync(FULL, before >> 9, RB + 1);
+    const uint32_t span = total - lim;
+    limit = span ? lim : 32768u;
+    lsh = span <= LNG ? 0u : 32u - (uint32_t)__clz((int)((span - 1) / LNG));
+    const int slots = LIT ? (int)((span + (1u << lsh) - 1) >> lsh) : 0;  // at most LNG
+    uint32_t* lng = W.lit + (1 << ROOT);
+    for (int i = lane; i < (1 << RB); i += 32) root[i] = 0;
+    for (int i = lane; i < ((slots + 31) & ~31); i += 32) lng[i] = 0;
+    __syncwarp();
+    const uint32_t lmax = 15 - lsh;  // longest code with slots of lng
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+        const uint32_t s = b * 32 + lane, L = lr[b] & 15u, r = lr[b] >> 4;
+        if (L) {
+            const uint32_t c = first[L] + (r << (15 - L));
+            const uint32_t e = LIT ? lit_entry(s, L) : dist_entry(s, L);
+            if (L <= (uint32_t)RB) {
+                root[c >> (15 - RB)] = e;
+            } else {
+                (LIT ? W.lsym : W.dsym)[index[L] + r] = (uint16_t)s;
+                if (LIT && L <= lmax) lng[(c - lim) >> lsh] = e;
+            }
+        }
+    }
+    if (lane == 0) {
+        if (span) root[lim >> (15 - RB)] = SLOW;
+        if (total < 32768u) root[total >> (15 - RB)] = LIT ? F_BAD | 1u : (SEQ_BAD << 16) | 1u;
+        if (LIT && span && first[lmax + 1] < total) lng[(first[lmax + 1] - lim) >> lsh] = SLOW;
+    }
+    __syncwarp();
+    fill_forward(root, 1 << RB);
+    fill_forward(lng, (slots + 31) & ~31);
+    return true;
+}
+
+// The entry of a code whose next 15 bits are c (first bit highest), found by the limits of the code
+// lengths from L0 up.
+template <bool LIT>
+__device__ __noinline__ uint32_t long_entry(const DecWarp& W, uint32_t c, uint32_t L0) {
+    const uint32_t* first = LIT ? W.lfirst : W.dfirst;
+    uint32_t L = L0;
+    while (L < 15 && c >= first[L + 1]) L++;
+    const uint32_t i = (LIT ? W.lindex : W.dindex)[L] + ((c - first[L]) >> (15 - L));
+    if (c >= first[16] || i >= (LIT ? 288u : 32u)) return LIT ? F_BAD | 1u : (SEQ_BAD << 16) | 1u;
+    return LIT ? lit_entry(W.lsym[i], L) : dist_entry(W.dsym[i], L);
+}
+
+// Word w of the input (words nvalid and up read as zero); block k: words 4k to 4k + 3.
 __device__ __forceinline__ uint32_t load_word(const uint32_t* wbase, uint32_t nvalid, uint32_t w) {
     return w < nvalid ? __ldg(wbase + w) : 0u;
 }
-
-// Block k (16 bytes, words 4k..4k+3) of a lane's input: one 16-byte load when the whole block lies
-// within the nvalid readable words, else word by word (zero past the end).
-__device__ __forceinline__ uint4 load_block(const uint32_t* base16, uint32_t nvalid, uint32_t k) {
+__device__ __forceinline__ uint4 load_block(const uint32_t* wbase, uint32_t nvalid, uint32_t k) {
     const uint32_t w = 4 * k;
-    if (w + 3 < nvalid) return __ldg(reinterpret_cast<const uint4*>(base16) + k);
-    uint4 v;
-    v.x = w < nvalid ? __ldg(base16 + w) : 0u;
-    v.y = w + 1 < nvalid ? __ldg(base16 + w + 1) : 0u;
-    v.z = w + 2 < nvalid ? __ldg(base16 + w + 2) : 0u;
-    v.w = w + 3 < nvalid ? __ldg(base16 + w + 3) : 0u;
-    return v;
+    if (w + 3 < nvalid) return __ldg(reinterpret_cast<const uint4*>(wbase) + k);
+    return make_uint4(load_word(wbase, nvalid, w), load_word(wbase, nvalid, w + 1), load_word(wbase, nvalid, w + 2),
+                      load_word(wbase, nvalid, w + 3));
 }
 
-// A hint to bring the 128-byte line of p into L2 (a prefetch, no load into registers).
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// The warp's reader of block headers: lane l holds word base + l of the input.
+struct HeadBits {
+    const uint32_t* wbase;
+    uint32_t nvalid, base, word;
+    __device__ __forceinline__ void at(uint32_t p) {  // words from bit p on
+        base = p >> 5;
+        word = load_word(wbase, nvalid, base + (threadIdx.x & 31));
+    }
+    __device__ __forceinline__ void cover(uint32_t p) {  // at least the 96 bits from p on
+        if ((p >> 5) - base > 28u) at(p);
+    }
+    __device__ __forceinline__ uint32_t get(uint32_t p) const {  // 32 bits from bit p (per lane) on
+        const uint32_t w = (p >> 5) - base;
+        return __funnelshift_r(__shfl_sync(FULL, word, w), __shfl_sync(FULL, word, w + 1), p);
+    }
+};
 
-template <class C>
-__global__ void __launch_bounds__(C::WARPS * 32)
+// The code lengths of a dynamic block whose header fields start at bit p (after the three header bits),
+// into lens; p is left after them.  The 32 lanes decode the code at 32 bit positions at once; which of
+// those are symbols follows from the chain that starts at the first (pointer doubling).  Returns
+// literal/length codes | all codes << 16, or 0 on error.
+__device__ __noinline__ uint32_t read_lengths(DecWarp& W, HeadBits& hb, uint32_t& p, uint8_t* lens) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    hb.cover(p);
+    const uint32_t h = hb.get(p);
+    const uint32_t hlit = (h & 31u) + 257, hdist = ((h >> 5) & 31u) + 1, hclen = ((h >> 10) & 15u) + 4;
+    p += 14;
+    if (hlit > 286 || hdist > 30) return 0;
+    // the code-length code: lane s its symbol's length and code (left-justified to 7 bits)
+    uint8_t* cl = reinterpret_cast<uint8_t*>(W.count);
+    if (lane < 16) W.count[lane] = 0;
+    for (int i = lane; i < 80; i += 32) reinterpret_cast<uint32_t*>(lens)[i] = 0;
+    __syncwarp();
+    hb.cover(p);
+    const uint32_t x3 = hb.get(p + 3 * (lane < 19 ? lane : 0)) & 7u;
+    if (lane < (int)hclen) cl[kClOrder[lane]] = (uint8_t)x3;
+    p += 3 * hclen;
+    __syncwarp();
+    const uint32_t L = lane < 19 ? cl[lane] : 0u;
+    const uint32_t space = L ? 128u >> L : 0u;
+    uint32_t code = 0;
+    for (int t = 0; t < 19; t++) {
+        const uint32_t Lt = __shfl_sync(FULL, L, t);
+        if (Lt && (Lt < L || (Lt == L && t < lane))) code += 128u >> Lt;
+    }
+    if (__reduce_add_sync(FULL, space) != 128u) return 0;
+    uint32_t* tab4 = W.sst;  // 128 entries of a byte: length << 5 | symbol, never 0
+    uint8_t* tab = reinterpret_cast<uint8_t*>(tab4);
+    tab4[lane] = 0;
+    __syncwarp();
+    if (L) tab[code] = (uint8_t)((L << 5) | lane);
+    __syncwarp();
+    {  // spread each entry up to the next one, four slots per lane
+        uint32_t v = tab4[lane];
+        const uint32_t last = v >> 24 ? v >> 24 : (v >> 16) & 255u ? (v >> 16) & 255u : (v >> 8) & 255u ? (v >> 8) & 255u : v & 255u;
+        const uint32_t below = __ballot_sync(FULL, v != 0) & lt;
+        uint32_t c = __shfl_sync(FULL, last, below ? 31 - __clz(below) : 0);
+        uint32_t y = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t b = (v >> (8 * k)) & 255u;
+            c = b ? b : c;
+            y |= c << (8 * k);
+        }
+        tab4[lane] = y;
+    }
+    __syncwarp();
+    const uint32_t total = hlit + hdist;
+    uint32_t ci = 0, last = 0;
+    while (ci < total) {
+        hb.cover(p);
+        const uint32_t x = hb.get(p + lane);
+        const uint32_t t = tab[__brev(x) >> 25];
+        const uint32_t CL = t >> 5, s = t & 31u;
+        const uint32_t eb = s < 16 ? 0u : s == 16 ? 2u : s == 17 ? 3u : 7u;
+        const uint32_t n = CL + eb;
+        const uint32_t ext = (x >> CL) & ((1u << eb) - 1u);
+        // the symbols: positions reached from lane 0
+        uint32_t reach = 1u << lane, nx = lane + n;
+#pragma unroll
+        for (int r = 0; r < 5; r++) {
+            const uint32_t orr = __shfl_sync(FULL, reach, nx & 31u), onx = __shfl_sync(FULL, nx, nx & 31u);
+            if (nx < 32) {
+                reach |= orr;
+                nx = onx;
+            }
+        }
+        reach = __shfl_sync(FULL, reach, 0);
+        const uint32_t exit = __shfl_sync(FULL, nx, 0);
+        const bool on = (reach >> lane) & 1u;
+        const uint32_t rep = !on ? 0u : s < 16 ? 1u : (s == 18 ? 11u : 3u) + ext;
+        uint32_t tot;
+        const uint32_t pos = ci + warp_exclusive_scan(rep, tot);
+        const bool act = on && pos < total;
+        if (__any_sync(FULL, act && (pos + rep > total || (s == 16 && pos == 0)))) return 0;
+        // a repeat copies the length before it: the nearest earlier symbol that is not one
+        const uint32_t own = __ballot_sync(FULL, act && s != 16);
+        const uint32_t sv = s < 16 ? s : 0u;
+        const uint32_t prior = own & lt;
+        const uint32_t pv = __shfl_sync(FULL, sv, prior ? 31 - __clz(prior) : 0);
+        const uint32_t v = s != 16 ? sv : prior ? pv : last;
+        if (act && v)  // lengths start at zero
+            for (uint32_t r = 0; r < rep; r++) lens[pos + r] = (uint8_t)v;
+        last = own ? __shfl_sync(FULL, sv, 31 - __clz(own)) : last;
+        if (ci + tot >= total) {
+            const uint32_t end = __ballot_sync(FULL, act && pos + rep == total);
+            p = __shfl_sync(FULL, p + lane + n, __ffs(end) - 1);
+        } else {
+            p += exit;
+        }
+        ci += tot;
+    }
+    __syncwarp();
+    if (lens[256] == 0) return 0;  // no end-of-block code
+    return hlit | (total << 16);
+}
+
+// What a lane has decoded of its segment.
+struct LaneOut {
+    uint32_t nl, ns, lc;   // literals, sequences, literals since the last sequence
+    uint32_t fl, fs;       // stored in the slot so far
+    uint32_t stop;         // 0, 1 at an end-of-block code, 2 at an invalid code
+    bool over;             // more than the run holds (counted on, not stored)
+};
+
+// Store 16 staged literals (l) or 4 staged sequences, when the run holds them.
+__device__ __forceinline__ void store_lits(const DecWarp& W, LaneOut& o, uint8_t* run, uint32_t cap) {
+    const uint32_t* c = W.lst + ((o.fl >> 2) & (LROWS - 1)) * 32 + (threadIdx.x & 31);  // fl: a multiple of 16
+    o.fl += 16;
+    if (16 + o.fl + 4 * o.fs > cap) o.over = true;
+    if (!o.over) *reinterpret_cast<uint4*>(run + o.fl) = make_uint4(c[0], c[32], c[64], c[96]);
+}
+__device__ __forceinline__ void store_seqs(const DecWarp& W, LaneOut& o, uint8_t* run, uint32_t cap) {
+    const uint32_t* c = W.sst + (o.fs & (SROWS - 1)) * 32 + (threadIdx.x & 31);  // fs: a multiple of 4
+    o.fs += 4;
+    if (16 + o.fl + 4 * o.fs > cap) o.over = true;
+    if (!o.over) *reinterpret_cast<uint4*>(run + cap - 4 * o.fs) = make_uint4(c[96], c[64], c[32], c[0]);
+}
+
+// A lane's input: 16 words in its column; the block after them is loaded a round ahead.
+struct LaneIn {
+    const uint32_t* wbase;
+    uint32_t nvalid, fill;  // words up to fill are in the column
+    bool coming;            // next is being loaded
+    uint4 next;
+};
+__device__ __forceinline__ void put_block(uint32_t* col, uint32_t fill, uint4 v) {
+    uint32_t* c = col + (fill & (ROWS - 1)) * 32;
+    c[0] = v.x;
+    c[32] = v.y;
+    c[64] = v.z;
+    c[96] = v.w;
+    if ((fill & (ROWS - 1)) == 0) {
+        col[ROWS * 32] = v.x;
+        col[(ROWS + 1) * 32] = v.y;
+    }
+}
+__device__ __forceinline__ void start_input(LaneIn& in, uint32_t* col, uint32_t p) {
+    const uint32_t k = p >> 7;
+    const uint4 a = load_block(in.wbase, in.nvalid, k), b = load_block(in.wbase, in.nvalid, k + 1),
+                c = load_block(in.wbase, in.nvalid, k + 2);
+    put_block(col, 4 * k, a);
+    put_block(col, 4 * k + 4, b);
+    put_block(col, 4 * k + 8, c);
+    in.fill = 4 * k + 12;
+    in.coming = false;
+}
+// Take the block that was loaded and load the next one when there is room for it; returns the bit up to
+// which steps may start (a step reads three words).
+__device__ __forceinline__ uint32_t refill(LaneIn& in, uint32_t* col, uint32_t p) {
+    if (in.coming) {
+        put_block(col, in.fill, in.next);
+        in.fill += 4;
+    }
+    in.coming = in.fill - (p >> 5) <= ROWS - 4;
+    if (in.coming) in.next = load_block(in.wbase, in.nvalid, in.fill >> 2);
+    return (in.fill - 2) * 32;
+}
+
+// A symbol whose codes the tables do not resolve or that takes more than 32 bits (rare): x its first 32
+// bits, hi the next ones.  Returns its bits; e, d: its entries, y: the bits after the literal/length.
+__device__ __noinline__ uint32_t slow_symbol(const DecWarp& W, uint32_t x, uint32_t hi, uint32_t lsh, uint32_t& e,
+                                             uint32_t& d, uint32_t& y) {
+    if ((e & 63u) == SLOW) e = long_entry<true>(W, __brev(x) >> 17, 15 - lsh);
+    const uint32_t n = e & 63u;
+    y = __funnelshift_r(x, hi, n);
+    d = W.dst[__brev(y) >> (32 - DROOT)];
+    if ((d & 63u) == SLOW) d = long_entry<false>(W, __brev(y) >> 17, DROOT + 1);
+    return n + (e & F_MATCH ? d & 63u : 0u);
+}
+
+// One symbol at bit p of the lane's input: p moves past it.  With STORE it is staged and the lane stops
+// at an end-of-block or invalid code (end becomes 0); without, every code is passed over.  Literals and
+// matches take the same path (a warp has both at nearly every step); lim: where the codes longer than
+// the root begin, lim2: the table index of the first of them, as lim - (index << lsh).
+template <bool STORE>
+__device__ __forceinline__ void decode_step(DecWarp& W, uint32_t* col, uint32_t& p, uint32_t& end, uint32_t lim,
+                                            uint32_t lim2, uint32_t lsh, LaneOut& o) {
+    const uint32_t* r = col + ((p >> 5) & (ROWS - 1)) * 32;
+    const uint32_t w0 = r[0], w1 = r[32];
+    const uint32_t x = __funnelshift_r(w0, w1, p);
+    const uint32_t c = __brev(x) >> 17;
+    uint32_t e = W.lit[c >= lim ? (c - lim2) >> lsh : c >> (15 - ROOT)];
+    uint32_t y = __funnelshift_r(x, 0u, e);  // shifts by bits 0-4
+    uint32_t d = W.dst[__brev(y) >> (32 - DROOT)];
+    uint32_t t = (e & 63u) + (e & F_MATCH ? d & 63u : 0u);
+    if (t >= 32) t = slow_symbol(W, x, __funnelshift_r(w1, r[64], p), lsh, e, d, y);
+    p += t;
+    if (STORE) {
+        const int lane = threadIdx.x & 31;
+        const bool match = (e & F_MATCH) != 0, lit = e < F_BAD;
+        const uint32_t len3 = ((e >> 16) & 255u) + __funnelshift_r(x & low_bits(e & 31u), 0u, e >> 6);
+        const uint32_t dist = (d >> 16) + __funnelshift_r(y & low_bits(d & 31u), 0u, d >> 6);
+        const uint32_t q = (o.lc << 24) | (len3 << 16) | dist;
+        if (match) W.sst[(o.ns & (SROWS - 1)) * 32 + lane] = q;
+        if (lit)
+            reinterpret_cast<uint8_t*>(W.lst)[((o.nl >> 2) & (LROWS - 1)) * 128 + lane * 4 + (o.nl & 3u)] =
+                (uint8_t)(e >> 16);
+        o.nl += lit;
+        o.ns += match;
+        o.lc = match ? 0u : o.lc + lit;
+        if (e & (F_EOB | F_BAD)) {
+            o.stop = e & F_BAD ? 2u : 1u;
+            end = 0;
+        }
+    }
+}
+
+// The Huffman-coded symbols of one block from bit p on, as runs from offset `at` of the member's slot;
+// p and at are left after them.  `last`: the block is the member's last.  CB_OK, CB_ERR_INFLATE or
+// ST_LISTED (they do not fit the slot).
+__device__ uint32_t decode_block(DecWarp& W, LaneIn& in, uint32_t& p0, uint32_t E, uint8_t* slot, uint32_t slot_n,
+                                 uint32_t& at, bool final_block, uint32_t limit, uint32_t lsh) {
+    const int lane = threadIdx.x & 31;
+    uint32_t* col = W.in + lane;
+    const uint32_t lim2 = limit - ((1u << ROOT) << lsh);
+    for (;;) {  // windows of up to 32 segments
+        if (p0 >= E) return CB_ERR_INFLATE;
+        const uint32_t R = E - p0;
+        const uint32_t seg = max(SEG_MIN, min(SEG_MAX, (R + 31) / 32));
+        const int A = (int)min(32u, (R + seg - 1) / seg);
+        const uint32_t b0 = p0 + lane * seg, b1 = min(b0 + seg, E);
+        const bool act = lane < A;
+        LaneOut o;
+        uint32_t p = lane * seg <= OVERLAP ? p0 : b0 - OVERLAP;
+        if (act) start_input(in, col, p);
+        __syncwarp();
+        {
+            const uint32_t end = act ? b0 : 0u;
+            while (__any_sync(FULL, p < end)) {
+                uint32_t to = 0;
+                if (p < end) to = min(end, refill(in, col, p));
+#pragma unroll
+                for (int k = 0; k < STEPS; k++)
+                    if (p < to) decode_step<false>(W, col, p, to, limit, lim2, lsh, o);
+            }
+        }
+        uint32_t s = p;  // the first symbol of the lane's segment
+        // three quarters of the slot's free bytes by bits of input (symbols usually need a third of them;
+        // the last quarter is for a block that starts in the last segment)
+        const uint32_t share = (uint32_t)((unsigned long long)(slot_n - at) * min(R, 32 * seg) * 3 / (4ull * R));
+        uint32_t cap = (share / A) & ~15u;
+        if (cap < 48) cap = 0;
+        uint32_t run = at + lane * cap, next_at = at;
+        bool need = act, exact = false;
+        int F;
+        for (;;) {
+            uint32_t end = 0;
+            if (need) {
+                o.nl = o.ns = o.lc = o.fl = o.fs = o.stop = 0;
+                o.over = cap == 0;
+                end = b1;
+            }
+            while (__any_sync(FULL, p < end)) {
+                uint32_t to = 0;
+                if (p < end) to = min(end, refill(in, col, p));
+#pragma unroll
+                for (int k = 0; k < STEPS; k++)
+                    if (p < to) decode_step<true>(W, col, p, to, limit, lim2, lsh, o);
+                if (need) {
+                    if (o.stop) end = 0;
+                    if (o.nl - o.fl >= 16) store_lits(W, o, slot + run, cap);
+                    if (o.ns - o.fs >= 4) store_seqs(W, o, slot + run, cap);
+                    if (o.lc > LC_MAX) {  // a sequence's literal count has 8 bits
+                        W.sst[(o.ns & (SROWS - 1)) * 32 + lane] = o.lc << 24;
+                        o.ns++;
+                        o.lc = 0;
+                    }
+                    if (o.ns - o.fs >= 4) store_seqs(W, o, slot + run, cap);
+                }
+            }
+            if (need) {  // what is left, and the literals after the last match
+                if (o.lc) {
+                    W.sst[(o.ns & (SROWS - 1)) * 32 + lane] = o.lc << 24;
+                    o.ns++;
+                }
+                if (o.nl > o.fl) store_lits(W, o, slot + run, cap);
+                if (o.ns > o.fs) store_seqs(W, o, slot + run, cap);
+            }
+            // every segment up to the block's end must begin where the one before it ended
+            const uint32_t stopped = __ballot_sync(FULL, act && o.stop != 0);
+            F = stopped ? __ffs(stopped) - 1 : A - 1;
+            const uint32_t pe = __shfl_up_sync(FULL, p, 1);
+            need = lane > 0 && lane <= F && s != pe;
+            if (__any_sync(FULL, need)) {
+                if (need) s = p = pe;
+            } else {
+                const bool over = __any_sync(FULL, lane <= F && o.over);
+                if (!over) break;
+                // some run was too short: lay the runs out by their sizes and decode them again
+                const uint32_t size = lane <= F ? 16 + ((o.nl + 15) & ~15u) + ((o.ns + 3) & ~3u) * 4 : 0u;
+                uint32_t tot;
+                const uint32_t ex = warp_exclusive_scan(size, tot);
+                if (exact || tot > slot_n - at) return ST_LISTED;
+                exact = true;
+                run = at + ex;
+                cap = size;
+                next_at = at + tot;
+                need = lane <= F;
+                p = s;
+            }
+            if (need) start_input(in, col, p);
+            __syncwarp();
+        }
+        const uint32_t stop = __shfl_sync(FULL, o.stop, F);
+        p0 = __shfl_sync(FULL, p, F);
+        if (stop == 2 || p0 > E) return CB_ERR_INFLATE;
+        if (!exact) next_at = at + (F + 1) * cap;
+        const uint32_t nrun = __shfl_down_sync(FULL, run, 1);
+        if (lane <= F)
+            *reinterpret_cast<uint4*>(slot + run) =
+                make_uint4(o.nl, o.ns, lane < F ? nrun : stop && final_block ? RUN_END : next_at, run + cap);
+        at = next_at;
+        __syncwarp();
+        if (stop) return CB_OK;
+    }
+}
+
+// One member's symbols into its slot.  CB_OK, CB_ERR_INFLATE or ST_LISTED.
+__device__ uint32_t decode_member(DecWarp& W, const cb_member_job& job, uint8_t* slot) {
+    const int lane = threadIdx.x & 31;
+    LaneIn in;
+    const uintptr_t src = (uintptr_t)job.in;
+    in.wbase = reinterpret_cast<const uint32_t*>(src & ~(uintptr_t)15);
+    in.nvalid = (uint32_t)((src + job.in_len + 8 - (uintptr_t)in.wbase) >> 2);
+    HeadBits hb;
+    hb.wbase = in.wbase;
+    hb.nvalid = in.nvalid;
+    uint32_t p = (uint32_t)(src & 15) * 8;
+    const uint32_t s0 = p, E = p + job.in_len * 8u;
+    const uint32_t slot_n = (uint32_t)slot_bytes(job.isize);
+    uint32_t at = 0;
+    uint8_t* lens = reinterpret_cast<uint8_t*>(W.lst);
+    for (;;) {
+        if (p > E) return CB_ERR_INFLATE;
+        hb.at(p);
+        const uint32_t h = hb.get(p);
+        p += 3;
+        const bool final_block = h & 1u;
+        const uint32_t btype = (h >> 1) & 3u;
+        if (btype == 3) return CB_ERR_INFLATE;
+        if (btype == 0) {
+            p = s0 + ((p - s0 + 7) & ~7u);
+            const uint32_t y = hb.get(p), len = y & 0xFFFFu;
+            p += 32;
+            if (len != (~y >> 16) || p > E || 8ull * len > E - p) return CB_ERR_INFLATE;
+            const uint32_t ns = (len + 254) / 255, size = 16 + ((len + 15) & ~15u) + ((ns + 3) & ~3u) * 4;
+            if (slot_n - at < size) return ST_LISTED;
+            uint8_t* run = slot + at;
+            for (uint32_t i = lane; i < (len + 3) / 4; i += 32) {
+                const uint32_t b = p + 32 * i, w = b >> 5;
+                reinterpret_cast<uint32_t*>(run + 16)[i] =
+                    __funnelshift_r(load_word(in.wbase, in.nvalid, w), load_word(in.wbase, in.nvalid, w + 1), b);
+            }
+            for (uint32_t i = lane; i < ns; i += 32)
+                reinterpret_cast<uint32_t*>(run + size)[-1 - (int)i] = min(255u, len - 255 * i) << 24;
+            p += 8 * len;
+            if (lane == 0)
+                *reinterpret_cast<uint4*>(run) = make_uint4(len, ns, final_block ? RUN_END : at + size, at + size);
+            at += size;
+        } else {
+            uint32_t limit, lsh, dl, dsh;
+            int nl = 288, nd = 32;
+            if (btype == 1) {
+                for (int i = lane; i < 320; i += 32) lens[i] = i < 144 ? 8 : i < 256 ? 9 : i < 280 ? 7 : i < 288 ? 8 : 5;
+                __syncwarp();
+            } else {
+                const uint32_t r = read_lengths(W, hb, p, lens);
+                if (!r) return CB_ERR_INFLATE;
+                nl = (int)(r & 0xFFFFu);
+                nd = (int)(r >> 16) - nl;
+            }
+            if (!build_tables<true>(W, lens, nl, limit, lsh)) return CB_ERR_INFLATE;
+            if (!build_tables<false>(W, lens + nl, nd, dl, dsh)) return CB_ERR_INFLATE;
+            const uint32_t st = decode_block(W, in, p, E, slot, slot_n, at, final_block, limit, lsh);
+            if (st != CB_OK) return st;
+        }
+        if (final_block) return p > E ? (uint32_t)CB_ERR_INFLATE : (uint32_t)CB_OK;
+        if (slot_n - at < 16) return ST_LISTED;
+    }
+}
+
+__global__ void __launch_bounds__(DEC_WARPS * 32)
     k_decode(const cb_member_job* __restrict__ jobs, int64_t n_jobs, const int64_t* __restrict__ d_n_jobs,
-             uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws, unsigned long long arena_bytes,
-             int steps, uint32_t ahead, long long j0, long long j1, int qi) {
+             uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws, uint8_t* arena,
+             unsigned long long arena_bytes, bool list_unfit, long long j0, long long j1, int qi) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    typename C::CtaSmem& S = *reinterpret_cast<typename C::CtaSmem*>(smem_raw);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    typename C::WarpSmem& W = S.w[warp];
-    unsigned long long* queue = reinterpret_cast<unsigned long long*>(ws) + qi;  // this launch's counter
-    uint32_t* per_job = reinterpret_cast<uint32_t*>(ws + WS_HEAD);  // (units, status, slot lo, slot hi) per job
-    uint8_t* arena = ws + arena_offset(n_jobs);
+    DecWarp& W = reinterpret_cast<DecWarp*>(smem_raw)[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    unsigned long long* queue = reinterpret_cast<unsigned long long*>(ws);
+    uint32_t* per_job = reinterpret_cast<uint32_t*>(ws + WS_HEAD);
     long long n = n_jobs;
     if (d_n_jobs) n = min((long long)n, (long long)*d_n_jobs);
     n = min(n, j1);  // this launch's jobs: [j0, j1)
-
-    uint8_t* const my_base = W.lane[lane];
-    const uint16_t* my_lit = reinterpret_cast<const uint16_t*>(my_base + C::LIT);
-    const uint16_t* my_dist = reinterpret_cast<const uint16_t*>(my_base + C::DIST);
-    const uint16_t* my_dsym = reinterpret_cast<const uint16_t*>(my_base + C::DSYM);
-    const uint8_t* my_lsym = my_base + C::LSYM;
-    const uint32_t* my_lhi = reinterpret_cast<const uint32_t*>(my_base + C::LHI);
-    const uint16_t* my_cltab = reinterpret_cast<const uint16_t*>(my_base);  // while a header is read
-    uint8_t* my_lens = my_base + C::LSYM;  // code lengths while a header is read (after the 19 below)
-
-    // the member of this lane
-    int st = S_IDLE;
-    long long j = 0;
-    // bit reader: bb holds bc bits (LSB first), fed from registers: a0-a3 the words left of the current
-    // 16-byte block (acnt of them, a0 next), blk the next block, loaded a block ahead (nb: the block
-    // after it); wfed words went into bb so far
-    const uint32_t* wbase = nullptr;  // 16-byte aligned start at or before the payload
-    uint64_t bb = 0;
-    uint32_t bc = 0, a0 = 0, a1 = 0, a2 = 0, a3 = 0, acnt = 0, nb = 0, wfed = 0, nvalid = 0;
-    uint4 blk = make_uint4(0, 0, 0, 0);
-    uint32_t s0 = 0, in_bits = 0, isize = 0, pos = 0;
-    bool final_block = false;
-    uint32_t rem = 0, hlit = 0, total = 0, ci = 0;  // stored bytes left; code lengths read
-    uint32_t* slot = nullptr;
-    uint32_t nunits = 0, nwords = 0, half = 0, has = 0;  // units written, u32 words stored, a pending unit
-    uint32_t err = CB_OK;
-    uint32_t llim[C::NLL], dlim[C::NLD];
-#pragma unroll
-    for (int i = 0; i < C::NLL; i++) llim[i] = 0;
-#pragma unroll
-    for (int i = 0; i < C::NLD; i++) dlim[i] = 0;
-
-    auto next_word = [&]() {  // a0 went into bb: the next word becomes a0
-        a0 = a1;
-        a1 = a2;
-        a2 = a3;
-        wfed++;
-        if (--acnt == 0) {
-            a0 = blk.x;
-            a1 = blk.y;
-            a2 = blk.z;
-            a3 = blk.w;
-            acnt = 4;
-            blk = load_block(wbase, nvalid, nb);
-            // entering a new 128-byte line of input: ask L2 for the line `ahead` lines further on, so
-            // that the block loads find the lane's stream in L2 rather than DRAM
-            if (ahead && (nb & 7u) == 0 && 4 * (nb + 8 * ahead) < nvalid) prefetch_l2(wbase + 4 * (nb + 8 * ahead));
-            nb++;
-        }
-    };
-    auto refill = [&]() {  // afterwards bc >= 33
-        if (bc <= 32) {
-            bb |= (uint64_t)a0 << bc;
-            bc += 32;
-            next_word();
-        }
-    };
-    auto consume = [&](uint32_t k) {  // k <= bc
-        bb >>= k;
-        bc -= k;
-    };
-    auto consumed = [&]() { return wfed * 32u - bc - s0; };  // bits of the payload used
-    auto put = [&](uint32_t v, uint32_t k) {  // append k (0, 1 or 2) units, packed low unit first
-        if (k) {
-            const uint32_t wv = has ? (half | (v << 16)) : v;
-            if (k == 2 || has) slot[nwords++] = wv;
-            half = has ? (v >> 16) : v;
-            has ^= k & 1u;
-            nunits += k;
-        }
-    };
-    auto fail = [&](uint32_t code) {
-        err = code;
-        st = S_FIN;
-    };
-
     for (;;) {
-        // ---- lanes without a member take the next ones (one atomic per warp)
-        const unsigned idle = __ballot_sync(FULL, st == S_IDLE);
-        if (idle) {
-            const int leader = __ffs(idle) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(queue, (unsigned long long)__popc(idle));
-            base = __shfl_sync(FULL, base, leader);
-            if (st == S_IDLE) {
-                j = j0 + (long long)base + __popc(idle & ((1u << lane) - 1u));
-                if (j >= n) {
-                    st = S_DONE;
-                } else {
-                    const cb_member_job job = jobs[j];
-                    const uintptr_t in = (uintptr_t)job.in;
-                    wbase = reinterpret_cast<const uint32_t*>(in & ~(uintptr_t)15);
-                    s0 = (uint32_t)(in & 15) * 8;  // bits of the first block before the payload
-                    nvalid = (uint32_t)((in + job.in_len + 8 - (uintptr_t)wbase) >> 2);
-                    in_bits = job.in_len * 8u;
-                    isize = job.isize;
-                    bb = 0;
-                    bc = 0;
-                    wfed = 0;
-                    const uint4 b0 = load_block(wbase, nvalid, 0);
-                    a0 = b0.x;
-                    a1 = b0.y;
-                    a2 = b0.z;
-                    a3 = b0.w;
-                    acnt = 4;
-                    blk = load_block(wbase, nvalid, 1);
-                    nb = 2;
-                    for (uint32_t q = 0; q < (s0 >> 5); q++) next_word();  // whole words before the payload
-                    refill();
-                    refill();
-                    consume(s0 & 31u);
-                    pos = 0;
-                    final_block = false;
-                    nunits = nwords = half = has = 0;
-                    err = CB_OK;
-                    st = S_HDR;
-                    const unsigned long long so = reinterpret_cast<const unsigned long long*>(per_job)[2 * j + 1];
-                    slot = reinterpret_cast<uint32_t*>(arena + so);
-                    if (so + slot_bytes(isize) > arena_bytes) fail(CB_ERR_CAPACITY);
-                }
-            }
+        unsigned long long jj = 0;
+        if (lane == 0) jj = atomicAdd(queue + qi, 1ull);
+        const long long j = j0 + (long long)__shfl_sync(FULL, jj, 0);
+        if (j >= n) break;
+        const cb_member_job job = jobs[j];
+        const unsigned long long so = reinterpret_cast<const unsigned long long*>(per_job)[2 * j + 1];
+        const uint32_t st = so + slot_bytes(job.isize) <= arena_bytes ? decode_member(W, job, arena + so)
+                            : list_unfit                              ? ST_LISTED
+                                                                      : (uint32_t)CB_ERR_CAPACITY;
+        if (lane == 0) {
+            per_job[4 * j + 1] = st;
+            if (st == ST_LISTED) per_job[4 * atomicAdd(queue + Q_LISTED, 1ull)] = (uint32_t)j;
+            else report(summary, job_status, j, st);
         }
-        if (__all_sync(FULL, st == S_DONE)) break;
-
-        // ---- code tables, built by the whole warp for one lane at a time
-        for (unsigned b = __ballot_sync(FULL, st == S_BUILD_CL || st == S_BUILD); b; b &= b - 1) {
-            const int t = __ffs(b) - 1;
-            const int tst = __shfl_sync(FULL, st, t);
-            bool ok;
-            uint8_t* tb = W.lane[t];
-            if (tst == S_BUILD_CL) {
-                // the code-length code: its 19 lengths wait at LSYM; its table goes to the region's start,
-                // then the code lengths to come start from zero (runs of zeros are not written)
-                if (lane < 19) W.lens[lane] = tb[C::LSYM + lane];
-                __syncwarp();
-                ok = build_lane(W.lens, 19, 7, T_CL, reinterpret_cast<uint16_t*>(tb), nullptr, nullptr, nullptr,
-                                nullptr, W.scratch);
-                for (int k = lane; k < 80; k += 32) reinterpret_cast<uint32_t*>(tb + C::LSYM)[k] = 0;
-            } else {
-                // literal/length and distance codes: fixed (hlit 0 marks a fixed block) or lane t's lengths
-                const uint32_t th = __shfl_sync(FULL, hlit, t);
-                const uint32_t ttot = __shfl_sync(FULL, total, t);
-                int nl, nd;
-                if (th == 0) {
-                    for (int s = lane; s < 320; s += 32)
-                        W.lens[s] = s < 144 ? 8 : s < 256 ? 9 : s < 280 ? 7 : s < 288 ? 8 : 5;
-                    nl = 288;
-                    nd = 32;
-                } else {
-                    for (uint32_t s = lane; s < ttot; s += 32) W.lens[s] = tb[C::LSYM + s];
-                    nl = (int)th;
-                    nd = (int)(ttot - th);
-                }
-                __syncwarp();
-                ok = build_lane(W.lens, nl, C::LB, T_LIT, reinterpret_cast<uint16_t*>(tb + C::LIT), W.lim, nullptr,
-                                tb + C::LSYM, reinterpret_cast<uint32_t*>(tb + C::LHI), W.scratch) &&
-                     build_lane(W.lens + nl, nd, C::DB, T_DIST, reinterpret_cast<uint16_t*>(tb + C::DIST),
-                                W.lim + C::NLL, reinterpret_cast<uint16_t*>(tb + C::DSYM), nullptr, nullptr, W.scratch);
-            }
-            __syncwarp();
-            if (lane == t) {
-                if (!ok) {
-                    fail(CB_ERR_INFLATE);
-                } else if (tst == S_BUILD_CL) {
-                    st = S_CLENS;
-                    ci = 0;
-                } else {
-#pragma unroll
-                    for (int i = 0; i < C::NLL; i++) llim[i] = W.lim[i];
-#pragma unroll
-                    for (int i = 0; i < C::NLD; i++) dlim[i] = W.lim[C::NLL + i];
-                    st = S_RUN;
-                }
-            }
-            __syncwarp();
-        }
-
-        // ---- block headers and member ends (each lane its own; rare)
-        if (st == S_HDR) {
-            if (consumed() > in_bits) {
-                fail(CB_ERR_INFLATE);
-            } else {
-                refill();
-                const uint32_t h = (uint32_t)bb & 7u;
-                consume(3);
-                final_block = (h & 1u) != 0;
-                const uint32_t btype = h >> 1;
-                if (btype == 0) {
-                    consume(bc & 7u);  // to a byte boundary: whole words are loaded, so bc & 7 bits remain
-                    refill();
-                    const uint32_t x = (uint32_t)bb;
-                    const uint32_t len = x & 0xFFFFu, nlen = x >> 16;
-                    consume(32);
-                    if (len != (~nlen & 0xFFFFu) || len > isize - pos || consumed() + 8ull * len > in_bits) {
-                        fail(CB_ERR_INFLATE);
-                    } else {
-                        rem = len;
-                        st = len ? S_STORED : (final_block ? S_FIN : S_HDR);
-                    }
-                } else if (btype == 1) {
-                    hlit = 0;  // fixed codes
-                    st = S_BUILD;
-                } else if (btype == 2) {
-                    refill();
-                    const uint32_t x = (uint32_t)bb;
-                    hlit = (x & 31u) + 257;
-                    const uint32_t hdist = ((x >> 5) & 31u) + 1, hclen = ((x >> 10) & 15u) + 4;
-                    consume(14);
-                    if (hlit > 286 || hdist > 30) {
-                        fail(CB_ERR_INFLATE);
-                    } else {
-                        total = hlit + hdist;
-                        uint32_t* zc = reinterpret_cast<uint32_t*>(my_lens);
-#pragma unroll
-                        for (int k = 0; k < 5; k++) zc[k] = 0;
-                        for (uint32_t i = 0; i < hclen; i++) {
-                            refill();
-                            my_lens[kClOrder[i]] = (uint8_t)(bb & 7u);
-                            consume(3);
-                        }
-                        st = S_BUILD_CL;
-                    }
-                } else {
-                    fail(CB_ERR_INFLATE);
-                }
-            }
-        }
-        if (st == S_FIN) {
-            if (err == CB_OK && (consumed() > in_bits || pos != isize)) err = CB_ERR_INFLATE;
-            if (err == CB_OK && has) slot[nwords] = half;  // the last unit (the slot has 8 spare bytes)
-            per_job[4 * j] = nunits;
-            per_job[4 * j + 1] = err;
-            report(summary, job_status, j, err);
-            st = S_IDLE;
-        }
-
-        // ---- decode steps (lock step over the lanes' own streams); one straight path per symbol
-#pragma unroll 1
-        for (int k = 0; k < steps; k++) {
-            if (st == S_RUN) {
-                refill();
-                const uint32_t x = (uint32_t)bb;
-                uint32_t e = my_lit[x & C::LMASK];
-                if (e == E_LONG) e = long_lit_entry<C::NLL>(x, llim, my_lsym, my_lhi);
-                const uint32_t L = e_len(e);
-                const bool is_len = (e & 0x8000u) != 0;
-                const bool is_lit = e < 0x1000u;
-                const bool is_eob = !is_len && e_kind(e) == E_EOB;
-                const uint32_t ext = is_len ? (e >> 12) & 7u : 0u;
-                const uint32_t len = (e & 255u) + 3 + ((x >> L) & ((1u << ext) - 1u));
-                const uint32_t n1 = L + ext;  // <= 20 < bc
-                // the distance (used by lengths only) from the 32 bits after n1: the rest of bb and,
-                // past its bc bits, the next word a0 -- no refill inside the step
-                const uint32_t avail = bc - n1;
-                const uint32_t y = (uint32_t)(bb >> n1) | (avail < 32 ? a0 << avail : 0u);
-                uint32_t d = my_dist[y & C::DMASK];
-                if (is_len && d == E_LONG) d = long_entry<C::NLD, 32>(y, dlim, my_dsym);
-                const uint32_t dl = e_len(d);
-                uint32_t dbase, dext;
-                dist_code(d & 31u, dbase, dext);
-                const uint32_t dist = dbase + ((y >> dl) & ((1u << dext) - 1u));
-                // a literal may take the next code too when it is a literal of the root table: at most 15
-                // bits went to the first, and bb holds 33 or more (the step's second symbol)
-                const uint32_t xb = (uint32_t)(bb >> L);
-                const uint32_t eb = my_lit[xb & C::LMASK];
-                const bool two = is_lit && eb < 0x1000u && pos + 1 < isize;
-                const uint32_t k = n1 + (is_len ? dl + dext : two ? e_len(eb) : 0u);  // <= 48
-                if (k < bc) {
-                    consume(k);
-                } else {  // the step used bits of a0: it becomes the buffer
-                    const uint32_t r = k - bc;  // < 16
-                    bb = (uint64_t)(a0 >> r);
-                    bc = 32 - r;
-                    next_word();
-                }
-                const bool bad = (!is_len && !is_lit && !is_eob) || (is_lit && pos >= isize) ||
-                                 (is_len && (e_kind(d) != E_DIST || (d & 0x8000u) || dist > pos || len > isize - pos));
-                if (bad) {
-                    fail(CB_ERR_INFLATE);
-                } else {
-                    put(is_len ? unit_match(len, dist) : two ? ((e & 255u) | ((eb & 255u) << 16)) : (e & 255u),
-                        is_len ? 2u : two ? 2u : is_lit ? 1u : 0u);
-                    pos += is_len ? len : two ? 2u : is_lit ? 1u : 0u;
-                    if (is_eob) st = final_block ? S_FIN : S_HDR;
-                }
-            } else if (st == S_CLENS) {
-                refill();
-                const uint32_t x = (uint32_t)bb;
-                const uint32_t e = my_cltab[x & 127u];
-                const uint32_t L = e_len(e), s = e & 255u;
-                const uint32_t eb = s < 16 ? 0u : s == 16 ? 2u : s == 17 ? 3u : 7u;
-                const uint32_t rep = s < 16 ? 1u : (s == 18 ? 11u : 3u) + ((x >> L) & ((1u << eb) - 1u));
-                // a second plain length in the same step when its code follows (14 bits at most went to
-                // the first, bb holds 33 or more)
-                const uint32_t e2 = my_cltab[(uint32_t)(bb >> (L + eb)) & 127u];
-                const uint32_t s2 = e2 & 255u, L2 = e_len(e2);
-                const bool two = e_kind(e2) == E_CL && !(e2 & 0x8000u) && L2 != 0 && s2 < 16 && ci + rep < total;
-                consume(L + eb + (two ? L2 : 0u));
-                if (e_kind(e) != E_CL || (e & 0x8000u) || L == 0 || (s == 16 && ci == 0) || ci + rep > total) {
-                    fail(CB_ERR_INFLATE);
-                } else {
-                    if (s < 16) {
-                        my_lens[ci] = (uint8_t)s;
-                    } else if (s == 16) {
-                        const uint8_t v = my_lens[ci - 1];
-                        for (uint32_t r = 0; r < rep; r++) my_lens[ci + r] = v;  // 3-6 copies
-                    }
-                    ci += rep;
-                    if (two) my_lens[ci++] = (uint8_t)s2;
-                    if (ci == total) {
-                        if (my_lens[256] == 0) fail(CB_ERR_INFLATE);  // no end-of-block code
-                        else st = S_BUILD;
-                    }
-                }
-            } else if (st == S_STORED) {
-                refill();
-                const uint32_t x = (uint32_t)bb;
-                const uint32_t k2 = rem >= 2 ? 2u : 1u;
-                consume(8 * k2);
-                put(k2 == 2 ? ((x & 255u) | ((x << 8) & 0xFF0000u)) : (x & 255u), k2);
-                pos += k2;
-                rem -= k2;
-                if (rem == 0) st = final_block ? S_FIN : S_HDR;
-            }
-        }
+        __syncwarp();
     }
 }
 
 // ---------------------------------------------------------------- k_copy: one member per warp
 
-constexpr int WIN = 1024;                 // flush and CRC window
-static_assert(WIN == 32 * 32, "one 32-byte CRC column per lane");
+constexpr int COPY_WARPS = 2;             // warps per CTA
+constexpr uint32_t LINE = 128;            // output bytes of a round: a word per lane
+constexpr uint32_t GMAX = 1152;           // output bytes of a group of 64 sequences, at most
+constexpr uint32_t FAR_N = 32;            // sources fetched from HBM per group, of up to FAR_LEN bytes each
+constexpr uint32_t FAR_WORDS = 8, FAR_LEN = 4 * FAR_WORDS - 3;
+static_assert(GMAX >= 2 * (255 + 258), "two sequences fit a group");
 
-// WARPS_ warps per CTA, each with a ring of RING_ bytes: sources up to RING_ - 32 bytes back read
-// the ring, older ones the output already stored in HBM.
-template <int WARPS_, uint32_t RING_, int UPL_ = 1>
+// RING_: bytes of output each warp keeps in shared memory: sources up to RING_ - GMAX - LINE bytes back
+// read it, older ones the output already stored.
+template <uint32_t RING_>
 struct CopyCfg {
-    static constexpr int WARPS = WARPS_;
-    static constexpr int UPL = UPL_;              // units per lane in a group
-    static constexpr uint32_t GU = 32 * UPL_;     // units per group
     static constexpr uint32_t RING = RING_, RMASK = RING_ - 1;
-    // a group's tokens start within GMAX bytes: its output (GMAX + 258 at most) and the unflushed
-    // window before it (under WIN bytes) stay in the ring while the group is written
-    static constexpr uint32_t GMAX = RING_ - WIN - 258 - 64;
-    static_assert((RING_ & (RING_ - 1)) == 0 && RING_ >= 4096, "ring size");
-    struct CtaSmem {
-        uint32_t crc8[8][256];
-        uint32_t mulk[4][256];   // x * x^(8 (WIN - 32)) by bytes: moves a column past the other lanes
-        uint32_t tok[WARPS_][32 * UPL_];  // the tokens of the warp's current group, in order
-        alignas(16) uint8_t ring[WARPS_][RING_];
+    static_assert((RING_ & (RING_ - 1)) == 0 && RING_ >= 4096 && RING_ <= 16384, "ring size");
+    struct WarpSmem {
+        alignas(16) uint8_t ring[RING_];
+        uint32_t lit[64];                // the group's first literals (256 bytes)
+        uint32_t far[FAR_N * 9];         // fetched sources (and one word more each: fewer conflicts)
+        uint32_t tok[132], aux[132];
+        uint32_t map[(GMAX + LINE) / 4]; // per byte of the group's lines: the number of the token that starts there
     };
 };
 
-template <class S>
-__device__ __forceinline__ uint32_t mulk(const S& s, uint32_t x) {
-    return s.mulk[0][x & 255] ^ s.mulk[1][(x >> 8) & 255] ^ s.mulk[2][(x >> 16) & 255] ^ s.mulk[3][x >> 24];
-}
+// A group's tokens are the literal runs and matches of its sequences, numbered 4 l + 1 to 4 l + 4 for lane
+// l's two.  tok: in 16 bits what to add to a byte's place (from the group's first line) to get its source's
+// offset from the ring's start in shared memory.  The few tokens with a flag find it through aux: a match
+// closer than a line, whose source may be in the round itself, or across the ring's end (T_RING; aux: the
+// distance above bit 16, the start), and sources read from HBM (T_DIRECT; aux the same, or with T_PLAIN
+// what to add to get a literal's place from the group's first word of them).
+constexpr uint32_t T_RING = 1u << 16, T_DIRECT = 1u << 17, T_PLAIN = 1u << 18;
+constexpr uint32_t T_FLAGS = T_RING | T_DIRECT;
 
-// Store output bytes [ws, we) from the ring (byte p at slot p + a) to out, and fold them into this
-// lane's CRC column (window kwin; windows are aligned to the end of the member, the first one
-// padded by `pad` zero bytes in front).
-template <uint32_t RMASK, class S>
-__device__ __noinline__ uint32_t flush_window(uint8_t* out, uint32_t a, uint32_t ws, uint32_t we, uint32_t kwin,
-                                              uint32_t pad, uint32_t col, const uint8_t* ring, const S& s, bool crc) {
-    const int lane = threadIdx.x & 31;
-    const uintptr_t o16 = (uintptr_t)out & ~(uintptr_t)15;
-    const uintptr_t lo = (uintptr_t)out + ws, hi = (uintptr_t)out + we;
-    const uintptr_t A0 = lo & ~(uintptr_t)15;
-    const uint32_t nunits = (uint32_t)(((hi + 15) & ~(uintptr_t)15) - A0) >> 4;
-    for (uint32_t u = lane; u < nunits; u += 32) {
-        const uintptr_t ga = A0 + 16 * (uintptr_t)u;
-        const uint32_t sl = (uint32_t)(ga - o16) & RMASK;
-        if (ga >= lo && ga + 16 <= hi) {
-            *reinterpret_cast<uint4*>(ga) = *reinterpret_cast<const uint4*>(ring + sl);
-        } else {
-            for (uint32_t k = 0; k < 16; k++)
-                if (ga + k >= lo && ga + k < hi) *reinterpret_cast<uint8_t*>(ga + k) = ring[(sl + k) & RMASK];
-        }
-    }
-    if (crc) {
-        uint32_t c = mulk(s, col);
-        const long long v0 = (long long)kwin * WIN + 32 * lane - (long long)pad;  // position of the column
-        uint32_t wv[8];
-        if (v0 >= 0) {
-            // the column's 32 bytes from 9 aligned ring words (funnel shifts for the byte phase)
-            const uint32_t sl = (uint32_t)(v0 + a) & RMASK, w = sl >> 2, sh = (sl & 3u) * 8;
-            const uint32_t* rw = reinterpret_cast<const uint32_t*>(ring);
-            uint32_t r[9];
-#pragma unroll
-            for (int k = 0; k < 9; k++) r[k] = rw[(w + k) & (RMASK >> 2)];
-#pragma unroll
-            for (int k = 0; k < 8; k++) wv[k] = __funnelshift_r(r[k], r[k + 1], sh);
-        } else {
-            // the first window: zero bytes stand before the member's start
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                uint32_t v = 0;
-#pragma unroll
-                for (int t = 0; t < 4; t++) {
-                    const long long r0 = v0 + 4 * k + t;
-                    v |= (r0 >= 0 ? (uint32_t)ring[(uint32_t)(r0 + a) & RMASK] : 0u) << (8 * t);
-                }
-                wv[k] = v;
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 8; q += 2) c = crc_step8(s.crc8, c, wv[q], wv[q + 1]);
-        col = c;
-    }
-    __syncwarp();
-    return col;
-}
+// All ones, shifted left by n (0 from 32 on).
+__device__ __forceinline__ uint32_t shl_clamp(uint32_t n) { return __funnelshift_lc(0u, 0xFFFFFFFFu, n); }
 
-// zlib's CRC32 of the member from the lane columns.
-__device__ __noinline__ uint32_t finish_crc(uint32_t col, uint32_t isize) {
-    const int lane = threadIdx.x & 31;
-    uint32_t v = col;
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-        const int d = 1 << k;
-        const uint32_t other = __shfl_down_sync(FULL, v, d);
-        if ((lane & (2 * d - 1)) == 0) v = gf_mul(v, kCrc.seg[k]) ^ other;
-    }
-    v = __shfl_sync(FULL, v, 0);
-    return crc_finish(v, isize);
-}
-
+// Positions below are slots: bytes from the 128-byte line of the member's first output byte (a bytes
+// before it).  A group's output is written in rounds of one line, a word per lane: each byte of the word
+// belongs to the last token that starts at or before it.
 template <class C>
-__global__ void __launch_bounds__(C::WARPS * 32)
+__global__ void __launch_bounds__(COPY_WARPS * 32)
     k_copy(const cb_member_job* __restrict__ jobs, int64_t n_jobs, const int64_t* __restrict__ d_n_jobs,
-           uint8_t* out_base, int check_crc, uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws,
-           long long j0, long long j1, int qi) {
+           uint8_t* out_base, uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws,
+           const uint8_t* arena, long long j0, long long j1, int qi) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    typename C::CtaSmem& S = *reinterpret_cast<typename C::CtaSmem*>(smem_raw);
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-#pragma unroll
-        for (int b = 0; b < 4; b++) S.mulk[b][i] = gf_mul((uint32_t)i << (8 * b), kCrc.k992);
-    }
-    init_crc8(S.crc8);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint8_t* ring = S.ring[warp];
-    uint32_t* tokw = S.tok[warp];
-    const uint32_t incl = lane == 31 ? 0xFFFFFFFFu : (2u << lane) - 1u;  // lanes 0..lane
+    using WarpSmem = typename C::WarpSmem;
+    WarpSmem& W = reinterpret_cast<WarpSmem*>(smem_raw)[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint8_t* smem = W.ring;
+    uint32_t* ring4 = reinterpret_cast<uint32_t*>(W.ring);
+    const uint32_t LIT_AT = (uint32_t)(reinterpret_cast<const uint8_t*>(W.lit) - smem);
+    const uint32_t FAR_AT = (uint32_t)(reinterpret_cast<const uint8_t*>(W.far) - smem);
+    uint8_t* map1 = reinterpret_cast<uint8_t*>(W.map);
     unsigned long long* queue = reinterpret_cast<unsigned long long*>(ws) + qi;  // this launch's counter
-    const uint32_t* per_job = reinterpret_cast<const uint32_t*>(ws + WS_HEAD);
-    const uint8_t* arena = ws + arena_offset(n_jobs);
+    uint32_t* per_job = reinterpret_cast<uint32_t*>(ws + WS_HEAD);
     long long n = n_jobs;
     if (d_n_jobs) n = min((long long)n, (long long)*d_n_jobs);
     n = min(n, j1);  // this launch's jobs: [j0, j1)
-    const bool crc = check_crc != 0;
+    for (uint32_t i = lane; i < (GMAX + LINE) / 4; i += 32) W.map[i] = 0;
+    if (lane == 0) W.tok[0] = 0;  // bytes before the group's first
+    __syncwarp();
 
     for (;;) {
         unsigned long long jj = 0;
         if (lane == 0) jj = atomicAdd(queue, 1ull);
         const long long j = j0 + (long long)__shfl_sync(FULL, jj, 0);
         if (j >= n) break;
-        if (per_job[4 * j + 1] != CB_OK) continue;  // k_decode reported it
+        if (per_job[4 * j + 1] != CB_OK) continue;  // k_decode reported or listed it
         const cb_member_job job = jobs[j];
-        const uint32_t nu = per_job[4 * j];
-        const uint16_t* U =
-            reinterpret_cast<const uint16_t*>(arena + reinterpret_cast<const unsigned long long*>(per_job)[2 * j + 1]);
-        uint8_t* out = out_base + job.out_off;
-        const uint32_t a = (uint32_t)((uintptr_t)out & 15);
-        const uint32_t isize = job.isize;
-        const uint32_t pad = (uint32_t)(-(int32_t)isize) & (WIN - 1);
-        uint32_t p = 0, ws_ = 0, we = min((uint32_t)WIN - pad, isize), kwin = 0, col = 0;
-        uint32_t st = (nu > isize) ? (uint32_t)CB_ERR_INFLATE : (uint32_t)CB_OK;
-        // groups of GU = 32 * UPL units, lane l holding units UPL * l ... UPL * l + UPL - 1 of the group
-        constexpr int UPL = C::UPL;
-        constexpr uint32_t GU = C::GU;
-        uint32_t g = 0;
-        uint32_t u[UPL];
-#pragma unroll
-        for (int h = 0; h < UPL; h++) {
-            const uint32_t i = UPL * lane + h;
-            u[h] = (i < nu && st == CB_OK) ? (uint32_t)__ldcs(U + i) : 0u;
-        }
-        while (st == CB_OK && g < nu) {
-            // this group: units [g, g + cnt); a match head as the group's last unit waits for the next group
-            const uint32_t avail = min(GU, nu - g);
-            const uint32_t nl = __shfl_down_sync(FULL, u[0], 1);  // the unit after this lane's last
-            const bool head_last = avail == GU && (__shfl_sync(FULL, u[UPL - 1], 31) & 0xC000u) == 0x8000u;
-            uint32_t cnt = avail - (head_last ? 1u : 0u);
-            uint32_t len[UPL], ex[UPL];
-            uint32_t glen;
-            auto lengths = [&](uint32_t c) {  // bytes of each unit's token, and where each starts
-                uint32_t tot = 0;
-#pragma unroll
-                for (int h = 0; h < UPL; h++) {
-                    const uint32_t x = u[h];
-                    len[h] = UPL * lane + h < c ? (!(x & 0x8000u) ? 1u : (x & 0xC000u) == 0x8000u ? ((x >> 6) & 255u) + 3 : 0u)
-                                                : 0u;
-                    tot += len[h];
+        const uint8_t* slot = arena + reinterpret_cast<const unsigned long long*>(per_job)[2 * j + 1];
+        const uint32_t a = (uint32_t)((uintptr_t)(out_base + job.out_off) & 127);
+        uint8_t* base = out_base + job.out_off - a;  // slot 0
+        const uint32_t Eend = a + job.isize;
+        uint32_t P = a, st = CB_OK, run = 0;
+        uint4 head = __ldcg(reinterpret_cast<const uint4*>(slot));
+        for (;;) {  // runs
+            const uint32_t nl = head.x, ns = head.y, next = head.z;
+            const uint2* sq = reinterpret_cast<const uint2*>(slot + head.w) - 1;  // sequences 1, 0
+            const uint8_t* lits = slot + run + 16;
+            if (next != RUN_END) head = __ldcg(reinterpret_cast<const uint4*>(slot + next));
+            uint32_t g = 0, lbase = 0;  // sequences (an even number) and literals done
+            const uint2 none = make_uint2(0, 0);
+            uint2 seq = 2 * lane < ns ? __ldcg(sq - lane) : none;
+            uint32_t lw0 = 4 * lane < nl ? __ldcg(reinterpret_cast<const uint32_t*>(lits) + lane) : 0u;
+            uint32_t lw1 = 4 * lane + 128 < nl ? __ldcg(reinterpret_cast<const uint32_t*>(lits) + lane + 32) : 0u;
+            while (g < ns) {
+                // this lane's two sequences
+                uint32_t s0 = g + 2 * lane < ns ? seq.y : 0u, s1 = g + 2 * lane + 1 < ns ? seq.x : 0u;
+                uint32_t c0 = s0 >> 24, m0 = s0 & SEQ_MATCH ? ((s0 >> 16) & 255u) + 3 : 0u;
+                uint32_t c1 = s1 >> 24, m1 = s1 & SEQ_MATCH ? ((s1 >> 16) & 255u) + 3 : 0u;
+                const bool none0 = (s0 & 0xFFFFu) && !m0, none1 = (s1 & 0xFFFFu) && !m1;
+                const uint32_t v = (c0 + m0 + c1 + m1) | ((c0 + c1) << 16);
+                uint32_t gv;
+                uint32_t ex = warp_exclusive_scan(v, gv);
+                uint32_t cnt = min(64u, ns - g);
+                if ((gv & 0xFFFFu) > GMAX) {  // the lanes whose sequences end within GMAX bytes (at least one)
+                    const uint32_t keep = __popc(__ballot_sync(FULL, ((ex + v) & 0xFFFFu) <= GMAX));
+                    gv = __shfl_sync(FULL, ex + v, keep - 1);
+                    cnt = 2 * keep;
+                    if (lane >= (int)keep) {
+                        c0 = m0 = c1 = m1 = 0;
+                        ex = gv;
+                    }
                 }
-                uint32_t e0 = warp_exclusive_scan(tot, glen);
-#pragma unroll
-                for (int h = 0; h < UPL; h++) {
-                    ex[h] = e0;
-                    e0 += len[h];
+                const uint32_t glen = gv & 0xFFFFu, phase = lbase & 3u;
+                const uint8_t* lsrc = lits + (lbase & ~3u);  // byte 0 of lit
+                W.lit[lane] = lw0;
+                W.lit[lane + 32] = lw1;
+                // the next group's sequences and literals are loaded while this one is written
+                g += cnt;
+                lbase += gv >> 16;
+                {
+                    const uint32_t lb = lbase & ~3u;
+                    const uint32_t* lp = reinterpret_cast<const uint32_t*>(lits + lb) + lane;
+                    seq = g + 2 * lane < ns ? __ldcg(sq - (g >> 1) - lane) : none;
+                    lw0 = lb + 4 * lane < nl ? __ldcg(lp) : 0u;
+                    lw1 = lb + 4 * lane + 128 < nl ? __ldcg(lp + 32) : 0u;
                 }
-            };
-            lengths(cnt);
-            if (glen > C::GMAX) {
-                // keep the units whose token starts within GMAX bytes (a tail goes with its head); the
-                // starts only grow along the units, so the kept units are a prefix
-                const uint32_t prev_ex = __shfl_up_sync(FULL, ex[UPL - 1], 1);
-                uint32_t kept = 0;
-#pragma unroll
-                for (int h = 0; h < UPL; h++) {
-                    const bool tail = (u[h] & 0xC000u) == 0xC000u;
-                    const uint32_t start = tail ? (h > 0 ? ex[h > 0 ? h - 1 : 0] : (lane > 0 ? prev_ex : ex[h])) : ex[h];
-                    kept += __popc(__ballot_sync(FULL, UPL * lane + h < cnt && start < C::GMAX));
+                // places from the group's first line: its start, this lane's, and after each of its parts
+                const uint32_t R0 = P & ~(LINE - 1), p0 = P - R0, pe = p0 + glen;
+                const uint32_t b0 = p0 + (ex & 0xFFFFu), b1 = b0 + c0, b2 = b1 + m0, b3 = b2 + c1, b4 = b3 + m1;
+                const uint32_t d0 = (s0 & 0x7FFFu) + 1, d1 = (s1 & 0x7FFFu) + 1;
+                if (__any_sync(FULL, none0 || none1 || (m0 && d0 > R0 + b1 - a) || (m1 && d1 > R0 + b3 - a)) ||
+                    glen > Eend - P) {
+                    st = CB_ERR_INFLATE;
+                    break;
                 }
-                cnt = kept;
-                lengths(cnt);
-            }
-            // match heads: the distance from the head and its tail (the next unit; a head that is the
-            // last of the units, or not followed by a tail, is an error)
-            bool bad = false;
-            uint32_t tokv[UPL], myr[UPL], mybit[UPL];
-            bool is_tok[UPL];
+                // sources older than the ring will hold come to `far`
+                const uint32_t x0 = R0 + b1 - d0, x1 = R0 + b3 - d1;
+                const uint32_t old = R0 + ((pe + LINE - 1) & ~(LINE - 1));  // slots below old - RING
+                const bool old0 = m0 && x0 + C::RING < old, old1 = m1 && x1 + C::RING < old;
+                uint32_t f0 = FAR_N, f1 = FAR_N;  // their places there
+                const uint32_t any0 = __ballot_sync(FULL, old0), any1 = __ballot_sync(FULL, old1);
+                if (any0 | any1) {
+                    if (old0 && m0 <= FAR_LEN) f0 = __popc(any0 & lt);
+                    if (old1 && m1 <= FAR_LEN) f1 = __popc(any0) + __popc(any1 & lt);
+                    const uint32_t n0 = f0 < FAR_N ? ((x0 & 3u) + m0 + 3) >> 2 : 0u;
+                    const uint32_t n1 = f1 < FAR_N ? ((x1 & 3u) + m1 + 3) >> 2 : 0u;
+                    const uint32_t* q0 = reinterpret_cast<const uint32_t*>(base + (x0 & ~3u));
+                    const uint32_t* q1 = reinterpret_cast<const uint32_t*>(base + (x1 & ~3u));
+                    uint32_t w0[FAR_WORDS / 2], w1[FAR_WORDS / 2];
 #pragma unroll
-            for (int h = 0; h < UPL; h++) {
-                const uint32_t i = UPL * lane + h;
-                const uint32_t x = u[h];
-                const uint32_t nx = h + 1 < UPL ? u[h + 1 < UPL ? h + 1 : 0] : nl;
-                const bool head = i < cnt && (x & 0xC000u) == 0x8000u;
-                const uint32_t dist = head ? ((((x & 63u) << 9) | (nx & 511u)) + 1) : 0u;
-                bad |= (head && (i + 1 >= cnt || (nx & 0xC000u) != 0xC000u)) || (head && dist > p + ex[h]);
-                is_tok[h] = len[h] != 0;
-                tokv[h] = head ? (0x80000000u | dist) : (x & 255u);
-                // a token starts in round ex >> 5 of the group, at bit ex & 31 of that round's start mask
-                myr[h] = is_tok[h] ? ex[h] >> 5 : 0xFFFFFFFFu;
-                mybit[h] = 1u << (ex[h] & 31u);
-            }
-            // the next group's units are loaded while this one is written
-            const uint32_t g2 = g + cnt;
-            uint32_t u2[UPL];
+                    for (uint32_t h = 0; h < FAR_WORDS; h += FAR_WORDS / 2) {
+                        if (h && !__any_sync(FULL, n0 > h || n1 > h)) break;
 #pragma unroll
-            for (int h = 0; h < UPL; h++) {
-                const uint32_t i = g2 + UPL * lane + h;
-                u2[h] = i < nu ? (uint32_t)__ldcs(U + i) : 0u;
-            }
-            if (__any_sync(FULL, bad) || glen > isize - p) {
-                st = CB_ERR_INFLATE;
-                break;
-            }
-            // the group's tokens in order (tails are not tokens): literal byte, or 0x80000000 | distance
-            {
-                uint32_t ord = 0;
-                const uint32_t lower = (1u << lane) - 1u;
+                        for (uint32_t k = 0; k < FAR_WORDS / 2; k++) {
+                            w0[k] = h + k < n0 ? __ldcg(q0 + h + k) : 0u;
+                            w1[k] = h + k < n1 ? __ldcg(q1 + h + k) : 0u;
+                        }
 #pragma unroll
-                for (int h = 0; h < UPL; h++) ord += __popc(__ballot_sync(FULL, is_tok[h]) & lower);
-#pragma unroll
-                for (int h = 0; h < UPL; h++)
-                    if (is_tok[h]) tokw[ord++] = tokv[h];
-            }
-            __syncwarp();
-            uint32_t before = 0;  // tokens that start before this round
-            uint32_t ri = 0;
-#pragma unroll 2
-            for (uint32_t r0 = 0; r0 < glen; r0 += 32, ri++) {
-                const uint32_t rel = r0 + lane;
-                // the token of byte rel: tokens starting in this round set bits of a mask; the byte's
-                // token is the last one starting at or before it
-                uint32_t mine = 0;
-#pragma unroll
-                for (int h = 0; h < UPL; h++) mine |= myr[h] == ri ? mybit[h] : 0u;
-                const uint32_t sm = __reduce_or_sync(FULL, mine);
-                const uint32_t ord = before + __popc(sm & incl) - 1;
-                before += __popc(sm);
-                const uint32_t t = tokw[ord & (GU - 1)];
-                const uint32_t b = p + rel;
-                uint32_t val = t & 255u;
-                int src = lane;  // the lane of this round holding the byte's source
-                if (rel < glen && (t & 0x80000000u)) {
-                    const uint32_t x = b - (t & 0x7FFFFFFFu);
-                    if (x >= p + r0) src = (int)(x - (p + r0));
-                    else if (x + C::RING >= p + r0 + 32) val = ring[(x + a) & C::RMASK];
-                    else val = __ldcg(out + x);  // flushed long ago (the ring keeps the last RING - 32 bytes)
-                }
-                bool need = src != lane;
-                for (int it = 0; it < 6 && __any_sync(FULL, need); it++) {
-                    const uint32_t v2 = __shfl_sync(FULL, val, src);
-                    const int s2 = __shfl_sync(FULL, src, src);
-                    const bool n2 = __shfl_sync(FULL, (int)need, src) != 0;
-                    if (need) {
-                        if (!n2) {
-                            val = v2;
-                            need = false;
-                        } else {
-                            src = s2;
+                        for (uint32_t k = 0; k < FAR_WORDS / 2; k++) {
+                            if (h + k < n0) W.far[9 * f0 + h + k] = w0[k];
+                            if (h + k < n1) W.far[9 * f1 + h + k] = w1[k];
                         }
                     }
                 }
-                if (rel < glen) ring[(b + a) & C::RMASK] = (uint8_t)val;
+                {
+                    const uint32_t l0 = phase + (ex >> 16), l1 = l0 + c0;
+                    auto literals = [&](uint32_t id, uint32_t start, uint32_t c, uint32_t l) {
+                        map1[start] = (uint8_t)id;
+                        const bool held = l + c <= 256;
+                        W.tok[id] = (((held ? LIT_AT + l : 0u) - start) & 0xFFFFu) | (held ? 0u : T_DIRECT | T_PLAIN);
+                        W.aux[id] = l - start;
+                    };
+                    auto match = [&](uint32_t id, uint32_t start, uint32_t len, uint32_t d, uint32_t x, bool is_old, uint32_t f) {
+                        const uint32_t at = x & C::RMASK;
+                        map1[start] = (uint8_t)id;
+                        const bool held = is_old ? f < FAR_N : d >= LINE && at + len <= C::RING;
+                        W.tok[id] = (((!held ? 0u : is_old ? FAR_AT + 36 * f + (x & 3u) : at) - start) & 0xFFFFu) |
+                                    (held ? 0u : is_old ? T_DIRECT : T_RING);
+                        W.aux[id] = start | (d << 16);
+                    };
+                    if (c0) literals(4 * lane + 1, b0, c0, l0);
+                    if (m0) match(4 * lane + 2, b1, m0, d0, x0, old0, f0);
+                    if (c1) literals(4 * lane + 3, b2, c1, l1);
+                    if (m1) match(4 * lane + 4, b3, m1, d1, x1, old1, f1);
+                }
                 __syncwarp();
-            }
-            __syncwarp();  // the round loop read tokw; the next group writes it
-            p += glen;
-            while (we > ws_ && p >= we) {
-                col = flush_window<C::RMASK>(out, a, ws_, we, kwin, pad, col, ring, S, crc);
-                ws_ = we;
-                we = min(we + WIN, isize);
-                kwin++;
-            }
-            g = g2;
+                uint32_t carry = 0;
+                for (uint32_t rr = 0; rr < pe; rr += LINE) {
+                    const uint32_t rel = rr + 4 * lane, w = R0 + rel;
+                    const uint32_t m = W.map[rel >> 2];
+                    W.map[rel >> 2] = 0;
+                    // the token of the byte before the word: the last one that starts in a lane below, or
+                    // in an earlier round
+                    const uint32_t mlast = (m >> (24 - (__clz((int)m) & 24))) & 255u;
+                    const uint32_t has = __ballot_sync(FULL, m != 0), below = has & lt;
+                    uint32_t id = __shfl_sync(FULL, mlast, below ? 31 - __clz((int)below) : 0);
+                    if (!below) id = carry;
+                    if (has) carry = __shfl_sync(FULL, mlast, 31 - __clz((int)has));
+                    uint32_t ids[4], tk[4], v[4];
 #pragma unroll
-            for (int h = 0; h < UPL; h++) u[h] = u2[h];
+                    for (int k = 0; k < 4; k++) {
+                        const uint32_t b = (m >> (8 * k)) & 255u;
+                        id = b ? b : id;
+                        ids[k] = id;
+                        tk[k] = W.tok[id];
+                        v[k] = smem[(rel + k + tk[k]) & 0xFFFFu];
+                    }
+                    uint32_t word = v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24);
+                    // bytes before the group's first are there already
+                    const uint32_t mine = shl_clamp(w < P ? 8 * (P - w) : 0u);
+                    if (w < P) word = (word & mine) | (ring4[(w & C::RMASK) >> 2] & ~mine);
+                    const uint32_t fl = tk[0] | tk[1] | tk[2] | tk[3];
+                    if (__any_sync(FULL, rel < pe && (fl & T_FLAGS))) {
+                        const uint32_t fresh = max(R0 + rr, P);  // slots from here on are written in this round
+                        uint32_t pend = 0, ax[4];
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const uint32_t s = w + k;
+                            ax[k] = 0;
+                            if ((tk[k] & T_FLAGS) && s >= P && s < R0 + pe) {
+                                ax[k] = W.aux[ids[k]];
+                                const uint32_t x = s - (ax[k] >> 16);
+                                uint32_t b = 0;
+                                if (tk[k] & T_DIRECT) b = __ldcg(tk[k] & T_PLAIN ? lsrc + (rel + k + ax[k]) : base + x);
+                                else if (x >= fresh) pend |= 1u << k;
+                                else b = W.ring[x & C::RMASK];
+                                word = (word & ~(0xFFu << (8 * k))) | (b << (8 * k));
+                            }
+                        }
+                        while (__any_sync(FULL, pend != 0)) {
+                            // bytes whose sources are in this round: at each pass those below the first byte
+                            // still missing; a match that overlaps itself repeats the bytes before its start
+                            const uint32_t Q = __reduce_min_sync(FULL, pend ? w + __ffs((int)pend) - 1 : 0xFFFFFFFFu);
+                            ring4[(w & C::RMASK) >> 2] = word;
+                            __syncwarp();
+#pragma unroll
+                            for (int k = 0; k < 4; k++) {
+                                if (pend >> k & 1) {
+                                    const uint32_t d = ax[k] >> 16, start = R0 + (ax[k] & 0xFFFFu);
+                                    uint32_t x = w + k - d;
+                                    if (x >= start) x = start - d + (x - start) % d;
+                                    if (x < Q) {
+                                        word = (word & ~(0xFFu << (8 * k))) | ((uint32_t)W.ring[x & C::RMASK] << (8 * k));
+                                        pend &= ~(1u << k);
+                                    }
+                                }
+                            }
+                            __syncwarp();
+                        }
+                    }
+                    ring4[(w & C::RMASK) >> 2] = word;
+                    if (rel < pe && mine) {
+                        if (w >= a && w + 4 <= Eend) {
+                            // bytes of the word after the group's end are overwritten by the next one
+                            *reinterpret_cast<uint32_t*>(base + w) = word;
+                        } else {  // the member's first or last word: its own bytes only
+                            for (uint32_t s = max(w, P); s < min(w + 4, R0 + pe); s++)
+                                base[s] = (uint8_t)(word >> (8 * (s - w)));
+                        }
+                    }
+                    __syncwarp();
+                }
+                P += glen;
+            }
+            if (st != CB_OK || next == RUN_END || next <= run) break;  // runs only go forward
+            run = next;
         }
-        if (st == CB_OK && p != isize) st = CB_ERR_INFLATE;
-        if (st == CB_OK && crc && finish_crc(col, isize) != job.crc) st = CB_ERR_CRC;
-        if (lane == 0 && st != CB_OK) report(summary, job_status, j, st);
+        if (st == CB_OK && P != Eend) st = CB_ERR_INFLATE;
+        if (lane == 0 && st != CB_OK) {
+            per_job[4 * j + 1] = st;
+            report(summary, job_status, j, st);
+        }
         __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------- k_crc: one member per warp
+//
+// The polynomial P divides P(x^1024) (= P^1024 in characteristic 2), so a message may be reduced by
+// P(x^1024) first: rows of 1024 bits (a 4-byte word per lane) take the place of the polynomial's
+// single bits, and eliminating a row is an XOR of it into the 14 rows that P's other terms name --
+// seven three-input XORs per row of 128 bytes, in registers.  What is left are 32 rows; each lane
+// folds its words of them with a table of x^1024 and the lanes join with one multiplication each.
+// (Tables for every byte took a shared-memory access with conflicts per byte.)
+
+constexpr int CRC_NT = 256;
+
+struct CrcLane {
+    uint32_t x1024, k[32];  // x^1024; x^(32 (32 - l)): the bits after lane l's word of a row, and 32 more
+};
+constexpr CrcLane make_crc_lane() {
+    CrcLane c{};
+    const CrcConst q = make_crc_const();
+    c.x1024 = xpow_from(q.x2n, 1024);
+    uint32_t v = xpow_from(q.x2n, 32);
+    const uint32_t x32 = v;
+    for (int l = 31; l >= 0; l--) {
+        c.k[l] = v;
+        v = gf_mul(v, x32);
+    }
+    return c;
+}
+static __constant__ CrcLane kCrcLane = make_crc_lane();
+
+// v[i] ^= the rows d before it, d over the terms of the polynomial (x^(32 - d)).
+template <bool LAST>
+__device__ __forceinline__ void crc_rows(uint32_t (&v)[32], const uint32_t (&w)[8], int i0) {
+    constexpr int D[13] = {6, 9, 10, 16, 20, 21, 22, 24, 25, 27, 28, 30, 31};
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+        if (i < i0 || i >= i0 + 8) continue;
+        uint32_t x = v[i] ^ w[i & 7];  // v[i] so far: the row 32 before
+#pragma unroll
+        for (int t = 0; t < 13; t++)
+            if (!LAST || D[t] > i) x ^= v[(i - D[t]) & 31];
+        v[i] = x;
+    }
+}
+
+// The word of the message at byte position q (negative positions are zero bytes); with INV the first
+// four bytes are inverted (the CRC's initial value).
+__device__ __forceinline__ uint32_t crc_word_careful(const uint8_t* m, long long q, bool inv) {
+    uint32_t x = 0;
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        const long long r = q + t;
+        if (r >= 0) x |= ((uint32_t)m[r] ^ (inv && r < 4 ? 0xFFu : 0u)) << (8 * t);
+    }
+    return x;
+}
+
+__global__ void __launch_bounds__(CRC_NT)
+    k_crc(const cb_member_job* __restrict__ jobs, int64_t n_jobs, const int64_t* __restrict__ d_n_jobs,
+          const uint8_t* __restrict__ out_base, uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws,
+          long long j0, long long j1) {
+    __shared__ uint32_t fold[4][256];
+    for (int i = threadIdx.x; i < 1024; i += CRC_NT) fold[i >> 8][i & 255] = gf_mul((uint32_t)(i & 255) << (8 * (i >> 8)), kCrcLane.x1024);
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    uint32_t* per_job = reinterpret_cast<uint32_t*>(ws + WS_HEAD);
+    long long n = n_jobs;
+    if (d_n_jobs) n = min((long long)n, (long long)*d_n_jobs);
+    n = min(n, j1);
+    const long long warps = (long long)gridDim.x * (CRC_NT / 32);
+    for (long long j = j0 + (long long)blockIdx.x * (CRC_NT / 32) + (threadIdx.x >> 5); j < n; j += warps) {
+        if (per_job[4 * j + 1] != CB_OK) continue;
+        const cb_member_job job = jobs[j];
+        const uint8_t* m = out_base + job.out_off;
+        const uint32_t len = job.isize;
+        const bool inv = len >= 4;
+        const long long pad = (long long)((4096u - (len & 4095u)) & 4095u);
+        const long long iters = ((long long)len + pad) >> 12;
+        uint32_t v[32];
+#pragma unroll
+        for (int i = 0; i < 32; i++) v[i] = 0;
+        for (long long it = 0; it < iters; it++) {
+            const bool last = it + 1 == iters;
+#pragma unroll
+            for (int i0 = 0; i0 < 32; i0 += 8) {
+                uint32_t w[8];
+                const long long q0 = it * 4096 + i0 * 128 + 4 * lane - pad;
+                if (it * 4096 - pad < 4) {  // rows with bytes before the member or its first four
+#pragma unroll
+                    for (int i = 0; i < 8; i++) w[i] = crc_word_careful(m, q0 + 128 * i, inv);
+                } else {
+                    const uintptr_t ad = (uintptr_t)(m + q0);
+                    const uint32_t* wp = reinterpret_cast<const uint32_t*>(ad & ~(uintptr_t)3);
+                    const uint32_t sh = (uint32_t)(ad & 3) * 8;
+                    if (sh) {
+                        uint32_t hi[8];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) w[i] = __ldg(wp + 32 * i);
+#pragma unroll
+                        for (int i = 0; i < 8; i++) hi[i] = __ldg(wp + 32 * i + 1);
+#pragma unroll
+                        for (int i = 0; i < 8; i++) w[i] = __funnelshift_r(w[i], hi[i], sh);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; i++) w[i] = __ldg(wp + 32 * i);
+                    }
+                }
+                if (last) crc_rows<true>(v, w, i0);
+                else crc_rows<false>(v, w, i0);
+            }
+        }
+        uint32_t c = 0;
+#pragma unroll
+        for (int i = 0; i < 32; i++)
+            c = fold[0][c & 255] ^ fold[1][(c >> 8) & 255] ^ fold[2][(c >> 16) & 255] ^ fold[3][c >> 24] ^ v[i];
+        c = __reduce_xor_sync(FULL, gf_mul(c, kCrcLane.k[lane]));
+        const uint32_t crc = inv ? ~c : crc_finish(c, len);
+        if (lane == 0 && crc != job.crc) {
+            per_job[4 * j + 1] = CB_ERR_CRC;
+            report(summary, job_status, j, CB_ERR_CRC);
+        }
     }
 }
 
@@ -998,7 +1163,7 @@ __global__ void k_split_init(cb_inflate_summary* summary, unsigned long long* qu
     summary->reserved = 0;
     summary->n_bad = 0;
     summary->first_bad = INT64_MAX;
-    for (int q = 0; q < 4; q++) queue[q] = 0;  // decode and copy counters of up to two job ranges
+    for (int q = 0; q < 8; q++) queue[q] = 0;  // decode and copy counters of up to two job ranges, the list's
 }
 
 __global__ void k_split_finish(cb_inflate_summary* summary) {
@@ -1011,6 +1176,13 @@ __global__ void k_split_finish(cb_inflate_summary* summary) {
 using namespace cb;
 
 int cb_set_error(cudaError_t e);  // abi.cu
+int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base,
+                         int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
+                         size_t workspace_bytes, bool list_unfit, void* stream);
+// inflate.cu: the one-kernel form for the jobs list[4 * k], k < *count (on the device)
+int cb_inflate_listed(const cb_member_job* jobs, const uint32_t* list, const unsigned long long* count,
+                      uint8_t* out_base, int check_crc, uint32_t* job_status, cb_inflate_summary* summary,
+                      unsigned long long* queue, cudaStream_t s);
 
 namespace {
 
@@ -1033,65 +1205,68 @@ int occupancy(int (&cache)[MAX_DEVICES], K kernel, int threads, size_t smem) {
 
 int fail_occ(int o) { return cb_set_error(o == -1 ? cudaErrorInvalidDevice : (cudaError_t)(-o)); }
 
+// One inflate call's arguments.
+struct Call {
+    const cb_member_job* jobs;
+    int64_t n_jobs;
+    const int64_t* d_n_jobs;
+    uint8_t* out_base;
+    int check_crc;
+    uint32_t* job_status;
+    cb_inflate_summary* summary;
+    uint8_t *ws, *arena;
+    unsigned long long arena_bytes;
+    bool list_unfit;
+};
+
 // One launch's jobs: [j0, j1) of the table, and its queue counters (decode at qd, copy at qd + 1).
 struct Range {
     long long j0, j1;
     int qd;
 };
 
-template <class D>
-int launch_decode(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint32_t* job_status,
-                  cb_inflate_summary* summary, uint8_t* ws, unsigned long long arena_bytes, Range r, cudaStream_t s) {
+// CTAs for a persistent grid of `occ` per SM, `warps` members each, no more than the range has work for.
+unsigned grid_for(const Call& c, Range r, int occ, int warps) {
+    long long grid = (long long)cb_device_sm_count() * occ;
+    const long long by_work = (r.j1 - r.j0 + warps - 1) / warps;
+    if (!c.d_n_jobs && by_work < grid) grid = by_work;
+    return (unsigned)(grid < 1 ? 1 : grid);
+}
+
+int decode_range(const Call& c, Range r, cudaStream_t s) {
     static int cache[MAX_DEVICES];
-    const size_t smem = sizeof(typename D::CtaSmem);
-    const int o = occupancy(cache, split::k_decode<D>, D::WARPS * 32, smem);
+    const size_t smem = split::DEC_WARPS * sizeof(split::DecWarp);
+    const int o = occupancy(cache, split::k_decode, split::DEC_WARPS * 32, smem);
     if (o <= 0) return fail_occ(o);
-    long long grid = (long long)cb_device_sm_count() * o;
-    const long long by_work = (r.j1 - r.j0 + 32 * D::WARPS - 1) / (32 * D::WARPS);
-    if (!d_n_jobs && by_work < grid) grid = by_work;
-    split::k_decode<D><<<(unsigned)(grid < 1 ? 1 : grid), D::WARPS * 32, smem, s>>>(
-        jobs, n_jobs, d_n_jobs, job_status, summary, ws, arena_bytes, (int)cb_param(CB_PARAM_DECODE_STEPS),
-        (uint32_t)cb_param(CB_PARAM_DECODE_PREFETCH), r.j0, r.j1, r.qd);
+    split::k_decode<<<grid_for(c, r, o, split::DEC_WARPS), split::DEC_WARPS * 32, smem, s>>>(
+        c.jobs, c.n_jobs, c.d_n_jobs, c.job_status, c.summary, c.ws, c.arena, c.arena_bytes, c.list_unfit, r.j0, r.j1, r.qd);
     return CB_OK;
 }
 
 template <class C>
-int launch_copy(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base, int check_crc,
-                uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws, Range r, cudaStream_t s) {
+int launch_copy(const Call& c, Range r, cudaStream_t s) {
     static int cache[MAX_DEVICES];
-    const size_t smem = sizeof(typename C::CtaSmem);
-    const int o = occupancy(cache, split::k_copy<C>, C::WARPS * 32, smem);
+    const size_t smem = split::COPY_WARPS * sizeof(typename C::WarpSmem);
+    const int o = occupancy(cache, split::k_copy<C>, split::COPY_WARPS * 32, smem);
     if (o <= 0) return fail_occ(o);
-    long long grid = (long long)cb_device_sm_count() * o;
-    const long long by_work = (r.j1 - r.j0 + C::WARPS - 1) / C::WARPS;
-    if (!d_n_jobs && by_work < grid) grid = by_work;
-    split::k_copy<C><<<(unsigned)(grid < 1 ? 1 : grid), C::WARPS * 32, smem, s>>>(
-        jobs, n_jobs, d_n_jobs, out_base, check_crc, job_status, summary, ws, r.j0, r.j1, r.qd + 1);
+    split::k_copy<C><<<grid_for(c, r, o, split::COPY_WARPS), split::COPY_WARPS * 32, smem, s>>>(
+        c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status, c.summary, c.ws, c.arena, r.j0, r.j1, r.qd + 1);
     return CB_OK;
 }
 
-int decode_range(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint32_t* job_status,
-                 cb_inflate_summary* summary, uint8_t* ws, unsigned long long arena_bytes, Range r, cudaStream_t s) {
-    const int rb = (int)cb_param(CB_PARAM_DECODE_ROOT);
-    if (rb == 8)
-        return launch_decode<split::DecCfg<8, 6, 1>>(jobs, n_jobs, d_n_jobs, job_status, summary, ws, arena_bytes, r, s);
-    if (rb == 7)
-        return launch_decode<split::DecCfg<7, 5, 1>>(jobs, n_jobs, d_n_jobs, job_status, summary, ws, arena_bytes, r, s);
-    return launch_decode<split::DecCfg<6, 5, 1>>(jobs, n_jobs, d_n_jobs, job_status, summary, ws, arena_bytes, r, s);
-}
-
-int copy_range(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base, int check_crc,
-               uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws, Range r, cudaStream_t s) {
+int copy_range(const Call& c, Range r, cudaStream_t s) {
     const int cw = (int)cb_param(CB_PARAM_COPY_WARPS);
-    const int units = (int)cb_param(CB_PARAM_COPY_UNITS);
-#define CB_COPY(W, R, UPL) \
-    launch_copy<split::CopyCfg<W, R, UPL>>(jobs, n_jobs, d_n_jobs, out_base, check_crc, job_status, summary, ws, r, s)
-    if (cw == 2) return CB_COPY(2, 16384, 1);
-    if (cw == 3) return CB_COPY(3, 16384, 1);
-    if (cw == 12) return units == 4 ? CB_COPY(12, 8192, 4) : units == 2 ? CB_COPY(12, 8192, 2) : CB_COPY(12, 8192, 1);
-    if (cw == 24) return units >= 2 ? CB_COPY(24, 4096, 2) : CB_COPY(24, 4096, 1);
-    return units == 4 ? CB_COPY(6, 16384, 4) : units == 2 ? CB_COPY(6, 16384, 2) : CB_COPY(6, 16384, 1);
-#undef CB_COPY
+    // 4 KB: 28 warps per SM, 4.04 ms on 15,456 GEX members, 8 KB 16 warps and 4.39 ms
+    const int rc = cw == 12   ? launch_copy<split::CopyCfg<4096>>(c, r, s)
+                   : cw == 24 ? launch_copy<split::CopyCfg<8192>>(c, r, s)
+                              : launch_copy<split::CopyCfg<16384>>(c, r, s);
+    if (rc != CB_OK || !c.check_crc) return rc;
+    static int cache[MAX_DEVICES];
+    const int o = occupancy(cache, split::k_crc, split::CRC_NT, 0);
+    if (o <= 0) return fail_occ(o);
+    split::k_crc<<<grid_for(c, r, o, split::CRC_NT / 32), split::CRC_NT, 0, s>>>(
+        c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status, c.summary, c.ws, r.j0, r.j1);
+    return CB_OK;
 }
 
 // Two side streams per device for the pipelined form, and the events that join them to the caller's
@@ -1124,30 +1299,39 @@ int side_for(int dev, Side*& out) {
 
 extern "C" size_t cb_inflate_split_workspace_bytes(int64_t n_jobs, int64_t out_bytes) {
     if (n_jobs < 0 || out_bytes < 0) return 0;
-    return split::arena_offset(n_jobs) + 2 * (size_t)out_bytes + 16 * (size_t)n_jobs + 16;
+    return split::arena_offset(n_jobs) + 2 * (size_t)out_bytes + 80 * (size_t)n_jobs + 32;
 }
 
 extern "C" int cb_inflate_split(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base,
                                 int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
                                 size_t workspace_bytes, void* stream) {
+    return cb_inflate_split_any(jobs, n_jobs, d_n_jobs, out_base, check_crc, job_status, summary, workspace,
+                                workspace_bytes, false, stream);
+}
+
+int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base,
+                         int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
+                         size_t workspace_bytes, bool list_unfit, void* stream) {
     if (!summary || !workspace || n_jobs < 0 || workspace_bytes < split::arena_offset(n_jobs) + 16) return CB_ERR_ARG;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
-    const unsigned long long arena_bytes = workspace_bytes - split::arena_offset(n_jobs);
-    split::k_split_init<<<1, 1, 0, s>>>(summary, reinterpret_cast<unsigned long long*>(ws));
+    uint8_t* arena = reinterpret_cast<uint8_t*>(((uintptr_t)(ws + split::arena_offset(n_jobs)) + 15) & ~(uintptr_t)15);
+    const Call c{jobs, n_jobs, d_n_jobs, out_base, check_crc, job_status, summary, ws, arena,
+                 (unsigned long long)(ws + workspace_bytes - arena), list_unfit};
+    auto* queue = reinterpret_cast<unsigned long long*>(ws);
+    split::k_split_init<<<1, 1, 0, s>>>(summary, queue);
     if (n_jobs > 0) {
         split::k_slots<<<1, split::SLOT_NT, 0, s>>>(jobs, n_jobs, d_n_jobs, ws);
         // Pipelined: the jobs in two ranges, each decoded and then copied on its own stream, so that
-        // the second range's decode and the first range's copy take the GPU while the other decode
-        // runs out of members (one member per lane leaves lanes idle at its end).  Only with the job
-        // count known on the host.
+        // the second range's decode and the first range's copy fill the warps that the other's end
+        // leaves idle.  Only with the job count known on the host.
         const long long pipe = cb_param(CB_PARAM_DECODE_PIPELINE);
         const bool two = !d_n_jobs && n_jobs >= 2 && (pipe == 2 || (pipe == 1 && n_jobs >= 65536));
         int rc = CB_OK;
         if (!two) {
             const Range all{0, n_jobs, 0};
-            rc = decode_range(jobs, n_jobs, d_n_jobs, job_status, summary, ws, arena_bytes, all, s);
-            if (rc == CB_OK) rc = copy_range(jobs, n_jobs, d_n_jobs, out_base, check_crc, job_status, summary, ws, all, s);
+            rc = decode_range(c, all, s);
+            if (rc == CB_OK) rc = copy_range(c, all, s);
             if (rc != CB_OK) return rc;
         } else {
             int dev = 0;
@@ -1163,12 +1347,10 @@ extern "C" int cb_inflate_split(const cb_member_job* jobs, int64_t n_jobs, const
             if (e == cudaSuccess) e = cudaStreamWaitEvent(sd->x, sd->start, 0);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(sd->y, sd->start, 0);
             if (e != cudaSuccess) return cb_set_error(e);
-            rc = decode_range(jobs, n_jobs, d_n_jobs, job_status, summary, ws, arena_bytes, ra, sd->x);
-            if (rc == CB_OK) rc = decode_range(jobs, n_jobs, d_n_jobs, job_status, summary, ws, arena_bytes, rb, sd->y);
-            if (rc == CB_OK)
-                rc = copy_range(jobs, n_jobs, d_n_jobs, out_base, check_crc, job_status, summary, ws, ra, sd->x);
-            if (rc == CB_OK)
-                rc = copy_range(jobs, n_jobs, d_n_jobs, out_base, check_crc, job_status, summary, ws, rb, sd->y);
+            rc = decode_range(c, ra, sd->x);
+            if (rc == CB_OK) rc = decode_range(c, rb, sd->y);
+            if (rc == CB_OK) rc = copy_range(c, ra, sd->x);
+            if (rc == CB_OK) rc = copy_range(c, rb, sd->y);
             // join both side streams back to the caller's stream whatever happened above
             e = cudaEventRecord(sd->done_x, sd->x);
             if (e == cudaSuccess) e = cudaEventRecord(sd->done_y, sd->y);
@@ -1177,6 +1359,9 @@ extern "C" int cb_inflate_split(const cb_member_job* jobs, int64_t n_jobs, const
             if (rc != CB_OK) return rc;
             if (e != cudaSuccess) return cb_set_error(e);
         }
+        rc = cb_inflate_listed(jobs, reinterpret_cast<const uint32_t*>(ws + split::WS_HEAD), queue + split::Q_LISTED,
+                               out_base, check_crc, job_status, summary, queue + split::Q_LISTED + 1, s);
+        if (rc != CB_OK) return rc;
     }
     split::k_split_finish<<<1, 1, 0, s>>>(summary);
     return cb_set_error(cudaGetLastError());

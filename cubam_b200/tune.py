@@ -2,9 +2,8 @@
 
 cubam launches its kernels with fixed shapes (``src/cubam/_kernels.py:637-641``) and reads with a
 fixed chunk policy (``src/cubam/_memory.py:11-23``).  Here the shapes that matter are launch
-parameters of the library (``cb_set_param``): the inflate form, the root bits of form 3's lane
-decoder, the warps, window and group size of form 3's copy kernel, the decode steps between lane scheduling
-rounds, the input prefetch distance, and the tile of the record chain's walk.  :func:`tune` times
+parameters of the library (``cb_set_param``): the inflate form, the window of form 3's copy kernel, its
+two-range pipeline, and the tile of the record chain's walk.  :func:`tune` times
 candidates on a real batch (a :class:`~cubam_b200.batch.BatchPlan`), one parameter at a time in the
 order of their effect (coordinate descent from the current values), keeps the fastest, applies it
 to the process and stores it in a JSON cache:
@@ -31,11 +30,11 @@ from cubam_b200 import _lib
 #: candidate values per parameter, in the order they are tuned
 CANDIDATES = {
     "inflate_form": (_lib.PARAM_INFLATE_FORM, (1, 2, 3)),
-    "decode_root": (_lib.PARAM_DECODE_ROOT, (6, 7, 8)),
+    "decode_root": (_lib.PARAM_DECODE_ROOT, (7,)),  # no effect any more (nor copy_units, decode_steps, decode_prefetch)
     "copy_warps": (_lib.PARAM_COPY_WARPS, (6, 12, 24)),
-    "copy_units": (_lib.PARAM_COPY_UNITS, (1, 2, 4)),
-    "decode_steps": (_lib.PARAM_DECODE_STEPS, (8, 16, 32)),
-    "decode_prefetch": (_lib.PARAM_DECODE_PREFETCH, (0, 4, 8)),
+    "copy_units": (_lib.PARAM_COPY_UNITS, (2,)),
+    "decode_steps": (_lib.PARAM_DECODE_STEPS, (16,)),
+    "decode_prefetch": (_lib.PARAM_DECODE_PREFETCH, (4,)),
     "decode_pipeline": (_lib.PARAM_DECODE_PIPELINE, (0, 2)),
     "chain_tile": (_lib.PARAM_CHAIN_TILE, (0, 16384, 32768)),
 }
@@ -132,7 +131,7 @@ def tune(plan, reps: int = 2, path: Path | None = None, names=None, use_cache: b
     best["inflate_form"] = plan.form or best["inflate_form"]
     measured = {}
     for name in names or CANDIDATES:
-        if name in FORM3 and best["inflate_form"] != 3:
+        if len(CANDIDATES[name][1]) < 2 or (name in FORM3 and best["inflate_form"] != 3):
             continue
         stage = STAGE.get(name, "inflated")
         times = {}

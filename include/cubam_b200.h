@@ -93,18 +93,14 @@ int cb_device_sm_count(void);
  *                          shared memory 8 KiB at a time): a power of two, 2-64 KiB, or 0: 64 KiB,
  *                          less for chunks too small to give 16 tiles per SM (0)
  *   CB_PARAM_INFLATE_FORM  the form cb_inflate runs: 1 member per warp, 2 per lane, 3 split (3)
- *   CB_PARAM_DECODE_ROOT   literal/length root bits of form 3's lane decoder: 6, 7 or 8 (7)
- *   CB_PARAM_COPY_WARPS    warps per CTA of form 3's copy kernel: 2, 3 or 6 with a 16 KiB window per
- *                          warp, 12 with an 8 KiB window, 24 with a 4 KiB window (12)
- *   CB_PARAM_DECODE_STEPS  decode steps of form 3 between lane scheduling rounds: 1-64 (16)
- *   CB_PARAM_DECODE_PREFETCH  lines (128 B) of compressed input form 3's decoder asks L2 for ahead of
- *                          each lane's position: 0-16, 0 = none (4)
- *   CB_PARAM_SPLIT_MIN_JOBS   with CB_PARAM_INFLATE_FORM 3, form 0 runs form 1 for calls of fewer jobs
- *                          (form 3 decodes one member per lane, so it needs many members to fill the GPU):
- *                          0 or more (8192; on 15,456 GEX members form 3 took 16.7 ms, form 1 22.0)
- *   CB_PARAM_COPY_UNITS    DEFLATE units each lane of form 3's copy kernel takes per group: 1 (groups of
- *                          32 units), 2 (64; with 6, 12 or 24 copy warps) or 4 (128; with 6 or 12 copy
- *                          warps, else 2) (2)
+ *   CB_PARAM_DECODE_ROOT   no effect (kept for callers that set it): 6, 7 or 8 (7)
+ *   CB_PARAM_COPY_WARPS    the window of output that each warp of form 3's copy kernel keeps in shared
+ *                          memory: 16 KiB for 2, 3 or 6, 4 KiB for 12, 8 KiB for 24 (12)
+ *   CB_PARAM_DECODE_STEPS  no effect (kept for callers that set it): 1-64 (16)
+ *   CB_PARAM_DECODE_PREFETCH  no effect (kept for callers that set it): 0-16 (4)
+ *   CB_PARAM_SPLIT_MIN_JOBS   with CB_PARAM_INFLATE_FORM 3, form 0 runs form 1 for calls of fewer jobs: 0
+ *                          or more (CB_SPLIT_MIN_JOBS_ANY, the default: form 3 for any number of jobs)
+ *   CB_PARAM_COPY_UNITS    no effect (kept for callers that set it): 1, 2 or 4 (2)
  *   CB_PARAM_DECODE_PIPELINE  form 3 in two job ranges, each decoded and then copied on its own stream
  *                          (side streams joined back to the caller's by events), so that one range's
  *                          decode and the other's copy fill the lanes a decode leaves idle at its end:
@@ -124,6 +120,7 @@ enum {
     CB_PARAM_COPY_UNITS = 8,
     CB_PARAM_DECODE_PIPELINE = 9
 };
+#define CB_SPLIT_MIN_JOBS_ANY 8192
 int cb_set_param(int key, int64_t value);
 int64_t cb_get_param(int key);
 
@@ -177,10 +174,10 @@ int cb_inflate(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_job
                void* stream);
 
 /* cb_inflate with the form given: 1 = one member per warp, 2 = one member per lane (most
- * members in flight), 3 = cb_inflate_split, 0 = CB_PARAM_INFLATE_FORM (form 1 in place of form 3 for
- * fewer than CB_PARAM_SPLIT_MIN_JOBS jobs).  Form 3 runs only with a
- * workspace larger than cb_inflate_workspace_bytes() (sized by cb_inflate_split_workspace_bytes);
- * with the small workspace form 1 runs in its place.  Every form gives the same bytes and the same
+ * members in flight), 3 = cb_inflate_split, 0 = CB_PARAM_INFLATE_FORM (see CB_PARAM_SPLIT_MIN_JOBS).
+ * Form 3 runs only with a workspace larger than cb_inflate_workspace_bytes() (sized by
+ * cb_inflate_split_workspace_bytes); with the small workspace form 1 runs in its place.  With form 0 and
+ * fewer than 8192 jobs any workspace will do: jobs that form 3 has no room for run as in form 1.  Every form gives the same bytes and the same
  * per-job codes.  No cubam counterpart (cubam has one nvCOMP call, src/cubam/bgzf.py:595). */
 int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base,
                     int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
@@ -189,11 +186,11 @@ int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_
 /* Members the one-member-per-lane form keeps in flight on the current device (0 on error). */
 int64_t cb_inflate_lane_slots(void);
 
-/* ---- Inflate, form 3: the Huffman decode and the copy as two kernels (same contract as cb_inflate,
- *      replacing the same nvCOMP call, src/cubam/bgzf.py:587-611) ---------------------------------
- * k_decode decodes one member per lane (32 members per warp in lock step) into 16-bit units in a
- * token arena inside the workspace (a slot of 2 isize + 8 bytes per job, rounded up to 8); k_copy writes each member
- * with one warp through a shared-memory window (CB_PARAM_COPY_WARPS) and checks its CRC32.
+/* ---- Inflate, form 3: the Huffman decode, the copy and the CRC32 as three kernels (same contract as
+ *      cb_inflate, replacing the same nvCOMP call, src/cubam/bgzf.py:587-611) ------------------------
+ * Each takes a warp per member.  The decode's lanes decode 32 segments of the member at once into an
+ * arena inside the workspace (a slot of 2 isize + 64 bytes per job, rounded up to 16); the copy writes
+ * the member through a window in shared memory (CB_PARAM_COPY_WARPS).
  * out_bytes: the sum of isize over the jobs (or more); a job whose slot does not fit a smaller
  * workspace fails with CB_ERR_CAPACITY. */
 size_t cb_inflate_split_workspace_bytes(int64_t n_jobs, int64_t out_bytes);

@@ -1,0 +1,156 @@
+"""The split inflater (decode of 32 segments at once, copy by rounds, CRC32 by rows) against zlib where its
+tiles, windows and slots have edges."""
+
+import random
+import zlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA GPU", allow_module_level=True)
+
+from cubam_b200 import _lib, bgzf as G  # noqa: E402
+
+BLOCK = 0xFF00
+
+
+def _raw(data, level=6, strategy=zlib.Z_DEFAULT_STRATEGY, flush_every=0, mem=8):
+    z = zlib.compressobj(level, zlib.DEFLATED, -15, mem, strategy)
+    if not flush_every:
+        return z.compress(data) + z.flush()
+    parts = [z.compress(data[i : i + flush_every]) + z.flush(zlib.Z_FULL_FLUSH) for i in range(0, len(data), flush_every)]
+    return b"".join(parts) + z.flush()
+
+
+def _edges():
+    """Sizes at the edges of words, lines (128), CRC rows (4096) and members, as text, noise and runs."""
+    rng = random.Random(5)
+    out = []
+    for n in (1, 2, 3, 4, 5, 31, 32, 127, 128, 129, 255, 256, 257, 4093, 4095, 4096, 4097, 4100, 8191, 8193, BLOCK):
+        text = bytes(rng.choices(b"ACGT\n0123", k=n))
+        noise = rng.randbytes(n)
+        for p, kw in ((text, {}), (noise, {}), (b"x" * n, {}), (text, {"strategy": zlib.Z_FIXED}),
+                      (noise, {"strategy": zlib.Z_HUFFMAN_ONLY}), (text, {"level": 0})):
+            out.append((p, kw))
+    return out
+
+
+def _distances():
+    """Matches from just inside to just outside each window of the copy, and that overlap themselves."""
+    rng = random.Random(6)
+    out = []
+    for d in (1, 2, 3, 7, 8, 31, 127, 128, 129, 4095 - 1280, 4096, 8192 - 1280, 8192, 16384, 32767, 32768):
+        base = rng.randbytes(d)
+        out.append((base * (BLOCK // d) + base[: BLOCK % d], {}))
+        mixed = bytearray(base)
+        while len(mixed) < BLOCK - 300:  # short matches among literals
+            k = rng.randint(3, 40)
+            mixed += bytes(mixed[-d + i % d] for i in range(k)) + rng.randbytes(rng.randint(0, 3))
+        out.append((bytes(mixed), {"level": 9}))
+    return out
+
+
+def _blocks():
+    """Many blocks per member, down to ones whose runs do not fit the member's slot, and skewed codes."""
+    rng = random.Random(7)
+    text = bytes(rng.choices(b"ACGTN\tchr12345", k=BLOCK))
+    out = [(text[:30000], {"flush_every": k}) for k in (7, 40, 300, 2000, 9000)]
+    skew = bytes(rng.choices(range(64), weights=[1.0 / (1 << min(i, 20)) for i in range(64)], k=BLOCK // 2))
+    out.append((skew + rng.randbytes(BLOCK // 2 - 200), {"strategy": zlib.Z_HUFFMAN_ONLY}))
+    out.append((skew * 2, {"strategy": zlib.Z_HUFFMAN_ONLY}))
+    out.append((text, {"mem": 1}))
+    fib = [1, 1]
+    while len(fib) < 24:
+        fib.append(fib[-1] + fib[-2])
+    deep = [b for i, f in enumerate(fib) for b in [i * 11 % 256] * min(f, 9000)][: BLOCK]  # codes of all lengths
+    rng.shuffle(deep)
+    out.append((bytes(deep), {"strategy": zlib.Z_HUFFMAN_ONLY}))
+    return out
+
+
+def _table(cases, out_shift=0, gap=0):
+    """The members' bytes on the GPU and their job table (``gap`` unused bytes after each member's output)."""
+    blob, rows, off = bytearray(), [], out_shift
+    for data, kw in cases:
+        raw = _raw(data, **kw)
+        blob += bytes(18)
+        rows.append([len(blob), off, len(raw) | (len(data) << 32), zlib.crc32(data)])
+        blob += raw + zlib.crc32(data).to_bytes(4, "little") + len(data).to_bytes(4, "little")
+        off += len(data) + gap
+    buf = torch.frombuffer(blob, dtype=torch.uint8).cuda()
+    table = np.array(rows, dtype=np.int64)
+    table[:, 0] += buf.data_ptr()
+    return buf, torch.from_numpy(table).cuda(), off
+
+
+def _run(table, total, workspace_bytes, form, check_crc=True):
+    out = torch.full((total + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+    summ = torch.zeros(G.ctypes_sizeof(_lib.InflateSummary), dtype=torch.uint8, device="cuda")
+    codes = torch.full((len(table),), 99, dtype=torch.int32, device="cuda")
+    ws = torch.empty(workspace_bytes, dtype=torch.uint8, device="cuda")
+    G.launch_inflate(table.data_ptr(), len(table), out.data_ptr(), total, check_crc, summ.data_ptr(), ws, form,
+                     codes.data_ptr())
+    return out.cpu().numpy(), codes.cpu().numpy(), G.read_struct(summ, _lib.InflateSummary)
+
+
+@pytest.mark.parametrize("window", [6, 12, 24])
+@pytest.mark.parametrize("make", [_edges, _distances, _blocks], ids=["edges", "distances", "blocks"])
+def test_split_matches_zlib(make, window):
+    cases = make()
+    want = b"".join(d for d, _ in cases)
+    assert _lib.lib.cb_set_param(_lib.PARAM_COPY_WARPS, window) == 0
+    try:
+        for shift in (0, 5):
+            buf, table, total = _table(cases, shift)
+            out, codes, summ = _run(table, total, G.inflate_workspace_bytes(len(cases), total, 3), 3)
+            assert summ.status == 0 and summ.n_bad == 0 and summ.first_bad == -1 and not codes.any()
+            assert out[shift:total].tobytes() == want
+            assert (out[:shift] == 0xA5).all() and (out[total:] == 0xA5).all()
+    finally:
+        _lib.lib.cb_set_param(_lib.PARAM_COPY_WARPS, -1)
+
+
+def test_split_reports_crc_and_size():
+    """A wrong CRC32 (also unchecked), and an ISIZE one too small or too large, in members of every size."""
+    cases = [(d, kw) for d, kw in _edges() if len(d) > 1][::5]
+    buf, table, total = _table(cases, gap=1)  # room for the ISIZE that is one too large
+    rows = table.cpu().numpy().copy()
+    rows[0::4, 3] ^= 1
+    rows[1::4, 2] -= 1 << 32
+    rows[2::4, 2] += 1 << 32
+    bad = torch.from_numpy(rows).cuda()
+    size = G.inflate_workspace_bytes(len(cases), total + len(cases), 3)
+    kinds = np.arange(len(cases)) % 4
+    want = np.array([_lib.CRC, _lib.INFLATE, _lib.INFLATE, _lib.OK])[kinds]
+    out, codes, summ = _run(bad, total, size, 3)
+    assert codes.tolist() == want.tolist()
+    assert summ.n_bad == int((want != 0).sum()) and summ.first_bad == 0 and summ.status == _lib.CRC
+    _, codes, _ = _run(bad, total, size, 3, check_crc=False)
+    assert codes.tolist() == np.where(want == _lib.CRC, _lib.OK, want).tolist()
+
+
+@pytest.mark.parametrize("room", ["small", "head", "half", "full", "odd"])
+def test_any_workspace_for_few_jobs(room):
+    """A call of few jobs that leaves the form to the library takes every workspace from 256 bytes up."""
+    cases = _edges()
+    buf, table, total = _table(cases)
+    full = int(_lib.lib.cb_inflate_split_workspace_bytes(len(cases), total))
+    size = {"small": 256, "head": 256 + 16 * len(cases) + 600, "half": full - total, "full": full, "odd": full + 9}[room]
+    out, codes, summ = _run(table, total, size, 0)
+    assert summ.status == 0 and not codes.any()
+    assert out[:total].tobytes() == b"".join(d for d, _ in cases)
+
+
+def test_split_workspace_too_small_is_an_error():
+    """Form 3 asked for by name: the jobs whose slots the workspace does not hold fail, the others do not."""
+    cases = [c for c in _edges() if len(c[0]) >= 4093]
+    buf, table, total = _table(cases)
+    full = int(_lib.lib.cb_inflate_split_workspace_bytes(len(cases), total))
+    out, codes, summ = _run(table, total, full - total, 3)
+    assert set(codes.tolist()) == {_lib.OK, _lib.CAPACITY} and codes[0] == 0 and codes[-1] == _lib.CAPACITY
+    assert summ.status == _lib.CAPACITY
+    assert out[: len(cases[0][0])].tobytes() == cases[0][0]
