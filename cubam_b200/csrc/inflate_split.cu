@@ -20,8 +20,8 @@
 //     form (cb_inflate_listed, inflate.cu).
 //
 // Measured on 15,456 GEX members (398 MB to 1.01 GB; a member per lane in the decoder and a byte per lane in
-// the copy before): decode 3.05 ms (10.45), copy 4.04 (5.16, CRC32 included), CRC32 0.42.  39 members:
-// decode 0.5 ms, copy 0.5 (one kernel with one serial decoder per member: 4.2).
+// the copy before): decode 3.05 ms (10.45), copy 3.8 (5.16, CRC32 included), CRC32 0.42.  41 members:
+// decode 0.47 ms, copy 0.43 (one kernel with one serial decoder per member: 4.2).
 //
 // Every loop is bounded: a decode step consumes input bits, bounded per member, a repair round
 // confirms at least one more segment; every shared-memory index is masked or checked; arena and
@@ -786,6 +786,7 @@ struct CopyCfg {
         alignas(16) uint8_t ring[RING_];
         uint32_t lit[64];                // the group's first literals (256 bytes)
         uint32_t far[FAR_N * 9];         // fetched sources (and one word more each: fewer conflicts)
+        uint2 want[FAR_N];               // their slots and lengths
         uint32_t tok[132], aux[132];
         uint32_t map[(GMAX + LINE) / 4]; // per byte of the group's lines: the number of the token that starts there
     };
@@ -793,21 +794,32 @@ struct CopyCfg {
 
 // A group's tokens are the literal runs and matches of its sequences, numbered 4 l + 1 to 4 l + 4 for lane
 // l's two.  tok: in 16 bits what to add to a byte's place (from the group's first line) to get its source's
-// offset from the ring's start in shared memory.  The few tokens with a flag find it through aux: a match
-// closer than a line, whose source may be in the round itself, or across the ring's end (T_RING; aux: the
-// distance above bit 16, the start), and sources read from HBM (T_DIRECT; aux the same, or with T_PLAIN
-// what to add to get a literal's place from the group's first word of them).
-constexpr uint32_t T_RING = 1u << 16, T_DIRECT = 1u << 17, T_PLAIN = 1u << 18;
-constexpr uint32_t T_FLAGS = T_RING | T_DIRECT;
+// offset from the ring's start in shared memory; T_NEAR: a match closer than a line (its distance from bit
+// 20), some of whose bytes may have their source in the same round.  The few tokens with T_WRAP (a source
+// across the ring's end) or T_DIRECT (one read from HBM: a literal with T_PLAIN, of the next run with
+// T_NEXT) find it through aux: the distance above bit 16 and the start, or for T_PLAIN what to add to get a
+// literal's place in lit, had it room.
+constexpr uint32_t T_NEAR = 1u << 16, T_WRAP = 1u << 17, T_DIRECT = 1u << 18, T_PLAIN = 1u << 19, T_NEXT = 1u << 27;
+constexpr uint32_t T_FLAGS = T_NEAR | T_WRAP | T_DIRECT;
+
+// A run as k_copy reads it: offsets in the slot of its sequences 1, 0 (then 3, 2 before them) and of its
+// literals, their numbers and the next run's offset.
+struct Run {
+    uint32_t sq, lits, nl, ns, next;
+};
+__device__ __forceinline__ Run run_at(uint32_t at, uint4 head) {
+    return Run{head.w - 8, at + 16, head.x, head.y, head.z};
+}
 
 // All ones, shifted left by n (0 from 32 on).
 __device__ __forceinline__ uint32_t shl_clamp(uint32_t n) { return __funnelshift_lc(0u, 0xFFFFFFFFu, n); }
 
 // Positions below are slots: bytes from the 128-byte line of the member's first output byte (a bytes
-// before it).  A group's output is written in rounds of one line, a word per lane: each byte of the word
-// belongs to the last token that starts at or before it.
+// before it).  A group is 64 sequences of the current run, or its last ones and the first of the next.
+// Its output is written in rounds of one line, a word per lane: each byte of the word belongs to the
+// last token that starts at or before it.
 template <class C>
-__global__ void __launch_bounds__(COPY_WARPS * 32)
+__global__ void __launch_bounds__(COPY_WARPS * 32, C::RING == 4096 ? 14 : 8)
     k_copy(const cb_member_job* __restrict__ jobs, int64_t n_jobs, const int64_t* __restrict__ d_n_jobs,
            uint8_t* out_base, uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws,
            const uint8_t* arena, long long j0, long long j1, int qi) {
@@ -841,103 +853,137 @@ __global__ void __launch_bounds__(COPY_WARPS * 32)
         const uint32_t a = (uint32_t)((uintptr_t)(out_base + job.out_off) & 127);
         uint8_t* base = out_base + job.out_off - a;  // slot 0
         const uint32_t Eend = a + job.isize;
-        uint32_t P = a, st = CB_OK, run = 0;
-        uint4 head = __ldcg(reinterpret_cast<const uint4*>(slot));
-        for (;;) {  // runs
-            const uint32_t nl = head.x, ns = head.y, next = head.z;
-            const uint2* sq = reinterpret_cast<const uint2*>(slot + head.w) - 1;  // sequences 1, 0
-            const uint8_t* lits = slot + run + 16;
-            if (next != RUN_END) head = __ldcg(reinterpret_cast<const uint4*>(slot + next));
-            uint32_t g = 0, lbase = 0;  // sequences (an even number) and literals done
-            const uint2 none = make_uint2(0, 0);
-            uint2 seq = 2 * lane < ns ? __ldcg(sq - lane) : none;
-            uint32_t lw0 = 4 * lane < nl ? __ldcg(reinterpret_cast<const uint32_t*>(lits) + lane) : 0u;
-            uint32_t lw1 = 4 * lane + 128 < nl ? __ldcg(reinterpret_cast<const uint32_t*>(lits) + lane + 32) : 0u;
-            while (g < ns) {
+        uint32_t P = a, st = CB_OK;
+        const uint4 no_head = make_uint4(0, 0, RUN_END, 0);
+        auto head_at = [&](uint32_t at) { return at == RUN_END ? no_head : __ldcg(reinterpret_cast<const uint4*>(slot + at)); };
+        // the current run (g of its sequences and lbase of its literals done), the next one, and the head
+        // of the one after that
+        Run A = run_at(0, head_at(0));
+        uint32_t bat = A.next;
+        Run B = run_at(bat, head_at(bat));
+        uint32_t cat = B.next;
+        uint4 chead = head_at(cat);
+        uint32_t g = 0, lbase = 0;
+        // the group's make-up: lanes below inA have two sequences of A each, the others of B; B's literals
+        // follow A's in `lit` from byte boff
+        uint32_t nA, nB, boff;
+        uint2 seq;
+        uint32_t lw0, lw1;
+        auto compose = [&]() {
+            nA = min(64u, A.ns - g);
+            const uint32_t even = (nA + 1) & ~1u;
+            nB = min(64u - even, B.ns);
+            const uint32_t lb = lbase & ~3u;
+            boff = (A.nl - lb + 3) & ~3u;
+            const bool ofA = 2 * lane < even;
+            const uint32_t i = ofA ? g + 2 * lane : 2 * lane - even;
+            const uint32_t ns = ofA ? A.ns : B.ns;
+            seq = i < ns ? __ldcg(reinterpret_cast<const uint2*>(slot + ((ofA ? A.sq : B.sq) - 4 * i))) : make_uint2(0, 0);
+            if (i + 1 >= ns) seq.x = 0;
+            auto literals = [&](uint32_t o) {  // four, from byte o of lit
+                const bool isA = o < boff;
+                const uint32_t l = isA ? lb + o : o - boff;
+                return l < (isA ? A.nl : B.nl) ? __ldcg(reinterpret_cast<const uint32_t*>(slot + ((isA ? A.lits : B.lits) + l)))
+                                               : 0u;
+            };
+            lw0 = literals(4 * lane);
+            lw1 = literals(4 * lane + 128);
+        };
+        compose();
+        for (;;) {  // groups
+            {
                 // this lane's two sequences
-                uint32_t s0 = g + 2 * lane < ns ? seq.y : 0u, s1 = g + 2 * lane + 1 < ns ? seq.x : 0u;
+                const uint32_t s0 = seq.y, s1 = seq.x;
                 uint32_t c0 = s0 >> 24, m0 = s0 & SEQ_MATCH ? ((s0 >> 16) & 255u) + 3 : 0u;
                 uint32_t c1 = s1 >> 24, m1 = s1 & SEQ_MATCH ? ((s1 >> 16) & 255u) + 3 : 0u;
                 const bool none0 = (s0 & 0xFFFFu) && !m0, none1 = (s1 & 0xFFFFu) && !m1;
                 const uint32_t v = (c0 + m0 + c1 + m1) | ((c0 + c1) << 16);
                 uint32_t gv;
                 uint32_t ex = warp_exclusive_scan(v, gv);
-                uint32_t cnt = min(64u, ns - g);
+                const uint32_t even = (nA + 1) & ~1u;
+                uint32_t cA = nA, cB = nB;  // sequences done with this group
                 if ((gv & 0xFFFFu) > GMAX) {  // the lanes whose sequences end within GMAX bytes (at least one)
                     const uint32_t keep = __popc(__ballot_sync(FULL, ((ex + v) & 0xFFFFu) <= GMAX));
                     gv = __shfl_sync(FULL, ex + v, keep - 1);
-                    cnt = 2 * keep;
+                    cA = min(2 * keep, nA);
+                    cB = min(2 * keep > even ? 2 * keep - even : 0u, nB);
                     if (lane >= (int)keep) {
                         c0 = m0 = c1 = m1 = 0;
                         ex = gv;
                     }
                 }
-                const uint32_t glen = gv & 0xFFFFu, phase = lbase & 3u;
-                const uint8_t* lsrc = lits + (lbase & ~3u);  // byte 0 of lit
-                W.lit[lane] = lw0;
-                W.lit[lane + 32] = lw1;
-                // the next group's sequences and literals are loaded while this one is written
-                g += cnt;
-                lbase += gv >> 16;
-                {
-                    const uint32_t lb = lbase & ~3u;
-                    const uint32_t* lp = reinterpret_cast<const uint32_t*>(lits + lb) + lane;
-                    seq = g + 2 * lane < ns ? __ldcg(sq - (g >> 1) - lane) : none;
-                    lw0 = lb + 4 * lane < nl ? __ldcg(lp) : 0u;
-                    lw1 = lb + 4 * lane + 128 < nl ? __ldcg(lp + 32) : 0u;
-                }
+                const uint32_t glen = gv & 0xFFFFu;
                 // places from the group's first line: its start, this lane's, and after each of its parts
                 const uint32_t R0 = P & ~(LINE - 1), p0 = P - R0, pe = p0 + glen;
-                const uint32_t b0 = p0 + (ex & 0xFFFFu), b1 = b0 + c0, b2 = b1 + m0, b3 = b2 + c1, b4 = b3 + m1;
+                const uint32_t b0 = p0 + (ex & 0xFFFFu), b1 = b0 + c0, b2 = b1 + m0, b3 = b2 + c1;
                 const uint32_t d0 = (s0 & 0x7FFFu) + 1, d1 = (s1 & 0x7FFFu) + 1;
                 if (__any_sync(FULL, none0 || none1 || (m0 && d0 > R0 + b1 - a) || (m1 && d1 > R0 + b3 - a)) ||
                     glen > Eend - P) {
                     st = CB_ERR_INFLATE;
                     break;
                 }
+                // this lane's literals: place in lit; and lit
+                const bool ofB = 2 * lane >= even;
+                const uint32_t restA = A.nl - lbase;  // literals of A before B's
+                const uint32_t l0 = (ex >> 16) + (ofB ? boff - restA : lbase & 3u), l1 = l0 + c0;
+                const uint32_t srcA = A.lits + (lbase & ~3u), srcB = B.lits - boff;
+                W.lit[lane] = lw0;
+                W.lit[lane + 32] = lw1;
+                // the next group's sequences and literals are loaded while this one is written
+                g += cA;
+                lbase += min(gv >> 16, restA);
+                bool more = true;
+                if (g >= A.ns) {
+                    more = bat != RUN_END;
+                    if (more && cat <= bat) more = false;  // runs only go forward
+                    g = cB;
+                    lbase = (gv >> 16) - min(gv >> 16, restA);
+                    A = B;
+                    bat = cat;
+                    B = run_at(bat, chead);
+                    cat = B.next;
+                    if (more) chead = head_at(cat);
+                }
+                if (more) compose();
                 // sources older than the ring will hold come to `far`
                 const uint32_t x0 = R0 + b1 - d0, x1 = R0 + b3 - d1;
                 const uint32_t old = R0 + ((pe + LINE - 1) & ~(LINE - 1));  // slots below old - RING
                 const bool old0 = m0 && x0 + C::RING < old, old1 = m1 && x1 + C::RING < old;
                 uint32_t f0 = FAR_N, f1 = FAR_N;  // their places there
-                const uint32_t any0 = __ballot_sync(FULL, old0), any1 = __ballot_sync(FULL, old1);
+                const uint32_t any0 = __ballot_sync(FULL, old0 && m0 <= FAR_LEN);
+                const uint32_t any1 = __ballot_sync(FULL, old1 && m1 <= FAR_LEN);
                 if (any0 | any1) {
-                    if (old0 && m0 <= FAR_LEN) f0 = __popc(any0 & lt);
-                    if (old1 && m1 <= FAR_LEN) f1 = __popc(any0) + __popc(any1 & lt);
-                    const uint32_t n0 = f0 < FAR_N ? ((x0 & 3u) + m0 + 3) >> 2 : 0u;
-                    const uint32_t n1 = f1 < FAR_N ? ((x1 & 3u) + m1 + 3) >> 2 : 0u;
-                    const uint32_t* q0 = reinterpret_cast<const uint32_t*>(base + (x0 & ~3u));
-                    const uint32_t* q1 = reinterpret_cast<const uint32_t*>(base + (x1 & ~3u));
-                    uint32_t w0[FAR_WORDS / 2], w1[FAR_WORDS / 2];
+                    const uint32_t n0 = __popc(any0);
+                    if (any0 >> lane & 1u) f0 = __popc(any0 & lt);
+                    if (any1 >> lane & 1u) f1 = n0 + __popc(any1 & lt);
+                    if (f0 < FAR_N) W.want[f0] = make_uint2(x0, m0);
+                    if (f1 < FAR_N) W.want[f1] = make_uint2(x1, m1);
+                    __syncwarp();
+                    const uint2 t = lane < (int)(n0 + __popc(any1)) ? W.want[lane] : make_uint2(0, 0);
+                    const uint32_t nw = t.y ? ((t.x & 3u) + t.y + 3) >> 2 : 0u;
+                    const uint32_t* q = reinterpret_cast<const uint32_t*>(base + (t.x & ~3u));
+                    uint32_t* f = W.far + 9 * lane;
+                    uint32_t w[FAR_WORDS];
 #pragma unroll
-                    for (uint32_t h = 0; h < FAR_WORDS; h += FAR_WORDS / 2) {
-                        if (h && !__any_sync(FULL, n0 > h || n1 > h)) break;
+                    for (uint32_t k = 0; k < FAR_WORDS; k++) w[k] = k < nw ? __ldcg(q + k) : 0u;
 #pragma unroll
-                        for (uint32_t k = 0; k < FAR_WORDS / 2; k++) {
-                            w0[k] = h + k < n0 ? __ldcg(q0 + h + k) : 0u;
-                            w1[k] = h + k < n1 ? __ldcg(q1 + h + k) : 0u;
-                        }
-#pragma unroll
-                        for (uint32_t k = 0; k < FAR_WORDS / 2; k++) {
-                            if (h + k < n0) W.far[9 * f0 + h + k] = w0[k];
-                            if (h + k < n1) W.far[9 * f1 + h + k] = w1[k];
-                        }
-                    }
+                    for (uint32_t k = 0; k < FAR_WORDS; k++)
+                        if (k < nw) f[k] = w[k];
                 }
                 {
-                    const uint32_t l0 = phase + (ex >> 16), l1 = l0 + c0;
+                    const uint32_t plain = T_DIRECT | T_PLAIN | (ofB ? T_NEXT : 0u);
                     auto literals = [&](uint32_t id, uint32_t start, uint32_t c, uint32_t l) {
                         map1[start] = (uint8_t)id;
                         const bool held = l + c <= 256;
-                        W.tok[id] = (((held ? LIT_AT + l : 0u) - start) & 0xFFFFu) | (held ? 0u : T_DIRECT | T_PLAIN);
+                        W.tok[id] = (((held ? LIT_AT + l : 0u) - start) & 0xFFFFu) | (held ? 0u : plain);
                         W.aux[id] = l - start;
                     };
                     auto match = [&](uint32_t id, uint32_t start, uint32_t len, uint32_t d, uint32_t x, bool is_old, uint32_t f) {
                         const uint32_t at = x & C::RMASK;
                         map1[start] = (uint8_t)id;
-                        const bool held = is_old ? f < FAR_N : d >= LINE && at + len <= C::RING;
+                        const bool held = is_old ? f < FAR_N : at + len <= C::RING;
                         W.tok[id] = (((!held ? 0u : is_old ? FAR_AT + 36 * f + (x & 3u) : at) - start) & 0xFFFFu) |
-                                    (held ? 0u : is_old ? T_DIRECT : T_RING);
+                                    (!held ? (is_old ? T_DIRECT : T_WRAP) : d < LINE ? T_NEAR | (d << 20) : 0u);
                         W.aux[id] = start | (d << 16);
                     };
                     if (c0) literals(4 * lane + 1, b0, c0, l0);
@@ -947,6 +993,7 @@ __global__ void __launch_bounds__(COPY_WARPS * 32)
                 }
                 __syncwarp();
                 uint32_t carry = 0;
+                const uint32_t full0 = a > R0 ? a - R0 : 0u, full1 = Eend - R0;  // whole words of the member
                 for (uint32_t rr = 0; rr < pe; rr += LINE) {
                     const uint32_t rel = rr + 4 * lane, w = R0 + rel;
                     const uint32_t m = W.map[rel >> 2];
@@ -954,10 +1001,9 @@ __global__ void __launch_bounds__(COPY_WARPS * 32)
                     // the token of the byte before the word: the last one that starts in a lane below, or
                     // in an earlier round
                     const uint32_t mlast = (m >> (24 - (__clz((int)m) & 24))) & 255u;
-                    const uint32_t has = __ballot_sync(FULL, m != 0), below = has & lt;
+                    const uint32_t below = __ballot_sync(FULL, m != 0) & lt;
                     uint32_t id = __shfl_sync(FULL, mlast, below ? 31 - __clz((int)below) : 0);
                     if (!below) id = carry;
-                    if (has) carry = __shfl_sync(FULL, mlast, 31 - __clz((int)has));
                     uint32_t ids[4], tk[4], v[4];
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
@@ -967,52 +1013,67 @@ __global__ void __launch_bounds__(COPY_WARPS * 32)
                         tk[k] = W.tok[id];
                         v[k] = smem[(rel + k + tk[k]) & 0xFFFFu];
                     }
+                    carry = __shfl_sync(FULL, id, 31);
                     uint32_t word = v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24);
-                    // bytes before the group's first are there already
-                    const uint32_t mine = shl_clamp(w < P ? 8 * (P - w) : 0u);
-                    if (w < P) word = (word & mine) | (ring4[(w & C::RMASK) >> 2] & ~mine);
+                    if (rr == 0 && rel < p0) {  // bytes before the group's first are there already
+                        const uint32_t mine = shl_clamp(8 * (p0 - rel));
+                        word = (word & mine) | (ring4[(w & C::RMASK) >> 2] & ~mine);
+                    }
                     const uint32_t fl = tk[0] | tk[1] | tk[2] | tk[3];
                     if (__any_sync(FULL, rel < pe && (fl & T_FLAGS))) {
-                        const uint32_t fresh = max(R0 + rr, P);  // slots from here on are written in this round
-                        uint32_t pend = 0, ax[4];
+                        const int left = (int)(pe - rel), fresh = (int)max(rr, p0);  // written in this round from fresh on
+                        uint32_t pend = 0;  // bytes whose source is
 #pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            const uint32_t s = w + k;
-                            ax[k] = 0;
-                            if ((tk[k] & T_FLAGS) && s >= P && s < R0 + pe) {
-                                ax[k] = W.aux[ids[k]];
-                                const uint32_t x = s - (ax[k] >> 16);
-                                uint32_t b = 0;
-                                if (tk[k] & T_DIRECT) b = __ldcg(tk[k] & T_PLAIN ? lsrc + (rel + k + ax[k]) : base + x);
-                                else if (x >= fresh) pend |= 1u << k;
-                                else b = W.ring[x & C::RMASK];
-                                word = (word & ~(0xFFu << (8 * k))) | (b << (8 * k));
-                            }
-                        }
-                        while (__any_sync(FULL, pend != 0)) {
-                            // bytes whose sources are in this round: at each pass those below the first byte
-                            // still missing; a match that overlaps itself repeats the bytes before its start
-                            const uint32_t Q = __reduce_min_sync(FULL, pend ? w + __ffs((int)pend) - 1 : 0xFFFFFFFFu);
-                            ring4[(w & C::RMASK) >> 2] = word;
-                            __syncwarp();
+                        for (int k = 0; k < 4; k++)
+                            if ((tk[k] & T_NEAR) && k < left && (int)(rel + k - ((tk[k] >> 20) & (LINE - 1))) >= fresh)
+                                pend |= 1u << k;
+                        if (__any_sync(FULL, left > 0 && (fl & (T_WRAP | T_DIRECT)))) {
 #pragma unroll
                             for (int k = 0; k < 4; k++) {
-                                if (pend >> k & 1) {
-                                    const uint32_t d = ax[k] >> 16, start = R0 + (ax[k] & 0xFFFFu);
-                                    uint32_t x = w + k - d;
-                                    if (x >= start) x = start - d + (x - start) % d;
-                                    if (x < Q) {
-                                        word = (word & ~(0xFFu << (8 * k))) | ((uint32_t)W.ring[x & C::RMASK] << (8 * k));
-                                        pend &= ~(1u << k);
-                                    }
+                                if ((tk[k] & (T_WRAP | T_DIRECT)) && k < left) {
+                                    const uint32_t ax = W.aux[ids[k]], x = w + k - (ax >> 16);
+                                    uint32_t b = 0;
+                                    if (tk[k] & T_DIRECT)
+                                        b = __ldcg(tk[k] & T_PLAIN ? slot + ((tk[k] & T_NEXT ? srcB : srcA) + rel + k + ax) : base + x);
+                                    else if ((int)(x - R0) >= fresh) pend |= 1u << k;
+                                    else b = W.ring[x & C::RMASK];
+                                    word = (word & ~(0xFFu << (8 * k))) | (b << (8 * k));
                                 }
                             }
-                            __syncwarp();
+                        }
+                        if (__any_sync(FULL, pend != 0)) {
+                            // their sources; a match that overlaps itself repeats the bytes before its start
+                            int px[4];
+#pragma unroll
+                            for (int k = 0; k < 4; k++) {
+                                px[k] = 0x7FFFFFFF;
+                                if (pend >> k & 1) {
+                                    const uint32_t ax = W.aux[ids[k]], d = ax >> 16;
+                                    const int start = (int)(ax & 0xFFFFu);
+                                    px[k] = (int)(rel + k - d);
+                                    if (px[k] >= start) px[k] = start - (int)d + (int)((uint32_t)(px[k] - start) % d);
+                                }
+                            }
+                            do {
+                                // at each pass the bytes whose sources lie below the first one still missing
+                                const int Q = (int)__reduce_min_sync(FULL, pend ? rel + __ffs((int)pend) - 1 : 0x7FFFFFFFu);
+                                ring4[(w & C::RMASK) >> 2] = word;
+                                __syncwarp();
+#pragma unroll
+                                for (int k = 0; k < 4; k++) {
+                                    if (px[k] < Q) {
+                                        word = (word & ~(0xFFu << (8 * k))) | ((uint32_t)W.ring[(R0 + px[k]) & C::RMASK] << (8 * k));
+                                        pend &= ~(1u << k);
+                                        px[k] = 0x7FFFFFFF;
+                                    }
+                                }
+                                __syncwarp();
+                            } while (__any_sync(FULL, pend != 0));
                         }
                     }
                     ring4[(w & C::RMASK) >> 2] = word;
-                    if (rel < pe && mine) {
-                        if (w >= a && w + 4 <= Eend) {
+                    if (rel < pe && rel + 4 > p0) {
+                        if (rel >= full0 && rel + 4 <= full1) {
                             // bytes of the word after the group's end are overwritten by the next one
                             *reinterpret_cast<uint32_t*>(base + w) = word;
                         } else {  // the member's first or last word: its own bytes only
@@ -1023,9 +1084,8 @@ __global__ void __launch_bounds__(COPY_WARPS * 32)
                     __syncwarp();
                 }
                 P += glen;
+                if (!more) break;
             }
-            if (st != CB_OK || next == RUN_END || next <= run) break;  // runs only go forward
-            run = next;
         }
         if (st == CB_OK && P != Eend) st = CB_ERR_INFLATE;
         if (lane == 0 && st != CB_OK) {
