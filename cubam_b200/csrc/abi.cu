@@ -58,7 +58,7 @@ int64_t cb_param(int key) {
 }
 
 // CB_PARAM_INFLATE_FORM; for form 3 the caller may have set a number of jobs below which form 1 runs (form
-// 3 itself is the faster at every size: 39 GEX members take it 0.3 ms and form 1 4.2 ms).
+// 3 itself is the faster at every size: 39 GEX members take it 0.4 ms and form 1 4.2 ms).
 int cb_default_form(int64_t n_jobs) {
     const int form = (int)cb_param(CB_PARAM_INFLATE_FORM);
     const int64_t min_jobs = cb_param(CB_PARAM_SPLIT_MIN_JOBS);

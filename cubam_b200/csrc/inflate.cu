@@ -1187,9 +1187,9 @@ __global__ void __launch_bounds__(wm::WARPS * 32, 4)
     }
 }
 
-// The jobs list[4 * k], k < *count: the members that the two-kernel form leaves (usually none).
+// The jobs list[step * k], k < *count: the members that the two-kernel form leaves (usually none).
 __global__ void __launch_bounds__(wm::WARPS * 32, 4)
-    k_inflate_listed(const cb_member_job* __restrict__ jobs, const uint32_t* __restrict__ list,
+    k_inflate_listed(const cb_member_job* __restrict__ jobs, const uint32_t* __restrict__ list, int step,
                      const unsigned long long* __restrict__ count, uint8_t* out_base, int check_crc,
                      uint32_t* job_status, cb_inflate_summary* summary, unsigned long long* queue) {
     const unsigned long long n = *count;
@@ -1209,7 +1209,7 @@ __global__ void __launch_bounds__(wm::WARPS * 32, 4)
         if (lane == 0) k = atomicAdd(queue, 1ull);
         k = __shfl_sync(FULL, k, 0);
         if (k >= n) break;
-        const uint32_t j = list[4 * k];
+        const uint32_t j = list[step * k];
         const cb_member_job job = jobs[j];
         const uint32_t st = inflate_member(job, out_base, check_crc != 0, W, S);
         __syncwarp();
@@ -1447,7 +1447,7 @@ extern "C" int64_t cb_inflate_lane_slots(void) {
     return (int64_t)cb_device_sm_count() * b * Form2::WARPS * Form2::MLANES;
 }
 
-int cb_inflate_listed(const cb_member_job* jobs, const uint32_t* list, const unsigned long long* count,
+int cb_inflate_listed(const cb_member_job* jobs, const uint32_t* list, int step, const unsigned long long* count,
                       uint8_t* out_base, int check_crc, uint32_t* job_status, cb_inflate_summary* summary,
                       unsigned long long* queue, cudaStream_t s) {
     const size_t smem = sizeof(infl::wm::CtaSmem);
@@ -1460,7 +1460,7 @@ int cb_inflate_listed(const cb_member_job* jobs, const uint32_t* list, const uns
         if (dev >= 0) attr_set[dev].store(true, std::memory_order_release);
     }
     infl::k_inflate_listed<<<cb_device_sm_count() * 2, infl::wm::WARPS * 32, smem, s>>>(
-        jobs, list, count, out_base, check_crc, job_status, summary, queue);
+        jobs, list, step, count, out_base, check_crc, job_status, summary, queue);
     return cb_set_error(cudaGetLastError());
 }
 

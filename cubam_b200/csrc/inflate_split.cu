@@ -4,30 +4,35 @@
 // (src/cubam/bgzf.py:587-611) with the CRC32 check added (cubam's reader does not check it,
 // docs/reading.md:48-51).  DEFLATE is RFC 1951.
 //
-//  1. k_decode: one member per WARP, its 32 lanes decoding 32 segments of the member's bits at once.
-//     A Huffman decoder that starts at a wrong bit falls in step with the true symbols soon (on BAM
-//     members after 64 bits in half of the cases, after 512 in 99.5%), so every lane starts OVERLAP
-//     bits before its segment and notes the first symbol that begins in it; that must be where the
-//     lane before stopped, and a lane for which it is not decodes its segment again from there.  The
-//     lanes share one set of code tables in shared memory.  Their symbols go to the member's slot of
-//     an arena in HBM as runs (one per lane): literal bytes, and 4-byte sequences of a literal count
-//     and a match.
-//  2. k_copy: one member per WARP.  The warp takes 64 sequences at a time, places them by a prefix sum
-//     of their lengths and writes the output 128 bytes per round, a 4-byte word per lane, to a ring
-//     in shared memory (the sources of matches) and to HBM.
-//  3. k_crc: the CRC32 of every member's output, a warp per member, in registers.
-//  4. Members whose symbols do not fit their slot (many tiny blocks) are inflated by the one-kernel
-//     form (cb_inflate_listed, inflate.cu).
+//  1. k_decode: one member per CTA of W warps (W = 8, 4, 2 or 1, fewer the more members there are), its
+//     32 W lanes decoding as many segments of the member's bits at once.  A Huffman decoder that starts
+//     at a wrong bit falls in step with the true symbols soon (on BAM members after 64 bits in half of
+//     the cases, after 512 in 99.5%), so every lane starts OVERLAP bits before its segment and notes the
+//     first symbol that begins in it; that must be where the lane before stopped, and a lane for which
+//     it is not decodes its segment again from there.  The lanes share one set of code tables in shared
+//     memory.  Each lane writes its symbols, literal bytes and 4-byte sequences of a literal count and
+//     a match, to a run of its own in the member's output range, which is free until the copy; the
+//     warps then put the runs together in the member's slot of an arena in HBM.
+//  2. k_copy: one member per CTA of W warps.  They take 64 W sequences at a time, place them by a prefix
+//     sum of their lengths and write the output in rounds of 128 bytes per warp, a 4-byte word per lane,
+//     to a ring in shared memory (the sources of matches) and to HBM.
+//  3. k_crc: the CRC32 of every member's output, W warps per member, in registers.
+//  4. Members whose symbols do not fit their slot are inflated by the one-kernel form
+//     (cb_inflate_listed, inflate.cu).
 //
-// Measured on 15,456 GEX members (398 MB to 1.01 GB; a member per lane in the decoder and a byte per lane in
-// the copy before): decode 3.05 ms (10.45), copy 3.8 (5.16, CRC32 included), CRC32 0.42.  41 members:
-// decode 0.47 ms, copy 0.43 (one kernel with one serial decoder per member: 4.2).
+// What bounds them: with many members the issue of instructions (decode 0.54 per cycle and scheduler, at 18
+// warps per SM by shared memory); with few, the chain of steps of one lane and of rounds of one member,
+// which is why a member takes more warps then.  Measured, in ms (one serial decoder per member, in one
+// kernel, before; a warp per member in between):
+//   39 GEX members (10,000 records)      decode 0.21 (0.46), copy 0.16 (0.43), CRC32 0.02; one kernel 4.2
+//   about 70,000 (18 million records)    decode 12.6, copy 17.6, CRC32 2.5; all of it 47 with a member per lane
 //
 // Every loop is bounded: a decode step consumes input bits, bounded per member, a repair round
 // confirms at least one more segment; every shared-memory index is masked or checked; arena and
 // output writes stay within the member's slot and output range.
 
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "crc.cuh"
@@ -63,20 +68,24 @@ __constant__ uint8_t kClOrder[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12
 
 // ---------------------------------------------------------------- workspace
 
-// Workspace: [0, 256) queue counters; per job 16 bytes (u32 list of the members for the one-kernel
-// form, u32 status, u64 arena slot); the arena after that, 256-byte aligned.  Job j's slot is the
-// prefix sum of slot_bytes over the jobs before it (k_slots), so the arena holds
-// 2 sum(ISIZE) + 80 n_jobs bytes at most, whatever the jobs' output offsets are.
+// Workspace: [0, 256) queue counters; per job 32 bytes (u32 list of the members for the one-kernel
+// form, u32 status, u64 arena slot, u32 literals, u32 sequences); the arena after that, 256-byte
+// aligned.  Job j's slot is the prefix sum of slot_bytes over the jobs before it (k_slots), so the arena
+// holds 2 sum(ISIZE) + 80 n_jobs bytes at most, whatever the jobs' output offsets are.
 constexpr size_t WS_HEAD = 256;
-constexpr size_t PER_JOB = 16;
+constexpr size_t PER_JOB = 32;
+constexpr int JW = PER_JOB / 4;           // words per job
 constexpr int Q_LISTED = 6;               // queue counter: members for the one-kernel form
 constexpr uint32_t ST_LISTED = 0x100;     // internal status: on that list
 __host__ __device__ __forceinline__ size_t arena_offset(long long n_jobs) {
     return (WS_HEAD + PER_JOB * (size_t)n_jobs + 255) & ~(size_t)255;
 }
-// A slot's bytes, a multiple of 16 so that runs start 16-byte aligned.  Symbols take at most 4 bytes
-// per 3 output bytes (matches of length 3); the rest is room for the runs' heads and for lanes that
-// get more symbols than others.
+// A member's slot holds its symbols: literal bytes from its start up, sequences (a word each) from its end
+// down: bits 24-31 literals before the match, 16-23 match length - 3, 15 set when there is a match, 0-14
+// distance - 1.  Symbols take at most 4 bytes per 3 output bytes (matches of length 3); the rest is room
+// for sequences without a match (one per 255 literals, and at the end of a segment or block).
+constexpr uint32_t SEQ_MATCH = 0x8000u;
+constexpr uint32_t SEQ_BAD = 1u;  // without SEQ_MATCH: the match has no valid distance
 __host__ __device__ __forceinline__ unsigned long long slot_bytes(uint32_t isize) {
     return (2ull * isize + 64ull + 15ull) & ~15ull;
 }
@@ -133,22 +142,11 @@ __global__ void __launch_bounds__(SLOT_NT) k_slots(const cb_member_job* __restri
             const unsigned long long v = j < b ? (unsigned long long)slot_bytes(isz[k]) : 0ull;
             unsigned long long t;
             const unsigned long long x = warp_exclusive_scan(v, t);
-            if (j < b) slot[2 * j + 1] = carry + x;
+            if (j < b) slot[(JW / 2) * j + 1] = carry + x;
             carry += t;
         }
     }
 }
-
-// ---------------------------------------------------------------- runs
-//
-// A run is what one lane decoded of a block (or a stored block): at its start, 16-byte aligned, a head
-// of four words (literal bytes, sequences, offset of the next run in the slot or RUN_END, end of the
-// run), then the literals, and from its end downwards the sequences, one word each:
-//   bits 24-31 literals before the match, 16-23 match length - 3, 15 set when there is a match,
-//   0-14 distance - 1.
-constexpr uint32_t RUN_END = 0xFFFFFFFFu;
-constexpr uint32_t SEQ_MATCH = 0x8000u;
-constexpr uint32_t SEQ_BAD = 1u;  // without SEQ_MATCH: the match has no valid distance
 
 __device__ __forceinline__ void report(cb_inflate_summary* summary, uint32_t* job_status, long long j, uint32_t st) {
     if (job_status) job_status[j] = st;
@@ -159,38 +157,51 @@ __device__ __forceinline__ void report(cb_inflate_summary* summary, uint32_t* jo
     }
 }
 
-// ---------------------------------------------------------------- k_decode: one member per warp
+// ---------------------------------------------------------------- k_decode: one member per CTA of W warps
 
-// Entries of the literal/length table: bits 0-5 the bits of the code and its extra bits (SLOW: a code
-// longer than the table resolves), 6-9 the code length, 16-23 the literal or the length base - 3, and
+// Entries of the literal/length table: bits 0-5 the bits of the code and its extra bits (32: a code longer
+// than the table resolves), 6-9 the code length, 16-23 the literal or the length base - 3, and
 // flags; a literal has none.
 constexpr uint32_t F_MATCH = 1u << 31, F_EOB = 1u << 30, F_BAD = 1u << 29;
 // Entries of the distance table: bits 0-9 as above, 16-30 the distance base - 1, 31 set for a distance
 // (so the upper half is SEQ_MATCH | base - 1); a symbol that is none has bits 16-31 SEQ_BAD.
-constexpr uint32_t SLOW = 32;
+constexpr uint32_t SLOW = F_BAD | 32;  // (as a second literal: none)
 constexpr int ROOT = 9, DROOT = 8;     // bits that index the root tables
 constexpr uint32_t LNG = 512;          // entries for the longer literal/length codes, after the root's
+constexpr uint32_t DST = (1u << ROOT) + LNG;
 constexpr uint32_t OVERLAP = 512;      // bits a lane decodes before its segment to fall in step
-constexpr uint32_t SEG_MIN = 128, SEG_MAX = 4096;  // bits of a segment
+constexpr uint32_t SEG_MIN = 128;      // bits of a segment, at least
+constexpr uint32_t WINDOW = 179200;    // bits of a window of segments: a zlib block of 16,383 BAM symbols
+constexpr uint32_t BITS = (1u << 30) - 1;  // of a position in the member's input (its segments' ends have two flags)
+constexpr uint32_t RUN_MIN = 256;      // bytes of scratch per lane, at least (or one lane decodes alone)
 constexpr int ROWS = 16;               // words of input kept per lane
-constexpr int STEPS = 5;               // decode steps between refills
-constexpr int LROWS = 8, SROWS = 8;    // words of staged literals and sequences per lane
-constexpr uint32_t LC_MAX = 240;       // literals before a match, about (one sequence holds up to 255)
-constexpr int DEC_WARPS = 2;
-static_assert(STEPS + 15 <= 4 * LROWS && STEPS + 3 <= SROWS, "staging holds a round and what is left of the last");
+constexpr int STEPS = 8;               // decode steps between refills
+constexpr uint32_t LSTAGE = 32, SSTAGE = 16;  // staged literals (bytes) and sequences per lane
+constexpr uint32_t LC_MAX = 235;       // literals before a match, about (one sequence holds up to 255)
+static_assert(2 * STEPS + 15 <= (int)LSTAGE && STEPS + 4 <= (int)SSTAGE && LC_MAX + 2 * STEPS <= 255,
+              "staging holds a round and what is left of the last");
 
-// 10.3 KB per warp: 20 warps per SM.  The per-lane arrays (input, staging) are columns, word r of
-// lane l at r * 32 + l, so that their accesses never conflict.
-struct DecWarp {
-    uint32_t lit[(1 << ROOT) + LNG];
-    uint32_t dst[1 << DROOT];
-    uint32_t in[(ROWS + 2) * 32];   // rows ROWS, ROWS + 1 repeat rows 0, 1
-    uint32_t lst[LROWS * 32];       // while a header is read: the code lengths (bytes)
-    uint32_t sst[SROWS * 32];       // while a header is read: the code-length code's table (bytes)
+// Per member (a CTA of W warps): the code tables and what the warps tell each other.
+struct DecTables {
+    uint32_t tab[(1 << ROOT) + LNG + (1 << DROOT)];  // literal/length codes, then (from DST) distances
     uint32_t lfirst[17], lindex[17], dfirst[17], dindex[17];  // canonical codes by length, left-justified to 15 bits
-    uint32_t count[16];
+    uint32_t lcount[16], dcount[16];
     uint16_t lsym[288];             // symbols in canonical order
     uint16_t dsym[32];
+    unsigned long long job;
+    uint32_t say[9];
+};
+// Per warp.  The input is columns, word r of lane l at r * 32 + l (rows ROWS, ROWS + 1 repeat rows 0, 1);
+// the staging of a lane is contiguous, with odd word strides.
+struct DecWarp {
+    uint32_t in[(ROWS + 2) * 32];
+    uint32_t lst[32 * (LSTAGE / 4 + 1)];  // while a header is read: the code lengths (bytes)
+    uint32_t sst[32 * (SSTAGE + 1)];      // while a header is read: the code-length code's table (bytes)
+};
+template <int W> struct DecMember {
+    DecTables t;
+    uint32_t ends[32 * W], sums[2][W];
+    DecWarp w[W];
 };
 
 __device__ __forceinline__ uint32_t lit_entry(uint32_t s, uint32_t L) {
@@ -243,14 +254,15 @@ __device__ __forceinline__ void fill_forward(uint32_t* tab, int n) {
 // inflate: an over-subscribed code is an error, an incomplete one too unless its longest code has
 // length 1.  Returns false on error (the same in every lane).
 template <bool LIT>
-__device__ __noinline__ bool build_tables(DecWarp& W, const uint8_t* lens, int nsym, uint32_t& limit, uint32_t& lsh) {
+__device__ __noinline__ bool build_tables(DecTables& W, const uint8_t* lens, int nsym, uint32_t& limit, uint32_t& lsh) {
     constexpr int NB = LIT ? 9 : 1, RB = LIT ? ROOT : DROOT;
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
-    uint32_t* root = LIT ? W.lit : W.dst;
+    uint32_t* root = W.tab + (LIT ? 0u : DST);
     uint32_t* first = LIT ? W.lfirst : W.dfirst;
     uint32_t* index = LIT ? W.lindex : W.dindex;
-    if (lane < 16) W.count[lane] = 0;
+    uint32_t* count = LIT ? W.lcount : W.dcount;
+    if (lane < 16) count[lane] = 0;
     __syncwarp();
     uint32_t lr[NB];  // each symbol's code length, and its rank within the length
 #pragma unroll
@@ -258,13 +270,13 @@ __device__ __noinline__ bool build_tables(DecWarp& W, const uint8_t* lens, int n
         const int s = b * 32 + lane;
         const uint32_t L = s < nsym ? lens[s] : 0u;
         const uint32_t peers = __match_any_sync(FULL, L);
-        const uint32_t at = W.count[L];
+        const uint32_t at = count[L];
         __syncwarp();
-        if ((peers & lt) == 0) W.count[L] = at + __popc(peers);
+        if ((peers & lt) == 0) count[L] = at + __popc(peers);
         __syncwarp();
         lr[b] = L | ((at + __popc(peers & lt)) << 4);
     }
-    const uint32_t cnt = lane >= 1 && lane < 16 ? W.count[lane] : 0u;
+    const uint32_t cnt = lane >= 1 && lane < 16 ? count[lane] : 0u;
     uint32_t tot;
     // codes up to each length, left-justified (at most 288 << 14 < 2^23), and their number, in one sum
     const uint32_t before = warp_exclusive_scan(((lane < 16 ? cnt << (15 - lane) : 0u) << 9) | cnt, tot);
@@ -280,7 +292,7 @@ __device__ __noinline__ bool build_tables(DecWarp& W, const uint8_t* lens, int n
     limit = span ? lim : 32768u;
     lsh = span <= LNG ? 0u : 32u - (uint32_t)__clz((int)((span - 1) / LNG));
     const int slots = LIT ? (int)((span + (1u << lsh) - 1) >> lsh) : 0;  // at most LNG
-    uint32_t* lng = W.lit + (1 << ROOT);
+    uint32_t* lng = W.tab + (1 << ROOT);
     for (int i = lane; i < (1 << RB); i += 32) root[i] = 0;
     for (int i = lane; i < ((slots + 31) & ~31); i += 32) lng[i] = 0;
     __syncwarp();
@@ -313,7 +325,7 @@ __device__ __noinline__ bool build_tables(DecWarp& W, const uint8_t* lens, int n
 // The entry of a code whose next 15 bits are c (first bit highest), found by the limits of the code
 // lengths from L0 up.
 template <bool LIT>
-__device__ __noinline__ uint32_t long_entry(const DecWarp& W, uint32_t c, uint32_t L0) {
+__device__ __noinline__ uint32_t long_entry(const DecTables& W, uint32_t c, uint32_t L0) {
     const uint32_t* first = LIT ? W.lfirst : W.dfirst;
     uint32_t L = L0;
     while (L < 15 && c >= first[L + 1]) L++;
@@ -354,7 +366,7 @@ struct HeadBits {
 // into lens; p is left after them.  The 32 lanes decode the code at 32 bit positions at once; which of
 // those are symbols follows from the chain that starts at the first (pointer doubling).  Returns
 // literal/length codes | all codes << 16, or 0 on error.
-__device__ __noinline__ uint32_t read_lengths(DecWarp& W, HeadBits& hb, uint32_t& p, uint8_t* lens) {
+__device__ __noinline__ uint32_t read_lengths(DecTables& W, HeadBits& hb, uint32_t& p, uint8_t* lens, uint32_t* tab4) {
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
     hb.cover(p);
@@ -363,8 +375,8 @@ __device__ __noinline__ uint32_t read_lengths(DecWarp& W, HeadBits& hb, uint32_t
     p += 14;
     if (hlit > 286 || hdist > 30) return 0;
     // the code-length code: lane s its symbol's length and code (left-justified to 7 bits)
-    uint8_t* cl = reinterpret_cast<uint8_t*>(W.count);
-    if (lane < 16) W.count[lane] = 0;
+    uint8_t* cl = reinterpret_cast<uint8_t*>(W.lcount);
+    if (lane < 16) W.lcount[lane] = 0;
     for (int i = lane; i < 80; i += 32) reinterpret_cast<uint32_t*>(lens)[i] = 0;
     __syncwarp();
     hb.cover(p);
@@ -380,7 +392,7 @@ __device__ __noinline__ uint32_t read_lengths(DecWarp& W, HeadBits& hb, uint32_t
         if (Lt && (Lt < L || (Lt == L && t < lane))) code += 128u >> Lt;
     }
     if (__reduce_add_sync(FULL, space) != 128u) return 0;
-    uint32_t* tab4 = W.sst;  // 128 entries of a byte: length << 5 | symbol, never 0
+    // tab: 128 entries of a byte: length << 5 | symbol, never 0
     uint8_t* tab = reinterpret_cast<uint8_t*>(tab4);
     tab4[lane] = 0;
     __syncwarp();
@@ -459,18 +471,19 @@ struct LaneOut {
     bool over;             // more than the run holds (counted on, not stored)
 };
 
-// Store 16 staged literals (l) or 4 staged sequences, when the run holds them.
+// Store 16 staged literals or 4 staged sequences to the lane's run (cap bytes: literals from its start up,
+// sequences from its end down), when it holds them.  fl and fs are multiples of 16 and 4.
 __device__ __forceinline__ void store_lits(const DecWarp& W, LaneOut& o, uint8_t* run, uint32_t cap) {
-    const uint32_t* c = W.lst + ((o.fl >> 2) & (LROWS - 1)) * 32 + (threadIdx.x & 31);  // fl: a multiple of 16
-    o.fl += 16;
+    const uint32_t* c = W.lst + (threadIdx.x & 31) * (LSTAGE / 4 + 1) + ((o.fl & (LSTAGE - 1)) >> 2);
     if (16 + o.fl + 4 * o.fs > cap) o.over = true;
-    if (!o.over) *reinterpret_cast<uint4*>(run + o.fl) = make_uint4(c[0], c[32], c[64], c[96]);
+    if (!o.over) *reinterpret_cast<uint4*>(run + o.fl) = make_uint4(c[0], c[1], c[2], c[3]);
+    o.fl += 16;
 }
 __device__ __forceinline__ void store_seqs(const DecWarp& W, LaneOut& o, uint8_t* run, uint32_t cap) {
-    const uint32_t* c = W.sst + (o.fs & (SROWS - 1)) * 32 + (threadIdx.x & 31);  // fs: a multiple of 4
+    const uint32_t* c = W.sst + (threadIdx.x & 31) * (SSTAGE + 1) + (o.fs & (SSTAGE - 1));
     o.fs += 4;
-    if (16 + o.fl + 4 * o.fs > cap) o.over = true;
-    if (!o.over) *reinterpret_cast<uint4*>(run + cap - 4 * o.fs) = make_uint4(c[96], c[64], c[32], c[0]);
+    if (o.fl + 4 * o.fs > cap) o.over = true;
+    if (!o.over) *reinterpret_cast<uint4*>(run + cap - 4 * o.fs) = make_uint4(c[3], c[2], c[1], c[0]);
 }
 
 // A lane's input: 16 words in its column; the block after them is loaded a round ahead.
@@ -515,32 +528,37 @@ __device__ __forceinline__ uint32_t refill(LaneIn& in, uint32_t* col, uint32_t p
 
 // A symbol whose codes the tables do not resolve or that takes more than 32 bits (rare): x its first 32
 // bits, hi the next ones.  Returns its bits; e, d: its entries, y: the bits after the literal/length.
-__device__ __noinline__ uint32_t slow_symbol(const DecWarp& W, uint32_t x, uint32_t hi, uint32_t lsh, uint32_t& e,
+__device__ __noinline__ uint32_t slow_symbol(const DecTables& W, uint32_t x, uint32_t hi, uint32_t lsh, uint32_t& e,
                                              uint32_t& d, uint32_t& y) {
-    if ((e & 63u) == SLOW) e = long_entry<true>(W, __brev(x) >> 17, 15 - lsh);
+    if ((e & 63u) == 32u) e = long_entry<true>(W, __brev(x) >> 17, 15 - lsh);
     const uint32_t n = e & 63u;
     y = __funnelshift_r(x, hi, n);
-    d = W.dst[__brev(y) >> (32 - DROOT)];
-    if ((d & 63u) == SLOW) d = long_entry<false>(W, __brev(y) >> 17, DROOT + 1);
+    d = W.tab[DST + (__brev(y) >> (32 - DROOT))];
+    if ((d & 63u) == 32u) d = long_entry<false>(W, __brev(y) >> 17, DROOT + 1);
     return n + (e & F_MATCH ? d & 63u : 0u);
 }
 
-// One symbol at bit p of the lane's input: p moves past it.  With STORE it is staged and the lane stops
-// at an end-of-block or invalid code (end becomes 0); without, every code is passed over.  Literals and
-// matches take the same path (a warp has both at nearly every step); lim: where the codes longer than
-// the root begin, lim2: the table index of the first of them, as lim - (index << lsh).
+// One symbol at bit p of the lane's input, or two literals when the second one's code is in the root table
+// and starts below `end` (so that segments end at the same symbols whatever was taken together); p moves
+// past them.  With STORE they are staged and the lane stops at an end-of-block or invalid code (end
+// becomes 0); without, every code is passed over.  Literals and matches take the same path (a warp has
+// both at nearly every step): one access to the tables gives a match's distance code or the second
+// literal.  lim: where the codes longer than the root begin; lim2: the table index of the first of them, as
+// lim - (index << lsh).
 template <bool STORE>
-__device__ __forceinline__ void decode_step(DecWarp& W, uint32_t* col, uint32_t& p, uint32_t& end, uint32_t lim,
+__device__ __forceinline__ void decode_step(const DecTables& T, DecWarp& W, uint32_t* col, uint32_t& p, uint32_t& end, uint32_t lim,
                                             uint32_t lim2, uint32_t lsh, LaneOut& o) {
     const uint32_t* r = col + ((p >> 5) & (ROWS - 1)) * 32;
     const uint32_t w0 = r[0], w1 = r[32];
     const uint32_t x = __funnelshift_r(w0, w1, p);
     const uint32_t c = __brev(x) >> 17;
-    uint32_t e = W.lit[c >= lim ? (c - lim2) >> lsh : c >> (15 - ROOT)];
+    uint32_t e = T.tab[c >= lim ? (c - lim2) >> lsh : c >> (15 - ROOT)];
     uint32_t y = __funnelshift_r(x, 0u, e);  // shifts by bits 0-4
-    uint32_t d = W.dst[__brev(y) >> (32 - DROOT)];
-    uint32_t t = (e & 63u) + (e & F_MATCH ? d & 63u : 0u);
-    if (t >= 32) t = slow_symbol(W, x, __funnelshift_r(w1, r[64], p), lsh, e, d, y);
+    const uint32_t cy = __brev(y), n = e & 63u;
+    uint32_t d = T.tab[e & F_MATCH ? DST + (cy >> (32 - DROOT)) : cy >> (32 - ROOT)];
+    const bool lit2 = e < F_BAD && d < F_BAD && p + n < end;
+    uint32_t t = n + (lit2 || (e & F_MATCH) ? d & 63u : 0u);
+    if (t >= 32) t = slow_symbol(T, x, __funnelshift_r(w1, r[64], p), lsh, e, d, y);
     p += t;
     if (STORE) {
         const int lane = threadIdx.x & 31;
@@ -548,13 +566,14 @@ __device__ __forceinline__ void decode_step(DecWarp& W, uint32_t* col, uint32_t&
         const uint32_t len3 = ((e >> 16) & 255u) + __funnelshift_r(x & low_bits(e & 31u), 0u, e >> 6);
         const uint32_t dist = (d >> 16) + __funnelshift_r(y & low_bits(d & 31u), 0u, d >> 6);
         const uint32_t q = (o.lc << 24) | (len3 << 16) | dist;
-        if (match) W.sst[(o.ns & (SROWS - 1)) * 32 + lane] = q;
-        if (lit)
-            reinterpret_cast<uint8_t*>(W.lst)[((o.nl >> 2) & (LROWS - 1)) * 128 + lane * 4 + (o.nl & 3u)] =
-                (uint8_t)(e >> 16);
-        o.nl += lit;
+        if (match) W.sst[lane * (SSTAGE + 1) + (o.ns & (SSTAGE - 1))] = q;
+        uint8_t* l = reinterpret_cast<uint8_t*>(W.lst) + lane * (LSTAGE + 4);
+        if (lit) l[o.nl & (LSTAGE - 1)] = (uint8_t)(e >> 16);
+        if (lit2) l[(o.nl + 1) & (LSTAGE - 1)] = (uint8_t)(d >> 16);
+        const uint32_t k = (uint32_t)lit + lit2;
+        o.nl += k;
         o.ns += match;
-        o.lc = match ? 0u : o.lc + lit;
+        o.lc = match ? 0u : o.lc + k;
         if (e & (F_EOB | F_BAD)) {
             o.stop = e & F_BAD ? 2u : 1u;
             end = 0;
@@ -562,23 +581,109 @@ __device__ __forceinline__ void decode_step(DecWarp& W, uint32_t* col, uint32_t&
     }
 }
 
-// The Huffman-coded symbols of one block from bit p on, as runs from offset `at` of the member's slot;
-// p and at are left after them.  `last`: the block is the member's last.  CB_OK, CB_ERR_INFLATE or
-// ST_LISTED (they do not fit the slot).
-__device__ uint32_t decode_block(DecWarp& W, LaneIn& in, uint32_t& p0, uint32_t E, uint8_t* slot, uint32_t slot_n,
-                                 uint32_t& at, bool final_block, uint32_t limit, uint32_t lsh) {
-    const int lane = threadIdx.x & 31;
-    uint32_t* col = W.in + lane;
+// Barrier and vote over a member's W warps (W == 1: a CTA may hold several members).
+template <int W> __device__ __forceinline__ void sync_member() {
+    if (W == 1) __syncwarp();
+    else __syncthreads();
+}
+template <int W> __device__ __forceinline__ bool any_of_member(bool x) {
+    return W == 1 ? __any_sync(FULL, x) != 0 : __syncthreads_or(x) != 0;
+}
+
+// Exclusive sums over the member's threads of two values; their totals in ta and tb.
+template <int W>
+__device__ __forceinline__ void cta_scan2(DecMember<W>& M, uint32_t& a, uint32_t& b, uint32_t& ta, uint32_t& tb) {
+    const int warp = threadIdx.x >> 5;
+    a = warp_exclusive_scan(a, ta);
+    b = warp_exclusive_scan(b, tb);
+    if (W == 1) return;
+    if ((threadIdx.x & 31) == 0) {
+        M.sums[0][warp] = ta;
+        M.sums[1][warp] = tb;
+    }
+    __syncthreads();
+    ta = tb = 0;
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+        if (w == warp) {
+            a += ta;
+            b += tb;
+        }
+        ta += M.sums[0][w];
+        tb += M.sums[1][w];
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ uint32_t run_byte(const uint8_t* p) { return __ldcg(p); }
+
+// Move a run of n literals and k sequences (cap bytes) to dl and down from ds, by one warp: its loads are
+// issued ahead of its stores, eight words of each per lane.
+__device__ __forceinline__ void move_run(const uint8_t* run, uint32_t cap, uint32_t n, uint32_t k, uint8_t* dl,
+                                         uint32_t* ds) {
+    constexpr uint32_t U = 8;
+    const uint32_t lane = threadIdx.x & 31, h = min(n, (uint32_t)(-(intptr_t)dl & 3));
+    const uint32_t nw = (n - h) >> 2, tail = (n - h) & 3u;
+    const uint32_t* lw = reinterpret_cast<const uint32_t*>(run);
+    const uint32_t* sq = reinterpret_cast<const uint32_t*>(run + cap) - 1;
+    uint32_t* d = reinterpret_cast<uint32_t*>(dl + h);
+    // byte h + 4 i on of the literals in word i, and the head's and tail's bytes
+    const uint32_t hb = lane < h ? run_byte(run + lane) : 0u;
+    const uint32_t tb = lane < tail ? run_byte(run + n - tail + lane) : 0u;
+    for (uint32_t i0 = 0; i0 < k || i0 < nw; i0 += 32 * U) {
+        uint32_t q[U], a[U], b[U];
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++) {
+            const uint32_t i = i0 + 32 * u + lane;
+            q[u] = i < k ? __ldcg(sq - i) : 0u;
+            a[u] = i < nw ? __ldcg(lw + i) : 0u;
+            b[u] = i < nw && h ? __ldcg(lw + i + 1) : 0u;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++) {
+            const uint32_t i = i0 + 32 * u + lane;
+            if (i < k) ds[-(int)i] = q[u];
+            if (i < nw) d[i] = __funnelshift_r(a[u], b[u], 8 * h);
+        }
+    }
+    if (lane < h) dl[lane] = (uint8_t)hb;
+    if (lane < tail) dl[n - tail + lane] = (uint8_t)tb;
+}
+
+// Write n bytes to any dst, by one warp: word(i, h) gives the source's bytes h + 4 i to h + 4 i + 3, of which
+// h = 0 to 3 are before dst's first whole word.
+template <class F> __device__ __forceinline__ void put_bytes(uint8_t* dst, uint32_t n, F word) {
+    const uint32_t lane = threadIdx.x & 31, h = min(n, (uint32_t)(-(intptr_t)dst & 3));
+    if (lane < h) dst[lane] = (uint8_t)(word(0, 0) >> (8 * lane));
+    const uint32_t nw = (n - h) >> 2, tail = (n - h) & 3u;
+    uint32_t* d = reinterpret_cast<uint32_t*>(dst + h);
+    for (uint32_t i = lane; i < nw; i += 32) d[i] = word(i, h);
+    if (lane < tail) dst[n - tail + lane] = (uint8_t)(word(nw, h) >> (8 * lane));
+}
+
+// The Huffman-coded symbols of one block from bit p0 on, added to the nl literals and ns sequences in the
+// member's slot, by the whole CTA; p0, nl and ns are left after them.  scratch: scratch_n bytes, 16-byte
+// aligned, for the lanes' runs before they are put together.  CB_OK, CB_ERR_INFLATE or ST_LISTED (they do
+// not fit the slot), the same in every thread.
+template <int W>
+__device__ uint32_t decode_block(DecMember<W>& M, LaneIn& in, uint32_t& p0, uint32_t E, uint8_t* slot, uint32_t slot_n,
+                                 uint32_t& nl, uint32_t& ns, uint8_t* scratch, uint32_t scratch_n, uint32_t limit,
+                                 uint32_t lsh) {
+    constexpr uint32_t T = 32 * W;
+    const uint32_t tid = threadIdx.x % T, lane = tid & 31;
+    DecWarp& D = M.w[tid >> 5];
+    uint32_t* col = D.in + lane;
     const uint32_t lim2 = limit - ((1u << ROOT) << lsh);
-    for (;;) {  // windows of up to 32 segments
+    const uint32_t most = max(1u, min(T, scratch_n / RUN_MIN));  // lanes with room for a run
+    for (;;) {  // windows of up to T segments
         if (p0 >= E) return CB_ERR_INFLATE;
         const uint32_t R = E - p0;
-        const uint32_t seg = max(SEG_MIN, min(SEG_MAX, (R + 31) / 32));
-        const int A = (int)min(32u, (R + seg - 1) / seg);
-        const uint32_t b0 = p0 + lane * seg, b1 = min(b0 + seg, E);
-        const bool act = lane < A;
+        const uint32_t seg = max(SEG_MIN, (min(R, WINDOW) + most - 1) / most);
+        const uint32_t A = min(most, (R + seg - 1) / seg);
+        const uint32_t b0 = p0 + tid * seg, b1 = min(b0 + seg, E);
+        const bool act = tid < A;
         LaneOut o;
-        uint32_t p = lane * seg <= OVERLAP ? p0 : b0 - OVERLAP;
+        uint32_t p = tid * seg <= OVERLAP ? p0 : b0 - OVERLAP;
         if (act) start_input(in, col, p);
         __syncwarp();
         {
@@ -586,517 +691,596 @@ __device__ uint32_t decode_block(DecWarp& W, LaneIn& in, uint32_t& p0, uint32_t 
             while (__any_sync(FULL, p < end)) {
                 uint32_t to = 0;
                 if (p < end) to = min(end, refill(in, col, p));
-#pragma unroll
+#pragma unroll 1
                 for (int k = 0; k < STEPS; k++)
-                    if (p < to) decode_step<false>(W, col, p, to, limit, lim2, lsh, o);
+                    if (p < to) decode_step<false>(M.t, D, col, p, to, limit, lim2, lsh, o);
             }
         }
         uint32_t s = p;  // the first symbol of the lane's segment
-        // three quarters of the slot's free bytes by bits of input (symbols usually need a third of them;
-        // the last quarter is for a block that starts in the last segment)
-        const uint32_t share = (uint32_t)((unsigned long long)(slot_n - at) * min(R, 32 * seg) * 3 / (4ull * R));
-        uint32_t cap = (share / A) & ~15u;
-        if (cap < 48) cap = 0;
-        uint32_t run = at + lane * cap, next_at = at;
-        bool need = act, exact = false;
-        int F;
+        if (act) start_input(in, col, p);  // (decoded again from there, a segment gives the same sequences)
+        const uint32_t cap = (scratch_n / A) & ~15u;
+        uint8_t* run = scratch + tid * cap;
+        bool need = act, direct = false;
+        uint32_t F, al, as, tl, ts, my_l, my_s;
+        o.stop = 0;
         for (;;) {
             uint32_t end = 0;
             if (need) {
                 o.nl = o.ns = o.lc = o.fl = o.fs = o.stop = 0;
-                o.over = cap == 0;
+                o.over = false;
                 end = b1;
             }
             while (__any_sync(FULL, p < end)) {
                 uint32_t to = 0;
                 if (p < end) to = min(end, refill(in, col, p));
-#pragma unroll
+#pragma unroll 1
                 for (int k = 0; k < STEPS; k++)
-                    if (p < to) decode_step<true>(W, col, p, to, limit, lim2, lsh, o);
+                    if (p < to) decode_step<true>(M.t, D, col, p, to, limit, lim2, lsh, o);
                 if (need) {
                     if (o.stop) end = 0;
-                    if (o.nl - o.fl >= 16) store_lits(W, o, slot + run, cap);
-                    if (o.ns - o.fs >= 4) store_seqs(W, o, slot + run, cap);
-                    if (o.lc > LC_MAX) {  // a sequence's literal count has 8 bits
-                        W.sst[(o.ns & (SROWS - 1)) * 32 + lane] = o.lc << 24;
+                    if (!direct) {
+                        while (o.nl - o.fl >= 16) store_lits(D, o, run, cap);
+                        while (o.ns - o.fs >= 4) store_seqs(D, o, run, cap);
+                    }
+                    // a sequence's literal count has 8 bits; the literals after the last match have one of their own
+                    if (o.lc > LC_MAX || (p >= end && o.lc)) {
+                        D.sst[lane * (SSTAGE + 1) + (o.ns & (SSTAGE - 1))] = o.lc << 24;
                         o.ns++;
                         o.lc = 0;
                     }
-                    if (o.ns - o.fs >= 4) store_seqs(W, o, slot + run, cap);
+                    if (direct) {  // to their places, one by one (rare)
+                        for (; o.fl < o.nl && o.fl < my_l; o.fl++)
+                            slot[nl + al + o.fl] =
+                                reinterpret_cast<const uint8_t*>(D.lst)[lane * (LSTAGE + 4) + (o.fl & (LSTAGE - 1))];
+                        for (; o.fs < o.ns && o.fs < my_s; o.fs++)
+                            reinterpret_cast<uint32_t*>(slot + slot_n)[-1 - (int)(ns + as + o.fs)] =
+                                D.sst[lane * (SSTAGE + 1) + (o.fs & (SSTAGE - 1))];
+                    } else if (o.ns - o.fs >= 4 || (p >= end && o.ns > o.fs)) {
+                        store_seqs(D, o, run, cap);
+                    }
+                    if (p >= end) {
+                        need = false;
+                        if (!direct && o.nl > o.fl) store_lits(D, o, run, cap);
+                    }
                 }
-            }
-            if (need) {  // what is left, and the literals after the last match
-                if (o.lc) {
-                    W.sst[(o.ns & (SROWS - 1)) * 32 + lane] = o.lc << 24;
-                    o.ns++;
-                }
-                if (o.nl > o.fl) store_lits(W, o, slot + run, cap);
-                if (o.ns > o.fs) store_seqs(W, o, slot + run, cap);
             }
             // every segment up to the block's end must begin where the one before it ended
-            const uint32_t stopped = __ballot_sync(FULL, act && o.stop != 0);
-            F = stopped ? __ffs(stopped) - 1 : A - 1;
-            const uint32_t pe = __shfl_up_sync(FULL, p, 1);
-            need = lane > 0 && lane <= F && s != pe;
-            if (__any_sync(FULL, need)) {
+            M.ends[tid] = p | (act ? o.stop << 30 : 0u);
+            sync_member<W>();
+            F = A - 1;
+            for (uint32_t w = 0; w < T && w < A; w += 32) {
+                const uint32_t stopped = __ballot_sync(FULL, M.ends[w + lane] >> 30);
+                if (stopped) {
+                    F = w + __ffs((int)stopped) - 1;
+                    break;
+                }
+            }
+            const uint32_t pe = tid ? M.ends[tid - 1] & BITS : p0;
+            need = tid > 0 && tid <= F && s != pe;
+            if (any_of_member<W>(need)) {
                 if (need) s = p = pe;
             } else {
-                const bool over = __any_sync(FULL, lane <= F && o.over);
-                if (!over) break;
-                // some run was too short: lay the runs out by their sizes and decode them again
-                const uint32_t size = lane <= F ? 16 + ((o.nl + 15) & ~15u) + ((o.ns + 3) & ~3u) * 4 : 0u;
-                uint32_t tot;
-                const uint32_t ex = warp_exclusive_scan(size, tot);
-                if (exact || tot > slot_n - at) return ST_LISTED;
-                exact = true;
-                run = at + ex;
-                cap = size;
-                next_at = at + tot;
-                need = lane <= F;
+                if (direct) break;
+                my_l = al = tid <= F ? o.nl : 0u;
+                my_s = as = tid <= F ? o.ns : 0u;
+                cta_scan2<W>(M, al, as, tl, ts);
+                direct = any_of_member<W>(tid <= F && o.over);  // some run was too short: decode them again
+                if (!direct || nl + tl + 4ull * ((unsigned long long)ns + ts) > slot_n) break;
+                need = tid <= F;
                 p = s;
             }
             if (need) start_input(in, col, p);
             __syncwarp();
         }
-        const uint32_t stop = __shfl_sync(FULL, o.stop, F);
-        p0 = __shfl_sync(FULL, p, F);
+        const uint32_t stop = M.ends[F] >> 30;
+        p0 = M.ends[F] & BITS;
         if (stop == 2 || p0 > E) return CB_ERR_INFLATE;
-        if (!exact) next_at = at + (F + 1) * cap;
-        const uint32_t nrun = __shfl_down_sync(FULL, run, 1);
-        if (lane <= F)
-            *reinterpret_cast<uint4*>(slot + run) =
-                make_uint4(o.nl, o.ns, lane < F ? nrun : stop && final_block ? RUN_END : next_at, run + cap);
-        at = next_at;
-        __syncwarp();
+        if (nl + tl + 4ull * ((unsigned long long)ns + ts) > slot_n) return ST_LISTED;
+        if (!direct) {
+            // the runs, one after another, to the slot: each warp its lanes'
+            const uint32_t w0 = tid & ~31u;
+            for (uint32_t r = 0; r < 32 && w0 + r <= F; r++) {
+                const uint32_t n = __shfl_sync(FULL, my_l, r), k = __shfl_sync(FULL, my_s, r);
+                const uint32_t dl = nl + __shfl_sync(FULL, al, r), ds = ns + __shfl_sync(FULL, as, r);
+                move_run(scratch + (w0 + r) * cap, cap, n, k, slot + dl, reinterpret_cast<uint32_t*>(slot + slot_n) - 1 - ds);
+            }
+        }
+        nl += tl;
+        ns += ts;
+        sync_member<W>();  // the next window writes scratch and ends
         if (stop) return CB_OK;
     }
 }
 
-// One member's symbols into its slot.  CB_OK, CB_ERR_INFLATE or ST_LISTED.
-__device__ uint32_t decode_member(DecWarp& W, const cb_member_job& job, uint8_t* slot) {
-    const int lane = threadIdx.x & 31;
+// One member's symbols into its slot, by the whole CTA (out: the member's output, scratch until it is
+// written).  CB_OK, CB_ERR_INFLATE or ST_LISTED, the same in every thread.
+template <int W>
+__device__ uint32_t decode_member(DecMember<W>& M, const cb_member_job& job, uint8_t* slot, uint8_t* out, uint32_t& nl,
+                                  uint32_t& ns) {
+    const uint32_t tid = threadIdx.x % (32 * W), lane = tid & 31, warp = tid >> 5;
     LaneIn in;
     const uintptr_t src = (uintptr_t)job.in;
     in.wbase = reinterpret_cast<const uint32_t*>(src & ~(uintptr_t)15);
     in.nvalid = (uint32_t)((src + job.in_len + 8 - (uintptr_t)in.wbase) >> 2);
-    HeadBits hb;
-    hb.wbase = in.wbase;
-    hb.nvalid = in.nvalid;
     uint32_t p = (uint32_t)(src & 15) * 8;
     const uint32_t s0 = p, E = p + job.in_len * 8u;
     const uint32_t slot_n = (uint32_t)slot_bytes(job.isize);
-    uint32_t at = 0;
-    uint8_t* lens = reinterpret_cast<uint8_t*>(W.lst);
+    const uint32_t skip = (uint32_t)(-(intptr_t)out & 15);
+    uint8_t* scratch = out + skip;
+    const uint32_t scratch_n = job.isize > skip ? (job.isize - skip) & ~15u : 0u;
+    uint8_t* lens = reinterpret_cast<uint8_t*>(M.w[0].lst);
+    nl = ns = 0;
+    if (job.in_len > BITS / 16) return ST_LISTED;
     for (;;) {
         if (p > E) return CB_ERR_INFLATE;
-        hb.at(p);
-        const uint32_t h = hb.get(p);
-        p += 3;
-        const bool final_block = h & 1u;
-        const uint32_t btype = (h >> 1) & 3u;
-        if (btype == 3) return CB_ERR_INFLATE;
-        if (btype == 0) {
-            p = s0 + ((p - s0 + 7) & ~7u);
-            const uint32_t y = hb.get(p), len = y & 0xFFFFu;
-            p += 32;
-            if (len != (~y >> 16) || p > E || 8ull * len > E - p) return CB_ERR_INFLATE;
-            const uint32_t ns = (len + 254) / 255, size = 16 + ((len + 15) & ~15u) + ((ns + 3) & ~3u) * 4;
-            if (slot_n - at < size) return ST_LISTED;
-            uint8_t* run = slot + at;
-            for (uint32_t i = lane; i < (len + 3) / 4; i += 32) {
-                const uint32_t b = p + 32 * i, w = b >> 5;
-                reinterpret_cast<uint32_t*>(run + 16)[i] =
-                    __funnelshift_r(load_word(in.wbase, in.nvalid, w), load_word(in.wbase, in.nvalid, w + 1), b);
-            }
-            for (uint32_t i = lane; i < ns; i += 32)
-                reinterpret_cast<uint32_t*>(run + size)[-1 - (int)i] = min(255u, len - 255 * i) << 24;
-            p += 8 * len;
-            if (lane == 0)
-                *reinterpret_cast<uint4*>(run) = make_uint4(len, ns, final_block ? RUN_END : at + size, at + size);
-            at += size;
-        } else {
-            uint32_t limit, lsh, dl, dsh;
-            int nl = 288, nd = 32;
-            if (btype == 1) {
+        if (warp == 0) {  // the block's header, and its code lengths
+            HeadBits hb;
+            hb.wbase = in.wbase;
+            hb.nvalid = in.nvalid;
+            hb.at(p);
+            const uint32_t h = hb.get(p), btype = (h >> 1) & 3u;
+            uint32_t q = p + 3, a = 288, b = 32, bad = btype == 3;
+            if (btype == 0) {
+                q = s0 + ((q - s0 + 7) & ~7u);
+                const uint32_t y = hb.get(q);
+                q += 32;
+                a = y & 0xFFFFu;
+                bad = a != (~y >> 16) || q > E || 8ull * a > E - q;
+            } else if (btype == 1) {
                 for (int i = lane; i < 320; i += 32) lens[i] = i < 144 ? 8 : i < 256 ? 9 : i < 280 ? 7 : i < 288 ? 8 : 5;
-                __syncwarp();
-            } else {
-                const uint32_t r = read_lengths(W, hb, p, lens);
-                if (!r) return CB_ERR_INFLATE;
-                nl = (int)(r & 0xFFFFu);
-                nd = (int)(r >> 16) - nl;
+            } else if (btype == 2) {
+                const uint32_t r = read_lengths(M.t, hb, q, lens, M.w[0].sst);
+                bad = r == 0;
+                a = r & 0xFFFFu;
+                b = (r >> 16) - a;
             }
-            if (!build_tables<true>(W, lens, nl, limit, lsh)) return CB_ERR_INFLATE;
-            if (!build_tables<false>(W, lens + nl, nd, dl, dsh)) return CB_ERR_INFLATE;
-            const uint32_t st = decode_block(W, in, p, E, slot, slot_n, at, final_block, limit, lsh);
+            if (lane == 0) {
+                M.t.say[0] = h & 7u;
+                M.t.say[1] = q;
+                M.t.say[2] = a;
+                M.t.say[3] = b;
+                M.t.say[4] = bad;
+            }
+        }
+        sync_member<W>();
+        const uint32_t h = M.t.say[0], na = M.t.say[2], nb = M.t.say[3];
+        p = M.t.say[1];
+        const bool final_block = h & 1u;
+        if (M.t.say[4]) return CB_ERR_INFLATE;
+        if ((h >> 1) == 0) {
+            const uint32_t k = (na + 254) / 255;
+            if (nl + na + 4ull * ((unsigned long long)ns + k) > slot_n) return ST_LISTED;
+            // stored bytes, a part per warp
+            const uint32_t part = ((na + W - 1) / W + 3) & ~3u, from = min(na, warp * part), n = min(na, from + part) - from;
+            const uint32_t pb = p + 8 * from;
+            put_bytes(slot + nl + from, n, [&](uint32_t i, uint32_t h2) {
+                const uint32_t bit = pb + 8 * (4 * i + h2), w = bit >> 5;
+                return __funnelshift_r(load_word(in.wbase, in.nvalid, w), load_word(in.wbase, in.nvalid, w + 1), bit);
+            });
+            for (uint32_t i = tid; i < k; i += 32 * W)
+                reinterpret_cast<uint32_t*>(slot + slot_n)[-1 - (int)(ns + i)] = min(255u, na - 255 * i) << 24;
+            p += 8 * na;
+            nl += na;
+            ns += k;
+            sync_member<W>();  // say is written again
+        } else {
+            uint32_t limit, lsh;
+            if (warp == 0) {
+                const bool ok = build_tables<true>(M.t, lens, (int)na, limit, lsh);
+                if (lane == 0) {
+                    M.t.say[5] = ok;
+                    M.t.say[6] = limit;
+                    M.t.say[7] = lsh;
+                }
+            }
+            if (warp == (W > 1 ? 1u : 0u)) {
+                uint32_t dl, dsh;
+                const bool ok = build_tables<false>(M.t, lens + na, (int)nb, dl, dsh);
+                if (lane == 0) M.t.say[8] = ok;
+            }
+            sync_member<W>();
+            limit = M.t.say[6];
+            lsh = M.t.say[7];
+            if (!M.t.say[5] || !M.t.say[8]) return CB_ERR_INFLATE;
+            const uint32_t st = decode_block<W>(M, in, p, E, slot, slot_n, nl, ns, scratch, scratch_n, limit, lsh);
             if (st != CB_OK) return st;
         }
         if (final_block) return p > E ? (uint32_t)CB_ERR_INFLATE : (uint32_t)CB_OK;
-        if (slot_n - at < 16) return ST_LISTED;
     }
 }
 
-__global__ void __launch_bounds__(DEC_WARPS * 32)
+template <int W>
+__global__ void __launch_bounds__(W == 1 ? 64 : W * 32, W == 1 ? 9 : 1)
     k_decode(const cb_member_job* __restrict__ jobs, int64_t n_jobs, const int64_t* __restrict__ d_n_jobs,
-             uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws, uint8_t* arena,
+             uint8_t* out_base, uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws, uint8_t* arena,
              unsigned long long arena_bytes, bool list_unfit, long long j0, long long j1, int qi) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    DecWarp& W = reinterpret_cast<DecWarp*>(smem_raw)[threadIdx.x >> 5];
-    const int lane = threadIdx.x & 31;
+    DecMember<W>& M = reinterpret_cast<DecMember<W>*>(smem_raw)[threadIdx.x / (32 * W)];
+    const bool first = threadIdx.x % (32 * W) == 0;
     unsigned long long* queue = reinterpret_cast<unsigned long long*>(ws);
     uint32_t* per_job = reinterpret_cast<uint32_t*>(ws + WS_HEAD);
     long long n = n_jobs;
     if (d_n_jobs) n = min((long long)n, (long long)*d_n_jobs);
     n = min(n, j1);  // this launch's jobs: [j0, j1)
     for (;;) {
-        unsigned long long jj = 0;
-        if (lane == 0) jj = atomicAdd(queue + qi, 1ull);
-        const long long j = j0 + (long long)__shfl_sync(FULL, jj, 0);
+        if (first) M.t.job = atomicAdd(queue + qi, 1ull);
+        sync_member<W>();
+        const long long j = j0 + (long long)M.t.job;
         if (j >= n) break;
         const cb_member_job job = jobs[j];
-        const unsigned long long so = reinterpret_cast<const unsigned long long*>(per_job)[2 * j + 1];
-        const uint32_t st = so + slot_bytes(job.isize) <= arena_bytes ? decode_member(W, job, arena + so)
-                            : list_unfit                              ? ST_LISTED
-                                                                      : (uint32_t)CB_ERR_CAPACITY;
-        if (lane == 0) {
-            per_job[4 * j + 1] = st;
-            if (st == ST_LISTED) per_job[4 * atomicAdd(queue + Q_LISTED, 1ull)] = (uint32_t)j;
+        const unsigned long long so = reinterpret_cast<const unsigned long long*>(per_job)[(JW / 2) * j + 1];
+        uint32_t nl = 0, ns = 0;
+        const uint32_t st = so + slot_bytes(job.isize) <= arena_bytes
+                                ? decode_member<W>(M, job, arena + so, out_base + job.out_off, nl, ns)
+                            : list_unfit ? ST_LISTED
+                                         : (uint32_t)CB_ERR_CAPACITY;
+        sync_member<W>();
+        if (first) {
+            per_job[JW * j + 1] = st;
+            per_job[JW * j + 4] = nl;
+            per_job[JW * j + 5] = ns;
+            if (st == ST_LISTED) per_job[JW * atomicAdd(queue + Q_LISTED, 1ull)] = (uint32_t)j;
             else report(summary, job_status, j, st);
         }
-        __syncwarp();
     }
 }
 
-// ---------------------------------------------------------------- k_copy: one member per warp
+// ---------------------------------------------------------------- k_copy: one member per CTA of W warps
 
-constexpr int COPY_WARPS = 2;             // warps per CTA
-constexpr uint32_t LINE = 128;            // output bytes of a round: a word per lane
-constexpr uint32_t GMAX = 1152;           // output bytes of a group of 64 sequences, at most
-constexpr uint32_t FAR_N = 32;            // sources fetched from HBM per group, of up to FAR_LEN bytes each
+constexpr uint32_t LINE = 128;            // output bytes of a warp's round: a word per lane
+constexpr uint32_t FAR_N = 32;            // sources fetched from HBM per warp and group, of up to FAR_LEN bytes each
 constexpr uint32_t FAR_WORDS = 8, FAR_LEN = 4 * FAR_WORDS - 3;
-static_assert(GMAX >= 2 * (255 + 258), "two sequences fit a group");
 
-// RING_: bytes of output each warp keeps in shared memory: sources up to RING_ - GMAX - LINE bytes back
-// read it, older ones the output already stored.
-template <uint32_t RING_>
+// RING_: bytes of output kept in shared memory: sources up to RING_ - GMAX - SPAN bytes back read it, older
+// ones the output already stored.
+template <uint32_t RING_, int W_>
 struct CopyCfg {
-    static constexpr uint32_t RING = RING_, RMASK = RING_ - 1;
-    static_assert((RING_ & (RING_ - 1)) == 0 && RING_ >= 4096 && RING_ <= 16384, "ring size");
-    struct WarpSmem {
-        alignas(16) uint8_t ring[RING_];
-        uint32_t lit[64];                // the group's first literals (256 bytes)
-        uint32_t far[FAR_N * 9];         // fetched sources (and one word more each: fewer conflicts)
-        uint2 want[FAR_N];               // their slots and lengths
-        uint32_t tok[132], aux[132];
-        uint32_t map[(GMAX + LINE) / 4]; // per byte of the group's lines: the number of the token that starts there
+    static constexpr int W = W_;
+    static constexpr uint32_t T = 32 * W_, RING = RING_, RMASK = RING_ - 1;
+    static constexpr uint32_t SPAN = LINE * W_;   // output bytes of a round of all warps
+    static constexpr uint32_t GMAX = 1152 * W_;   // output bytes of a group of 64 sequences per warp, at most
+    static constexpr uint32_t LITS = 256 * W_;    // literals of a group held in shared memory
+    static_assert((RING_ & (RING_ - 1)) == 0 && RING_ >= GMAX + 2 * SPAN + 512 && RING_ <= 16384, "ring size");
+    static_assert(GMAX >= 2 * (255 + 258), "two sequences fit a group");
+    static_assert(SPAN <= 1024 && 4 * T < 65536, "a token's number and a near distance have their bits");
+    using Id = typename std::conditional<W_ == 1, uint8_t, uint16_t>::type;
+    struct alignas(16) Smem {
+        uint8_t ring[RING_];
+        uint32_t lit[LITS / 4];           // the group's first literals
+        uint32_t far[W_][FAR_N * 9];      // fetched sources (and one word more each: fewer conflicts)
+        uint2 want[W_][FAR_N];            // their slots and lengths
+        uint32_t tok[4 * T + 4], aux[4 * T + 4];
+        alignas(8) Id map[GMAX + SPAN];   // per byte of the group's lines: the number of the token that starts there
+        uint16_t head[(GMAX + SPAN) / LINE + 1];  // W > 1: per line, the token of its first byte
+        uint8_t missing[T];               // W > 1: per word of a round, the bytes that wait for others
+        unsigned long long sums[W_], job;
+        uint32_t count[W_];
     };
 };
 
-// A group's tokens are the literal runs and matches of its sequences, numbered 4 l + 1 to 4 l + 4 for lane
-// l's two.  tok: in 16 bits what to add to a byte's place (from the group's first line) to get its source's
-// offset from the ring's start in shared memory; T_NEAR: a match closer than a line (its distance from bit
+// A group's tokens are the literal runs and matches of its sequences, numbered 4 t + 1 to 4 t + 4 for thread
+// t's two.  tok: in 16 bits what to add to a byte's place (from the group's first line) to get its source's
+// offset from the ring's start in shared memory; T_NEAR: a match closer than a round (its distance from bit
 // 20), some of whose bytes may have their source in the same round.  The few tokens with T_WRAP (a source
-// across the ring's end) or T_DIRECT (one read from HBM: a literal with T_PLAIN, of the next run with
-// T_NEXT) find it through aux: the distance above bit 16 and the start, or for T_PLAIN what to add to get a
-// literal's place in lit, had it room.
-constexpr uint32_t T_NEAR = 1u << 16, T_WRAP = 1u << 17, T_DIRECT = 1u << 18, T_PLAIN = 1u << 19, T_NEXT = 1u << 27;
+// across the ring's end) or T_DIRECT (one read from HBM: a literal with T_PLAIN) find it through aux: the
+// distance above bit 16 and the start, or for T_PLAIN what to add to get a literal's place in the slot.
+constexpr uint32_t T_NEAR = 1u << 16, T_WRAP = 1u << 17, T_DIRECT = 1u << 18, T_PLAIN = 1u << 19;
 constexpr uint32_t T_FLAGS = T_NEAR | T_WRAP | T_DIRECT;
-
-// A run as k_copy reads it: offsets in the slot of its sequences 1, 0 (then 3, 2 before them) and of its
-// literals, their numbers and the next run's offset.
-struct Run {
-    uint32_t sq, lits, nl, ns, next;
-};
-__device__ __forceinline__ Run run_at(uint32_t at, uint4 head) {
-    return Run{head.w - 8, at + 16, head.x, head.y, head.z};
-}
 
 // All ones, shifted left by n (0 from 32 on).
 __device__ __forceinline__ uint32_t shl_clamp(uint32_t n) { return __funnelshift_lc(0u, 0xFFFFFFFFu, n); }
 
 // Positions below are slots: bytes from the 128-byte line of the member's first output byte (a bytes
-// before it).  A group is 64 sequences of the current run, or its last ones and the first of the next.
-// Its output is written in rounds of one line, a word per lane: each byte of the word belongs to the
-// last token that starts at or before it.
+// before it).  A group is 64 sequences per warp, two per thread.  Its output is written in rounds of one
+// line per warp, a word per lane: each byte of the word belongs to the last token that starts at or before
+// it.
 template <class C>
-__global__ void __launch_bounds__(COPY_WARPS * 32, C::RING == 4096 ? 14 : 8)
+__global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
     k_copy(const cb_member_job* __restrict__ jobs, int64_t n_jobs, const int64_t* __restrict__ d_n_jobs,
            uint8_t* out_base, uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws,
            const uint8_t* arena, long long j0, long long j1, int qi) {
+    constexpr int W = C::W;
+    constexpr uint32_t T = C::T;
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    using WarpSmem = typename C::WarpSmem;
-    WarpSmem& W = reinterpret_cast<WarpSmem*>(smem_raw)[threadIdx.x >> 5];
-    const int lane = threadIdx.x & 31;
+    typename C::Smem& M = *reinterpret_cast<typename C::Smem*>(smem_raw);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t lt = (1u << lane) - 1u;
-    const uint8_t* smem = W.ring;
-    uint32_t* ring4 = reinterpret_cast<uint32_t*>(W.ring);
-    const uint32_t LIT_AT = (uint32_t)(reinterpret_cast<const uint8_t*>(W.lit) - smem);
-    const uint32_t FAR_AT = (uint32_t)(reinterpret_cast<const uint8_t*>(W.far) - smem);
-    uint8_t* map1 = reinterpret_cast<uint8_t*>(W.map);
+    const uint8_t* smem = M.ring;
+    uint32_t* ring4 = reinterpret_cast<uint32_t*>(M.ring);
+    const uint32_t LIT_AT = (uint32_t)(reinterpret_cast<const uint8_t*>(M.lit) - smem);
+    const uint32_t FAR_AT = (uint32_t)(reinterpret_cast<const uint8_t*>(M.far[warp]) - smem);
     unsigned long long* queue = reinterpret_cast<unsigned long long*>(ws) + qi;  // this launch's counter
     uint32_t* per_job = reinterpret_cast<uint32_t*>(ws + WS_HEAD);
     long long n = n_jobs;
     if (d_n_jobs) n = min((long long)n, (long long)*d_n_jobs);
     n = min(n, j1);  // this launch's jobs: [j0, j1)
-    for (uint32_t i = lane; i < (GMAX + LINE) / 4; i += 32) W.map[i] = 0;
-    if (lane == 0) W.tok[0] = 0;  // bytes before the group's first
-    __syncwarp();
+    auto sync = [&]() {
+        if (W == 1) __syncwarp();
+        else __syncthreads();
+    };
+    auto any = [&](bool x) { return W == 1 ? __any_sync(FULL, x) != 0 : __syncthreads_or(x) != 0; };
+    for (uint32_t i = tid; i < C::GMAX + C::SPAN; i += T) M.map[i] = 0;
+    if (tid == 0) M.tok[0] = 0;  // bytes before the group's first
 
     for (;;) {
-        unsigned long long jj = 0;
-        if (lane == 0) jj = atomicAdd(queue, 1ull);
-        const long long j = j0 + (long long)__shfl_sync(FULL, jj, 0);
+        if (tid == 0) M.job = atomicAdd(queue, 1ull);
+        sync();
+        const long long j = j0 + (long long)M.job;
+        sync();
         if (j >= n) break;
-        if (per_job[4 * j + 1] != CB_OK) continue;  // k_decode reported or listed it
+        if (per_job[JW * j + 1] != CB_OK) continue;  // k_decode reported or listed it
         const cb_member_job job = jobs[j];
-        const uint8_t* slot = arena + reinterpret_cast<const unsigned long long*>(per_job)[2 * j + 1];
-        const uint32_t a = (uint32_t)((uintptr_t)(out_base + job.out_off) & 127);
+        const uint8_t* lits = arena + reinterpret_cast<const unsigned long long*>(per_job)[(JW / 2) * j + 1];
+        const uint2* sq = reinterpret_cast<const uint2*>(lits + slot_bytes(job.isize)) - 1;  // sequences 1, 0
+        const uint32_t nl = per_job[JW * j + 4], ns = per_job[JW * j + 5];
+        const uint32_t a = (uint32_t)((uintptr_t)(out_base + job.out_off) & (LINE - 1));
         uint8_t* base = out_base + job.out_off - a;  // slot 0
         const uint32_t Eend = a + job.isize;
         uint32_t P = a, st = CB_OK;
-        const uint4 no_head = make_uint4(0, 0, RUN_END, 0);
-        auto head_at = [&](uint32_t at) { return at == RUN_END ? no_head : __ldcg(reinterpret_cast<const uint4*>(slot + at)); };
-        // the current run (g of its sequences and lbase of its literals done), the next one, and the head
-        // of the one after that
-        Run A = run_at(0, head_at(0));
-        uint32_t bat = A.next;
-        Run B = run_at(bat, head_at(bat));
-        uint32_t cat = B.next;
-        uint4 chead = head_at(cat);
-        uint32_t g = 0, lbase = 0;
-        // the group's make-up: lanes below inA have two sequences of A each, the others of B; B's literals
-        // follow A's in `lit` from byte boff
-        uint32_t nA, nB, boff;
+        uint32_t g = 0, lbase = 0;  // sequences (an even number) and literals done
         uint2 seq;
         uint32_t lw0, lw1;
-        auto compose = [&]() {
-            nA = min(64u, A.ns - g);
-            const uint32_t even = (nA + 1) & ~1u;
-            nB = min(64u - even, B.ns);
-            const uint32_t lb = lbase & ~3u;
-            boff = (A.nl - lb + 3) & ~3u;
-            const bool ofA = 2 * lane < even;
-            const uint32_t i = ofA ? g + 2 * lane : 2 * lane - even;
-            const uint32_t ns = ofA ? A.ns : B.ns;
-            seq = i < ns ? __ldcg(reinterpret_cast<const uint2*>(slot + ((ofA ? A.sq : B.sq) - 4 * i))) : make_uint2(0, 0);
+        auto load = [&]() {  // the group's sequences and first literals
+            const uint32_t i = g + 2 * tid, l = (lbase & ~3u) + 4 * tid;
+            seq = i < ns ? __ldcg(sq - (i >> 1)) : make_uint2(0, 0);
             if (i + 1 >= ns) seq.x = 0;
-            auto literals = [&](uint32_t o) {  // four, from byte o of lit
-                const bool isA = o < boff;
-                const uint32_t l = isA ? lb + o : o - boff;
-                return l < (isA ? A.nl : B.nl) ? __ldcg(reinterpret_cast<const uint32_t*>(slot + ((isA ? A.lits : B.lits) + l)))
-                                               : 0u;
-            };
-            lw0 = literals(4 * lane);
-            lw1 = literals(4 * lane + 128);
+            lw0 = l < nl ? __ldcg(reinterpret_cast<const uint32_t*>(lits + l)) : 0u;
+            lw1 = l + 4 * T < nl ? __ldcg(reinterpret_cast<const uint32_t*>(lits + l + 4 * T)) : 0u;
         };
-        compose();
-        for (;;) {  // groups
-            {
-                // this lane's two sequences
-                const uint32_t s0 = seq.y, s1 = seq.x;
-                uint32_t c0 = s0 >> 24, m0 = s0 & SEQ_MATCH ? ((s0 >> 16) & 255u) + 3 : 0u;
-                uint32_t c1 = s1 >> 24, m1 = s1 & SEQ_MATCH ? ((s1 >> 16) & 255u) + 3 : 0u;
-                const bool none0 = (s0 & 0xFFFFu) && !m0, none1 = (s1 & 0xFFFFu) && !m1;
-                const uint32_t v = (c0 + m0 + c1 + m1) | ((c0 + c1) << 16);
+        load();
+        while (g < ns) {
+            // this thread's two sequences
+            const uint32_t s0 = seq.y, s1 = seq.x;
+            uint32_t c0 = s0 >> 24, m0 = s0 & SEQ_MATCH ? ((s0 >> 16) & 255u) + 3 : 0u;
+            uint32_t c1 = s1 >> 24, m1 = s1 & SEQ_MATCH ? ((s1 >> 16) & 255u) + 3 : 0u;
+            const bool none0 = (s0 & 0xFFFFu) && !m0, none1 = (s1 & 0xFFFFu) && !m1;
+            // output bytes and literals before it, and of the group
+            const uint32_t vb = c0 + m0 + c1 + m1, vl = c0 + c1;
+            uint32_t eb, el, glen, glit;
+            if (W == 1) {
                 uint32_t gv;
-                uint32_t ex = warp_exclusive_scan(v, gv);
-                const uint32_t even = (nA + 1) & ~1u;
-                uint32_t cA = nA, cB = nB;  // sequences done with this group
-                if ((gv & 0xFFFFu) > GMAX) {  // the lanes whose sequences end within GMAX bytes (at least one)
-                    const uint32_t keep = __popc(__ballot_sync(FULL, ((ex + v) & 0xFFFFu) <= GMAX));
-                    gv = __shfl_sync(FULL, ex + v, keep - 1);
-                    cA = min(2 * keep, nA);
-                    cB = min(2 * keep > even ? 2 * keep - even : 0u, nB);
-                    if (lane >= (int)keep) {
-                        c0 = m0 = c1 = m1 = 0;
-                        ex = gv;
+                const uint32_t ex = warp_exclusive_scan(vb | (vl << 16), gv);
+                eb = ex & 0xFFFFu;
+                el = ex >> 16;
+                glen = gv & 0xFFFFu;
+                glit = gv >> 16;
+            } else {
+                unsigned long long wt;
+                unsigned long long ex = warp_exclusive_scan((unsigned long long)vb | ((unsigned long long)vl << 32), wt);
+                if (lane == 0) M.sums[warp] = wt;
+                __syncthreads();
+                unsigned long long tot = 0;
+#pragma unroll
+                for (int w = 0; w < W; w++) {
+                    if (w == (int)warp) ex += tot;
+                    tot += M.sums[w];
+                }
+                eb = (uint32_t)ex;
+                el = (uint32_t)(ex >> 32);
+                glen = (uint32_t)tot;
+                glit = (uint32_t)(tot >> 32);
+            }
+            uint32_t cnt = min(2 * T, ns - g);
+            if (glen > C::GMAX) {  // the threads whose sequences end within GMAX bytes (at least one)
+                const uint32_t mine = __popc(__ballot_sync(FULL, eb + vb <= C::GMAX));
+                uint32_t keep = mine;
+                if (W > 1) {
+                    if (lane == 0) M.count[warp] = mine;
+                    __syncthreads();  // and every thread has read sums
+                    keep = 0;
+#pragma unroll
+                    for (int w = 0; w < W; w++) keep += M.count[w];
+                }
+                if (W == 1) {
+                    glen = __shfl_sync(FULL, eb + vb, keep - 1);
+                    glit = __shfl_sync(FULL, el + vl, keep - 1);
+                } else {
+                    if (tid == keep - 1) M.sums[0] = (unsigned long long)(eb + vb) | ((unsigned long long)(el + vl) << 32);
+                    __syncthreads();
+                    glen = (uint32_t)M.sums[0];
+                    glit = (uint32_t)(M.sums[0] >> 32);
+                }
+                cnt = min(cnt, 2 * keep);
+                if (tid >= keep) {
+                    c0 = m0 = c1 = m1 = 0;
+                    eb = glen;
+                    el = glit;
+                }
+            }
+            // places from the group's first line: its start, this thread's, and after each of its parts
+            const uint32_t R0 = P & ~(LINE - 1), p0 = P - R0, pe = p0 + glen;
+            const uint32_t b0 = p0 + eb, b1 = b0 + c0, b2 = b1 + m0, b3 = b2 + c1;
+            const uint32_t d0 = (s0 & 0x7FFFu) + 1, d1 = (s1 & 0x7FFFu) + 1;
+            if (any(none0 || none1 || (m0 && d0 > R0 + b1 - a) || (m1 && d1 > R0 + b3 - a)) || glen > Eend - P) {
+                st = CB_ERR_INFLATE;
+                break;
+            }
+            M.lit[tid] = lw0;
+            M.lit[tid + T] = lw1;
+            const uint32_t l0 = (lbase & 3u) + el, l1 = l0 + c0, lit0 = lbase & ~3u;
+            // the next group's sequences and literals are loaded while this one is written
+            g += cnt;
+            lbase += glit;
+            load();
+            // sources older than the ring will hold come to `far`
+            const uint32_t x0 = R0 + b1 - d0, x1 = R0 + b3 - d1;
+            const uint32_t old = R0 + (pe + C::SPAN - 1) / C::SPAN * C::SPAN;  // slots below old - RING
+            const bool old0 = m0 && x0 + C::RING < old, old1 = m1 && x1 + C::RING < old;
+            uint32_t f0 = FAR_N, f1 = FAR_N;  // their places there
+            const uint32_t any0 = __ballot_sync(FULL, old0 && m0 <= FAR_LEN);
+            const uint32_t any1 = __ballot_sync(FULL, old1 && m1 <= FAR_LEN);
+            if (any0 | any1) {
+                const uint32_t n0 = __popc(any0);
+                if (any0 >> lane & 1u) f0 = __popc(any0 & lt);
+                if (any1 >> lane & 1u) f1 = n0 + __popc(any1 & lt);
+                if (f0 < FAR_N) M.want[warp][f0] = make_uint2(x0, m0);
+                if (f1 < FAR_N) M.want[warp][f1] = make_uint2(x1, m1);
+                __syncwarp();
+                const uint2 t = lane < n0 + __popc(any1) ? M.want[warp][lane] : make_uint2(0, 0);
+                const uint32_t nw = t.y ? ((t.x & 3u) + t.y + 3) >> 2 : 0u;
+                const uint32_t* q = reinterpret_cast<const uint32_t*>(base + (t.x & ~3u));
+                uint32_t* f = M.far[warp] + 9 * lane;
+                uint32_t w[FAR_WORDS];
+#pragma unroll
+                for (uint32_t k = 0; k < FAR_WORDS; k++) w[k] = k < nw ? __ldcg(q + k) : 0u;
+#pragma unroll
+                for (uint32_t k = 0; k < FAR_WORDS; k++)
+                    if (k < nw) f[k] = w[k];
+            }
+            {
+                auto place = [&](uint32_t id, uint32_t start, uint32_t len) {
+                    M.map[start] = (typename C::Id)id;
+                    if (W > 1)  // and the lines whose first byte is the token's
+                        for (uint32_t L = (start + LINE - 1) / LINE; L * LINE < start + len; L++) M.head[L] = (uint16_t)id;
+                };
+                auto literals = [&](uint32_t id, uint32_t start, uint32_t c, uint32_t l) {
+                    place(id, start, c);
+                    const bool held = l + c <= C::LITS;
+                    M.tok[id] = (((held ? LIT_AT + l : 0u) - start) & 0xFFFFu) | (held ? 0u : T_DIRECT | T_PLAIN);
+                    M.aux[id] = lit0 + l - start;
+                };
+                auto match = [&](uint32_t id, uint32_t start, uint32_t len, uint32_t d, uint32_t x, bool is_old, uint32_t f) {
+                    place(id, start, len);
+                    const uint32_t at = x & C::RMASK;
+                    const bool held = is_old ? f < FAR_N : at + len <= C::RING;
+                    M.tok[id] = (((!held ? 0u : is_old ? FAR_AT + 36 * f + (x & 3u) : at) - start) & 0xFFFFu) |
+                                (!held ? (is_old ? T_DIRECT : T_WRAP) : d < C::SPAN ? T_NEAR | (d << 20) : 0u);
+                    M.aux[id] = start | (d << 16);
+                };
+                if (c0) literals(4 * tid + 1, b0, c0, l0);
+                if (m0) match(4 * tid + 2, b1, m0, d0, x0, old0, f0);
+                if (c1) literals(4 * tid + 3, b2, c1, l1);
+                if (m1) match(4 * tid + 4, b3, m1, d1, x1, old1, f1);
+                if (W > 1 && tid == 0 && p0) M.head[0] = 0;
+            }
+            sync();
+            uint32_t carry = 0;
+            const uint32_t full0 = a > R0 ? a - R0 : 0u, full1 = Eend - R0;  // whole words of the member
+            for (uint32_t sr = 0; sr < pe; sr += C::SPAN) {
+                const uint32_t rr = sr + LINE * warp, rel = rr + 4 * lane, w = R0 + rel;
+                // the numbers of the tokens that start in the word
+                uint32_t m[4];
+                if (W == 1) {
+                    const uint32_t x = *reinterpret_cast<const uint32_t*>(M.map + rel);
+                    *reinterpret_cast<uint32_t*>(M.map + rel) = 0;
+#pragma unroll
+                    for (int k = 0; k < 4; k++) m[k] = (x >> (8 * k)) & 255u;
+                } else {
+                    const uint2 x = *reinterpret_cast<const uint2*>(M.map + rel);
+                    *reinterpret_cast<uint2*>(M.map + rel) = make_uint2(0, 0);
+                    m[0] = x.x & 0xFFFFu;
+                    m[1] = x.x >> 16;
+                    m[2] = x.y & 0xFFFFu;
+                    m[3] = x.y >> 16;
+                    carry = rr < pe ? M.head[rr / LINE] : 0u;
+                }
+                // the token of the byte before the word: the last one that starts in a lane below, else the
+                // line's first (W > 1) or the last of the line before
+                const uint32_t mlast = m[3] ? m[3] : m[2] ? m[2] : m[1] ? m[1] : m[0];
+                const uint32_t below = __ballot_sync(FULL, mlast != 0) & lt;
+                uint32_t id = __shfl_sync(FULL, mlast, below ? 31 - __clz((int)below) : 0);
+                if (!below) id = carry;
+                uint32_t ids[4], tk[4], v[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    id = m[k] ? m[k] : id;
+                    ids[k] = id;
+                    tk[k] = M.tok[id];
+                    v[k] = smem[(rel + k + tk[k]) & 0xFFFFu];
+                }
+                if (W == 1) carry = __shfl_sync(FULL, id, 31);
+                uint32_t word = v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24);
+                if (rr == 0 && rel < p0) {  // bytes before the group's first are there already
+                    const uint32_t mine = shl_clamp(8 * (p0 - rel));
+                    word = (word & mine) | (ring4[(w & C::RMASK) >> 2] & ~mine);
+                }
+                const uint32_t fl = tk[0] | tk[1] | tk[2] | tk[3];
+                uint32_t pend = 0;  // bytes whose source is written in this round
+                const int left = (int)(pe - rel), fresh = (int)max(sr, p0);  // from fresh on
+                if (__any_sync(FULL, left > 0 && (fl & T_FLAGS))) {
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if ((tk[k] & T_NEAR) && k < left && (int)(rel + k - (tk[k] >> 20)) >= fresh) pend |= 1u << k;
+                    if (__any_sync(FULL, left > 0 && (fl & (T_WRAP | T_DIRECT)))) {
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            if ((tk[k] & (T_WRAP | T_DIRECT)) && k < left) {
+                                const uint32_t ax = M.aux[ids[k]], x = w + k - (ax >> 16);
+                                uint32_t b = 0;
+                                if (tk[k] & T_DIRECT) b = __ldcg(tk[k] & T_PLAIN ? lits + (uint32_t)(rel + k + ax) : base + x);
+                                else if ((int)(x - R0) >= fresh) pend |= 1u << k;
+                                else b = M.ring[x & C::RMASK];
+                                word = (word & ~(0xFFu << (8 * k))) | (b << (8 * k));
+                            }
+                        }
                     }
                 }
-                const uint32_t glen = gv & 0xFFFFu;
-                // places from the group's first line: its start, this lane's, and after each of its parts
-                const uint32_t R0 = P & ~(LINE - 1), p0 = P - R0, pe = p0 + glen;
-                const uint32_t b0 = p0 + (ex & 0xFFFFu), b1 = b0 + c0, b2 = b1 + m0, b3 = b2 + c1;
-                const uint32_t d0 = (s0 & 0x7FFFu) + 1, d1 = (s1 & 0x7FFFu) + 1;
-                if (__any_sync(FULL, none0 || none1 || (m0 && d0 > R0 + b1 - a) || (m1 && d1 > R0 + b3 - a)) ||
-                    glen > Eend - P) {
-                    st = CB_ERR_INFLATE;
-                    break;
-                }
-                // this lane's literals: place in lit; and lit
-                const bool ofB = 2 * lane >= even;
-                const uint32_t restA = A.nl - lbase;  // literals of A before B's
-                const uint32_t l0 = (ex >> 16) + (ofB ? boff - restA : lbase & 3u), l1 = l0 + c0;
-                const uint32_t srcA = A.lits + (lbase & ~3u), srcB = B.lits - boff;
-                W.lit[lane] = lw0;
-                W.lit[lane + 32] = lw1;
-                // the next group's sequences and literals are loaded while this one is written
-                g += cA;
-                lbase += min(gv >> 16, restA);
-                bool more = true;
-                if (g >= A.ns) {
-                    more = bat != RUN_END;
-                    if (more && cat <= bat) more = false;  // runs only go forward
-                    g = cB;
-                    lbase = (gv >> 16) - min(gv >> 16, restA);
-                    A = B;
-                    bat = cat;
-                    B = run_at(bat, chead);
-                    cat = B.next;
-                    if (more) chead = head_at(cat);
-                }
-                if (more) compose();
-                // sources older than the ring will hold come to `far`
-                const uint32_t x0 = R0 + b1 - d0, x1 = R0 + b3 - d1;
-                const uint32_t old = R0 + ((pe + LINE - 1) & ~(LINE - 1));  // slots below old - RING
-                const bool old0 = m0 && x0 + C::RING < old, old1 = m1 && x1 + C::RING < old;
-                uint32_t f0 = FAR_N, f1 = FAR_N;  // their places there
-                const uint32_t any0 = __ballot_sync(FULL, old0 && m0 <= FAR_LEN);
-                const uint32_t any1 = __ballot_sync(FULL, old1 && m1 <= FAR_LEN);
-                if (any0 | any1) {
-                    const uint32_t n0 = __popc(any0);
-                    if (any0 >> lane & 1u) f0 = __popc(any0 & lt);
-                    if (any1 >> lane & 1u) f1 = n0 + __popc(any1 & lt);
-                    if (f0 < FAR_N) W.want[f0] = make_uint2(x0, m0);
-                    if (f1 < FAR_N) W.want[f1] = make_uint2(x1, m1);
-                    __syncwarp();
-                    const uint2 t = lane < (int)(n0 + __popc(any1)) ? W.want[lane] : make_uint2(0, 0);
-                    const uint32_t nw = t.y ? ((t.x & 3u) + t.y + 3) >> 2 : 0u;
-                    const uint32_t* q = reinterpret_cast<const uint32_t*>(base + (t.x & ~3u));
-                    uint32_t* f = W.far + 9 * lane;
-                    uint32_t w[FAR_WORDS];
-#pragma unroll
-                    for (uint32_t k = 0; k < FAR_WORDS; k++) w[k] = k < nw ? __ldcg(q + k) : 0u;
-#pragma unroll
-                    for (uint32_t k = 0; k < FAR_WORDS; k++)
-                        if (k < nw) f[k] = w[k];
-                }
-                {
-                    const uint32_t plain = T_DIRECT | T_PLAIN | (ofB ? T_NEXT : 0u);
-                    auto literals = [&](uint32_t id, uint32_t start, uint32_t c, uint32_t l) {
-                        map1[start] = (uint8_t)id;
-                        const bool held = l + c <= 256;
-                        W.tok[id] = (((held ? LIT_AT + l : 0u) - start) & 0xFFFFu) | (held ? 0u : plain);
-                        W.aux[id] = l - start;
-                    };
-                    auto match = [&](uint32_t id, uint32_t start, uint32_t len, uint32_t d, uint32_t x, bool is_old, uint32_t f) {
-                        const uint32_t at = x & C::RMASK;
-                        map1[start] = (uint8_t)id;
-                        const bool held = is_old ? f < FAR_N : at + len <= C::RING;
-                        W.tok[id] = (((!held ? 0u : is_old ? FAR_AT + 36 * f + (x & 3u) : at) - start) & 0xFFFFu) |
-                                    (!held ? (is_old ? T_DIRECT : T_WRAP) : d < LINE ? T_NEAR | (d << 20) : 0u);
-                        W.aux[id] = start | (d << 16);
-                    };
-                    if (c0) literals(4 * lane + 1, b0, c0, l0);
-                    if (m0) match(4 * lane + 2, b1, m0, d0, x0, old0, f0);
-                    if (c1) literals(4 * lane + 3, b2, c1, l1);
-                    if (m1) match(4 * lane + 4, b3, m1, d1, x1, old1, f1);
-                }
-                __syncwarp();
-                uint32_t carry = 0;
-                const uint32_t full0 = a > R0 ? a - R0 : 0u, full1 = Eend - R0;  // whole words of the member
-                for (uint32_t rr = 0; rr < pe; rr += LINE) {
-                    const uint32_t rel = rr + 4 * lane, w = R0 + rel;
-                    const uint32_t m = W.map[rel >> 2];
-                    W.map[rel >> 2] = 0;
-                    // the token of the byte before the word: the last one that starts in a lane below, or
-                    // in an earlier round
-                    const uint32_t mlast = (m >> (24 - (__clz((int)m) & 24))) & 255u;
-                    const uint32_t below = __ballot_sync(FULL, m != 0) & lt;
-                    uint32_t id = __shfl_sync(FULL, mlast, below ? 31 - __clz((int)below) : 0);
-                    if (!below) id = carry;
-                    uint32_t ids[4], tk[4], v[4];
+                if (any(pend != 0)) {
+                    // their sources; a match that overlaps itself repeats the bytes before its start
+                    int px[4];
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
-                        const uint32_t b = (m >> (8 * k)) & 255u;
-                        id = b ? b : id;
-                        ids[k] = id;
-                        tk[k] = W.tok[id];
-                        v[k] = smem[(rel + k + tk[k]) & 0xFFFFu];
-                    }
-                    carry = __shfl_sync(FULL, id, 31);
-                    uint32_t word = v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24);
-                    if (rr == 0 && rel < p0) {  // bytes before the group's first are there already
-                        const uint32_t mine = shl_clamp(8 * (p0 - rel));
-                        word = (word & mine) | (ring4[(w & C::RMASK) >> 2] & ~mine);
-                    }
-                    const uint32_t fl = tk[0] | tk[1] | tk[2] | tk[3];
-                    if (__any_sync(FULL, rel < pe && (fl & T_FLAGS))) {
-                        const int left = (int)(pe - rel), fresh = (int)max(rr, p0);  // written in this round from fresh on
-                        uint32_t pend = 0;  // bytes whose source is
-#pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            if ((tk[k] & T_NEAR) && k < left && (int)(rel + k - ((tk[k] >> 20) & (LINE - 1))) >= fresh)
-                                pend |= 1u << k;
-                        if (__any_sync(FULL, left > 0 && (fl & (T_WRAP | T_DIRECT)))) {
-#pragma unroll
-                            for (int k = 0; k < 4; k++) {
-                                if ((tk[k] & (T_WRAP | T_DIRECT)) && k < left) {
-                                    const uint32_t ax = W.aux[ids[k]], x = w + k - (ax >> 16);
-                                    uint32_t b = 0;
-                                    if (tk[k] & T_DIRECT)
-                                        b = __ldcg(tk[k] & T_PLAIN ? slot + ((tk[k] & T_NEXT ? srcB : srcA) + rel + k + ax) : base + x);
-                                    else if ((int)(x - R0) >= fresh) pend |= 1u << k;
-                                    else b = W.ring[x & C::RMASK];
-                                    word = (word & ~(0xFFu << (8 * k))) | (b << (8 * k));
-                                }
-                            }
+                        px[k] = 0x7FFFFFFF;
+                        if (pend >> k & 1) {
+                            const uint32_t ax = M.aux[ids[k]], d = ax >> 16;
+                            const int start = (int)(ax & 0xFFFFu);
+                            px[k] = (int)(rel + k - d);
+                            if (px[k] >= start) px[k] = start - (int)d + (int)((uint32_t)(px[k] - start) % d);
                         }
-                        if (__any_sync(FULL, pend != 0)) {
-                            // their sources; a match that overlaps itself repeats the bytes before its start
-                            int px[4];
+                    }
+                    if (W > 1) {
+                        M.missing[tid] = (uint8_t)pend;
+                        ring4[(w & C::RMASK) >> 2] = word;
+                        __syncthreads();
+                    }
+                    do {
+                        // at each pass the bytes whose sources are there (W == 1: lie below the first missing)
+                        int Q = 0;
+                        if (W == 1) {
+                            Q = (int)__reduce_min_sync(FULL, pend ? rel + __ffs((int)pend) - 1 : 0x7FFFFFFFu);
+                            ring4[(w & C::RMASK) >> 2] = word;
+                            __syncwarp();
+                        }
 #pragma unroll
-                            for (int k = 0; k < 4; k++) {
+                        for (int k = 0; k < 4; k++) {
+                            bool ready = px[k] < Q;
+                            if (W > 1 && (pend >> k & 1))
+                                ready = px[k] < fresh || !(M.missing[(px[k] - sr) >> 2] >> (px[k] & 3) & 1);
+                            if (ready) {
+                                word = (word & ~(0xFFu << (8 * k))) | ((uint32_t)M.ring[(R0 + px[k]) & C::RMASK] << (8 * k));
+                                pend &= ~(1u << k);
                                 px[k] = 0x7FFFFFFF;
-                                if (pend >> k & 1) {
-                                    const uint32_t ax = W.aux[ids[k]], d = ax >> 16;
-                                    const int start = (int)(ax & 0xFFFFu);
-                                    px[k] = (int)(rel + k - d);
-                                    if (px[k] >= start) px[k] = start - (int)d + (int)((uint32_t)(px[k] - start) % d);
-                                }
                             }
-                            do {
-                                // at each pass the bytes whose sources lie below the first one still missing
-                                const int Q = (int)__reduce_min_sync(FULL, pend ? rel + __ffs((int)pend) - 1 : 0x7FFFFFFFu);
-                                ring4[(w & C::RMASK) >> 2] = word;
-                                __syncwarp();
-#pragma unroll
-                                for (int k = 0; k < 4; k++) {
-                                    if (px[k] < Q) {
-                                        word = (word & ~(0xFFu << (8 * k))) | ((uint32_t)W.ring[(R0 + px[k]) & C::RMASK] << (8 * k));
-                                        pend &= ~(1u << k);
-                                        px[k] = 0x7FFFFFFF;
-                                    }
-                                }
-                                __syncwarp();
-                            } while (__any_sync(FULL, pend != 0));
                         }
-                    }
-                    ring4[(w & C::RMASK) >> 2] = word;
-                    if (rel < pe && rel + 4 > p0) {
-                        if (rel >= full0 && rel + 4 <= full1) {
-                            // bytes of the word after the group's end are overwritten by the next one
-                            *reinterpret_cast<uint32_t*>(base + w) = word;
-                        } else {  // the member's first or last word: its own bytes only
-                            for (uint32_t s = max(w, P); s < min(w + 4, R0 + pe); s++)
-                                base[s] = (uint8_t)(word >> (8 * (s - w)));
+                        sync();
+                        if (W > 1) {
+                            M.missing[tid] = (uint8_t)pend;
+                            ring4[(w & C::RMASK) >> 2] = word;
                         }
-                    }
-                    __syncwarp();
+                    } while (any(pend != 0));
                 }
-                P += glen;
-                if (!more) break;
+                ring4[(w & C::RMASK) >> 2] = word;
+                if (rel < pe && rel + 4 > p0) {
+                    if (rel >= full0 && rel + 4 <= full1) {
+                        // bytes of the word after the group's end are overwritten by the next one
+                        *reinterpret_cast<uint32_t*>(base + w) = word;
+                    } else {  // the member's first or last word: its own bytes only
+                        for (uint32_t s = max(w, P); s < min(w + 4, R0 + pe); s++) base[s] = (uint8_t)(word >> (8 * (s - w)));
+                    }
+                }
+                sync();
             }
+            P += glen;
         }
         if (st == CB_OK && P != Eend) st = CB_ERR_INFLATE;
-        if (lane == 0 && st != CB_OK) {
-            per_job[4 * j + 1] = st;
+        if (tid == 0 && st != CB_OK) {
+            per_job[JW * j + 1] = st;
             report(summary, job_status, j, st);
         }
-        __syncwarp();
     }
 }
 
-// ---------------------------------------------------------------- k_crc: one member per warp
+// ---------------------------------------------------------------- k_crc: one member per W warps
 //
 // The polynomial P divides P(x^1024) (= P^1024 in characteristic 2), so a message may be reduced by
 // P(x^1024) first: rows of 1024 bits (a 4-byte word per lane) take the place of the polynomial's
@@ -1151,69 +1335,88 @@ __device__ __forceinline__ uint32_t crc_word_careful(const uint8_t* m, long long
     return x;
 }
 
+// W warps per member, each a part of its 4,096-byte rows of rows; parts are joined by x^(8 bytes after).
+template <int W>
 __global__ void __launch_bounds__(CRC_NT)
     k_crc(const cb_member_job* __restrict__ jobs, int64_t n_jobs, const int64_t* __restrict__ d_n_jobs,
           const uint8_t* __restrict__ out_base, uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws,
           long long j0, long long j1) {
     __shared__ uint32_t fold[4][256];
+    __shared__ uint32_t parts[CRC_NT / 32];
     for (int i = threadIdx.x; i < 1024; i += CRC_NT) fold[i >> 8][i & 255] = gf_mul((uint32_t)(i & 255) << (8 * (i >> 8)), kCrcLane.x1024);
     __syncthreads();
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t* per_job = reinterpret_cast<uint32_t*>(ws + WS_HEAD);
     long long n = n_jobs;
     if (d_n_jobs) n = min((long long)n, (long long)*d_n_jobs);
     n = min(n, j1);
-    const long long warps = (long long)gridDim.x * (CRC_NT / 32);
-    for (long long j = j0 + (long long)blockIdx.x * (CRC_NT / 32) + (threadIdx.x >> 5); j < n; j += warps) {
-        if (per_job[4 * j + 1] != CB_OK) continue;
-        const cb_member_job job = jobs[j];
-        const uint8_t* m = out_base + job.out_off;
-        const uint32_t len = job.isize;
-        const bool inv = len >= 4;
-        const long long pad = (long long)((4096u - (len & 4095u)) & 4095u);
-        const long long iters = ((long long)len + pad) >> 12;
-        uint32_t v[32];
+    constexpr int PER = CRC_NT / 32 / W;  // members per CTA at a time
+    for (long long jb = j0 + (long long)blockIdx.x * PER; jb < n; jb += (long long)gridDim.x * PER) {
+        const long long j = jb + warp / W;
+        uint32_t c = 0, want = 0;
+        const bool on = j < n && per_job[JW * j + 1] == CB_OK;
+        uint32_t len = 0;
+        if (on) {
+            const cb_member_job job = jobs[j];
+            const uint8_t* m = out_base + job.out_off;
+            len = job.isize;
+            want = job.crc;
+            const bool inv = len >= 4;
+            const long long pad = (long long)((4096u - (len & 4095u)) & 4095u);
+            const long long iters = ((long long)len + pad) >> 12;
+            const long long i0 = iters * (warp % W) / W, i1 = iters * (warp % W + 1) / W;
+            uint32_t v[32];
 #pragma unroll
-        for (int i = 0; i < 32; i++) v[i] = 0;
-        for (long long it = 0; it < iters; it++) {
-            const bool last = it + 1 == iters;
+            for (int i = 0; i < 32; i++) v[i] = 0;
+            for (long long it = i0; it < i1; it++) {
+                const bool last = it + 1 == i1;
 #pragma unroll
-            for (int i0 = 0; i0 < 32; i0 += 8) {
-                uint32_t w[8];
-                const long long q0 = it * 4096 + i0 * 128 + 4 * lane - pad;
-                if (it * 4096 - pad < 4) {  // rows with bytes before the member or its first four
+                for (int r0 = 0; r0 < 32; r0 += 8) {
+                    uint32_t w[8];
+                    const long long q0 = it * 4096 + r0 * 128 + 4 * lane - pad;
+                    if (it * 4096 - pad < 4) {  // rows with bytes before the member or its first four
 #pragma unroll
-                    for (int i = 0; i < 8; i++) w[i] = crc_word_careful(m, q0 + 128 * i, inv);
-                } else {
-                    const uintptr_t ad = (uintptr_t)(m + q0);
-                    const uint32_t* wp = reinterpret_cast<const uint32_t*>(ad & ~(uintptr_t)3);
-                    const uint32_t sh = (uint32_t)(ad & 3) * 8;
-                    if (sh) {
-                        uint32_t hi[8];
-#pragma unroll
-                        for (int i = 0; i < 8; i++) w[i] = __ldg(wp + 32 * i);
-#pragma unroll
-                        for (int i = 0; i < 8; i++) hi[i] = __ldg(wp + 32 * i + 1);
-#pragma unroll
-                        for (int i = 0; i < 8; i++) w[i] = __funnelshift_r(w[i], hi[i], sh);
+                        for (int i = 0; i < 8; i++) w[i] = crc_word_careful(m, q0 + 128 * i, inv);
                     } else {
+                        const uintptr_t ad = (uintptr_t)(m + q0);
+                        const uint32_t* wp = reinterpret_cast<const uint32_t*>(ad & ~(uintptr_t)3);
+                        const uint32_t sh = (uint32_t)(ad & 3) * 8;
+                        if (sh) {
+                            uint32_t hi[8];
 #pragma unroll
-                        for (int i = 0; i < 8; i++) w[i] = __ldg(wp + 32 * i);
+                            for (int i = 0; i < 8; i++) w[i] = __ldg(wp + 32 * i);
+#pragma unroll
+                            for (int i = 0; i < 8; i++) hi[i] = __ldg(wp + 32 * i + 1);
+#pragma unroll
+                            for (int i = 0; i < 8; i++) w[i] = __funnelshift_r(w[i], hi[i], sh);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 8; i++) w[i] = __ldg(wp + 32 * i);
+                        }
                     }
+                    if (last) crc_rows<true>(v, w, r0);
+                    else crc_rows<false>(v, w, r0);
                 }
-                if (last) crc_rows<true>(v, w, i0);
-                else crc_rows<false>(v, w, i0);
             }
-        }
-        uint32_t c = 0;
 #pragma unroll
-        for (int i = 0; i < 32; i++)
-            c = fold[0][c & 255] ^ fold[1][(c >> 8) & 255] ^ fold[2][(c >> 16) & 255] ^ fold[3][c >> 24] ^ v[i];
-        c = __reduce_xor_sync(FULL, gf_mul(c, kCrcLane.k[lane]));
-        const uint32_t crc = inv ? ~c : crc_finish(c, len);
-        if (lane == 0 && crc != job.crc) {
-            per_job[4 * j + 1] = CB_ERR_CRC;
-            report(summary, job_status, j, CB_ERR_CRC);
+            for (int i = 0; i < 32; i++)
+                c = fold[0][c & 255] ^ fold[1][(c >> 8) & 255] ^ fold[2][(c >> 16) & 255] ^ fold[3][c >> 24] ^ v[i];
+            c = __reduce_xor_sync(FULL, gf_mul(c, kCrcLane.k[lane]));
+            if (W > 1 && i1 < iters) c = gf_mul(c, xpow_from(kCrc.x2n, 32768ull * (unsigned long long)(iters - i1)));
+        }
+        if (W > 1) {
+            if (lane == 0) parts[warp] = c;
+            __syncthreads();
+            if (warp % W == 0)
+                for (int w = 1; w < W; w++) c ^= parts[warp + w];
+            __syncthreads();
+        }
+        if (on && warp % W == 0) {
+            const uint32_t crc = len >= 4 ? ~c : crc_finish(c, len);
+            if (lane == 0 && crc != want) {
+                per_job[JW * j + 1] = CB_ERR_CRC;
+                report(summary, job_status, j, CB_ERR_CRC);
+            }
         }
     }
 }
@@ -1239,8 +1442,8 @@ int cb_set_error(cudaError_t e);  // abi.cu
 int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base,
                          int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
                          size_t workspace_bytes, bool list_unfit, void* stream);
-// inflate.cu: the one-kernel form for the jobs list[4 * k], k < *count (on the device)
-int cb_inflate_listed(const cb_member_job* jobs, const uint32_t* list, const unsigned long long* count,
+// inflate.cu: the one-kernel form for the jobs list[step * k], k < *count (on the device)
+int cb_inflate_listed(const cb_member_job* jobs, const uint32_t* list, int step, const unsigned long long* count,
                       uint8_t* out_base, int check_crc, uint32_t* job_status, cb_inflate_summary* summary,
                       unsigned long long* queue, cudaStream_t s);
 
@@ -1285,48 +1488,76 @@ struct Range {
     int qd;
 };
 
-// CTAs for a persistent grid of `occ` per SM, `warps` members each, no more than the range has work for.
-unsigned grid_for(const Call& c, Range r, int occ, int warps) {
+// CTAs for a persistent grid of `occ` per SM, `members` each at a time, no more than the range has work for.
+unsigned grid_for(const Call& c, Range r, int occ, int members) {
     long long grid = (long long)cb_device_sm_count() * occ;
-    const long long by_work = (r.j1 - r.j0 + warps - 1) / warps;
+    const long long by_work = (r.j1 - r.j0 + members - 1) / members;
     if (!c.d_n_jobs && by_work < grid) grid = by_work;
     return (unsigned)(grid < 1 ? 1 : grid);
 }
 
-int decode_range(const Call& c, Range r, cudaStream_t s) {
+// Warps per member: one member's serial work bounds a call of few, so each takes more warps while all of
+// them stay resident (28 warps per SM).
+int warps_per_member(const Call& c) {
+    const long long room = (long long)cb_device_sm_count() * 28;
+    return c.n_jobs * 8 <= room ? 8 : c.n_jobs * 4 <= room ? 4 : c.n_jobs * 2 <= room ? 2 : 1;
+}
+
+template <int W>
+int launch_decode(const Call& c, Range r, cudaStream_t s) {
     static int cache[MAX_DEVICES];
-    const size_t smem = split::DEC_WARPS * sizeof(split::DecWarp);
-    const int o = occupancy(cache, split::k_decode, split::DEC_WARPS * 32, smem);
+    constexpr int MEMBERS = W == 1 ? 2 : 1, NT = 32 * W * MEMBERS;
+    const size_t smem = MEMBERS * sizeof(split::DecMember<W>);
+    const int o = occupancy(cache, split::k_decode<W>, NT, smem);
     if (o <= 0) return fail_occ(o);
-    split::k_decode<<<grid_for(c, r, o, split::DEC_WARPS), split::DEC_WARPS * 32, smem, s>>>(
-        c.jobs, c.n_jobs, c.d_n_jobs, c.job_status, c.summary, c.ws, c.arena, c.arena_bytes, c.list_unfit, r.j0, r.j1, r.qd);
+    split::k_decode<W><<<grid_for(c, r, o, MEMBERS), NT, smem, s>>>(c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status,
+                                                                    c.summary, c.ws, c.arena, c.arena_bytes,
+                                                                    c.list_unfit, r.j0, r.j1, r.qd);
     return CB_OK;
+}
+
+int decode_range(const Call& c, Range r, cudaStream_t s) {
+    const int w = warps_per_member(c);
+    return w == 8 ? launch_decode<8>(c, r, s) : w == 4 ? launch_decode<4>(c, r, s) : w == 2 ? launch_decode<2>(c, r, s)
+                                                                                          : launch_decode<1>(c, r, s);
 }
 
 template <class C>
 int launch_copy(const Call& c, Range r, cudaStream_t s) {
     static int cache[MAX_DEVICES];
-    const size_t smem = split::COPY_WARPS * sizeof(typename C::WarpSmem);
-    const int o = occupancy(cache, split::k_copy<C>, split::COPY_WARPS * 32, smem);
+    static_assert(sizeof(typename C::Smem) < 65536, "a source's offset has 16 bits");
+    const size_t smem = sizeof(typename C::Smem);
+    const int o = occupancy(cache, split::k_copy<C>, C::T, smem);
     if (o <= 0) return fail_occ(o);
-    split::k_copy<C><<<grid_for(c, r, o, split::COPY_WARPS), split::COPY_WARPS * 32, smem, s>>>(
-        c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status, c.summary, c.ws, c.arena, r.j0, r.j1, r.qd + 1);
+    split::k_copy<C><<<grid_for(c, r, o, 1), C::T, smem, s>>>(c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status,
+                                                              c.summary, c.ws, c.arena, r.j0, r.j1, r.qd + 1);
+    return CB_OK;
+}
+
+template <int W>
+int launch_crc(const Call& c, Range r, cudaStream_t s) {
+    static int cache[MAX_DEVICES];
+    const int o = occupancy(cache, split::k_crc<W>, split::CRC_NT, 0);
+    if (o <= 0) return fail_occ(o);
+    split::k_crc<W><<<grid_for(c, r, o, split::CRC_NT / 32 / W), split::CRC_NT, 0, s>>>(
+        c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status, c.summary, c.ws, r.j0, r.j1);
     return CB_OK;
 }
 
 int copy_range(const Call& c, Range r, cudaStream_t s) {
+    const int w = warps_per_member(c);
     const int cw = (int)cb_param(CB_PARAM_COPY_WARPS);
+    int rc;
+    if (w == 8) rc = launch_copy<split::CopyCfg<16384, 8>>(c, r, s);
+    else if (w == 4) rc = launch_copy<split::CopyCfg<16384, 4>>(c, r, s);
+    else if (w == 2) rc = launch_copy<split::CopyCfg<8192, 2>>(c, r, s);
     // 4 KB: 28 warps per SM, 4.04 ms on 15,456 GEX members, 8 KB 16 warps and 4.39 ms
-    const int rc = cw == 12   ? launch_copy<split::CopyCfg<4096>>(c, r, s)
-                   : cw == 24 ? launch_copy<split::CopyCfg<8192>>(c, r, s)
-                              : launch_copy<split::CopyCfg<16384>>(c, r, s);
+    else if (cw == 12) rc = launch_copy<split::CopyCfg<4096, 1>>(c, r, s);
+    else if (cw == 24) rc = launch_copy<split::CopyCfg<8192, 1>>(c, r, s);
+    else rc = launch_copy<split::CopyCfg<16384, 1>>(c, r, s);
     if (rc != CB_OK || !c.check_crc) return rc;
-    static int cache[MAX_DEVICES];
-    const int o = occupancy(cache, split::k_crc, split::CRC_NT, 0);
-    if (o <= 0) return fail_occ(o);
-    split::k_crc<<<grid_for(c, r, o, split::CRC_NT / 32), split::CRC_NT, 0, s>>>(
-        c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status, c.summary, c.ws, r.j0, r.j1);
-    return CB_OK;
+    return w == 8 ? launch_crc<8>(c, r, s) : w == 4 ? launch_crc<4>(c, r, s) : w == 2 ? launch_crc<2>(c, r, s)
+                                                                                      : launch_crc<1>(c, r, s);
 }
 
 // Two side streams per device for the pipelined form, and the events that join them to the caller's
@@ -1419,7 +1650,8 @@ int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_
             if (rc != CB_OK) return rc;
             if (e != cudaSuccess) return cb_set_error(e);
         }
-        rc = cb_inflate_listed(jobs, reinterpret_cast<const uint32_t*>(ws + split::WS_HEAD), queue + split::Q_LISTED,
+        rc = cb_inflate_listed(jobs, reinterpret_cast<const uint32_t*>(ws + split::WS_HEAD), split::JW,
+                               queue + split::Q_LISTED,
                                out_base, check_crc, job_status, summary, queue + split::Q_LISTED + 1, s);
         if (rc != CB_OK) return rc;
     }

@@ -177,8 +177,8 @@ int cb_inflate(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_job
  * members in flight), 3 = cb_inflate_split, 0 = CB_PARAM_INFLATE_FORM (see CB_PARAM_SPLIT_MIN_JOBS).
  * Form 3 runs only with a workspace larger than cb_inflate_workspace_bytes() (sized by
  * cb_inflate_split_workspace_bytes); with the small workspace form 1 runs in its place.  With form 0 and
- * fewer than 8192 jobs any workspace will do: jobs that form 3 has no room for run as in form 1.  Every form gives the same bytes and the same
- * per-job codes.  No cubam counterpart (cubam has one nvCOMP call, src/cubam/bgzf.py:595). */
+ * fewer than 8192 jobs any workspace will do: jobs that form 3 has no room for run as in form 1.  Every
+ * form gives the same bytes and the same per-job codes.  No cubam counterpart (cubam has one nvCOMP call, src/cubam/bgzf.py:595). */
 int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base,
                     int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
                     size_t workspace_bytes, int form, void* stream);
@@ -188,9 +188,10 @@ int64_t cb_inflate_lane_slots(void);
 
 /* ---- Inflate, form 3: the Huffman decode, the copy and the CRC32 as three kernels (same contract as
  *      cb_inflate, replacing the same nvCOMP call, src/cubam/bgzf.py:587-611) ------------------------
- * Each takes a warp per member.  The decode's lanes decode 32 segments of the member at once into an
- * arena inside the workspace (a slot of 2 isize + 64 bytes per job, rounded up to 16); the copy writes
- * the member through a window in shared memory (CB_PARAM_COPY_WARPS).
+ * Each takes a member per 1 to 8 warps, more the fewer jobs there are.  The decode's lanes decode 32
+ * segments per warp at once, with the member's output range as scratch, into an arena inside the workspace
+ * (32 bytes and a slot of 2 isize + 64 bytes per job, rounded up to 16); the copy writes the member through
+ * a window in shared memory (CB_PARAM_COPY_WARPS, where a member has one warp).
  * out_bytes: the sum of isize over the jobs (or more); a job whose slot does not fit a smaller
  * workspace fails with CB_ERR_CAPACITY. */
 size_t cb_inflate_split_workspace_bytes(int64_t n_jobs, int64_t out_bytes);

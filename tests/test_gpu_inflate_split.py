@@ -114,6 +114,28 @@ def test_split_matches_zlib(make, window):
         _lib.lib.cb_set_param(_lib.PARAM_COPY_WARPS, -1)
 
 
+@pytest.mark.parametrize("jobs,window", [(600, -1), (1100, -1), (2100, 6), (2100, 12), (2100, 24)])
+@pytest.mark.parametrize("make", [_edges, _distances, _blocks], ids=["edges", "distances", "blocks"])
+def test_split_matches_zlib_at_every_width(make, jobs, window):
+    """The same members many times over: members take 4, 2 and 1 warps as the calls hold more of them."""
+    cases = make()
+    times = -(-jobs // len(cases))
+    buf, table, total = _table(cases, 3)
+    rows = table.cpu().numpy()
+    total -= 3
+    many = np.concatenate([rows + np.array([0, k * total, 0, 0]) for k in range(times)])
+    _lib.lib.cb_set_param(_lib.PARAM_COPY_WARPS, window)
+    try:
+        size = G.inflate_workspace_bytes(len(many), times * total, 3)
+        out, codes, summ = _run(torch.from_numpy(many).cuda(), 3 + times * total, size, 3)
+    finally:
+        _lib.lib.cb_set_param(_lib.PARAM_COPY_WARPS, -1)
+    assert summ.status == 0 and summ.n_bad == 0 and not codes.any()
+    want = np.frombuffer(b"".join(d for d, _ in cases), dtype=np.uint8)
+    assert (out[3 : 3 + times * total].reshape(times, total) == want).all()
+    assert (out[:3] == 0xA5).all() and (out[3 + times * total :] == 0xA5).all()
+
+
 def test_split_reports_crc_and_size():
     """A wrong CRC32 (also unchecked), and an ISIZE one too small or too large, in members of every size."""
     cases = [(d, kw) for d, kw in _edges() if len(d) > 1][::5]
