@@ -81,4 +81,56 @@ __device__ __forceinline__ uint32_t crc_step8(const uint32_t (*T)[256], uint32_t
            T[2][(w1 >> 8) & 255] ^ T[1][(w1 >> 16) & 255] ^ T[0][w1 >> 24];
 }
 
+// ---- CRC by rows: the polynomial P divides P(x^1024) (= P^1024 in characteristic 2), so a message may
+// be reduced by P(x^1024) first: rows of 1024 bits (a 4-byte word per lane) take the place of the
+// polynomial's single bits, and eliminating a row is an XOR of it into the 14 rows that P's other terms
+// name -- seven three-input XORs per row of 128 bytes, in registers.  What is left are 32 rows; each lane
+// folds its words of them with a table of x^1024 and the lanes join with one multiplication each.
+
+struct CrcLane {
+    uint32_t x1024, k[32];  // x^1024; x^(32 (32 - l)): the bits after lane l's word of a row, and 32 more
+};
+constexpr CrcLane make_crc_lane() {
+    CrcLane c{};
+    const CrcConst q = make_crc_const();
+    c.x1024 = xpow_from(q.x2n, 1024);
+    uint32_t v = xpow_from(q.x2n, 32);
+    const uint32_t x32 = v;
+    for (int l = 31; l >= 0; l--) {
+        c.k[l] = v;
+        v = gf_mul(v, x32);
+    }
+    return c;
+}
+static __constant__ CrcLane kCrcLane = make_crc_lane();
+
+// v[i] ^= the rows d before it, d over the terms of the polynomial (x^(32 - d)).
+template <bool LAST>
+__device__ __forceinline__ void crc_rows(uint32_t (&v)[32], const uint32_t (&w)[8], int i0) {
+    constexpr int D[13] = {6, 9, 10, 16, 20, 21, 22, 24, 25, 27, 28, 30, 31};
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+        if (i < i0 || i >= i0 + 8) continue;
+        uint32_t x = v[i] ^ w[i & 7];  // v[i] so far: the row 32 before
+#pragma unroll
+        for (int t = 0; t < 13; t++)
+            if (!LAST || D[t] > i) x ^= v[(i - D[t]) & 31];
+        v[i] = x;
+    }
+}
+
+// The table that folds rows together (T[b][v] = v x^(8 (3 - b)) x^1024 in the reflected form), by the CTA.
+__device__ __forceinline__ void init_crc_fold(uint32_t (*T)[256]) {
+    for (int i = threadIdx.x; i < 1024; i += blockDim.x)
+        T[i >> 8][i & 255] = gf_mul((uint32_t)(i & 255) << (8 * (i >> 8)), kCrcLane.x1024);
+}
+
+// The raw column of the 4,096 bytes that crc_rows<true> left in v, the same in every lane.
+__device__ __forceinline__ uint32_t crc_fold_rows(const uint32_t (*T)[256], const uint32_t (&v)[32]) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int i = 0; i < 32; i++) c = T[0][c & 255] ^ T[1][(c >> 8) & 255] ^ T[2][(c >> 16) & 255] ^ T[3][c >> 24] ^ v[i];
+    return __reduce_xor_sync(FULL, gf_mul(c, kCrcLane.k[threadIdx.x & 31]));
+}
+
 }  // namespace cb

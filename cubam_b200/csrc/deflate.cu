@@ -7,25 +7,32 @@
 //
 // k_deflate: a persistent grid, one CTA of 512 threads per span (at most 64 KiB) at a time, all of
 // the span's work in shared memory:
-//   1. the span is staged with 16-byte loads; its CRC32 is taken there (one column per thread in
-//      8-byte steps, columns joined in a tree by shifts in GF(2)[x]);
+//   1. the span is staged with 16-byte loads; its CRC32 is taken there (a warp per 4,096 bytes, by rows:
+//      crc.cuh);
 //   2. match finding, 512 positions (one per thread) per tile: a hash of the 4 bytes at each
 //      position; candidates are the nearest earlier position of the same hash in the warp
-//      (__match_any_sync) and the latest one of earlier tiles (a table of hash heads kept with
-//      atomicMax, so the result does not depend on thread timing); the longer match is kept;
-//   3. the greedy parse of the tile without a serial walk: jmp[0][i] = i + the step at i (the
-//      match length, or 1), jmp[k+1][i] = jmp[k][jmp[k][i]], and thread m finds token m of the tile
-//      by advancing the entry position by the binary digits of m.  With level >= 2 a position
-//      whose successor has a longer match is a literal (zlib's lazy evaluation, one position of
-//      lookahead);
+//      and the latest one of earlier tiles (a table of hash heads kept with atomicMax, so the result
+//      does not depend on thread timing); the longer match is kept (match_lens);
+//   3. the greedy parse without a walk over its tokens: a position steps by its match length, or 1, and
+//      pointer doubling within the warp gives, for each of its 32 positions, the positions visited from
+//      there on and where they leave the warp's; for a batch of four tiles every position then hops on
+//      to where it leaves its 128 positions, and one warp from 128 to 128.  With level >= 2 a position whose successor in the tile has a longer match is a
+//      literal (zlib's lazy evaluation, one position of lookahead);
 //   4. tokens go to a per-CTA buffer in HBM (it stays in L2), symbol counts to shared memory;
 //   5. Huffman code lengths (ranking by counting, Moffat-Katajainen minimum-redundancy lengths,
 //      limited to 15 and 7 bits), the code-length code, and the exact sizes of a dynamic, a fixed
 //      and a stored block; the smallest is written;
-//   6. bits go out at offsets from a block-wide prefix sum of token sizes (atomicOr into shared
-//      memory words) and are copied to the span's slot.
+//   6. bits go out at offsets from a block-wide prefix sum of token sizes, four tokens per thread, into
+//      shared memory words, and are copied to the span's slot.
 // k_offsets (one CTA) sums the stream sizes into output offsets; k_pack copies each slot to its
 // offset, with the BGZF header and trailer when framing.
+//
+// What bounds k_deflate is the issue of instructions between barriers (0.5 per cycle and scheduler; two
+// CTAs per SM by shared memory, 64 registers): per span about 170,000 cycles for the hash heads, 145,000 for
+// the matches, 310,000 for the parse and its tokens, 55,000 for the codes, 85,000 for the bits.  Measured on 64 MB of
+// GEX records in 1,024 spans: 1.88 ms (2.39 with a parse of twelve barriers per tile, each position
+// comparing for itself, a serial merge that waited for each load, an atomic per token and tables for the
+// CRC32); 240 MB 6.07 ms; k_pack 19 us (57 by bytes).
 //
 // Every loop is bounded by the span's size or an alphabet; no thread waits on another CTA.
 
@@ -41,14 +48,16 @@ constexpr int MAXSPAN = 65536;                 // largest raw span
 constexpr int BGZF_SPAN = 0xFF00;              // largest span framed as a BGZF member (BLOCK_DATA)
 constexpr int INB = MAXSPAN + 32;              // staged bytes: the span at offset a < 16, then slack
 constexpr int HB = 13, NH = 1 << HB;           // hash-head table
-constexpr int LEVELS = 9;                      // jump levels: up to 2^9 tokens per tile
+constexpr int BATCH = 4;                       // tiles parsed at a time
+constexpr int EMIT = 4;                        // tokens per thread and chunk of the emitter
+constexpr int LEVELS = 9;                      // doublings that cover a tile or an alphabet
 constexpr uint32_t MIN_MATCH = 4, MAX_MATCH = 258, WSIZE = 32768;
 constexpr int64_t SLOT = MAXSPAN + 64;         // bytes per span slot (a stream is at most 65536 + 10)
 constexpr int MAX_CTAS = 320;                  // token buffers in the workspace
 constexpr int64_t TOKS = MAXSPAN;              // tokens per CTA buffer
 constexpr int META = 4;                        // per span: stream bytes, CRC32, kind, input bytes
 enum : uint32_t { K_STORED = 0, K_FIXED = 1, K_DYNAMIC = 2 };
-static_assert((1 << LEVELS) == NT, "token m of a tile has LEVELS binary digits");
+static_assert((1 << LEVELS) == NT, "LEVELS doublings cover a tile");
 
 // Code-length construction of one alphabet (par_lengths).
 struct LenScratch {
@@ -58,11 +67,11 @@ struct LenScratch {
     uint16_t dep[2][NLIT_ALL];
     uint32_t c[NLIT_ALL + 2];    // internal nodes per depth
     uint32_t cum[16];            // codes of length <= l
-    int32_t maxd;
+    int32_t maxd, m;             // deepest internal node, used symbols
 };
 
 struct HuffScratch {
-    LenScratch ls;
+    LenScratch ls[2];
     uint8_t rsym[NRLE];
     uint8_t rext[NRLE];
     uint32_t roff[NRLE];  // bit offset of each code-length symbol within the run-length part
@@ -73,19 +82,25 @@ struct HuffScratch {
 
 struct Smem {
     uint32_t in[INB / 4];       // the span's bytes; after tokenising, the output bit buffer
-    uint32_t head[NH];          // position + 1 of the latest earlier-tile position of each hash (0 = none)
     union {
-        uint16_t jmp[LEVELS][NT];  // jmp[k][i]: tile position after 2^k tokens from i (>= NT: beyond)
-        uint32_t crc8[8][256];     // slice-by-8 tables, while the CRC is taken
-        HuffScratch h;             // code construction, after the last tile
-    } u;
-    uint32_t mt[NT];            // match at each tile position: length << 16 | distance (0: none)
-    uint32_t lfreq[NLIT_ALL], dfreq[32], clfreq[20];
-    uint8_t llen[NLIT_ALL], dlen[32], cllen[20];
+        uint32_t head[NH];      // position + 1 of the latest earlier-tile position of each hash (0 = none)
+        HuffScratch h;          // code construction, after the last tile
+    };
+    struct {                    // the parse of a batch
+        uint16_t exit[BATCH * NT];  // per position: where a parse from it leaves its 32 (9 bits, from the first
+                                    // of them), and the tokens until then
+        uint16_t exit4[BATCH * NT]; // the same for its 128 (and the tokens less one)
+        uint32_t entry[BATCH * NT / 128]; // per 128 positions: tokens before << 8 | 128 | position entered (0: none)
+        uint32_t first[BATCH][NT / 32];   // match length at the first position of each 32
+        uint32_t ntok, next;        // the batch's tokens, and where the next batch is entered
+    } p;
+    uint32_t fold[4][256];      // CRC (init_crc_fold)
+    alignas(16) uint32_t lfreq[NLIT_ALL], dfreq[32], clfreq[20];
+    alignas(4) uint8_t llen[NLIT_ALL], dlen[32], cllen[20];
     uint32_t scan[33];
     uint32_t cnt[3][16], nxt[3][16];  // codes per length and first code per length: literal, distance, code-length
-    uint32_t crcw[16], crck[LEVELS];
-    int32_t ntok, exitp, nrle, hlit, hdist, hclen, kind, pad_;
+    uint32_t crcw[NT / 32], crck[NT / 32];  // CRC: a part's column; x^(8 * 4096 i)
+    int32_t nrle, hlit, hdist, hclen, kind, pad_;
     uint32_t hdr_bits, bits;
 };
 
@@ -101,20 +116,55 @@ __device__ __forceinline__ uint64_t u64at(const uint32_t* w, uint32_t byte) {
     return (uint64_t)__funnelshift_r(w0, w1, sh) | ((uint64_t)__funnelshift_r(w1, w2, sh) << 32);
 }
 
-// Bytes in common at byte offsets q and c (c < q) of the staged span, at most maxl, 8 bytes per
-// step.  Reads at most 11 bytes past q + maxl (inside the staging slack).
-__device__ __forceinline__ uint32_t match_len(const uint32_t* w, uint32_t q, uint32_t c, uint32_t maxl) {
-    uint32_t L = 0;
-    while (L < maxl) {
-        const uint64_t x = u64at(w, q + L) ^ u64at(w, c + L);
-        if (x) {
-            L += (uint32_t)(__ffsll((long long)x) - 1) >> 3;
-            break;
-        }
-        L += 8;
+// Match length of every lane's position (byte offset q of the staged span, x: its next 20 bytes) at distance
+// d (0: no candidate), at most maxl, by the whole warp.  Up to 20 bytes are compared at once; of longer matches
+// a lane whose successor has one at the same distance has one byte more than the successor, and the last
+// lanes of such runs are compared by the warp, 128 bytes per step.  (Each lane by itself, 8 bytes per step,
+// made a warp wait for its longest match at every position.)  Reads at most 23 bytes past an offset, or 7
+// past q + maxl (inside the staging slack).
+__device__ __forceinline__ uint32_t match_lens(const uint32_t* w, uint32_t q, uint32_t d, const uint32_t (&x)[5],
+                                               uint32_t maxl) {
+    const uint32_t lane = threadIdx.x & 31, c = q - d, sh = (c & 3) * 8;
+    const uint32_t* pc = w + (c >> 2);
+    uint32_t lo = pc[4], diff = x[4] ^ __funnelshift_r(lo, pc[5], sh), at = 16;
+#pragma unroll
+    for (int i = 3; i >= 0; i--) {
+        const uint32_t v = pc[i], e = x[i] ^ __funnelshift_r(v, lo, sh);
+        diff = e ? e : diff;
+        at = e ? 4u * i : at;
+        lo = v;
     }
-    return L < maxl ? L : maxl;
+    uint32_t L = diff ? at + ((uint32_t)(__ffs((int)diff) - 1) >> 3) : 20u;
+    const bool more = d != 0 && diff == 0 && maxl > 20;
+    const uint32_t ends = __ballot_sync(FULL, more);
+    if (ends) {
+        const uint32_t after = __shfl_down_sync(FULL, d, 1);
+        const uint32_t stop = __ballot_sync(FULL, !(more && lane < 31 && (ends >> (lane + 1) & 1u) && after == d));
+        for (uint32_t todo = stop & ends; todo; todo &= todo - 1) {
+            const int s = __ffs((int)todo) - 1;
+            const uint32_t qs = __shfl_sync(FULL, q, s) + 20, ds = __shfl_sync(FULL, d, s), ms = __shfl_sync(FULL, maxl, s) - 20;
+            uint32_t len = ms;
+            for (uint32_t o = 0; o < ms; o += 128) {
+                const uint32_t k = o + 4 * lane;
+                const uint32_t e = k < ms ? u32at(w, qs + k) ^ u32at(w, qs - ds + k) : 0u;
+                const uint32_t m = __ballot_sync(FULL, e != 0);
+                if (m) {
+                    const int f = __ffs((int)m) - 1;
+                    len = o + 4 * f + ((uint32_t)(__ffs((int)__shfl_sync(FULL, e, f)) - 1) >> 3);
+                    break;
+                }
+            }
+            if ((int)lane == s) L += min(len, ms);
+        }
+        const int last = __ffs((int)(stop >> lane)) - 1;  // (lane 31 stops)
+        const uint32_t Le = __shfl_sync(FULL, L, lane + last);
+        if (more) L = Le + last;
+    }
+    return d ? min(L, maxl) : 0u;
 }
+
+// The lowest n bits set (n < 32).
+__device__ __forceinline__ uint32_t low_mask(uint32_t n) { return (1u << n) - 1u; }
 
 // OR the low nb (<= 32) bits of v into the bit stream at bit pos (a stream is shorter than the
 // staging buffer by construction: a block longer than the stored one is never emitted; the bound
@@ -127,185 +177,277 @@ __device__ __forceinline__ void or_bits(uint32_t* buf, uint32_t pos, uint32_t v,
     if (s + nb > 32) atomicOr(&buf[w + 1], (uint32_t)(x >> 32));
 }
 
-// Rank of symbol s among the symbols with nonzero counts, by (count, symbol): sorted[rank] = s.
+// Rank of symbol s among the symbols with nonzero counts, by (count, symbol): sorted[rank] = s.  freq is
+// 16-byte aligned and zero from nsym up to a multiple of four.
 __device__ __forceinline__ void rank_symbol(const uint32_t* freq, int nsym, int s, uint16_t* sorted) {
     const uint32_t f = freq[s];
-    if (!f) return;
     int r = 0;
-    for (int j = 0; j < nsym; j++) {
-        const uint32_t g = freq[j];
-        r += (g != 0) & ((g < f) | ((g == f) & (j < s)));
+    for (int j = 0; j < nsym; j += 4) {
+        const uint4 g = *reinterpret_cast<const uint4*>(freq + j);
+        // a count f counts as less up to symbol s, 0 wraps to the largest
+        r += g.x - 1 < f - 1 + (j < s);
+        r += g.y - 1 < f - 1 + (j + 1 < s);
+        r += g.z - 1 < f - 1 + (j + 2 < s);
+        r += g.w - 1 < f - 1 + (j + 3 < s);
     }
     sorted[r] = (uint16_t)s;
 }
 
-// Per-size constants of span_crc, kept by thread 0 from one span to the next (spans mostly have
-// the same size).
-struct CrcCache {
-    uint32_t seg = 0xFFFFFFFFu, n = 0xFFFFFFFFu, fin = 0;
-};
-
-// The zlib CRC32 of the staged span (bytes a .. a + n of S.in), every thread taking part; the
-// result is valid in thread 0.
-__device__ uint32_t span_crc(Smem& S, uint32_t a, uint32_t n, CrcCache& cc) {
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint8_t* in8 = reinterpret_cast<const uint8_t*>(S.in);
-    init_crc8(S.u.crc8);
-    // thread t: bytes [t*seg - pad, (t+1)*seg - pad) of the span behind pad zero bytes (zeros in
-    // front leave a raw column unchanged), so all columns are seg bytes long
-    const uint32_t seg = ((n + NT - 1) / NT + 7) & ~7u;
-    const int32_t pad = (int32_t)(NT * seg) - (int32_t)n;
-    if (t == 0 && seg != cc.seg) {
-        cc.seg = seg;
-        uint32_t c = xpow_from(kCrc.x2n, 8ull * seg);
-        for (int k = 0; k < LEVELS; k++) {
-            S.crck[k] = c;
-            c = gf_mul(c, c);
-        }
-    }
-    __syncthreads();
-    uint32_t col = 0;
-    const int32_t r1 = (int32_t)(t * seg) + (int32_t)seg - pad;
-    if (r1 > 0) {
-        int32_t r = (int32_t)(t * seg) - pad;
-        if (r < 0) r = 0;
-        for (; (r1 - r) & 7; r++) col = S.u.crc8[0][(col ^ in8[a + r]) & 255] ^ (col >> 8);
-        for (; r < r1; r += 8) col = crc_step8(S.u.crc8, col, u32at(S.in, a + r), u32at(S.in, a + r + 4));
-    }
+// The zlib CRC32 of the staged span (bytes a .. a + n of S.in), every thread taking part, a warp per 4,096
+// bytes (counted from the end: zeros in front leave a raw column unchanged); the result is valid in thread 0.
+// (512 columns by tables were 6% of the kernel's time.)
+__device__ uint32_t span_crc(Smem& S, uint32_t a, uint32_t n) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    static_assert(MAXSPAN <= NT / 32 * 4096, "a warp per 4,096 bytes");
+    const int parts = (int)((n + 4095) >> 12);
+    uint32_t c = 0;
+    if (warp < parts) {
+        const int pad = parts * 4096 - (int)n;
+        uint32_t v[32];
 #pragma unroll
-    for (int k = 0; k < 5; k++) {
-        const uint32_t other = __shfl_down_sync(FULL, col, 1 << k);
-        if ((lane & ((2 << k) - 1)) == 0) col = gf_mul(col, S.crck[k]) ^ other;
-    }
-    if (lane == 0) S.crcw[warp] = col;
-    __syncthreads();
-    uint32_t crc = 0;
-    if (warp == 0) {
-        uint32_t v = lane < NT / 32 ? S.crcw[lane] : 0u;
+        for (int i = 0; i < 32; i++) v[i] = 0;
 #pragma unroll
-        for (int k = 5; k < LEVELS; k++) {
-            const uint32_t other = __shfl_down_sync(FULL, v, 1 << (k - 5));
-            if ((lane & ((2 << (k - 5)) - 1)) == 0) v = gf_mul(v, S.crck[k]) ^ other;
-        }
-        if (t == 0) {
-            if (n != cc.n) {
-                cc.n = n;
-                cc.fin = gf_mul(0xFFFFFFFFu, xpow_from(kCrc.x2n, 8ull * n));
+        for (int r0 = 0; r0 < 32; r0 += 8) {
+            uint32_t w[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int q = warp * 4096 + (r0 + i) * 128 + 4 * lane - pad;
+                uint32_t x = u32at(S.in, a + (uint32_t)max(q, 0));
+                if (q < 4) {  // bytes before the span are zero, its first four are inverted (the initial value)
+                    if (q < 0) x = q > -4 ? x << (-8 * q) : 0u;
+                    if (n >= 4 && q > -4) x ^= q < 0 ? FULL << (-8 * q) : FULL >> (8 * q);
+                }
+                w[i] = x;
             }
-            crc = v ^ cc.fin ^ 0xFFFFFFFFu;  // crc_finish(v, n)
+            crc_rows<true>(v, w, r0);
         }
+        c = gf_mul(crc_fold_rows(S.fold, v), S.crck[parts - 1 - warp]);
     }
-    return crc;
+    if (lane == 0) S.crcw[warp] = c;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < NT / 32; w++) c ^= S.crcw[w];
+    return n >= 4 ? ~c : crc_finish(c, n);
+}
+
+// The lanes with this lane's hash (none but itself without v4), by a vote on each of its bits.
+__device__ __forceinline__ uint32_t same_hash(uint32_t h, bool v4) {
+    uint32_t m = __ballot_sync(FULL, v4);
+#pragma unroll
+    for (int b = 0; b < HB; b++) {
+        const bool on = h >> b & 1u;
+        const uint32_t v = __ballot_sync(FULL, on);
+        m &= on ? v : ~v;
+    }
+    return m;
 }
 
 // Tokens of the span into tok[0..), symbol counts into S.lfreq / S.dfreq.  Returns the token count.
+// A tile takes two barriers for the hash heads, a batch of tiles four more (a parse by doubling over the whole
+// tile took twelve per tile).
 __device__ uint32_t tokenize(Smem& S, uint32_t a, uint32_t n, int level, uint32_t* __restrict__ tok) {
-    const int t = threadIdx.x, lane = t & 31;
+    constexpr uint32_t WARPS = NT / 32, SPAN = BATCH * NT;
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5, lt = (1u << lane) - 1u;
     const uint8_t* in8 = reinterpret_cast<const uint8_t*>(S.in);
     uint32_t entry = 0, tbase = 0;
-    for (uint32_t T0 = 0; T0 < n; T0 += NT) {
-        const uint32_t tend = min((uint32_t)NT, n - T0);
-        const uint32_t p = T0 + t;
-        const bool v4 = level > 0 && p + 4 <= n;
-        const uint32_t cur = v4 ? u32at(S.in, a + p) : 0u;
-        const uint32_t h = (cur * 0x9E3779B1u) >> (32 - HB);
-        const unsigned grp = __match_any_sync(FULL, v4 ? h : (0x80000000u | (uint32_t)t));
-        const uint32_t hv = v4 ? S.head[h] : 0u;
-        __syncthreads();  // every read of the heads before this tile's updates
-        if (t == 0) S.ntok = 0;
-        if (v4 && (grp >> lane) == 1u) atomicMax(&S.head[h], p + 1);
-        uint32_t best = 0;
-        if (v4) {
-            const uint32_t maxl = min(MAX_MATCH, n - p);
-            const unsigned below = grp & ((1u << lane) - 1u);
-            if (below) {
-                const uint32_t c = p - (uint32_t)lane + (31u - (uint32_t)__clz(below));
-                const uint32_t L = match_len(S.in, a + p, a + c, maxl);
-                if (L >= MIN_MATCH) best = (L << 16) | (p - c);
+    for (uint32_t P0 = 0; P0 < n; P0 += SPAN) {
+        // candidates: the nearest earlier position of the same hash in the warp (distance << 16) and the
+        // latest of earlier tiles
+        uint32_t cand[BATCH], hash[BATCH];
+#pragma unroll
+        for (int k = 0; k < BATCH; k++) {
+            const uint32_t p = P0 + k * NT + t;
+            const bool v4 = level > 0 && p + 4 <= n;
+            hash[k] = v4 ? (u32at(S.in, a + p) * 0x9E3779B1u) >> (32 - HB) : 0x80000000u | t;
+            // (one tile of four by votes: the matching unit takes 23 cycles per warp for 32 different hashes, and
+            // 64 MB then took 2.02 ms; all of them by it 2.07, two by votes 2.04, all by votes 2.19)
+            const uint32_t grp = k == 1 ? same_hash(hash[k], v4) : __match_any_sync(FULL, hash[k]);
+            const uint32_t below = v4 ? grp & lt : 0u;
+            cand[k] = below ? (lane - (31u - (uint32_t)__clz((int)below))) << 16 : 0u;
+            if (v4 && (grp >> lane) == 1u) hash[k] |= 0x40000000u;  // the warp's last position of this hash
+        }
+#pragma unroll
+        for (int k = 0; k < BATCH; k++) {
+            const uint32_t p = P0 + k * NT + t;
+            if (P0 + k * NT >= n) break;
+            if (!(hash[k] >> 31)) {
+                const uint32_t hv = S.head[hash[k] & (NH - 1)];
+                if (hv && p + 1 - hv <= WSIZE) cand[k] |= p + 1 - hv;
             }
-            if (hv && (best >> 16) < maxl) {  // a match of maxl cannot be beaten
-                const uint32_t c = hv - 1;
-                if (p - c <= WSIZE) {
-                    const uint32_t L = match_len(S.in, a + p, a + c, maxl);
-                    if (L >= MIN_MATCH && L > (best >> 16)) best = (L << 16) | (p - c);
+            __syncthreads();  // every read of the heads before this tile's updates (and of the last batch's parse)
+            if (hash[k] >> 30 == 1u) atomicMax(&S.head[hash[k] & (NH - 1)], p + 1);
+            if (k == 0 && t < SPAN / 128) S.p.entry[t] = 0;
+            __syncthreads();
+        }
+        uint32_t best[BATCH];  // length << 16 | distance (0: none)
+#pragma unroll
+        for (int k = 0; k < BATCH; k++) {
+            const uint32_t p = P0 + k * NT + t;
+            uint32_t b = 0;
+            if (__any_sync(FULL, cand[k] != 0)) {
+                const bool v4 = p + 4 <= n;
+                const uint32_t q = a + (v4 ? p : 0u), maxl = v4 ? min(MAX_MATCH, n - p) : 0u;
+                const uint32_t d1 = cand[k] >> 16, d2 = cand[k] & 0xFFFFu;
+                const uint32_t* pq = S.in + (q >> 2);
+                uint32_t x[5], lo = pq[0];
+#pragma unroll
+                for (int i = 0; i < 5; i++) {
+                    const uint32_t hi = pq[i + 1];
+                    x[i] = __funnelshift_r(lo, hi, (q & 3) * 8);
+                    lo = hi;
+                }
+                if (__any_sync(FULL, d1 != 0)) {
+                    const uint32_t L = match_lens(S.in, q, d1, x, maxl);
+                    if (L >= MIN_MATCH) b = (L << 16) | d1;
+                }
+                const uint32_t L = match_lens(S.in, q, d2, x, maxl);
+                if (L >= MIN_MATCH && L > (b >> 16)) b = (L << 16) | d2;
+            }
+            best[k] = b;
+            if (lane == 0) S.p.first[k][warp] = b >> 16;
+        }
+        __syncthreads();
+        uint32_t seen[BATCH], nx[BATCH];  // the positions of the warp that a parse from here visits, and where it leaves
+#pragma unroll
+        for (int k = 0; k < BATCH; k++) {
+            uint32_t after = __shfl_down_sync(FULL, best[k] >> 16, 1);
+            if (lane == 31) after = warp + 1 < WARPS ? S.p.first[k][warp + 1] : 0u;
+            if (level >= 2 && after > (best[k] >> 16)) best[k] = 0;
+            // to the next match or past the 32, or past the match; then doubled
+            const uint32_t ahead = __ballot_sync(FULL, best[k] != 0) >> lane;
+            nx[k] = ahead ? lane + (uint32_t)__ffs((int)ahead) - 1u : 32u;
+            seen[k] = (nx[k] < 32 ? low_mask(nx[k]) : FULL) & ~lt;
+            if (best[k]) {
+                nx[k] = lane + (best[k] >> 16);
+                seen[k] = 1u << lane;
+            }
+        }
+        for (;;) {
+            bool more = false;
+#pragma unroll
+            for (int k = 0; k < BATCH; k++) more |= nx[k] < 32;
+            if (!__any_sync(FULL, more)) break;
+#pragma unroll
+            for (int k = 0; k < BATCH; k++) {
+                const uint32_t m = __shfl_sync(FULL, seen[k], nx[k] & 31u), x = __shfl_sync(FULL, nx[k], nx[k] & 31u);
+                if (nx[k] < 32) {
+                    seen[k] |= m;
+                    nx[k] = x;
                 }
             }
         }
-        S.mt[t] = best;
-        __syncthreads();
-        uint32_t step = 1;
-        if ((uint32_t)t < tend) {
-            const uint32_t m0 = S.mt[t];
-            if (m0) {
-                step = m0 >> 16;
-                if (level >= 2 && (uint32_t)t + 1 < tend && (S.mt[t + 1] >> 16) > step) step = 1;
-            }
-        }
-        S.u.jmp[0][t] = (uint16_t)((uint32_t)t < tend ? t + step : NT);
-        __syncthreads();
-#pragma unroll 1
-        for (int k = 0; k + 1 < LEVELS; k++) {
-            const uint32_t x = S.u.jmp[k][t];
-            S.u.jmp[k + 1][t] = x < (uint32_t)NT ? S.u.jmp[k][x] : (uint16_t)x;
-            __syncthreads();
-        }
-        uint32_t pos = entry;
 #pragma unroll
-        for (int k = 0; k < LEVELS; k++)
-            if (((t >> k) & 1) && pos < (uint32_t)NT) pos = S.u.jmp[k][pos];
-        if (pos < tend) {
-            const uint32_t nx = S.u.jmp[0][pos], st = nx - pos;
-            uint32_t tk;
-            if (st >= MIN_MATCH) {
-                const uint32_t d = S.mt[pos] & 0xFFFFu;
-                tk = 0x80000000u | (st << 16) | (d - 1);
-                atomicAdd(&S.lfreq[len_sym(st)], 1u);
-                atomicAdd(&S.dfreq[dist_sym(d)], 1u);
-            } else {
-                tk = in8[a + T0 + pos];
-                atomicAdd(&S.lfreq[tk], 1u);
+        for (int k = 0; k < BATCH; k++) {
+            const uint32_t g0 = P0 + k * NT + warp * 32;
+            if (g0 + 31 >= n) seen[k] &= n > g0 ? low_mask(n - g0) : 0u;
+            S.p.exit[k * NT + t] = (uint16_t)(nx[k] | (__popc(seen[k]) << 9));
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < BATCH; k++) {  // hop on to where a parse leaves each 128 positions
+            const uint32_t g = k * NT + t, s0 = g & ~127u, x = S.p.exit[g];
+            uint32_t e = (g & ~31u) + (x & 511u), cnt = x >> 9;
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                if (e < s0 + 128) {
+                    const uint32_t y = S.p.exit[e];
+                    e = (e & ~31u) + (y & 511u);
+                    cnt += y >> 9;
+                }
             }
-            tok[tbase + t] = tk;
-            if (nx >= tend) {
-                S.ntok = t + 1;
-                S.exitp = (int32_t)nx - NT;
+            S.p.exit4[g] = (uint16_t)((e - s0) | ((cnt - 1) << 9));
+        }
+        __syncthreads();
+        if (warp == 0) {  // and one warp from 128 to 128
+            const uint32_t end = min(SPAN, n - P0);
+            uint32_t e = entry, cnt = 0;
+            while (e < end) {
+                const uint32_t x = S.p.exit4[e];
+                S.p.entry[e >> 7] = (cnt << 8) | 128u | (e & 127u);  // (by every lane alike)
+                e = (e & ~127u) + (x & 511u);
+                cnt += (x >> 9) + 1;
+            }
+            if (lane == 0) {
+                S.p.ntok = cnt;
+                S.p.next = e > SPAN ? e - SPAN : 0u;
             }
         }
         __syncthreads();
-        tbase += (uint32_t)S.ntok;
-        entry = S.exitp > 0 ? (uint32_t)S.exitp : 0u;
+#pragma unroll
+        for (int k = 0; k < BATCH; k++) {
+            const uint32_t p = P0 + k * NT + t, g0 = k * NT + warp * 32, s0 = g0 & ~127u;
+            const uint32_t x = S.p.entry[g0 >> 7];
+            uint32_t e = x ? s0 + (x & 127u) : g0 + 32u, before = x >> 8;
+#pragma unroll
+            for (int r = 0; r < 3; r++) {  // the 32s before this one
+                if (e < g0) {
+                    const uint32_t y = S.p.exit[e];
+                    e = (e & ~31u) + (y & 511u);
+                    before += y >> 9;
+                }
+            }
+            const uint32_t mine = __shfl_sync(FULL, seen[k], e & 31u);
+            if (e < g0 + 32 && (mine >> lane & 1u)) {
+                uint32_t tk;
+                if (best[k]) {
+                    const uint32_t L = best[k] >> 16, d = best[k] & 0xFFFFu;
+                    tk = 0x80000000u | (L << 16) | (d - 1);
+                    atomicAdd(&S.lfreq[len_sym(L)], 1u);
+                    atomicAdd(&S.dfreq[dist_sym(d)], 1u);
+                } else {
+                    tk = in8[a + p];
+                    atomicAdd(&S.lfreq[tk], 1u);
+                }
+                tok[tbase + before + __popc(mine & lt)] = tk;
+            }
+        }
+        tbase += S.p.ntok;
+        entry = S.p.next;
     }
+    __syncthreads();
     return tbase;
 }
 
-// Code lengths (at most L bits) of the symbols 0..nrank-1 with counts freq, into len[0..nlen), as
-// build_lengths gives them; every thread takes part.  Thread 0 runs the first, sequential pass of
-// the Moffat-Katajainen method (the merge of leaves and internal nodes); the depths of internal
-// nodes come from pointer jumping over its parent links, the leaves per depth from a histogram of
-// those depths, and each symbol's length from its rank (lengths_from_depths, length_of_rank).
-__device__ void par_lengths(Smem& S, const uint32_t* freq, int nrank, int nlen, uint32_t L, uint8_t* len) {
-    const int t = threadIdx.x;
-    LenScratch& P = S.u.h.ls;
-    if (t < nrank) rank_symbol(freq, nrank, t, P.sorted);
-    const int m = __syncthreads_count(t < nrank && freq[t] != 0);
-    if (t < nlen) len[t] = 0;
-    if (t < m) P.A[t] = freq[P.sorted[t]];
-    for (int i = t; i < m + 2; i += NT) P.c[i] = 0u;
-    if (t == 0) P.maxd = 0;
+// An alphabet whose code lengths par_lengths makes: counts of the symbols 0..nrank-1 (16-byte aligned, zero
+// up to a multiple of four), nlen lengths of at most L bits.
+struct Alphabet {
+    const uint32_t* freq;
+    int nrank, nlen;
+    uint32_t L;
+    uint8_t* len;
+    LenScratch* scratch;
+};
+
+// Code lengths of an alphabet as build_lengths gives them, by a group of at least nlen + 2 threads of whole
+// warps that the caller numbers t = 0 on; every thread of the CTA calls this, several alphabets may be made
+// at once (a thread of no group: any alphabet with t >= nlen + 2).  Thread 0 runs the first, sequential
+// pass of the Moffat-Katajainen method (the merge of leaves and internal nodes); the depths of internal
+// nodes come from pointer jumping over its parent links, the leaves per depth from a histogram of those
+// depths, and each symbol's length from its rank (lengths_from_depths, length_of_rank).
+__device__ void par_lengths(const Alphabet& al, int t) {
+    LenScratch& P = *al.scratch;
+    if (t == 0) P.m = P.maxd = 0;
+    if (t < al.nlen + 2) P.c[t] = 0u;
     __syncthreads();
-    if (m < 2) {  // a complete two-code all the same, as decoders want
-        if (t == 0) {
-            if (m == 0) {
-                len[0] = len[1] = 1;
-            } else {
-                len[P.sorted[0]] = 1;
-                len[P.sorted[0] == 0 ? 1 : 0] = 1;
-            }
-        }
-        __syncthreads();
-        return;
+    if (t < al.nrank && al.freq[t]) {
+        rank_symbol(al.freq, al.nrank, t, P.sorted);
+        atomicAdd(&P.m, 1);
     }
-    if (t == 0) mk_pass1(P.A, m);
+    if (t < al.nlen) al.len[t] = 0;
+    __syncthreads();
+    const int m = P.m;
+    if (t < m) P.A[t] = al.freq[P.sorted[t]];
+    __syncthreads();
+    if (t == 0) {
+        if (m >= 2) {
+            mk_pass1(P.A, m);
+        } else if (m == 0) {  // a complete two-code all the same, as decoders want
+            al.len[0] = al.len[1] = 1;
+        } else {
+            al.len[P.sorted[0]] = 1;
+            al.len[P.sorted[0] == 0 ? 1 : 0] = 1;
+        }
+    }
     __syncthreads();
     const int ni = m - 1, root = m - 2;  // internal nodes; the last one is the root
     if (t < ni) {
@@ -331,9 +473,9 @@ __device__ void par_lengths(Smem& S, const uint32_t* freq, int nrank, int nlen, 
         atomicMax(&P.maxd, (int)P.dep[cur][t]);
     }
     __syncthreads();
-    if (t == 0) lengths_from_depths(P.c, P.maxd, L, P.cum);
+    if (t == 0 && m >= 2) lengths_from_depths(P.c, P.maxd, al.L, P.cum);
     __syncthreads();
-    if (t < m) len[P.sorted[t]] = (uint8_t)length_of_rank((uint32_t)(m - 1 - t), P.cum);
+    if (m >= 2 && t < m) al.len[P.sorted[t]] = (uint8_t)length_of_rank((uint32_t)(m - 1 - t), P.cum);
     __syncthreads();
 }
 
@@ -348,12 +490,15 @@ __device__ __forceinline__ void first_codes(const uint32_t* cnt, uint32_t* nxt) 
 }
 
 // The canonical code of symbol s (as canonical_codes): the first code of its length plus the
-// number of earlier symbols of that length; length << 16 | the code's bits reversed.
+// number of earlier symbols of that length; length << 16 | the code's bits reversed.  len is 4-byte aligned.
 __device__ __forceinline__ uint32_t canonical_of(const uint8_t* len, int s, const uint32_t* nxt) {
     const uint32_t l = len[s];
     if (!l) return 0u;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(len);  // four at a time
     uint32_t r = 0;
-    for (int j = 0; j < s; j++) r += len[j] == l;
+    for (int j = 0; j < s >> 2; j++) r += __popc(__vcmpeq4(w[j], l * 0x01010101u));
+    r += __popc(__vcmpeq4(w[s >> 2], l * 0x01010101u) & low_mask(8 * (s & 3)));
+    r >>= 3;
     return (l << 16) | reverse_bits(nxt[l] + r, l);
 }
 
@@ -361,9 +506,11 @@ __device__ __forceinline__ uint32_t canonical_of(const uint8_t* len, int s, cons
 // part (the same results as the serial build_lengths, rle_lengths and canonical_codes).
 __device__ void build_codes(Smem& S, uint32_t n) {
     const int t = threadIdx.x;
-    HuffScratch& H = S.u.h;
-    par_lengths(S, S.lfreq, NLIT, NLIT_ALL, MAXBITS, S.llen);
-    par_lengths(S, S.dfreq, NDIST, NDIST, MAXBITS, S.dlen);
+    HuffScratch& H = S.h;
+    // literals and lengths by the first threads, distances by the warps after them
+    const Alphabet al = t < 320 ? Alphabet{S.lfreq, NLIT, NLIT_ALL, MAXBITS, S.llen, &H.ls[0]}
+                                : Alphabet{S.dfreq, NDIST, NDIST, MAXBITS, S.dlen, &H.ls[1]};
+    par_lengths(al, t < 320 ? t : t - 320);
     if (t == 0) {
         S.hlit = 257;
         S.hdist = 1;
@@ -394,7 +541,7 @@ __device__ void build_codes(Smem& S, uint32_t n) {
         for (int k = 0; k < cnt; k++) atomicAdd(&S.clfreq[H.rsym[ro + k]], 1u);
     }
     __syncthreads();
-    par_lengths(S, S.clfreq, NCL, NCL, CLBITS, S.cllen);
+    par_lengths(Alphabet{S.clfreq, NCL, NCL, CLBITS, S.cllen, &H.ls[0]}, t);
     if (t == 0) {
         int hclen = NCL;
         while (hclen > 4 && S.cllen[cl_order(hclen - 1)] == 0) hclen--;
@@ -455,7 +602,7 @@ __device__ void build_codes(Smem& S, uint32_t n) {
 // The chosen block into S.in as a bit stream (not for stored blocks).
 __device__ void emit(Smem& S, uint32_t ntok, const uint32_t* __restrict__ tok) {
     const int t = threadIdx.x;
-    const HuffScratch& H = S.u.h;
+    const HuffScratch& H = S.h;
     const uint32_t words = (S.bits + 31) / 32 + 1;
     for (uint32_t w = t; w < words && w < (uint32_t)(INB / 4); w += NT) S.in[w] = 0u;
     __syncthreads();
@@ -475,34 +622,60 @@ __device__ void emit(Smem& S, uint32_t ntok, const uint32_t* __restrict__ tok) {
             or_bits(S.in, pos + (c >> 16), H.rext[t], cl_extra_bits(s));
         }
     }
+    // EMIT tokens per thread and prefix sum; their bits are put together in registers, so that a word takes
+    // one access to shared memory (a token of 13 bits took two or three, each an atomic)
     uint32_t base = S.hdr_bits;
-    uint32_t next = (uint32_t)t < ntok ? tok[t] : 0u;  // each chunk's tokens are loaded a chunk ahead
-    for (uint32_t c0 = 0; c0 < ntok; c0 += NT) {
-        const uint32_t i = c0 + t;
-        const uint32_t tk = next;
-        next = i + NT < ntok ? tok[i + NT] : 0u;
-        uint32_t v1 = 0, n1 = 0, v2 = 0, n2 = 0;
-        if (i < ntok) {
-            if (tk & 0x80000000u) {
-                const uint32_t L = (tk >> 16) & 0x1FFu, d = (tk & 0xFFFFu) + 1;
-                const uint32_t ls = len_sym(L), lc = H.lcode[ls], lb = lc >> 16;
-                v1 = (lc & 0xFFFFu) | (len_extra_val(L) << lb);
-                n1 = lb + len_extra_bits(ls);
-                const uint32_t ds = dist_sym(d), dc = H.dcode[ds], db = dc >> 16;
-                v2 = (dc & 0xFFFFu) | (dist_extra_val(d) << db);
-                n2 = db + dist_extra_bits(ds);
-            } else {
-                const uint32_t lc = H.lcode[tk & 255u];
-                v1 = lc & 0xFFFFu;
-                n1 = lc >> 16;
+    uint32_t next[EMIT];  // each chunk's tokens are loaded a chunk ahead
+#pragma unroll
+    for (int k = 0; k < EMIT; k++) next[k] = EMIT * t + k < ntok ? tok[EMIT * t + k] : 0u;
+    for (uint32_t c0 = 0; c0 < ntok; c0 += EMIT * NT) {
+        const uint32_t i = c0 + EMIT * t;
+        uint32_t v1[EMIT], v2[EMIT], nb[EMIT], bits = 0;  // nb: bits of v1, of v2 << 8
+#pragma unroll
+        for (int k = 0; k < EMIT; k++) {
+            const uint32_t tk = next[k];
+            next[k] = i + k + EMIT * NT < ntok ? tok[i + k + EMIT * NT] : 0u;
+            v1[k] = v2[k] = nb[k] = 0;
+            if (i + k < ntok) {
+                if (tk & 0x80000000u) {
+                    const uint32_t L = (tk >> 16) & 0x1FFu, d = (tk & 0xFFFFu) + 1;
+                    const uint32_t ls = len_sym(L), lc = H.lcode[ls], lb = lc >> 16;
+                    v1[k] = (lc & 0xFFFFu) | (len_extra_val(L) << lb);
+                    const uint32_t ds = dist_sym(d), dc = H.dcode[ds], db = dc >> 16;
+                    v2[k] = (dc & 0xFFFFu) | (dist_extra_val(d) << db);
+                    nb[k] = (lb + len_extra_bits(ls)) | ((db + dist_extra_bits(ds)) << 8);
+                } else {
+                    const uint32_t lc = H.lcode[tk & 255u];
+                    v1[k] = lc & 0xFFFFu;
+                    nb[k] = lc >> 16;
+                }
             }
+            bits += (nb[k] & 255u) + (nb[k] >> 8);
         }
         uint32_t total;
-        const uint32_t off = base + block_exclusive_scan<NT>(n1 + n2, total, S.scan);
-        if (i < ntok) {
-            or_bits(S.in, off, v1, n1);
-            or_bits(S.in, off + n1, v2, n2);
+        const uint32_t off = base + block_exclusive_scan<NT>(bits, total, S.scan);
+        uint32_t* w = S.in + (off >> 5);
+        uint32_t fill = off & 31u;
+        uint64_t buf = 0;
+        bool first = true;  // the word that holds the end of the token before this thread's first
+        auto put = [&](uint32_t v, uint32_t b) {
+            buf |= (uint64_t)v << fill;
+            fill += b;
+            if (fill >= 32) {
+                if (first) atomicOr(w, (uint32_t)buf);
+                else *w = (uint32_t)buf;
+                first = false;
+                w++;
+                buf >>= 32;
+                fill -= 32;
+            }
+        };
+#pragma unroll
+        for (int k = 0; k < EMIT; k++) {
+            put(v1[k], nb[k] & 255u);
+            put(v2[k], nb[k] >> 8);
         }
+        if (bits && fill) atomicOr(w, (uint32_t)buf);
         base += total;
     }
     if (t == 0) {
@@ -521,7 +694,9 @@ __global__ void __launch_bounds__(NT, 2)
     const int t = threadIdx.x;
     uint8_t* in8 = reinterpret_cast<uint8_t*>(S.in);
     uint32_t* tok = tokens + (int64_t)blockIdx.x * TOKS;
-    CrcCache cc;
+    init_crc_fold(S.fold);
+    if (t < NT / 32) S.crck[t] = xpow_from(kCrc.x2n, 32768ull * t);
+    __syncthreads();
     for (int64_t sp = blockIdx.x; sp < n_spans; sp += gridDim.x) {
         const int64_t len = size[sp];
         if (len < 0 || len > max_span) {
@@ -542,7 +717,7 @@ __global__ void __launch_bounds__(NT, 2)
         for (uint32_t c = t; c < nch; c += NT) reinterpret_cast<uint4*>(S.in)[c] = __ldg(g + c);
         __syncthreads();
         if (t < 8 && a + n + t < (uint32_t)INB) in8[a + n + t] = 0;
-        const uint32_t crc = span_crc(S, a, n, cc);
+        const uint32_t crc = span_crc(S, a, n);
         for (int i = t; i < NH; i += NT) S.head[i] = 0u;
         for (int i = t; i < NLIT_ALL; i += NT) S.lfreq[i] = 0u;
         if (t < 32) S.dfreq[t] = 0u;
@@ -635,7 +810,13 @@ __global__ void __launch_bounds__(256) k_pack(const uint8_t* __restrict__ slots,
             const uint8_t hb[16] = {31, 139, 8, 4, 0, 0, 0, 0, 0, 255, 6, 0, 66, 67, 2, 0};
             d[t] = t < 16 ? hb[t] : (uint8_t)(t == 16 ? bsize & 255 : bsize >> 8);
         }
-        for (uint32_t i = t; i < cs; i += blockDim.x) d[h + i] = s[i];
+        // the stream by words of the destination (the slot is 4-byte aligned, with room after the stream)
+        const uint32_t e = min(cs, (uint32_t)(-(uintptr_t)(d + h) & 3)), nw = (cs - e) >> 2;
+        const uint32_t* sw = reinterpret_cast<const uint32_t*>(s);
+        uint32_t* dw = reinterpret_cast<uint32_t*>(d + h + e);
+        for (uint32_t i = t; i < nw; i += blockDim.x) dw[i] = e ? __funnelshift_r(sw[i], sw[i + 1], 8 * e) : sw[i];
+        if (t < e) d[h + t] = s[t];
+        if (t < ((cs - e) & 3u)) d[h + e + 4 * nw + t] = s[e + 4 * nw + t];
         if (frame && t < 8) d[h + cs + t] = (uint8_t)(t < 4 ? crc >> (8 * t) : isize >> (8 * (t - 4)));
     }
 }

@@ -1281,47 +1281,9 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
 }
 
 // ---------------------------------------------------------------- k_crc: one member per W warps
-//
-// The polynomial P divides P(x^1024) (= P^1024 in characteristic 2), so a message may be reduced by
-// P(x^1024) first: rows of 1024 bits (a 4-byte word per lane) take the place of the polynomial's
-// single bits, and eliminating a row is an XOR of it into the 14 rows that P's other terms name --
-// seven three-input XORs per row of 128 bytes, in registers.  What is left are 32 rows; each lane
-// folds its words of them with a table of x^1024 and the lanes join with one multiplication each.
-// (Tables for every byte took a shared-memory access with conflicts per byte.)
+// The rows of crc.cuh, in registers.  (Tables for every byte took a shared-memory access with conflicts per byte.)
 
 constexpr int CRC_NT = 256;
-
-struct CrcLane {
-    uint32_t x1024, k[32];  // x^1024; x^(32 (32 - l)): the bits after lane l's word of a row, and 32 more
-};
-constexpr CrcLane make_crc_lane() {
-    CrcLane c{};
-    const CrcConst q = make_crc_const();
-    c.x1024 = xpow_from(q.x2n, 1024);
-    uint32_t v = xpow_from(q.x2n, 32);
-    const uint32_t x32 = v;
-    for (int l = 31; l >= 0; l--) {
-        c.k[l] = v;
-        v = gf_mul(v, x32);
-    }
-    return c;
-}
-static __constant__ CrcLane kCrcLane = make_crc_lane();
-
-// v[i] ^= the rows d before it, d over the terms of the polynomial (x^(32 - d)).
-template <bool LAST>
-__device__ __forceinline__ void crc_rows(uint32_t (&v)[32], const uint32_t (&w)[8], int i0) {
-    constexpr int D[13] = {6, 9, 10, 16, 20, 21, 22, 24, 25, 27, 28, 30, 31};
-#pragma unroll
-    for (int i = 0; i < 32; i++) {
-        if (i < i0 || i >= i0 + 8) continue;
-        uint32_t x = v[i] ^ w[i & 7];  // v[i] so far: the row 32 before
-#pragma unroll
-        for (int t = 0; t < 13; t++)
-            if (!LAST || D[t] > i) x ^= v[(i - D[t]) & 31];
-        v[i] = x;
-    }
-}
 
 // The word of the message at byte position q (negative positions are zero bytes); with INV the first
 // four bytes are inverted (the CRC's initial value).
@@ -1335,7 +1297,7 @@ __device__ __forceinline__ uint32_t crc_word_careful(const uint8_t* m, long long
     return x;
 }
 
-// W warps per member, each a part of its 4,096-byte rows of rows; parts are joined by x^(8 bytes after).
+// W warps per member, each a part of its 4,096-byte steps; parts are joined by x^(8 bytes after).
 template <int W>
 __global__ void __launch_bounds__(CRC_NT)
     k_crc(const cb_member_job* __restrict__ jobs, int64_t n_jobs, const int64_t* __restrict__ d_n_jobs,
@@ -1343,7 +1305,7 @@ __global__ void __launch_bounds__(CRC_NT)
           long long j0, long long j1) {
     __shared__ uint32_t fold[4][256];
     __shared__ uint32_t parts[CRC_NT / 32];
-    for (int i = threadIdx.x; i < 1024; i += CRC_NT) fold[i >> 8][i & 255] = gf_mul((uint32_t)(i & 255) << (8 * (i >> 8)), kCrcLane.x1024);
+    init_crc_fold(fold);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t* per_job = reinterpret_cast<uint32_t*>(ws + WS_HEAD);
@@ -1398,10 +1360,7 @@ __global__ void __launch_bounds__(CRC_NT)
                     else crc_rows<false>(v, w, r0);
                 }
             }
-#pragma unroll
-            for (int i = 0; i < 32; i++)
-                c = fold[0][c & 255] ^ fold[1][(c >> 8) & 255] ^ fold[2][(c >> 16) & 255] ^ fold[3][c >> 24] ^ v[i];
-            c = __reduce_xor_sync(FULL, gf_mul(c, kCrcLane.k[lane]));
+            c = crc_fold_rows(fold, v);
             if (W > 1 && i1 < iters) c = gf_mul(c, xpow_from(kCrc.x2n, 32768ull * (unsigned long long)(iters - i1)));
         }
         if (W > 1) {

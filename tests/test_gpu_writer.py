@@ -213,6 +213,43 @@ def test_streams_equal_the_host_model_byte_for_byte(tmp_path, host_model, level)
         assert got[a : a + b] == want[i], (i, off[i], size[i])
 
 
+@pytest.mark.parametrize("level", [1, 2])
+def test_streams_equal_the_host_model_at_the_edges_of_the_parse(tmp_path, host_model, level):
+    """Spans that end around the parse's units (32, 128, 512 and 2,048 positions) and the CRC's (4 and 4,096
+    bytes), at every alignment, of matches that end around what is compared at once (20 and 128 bytes more)
+    and at the longest length, in the reach of a warp and out of it."""
+    import struct
+    import subprocess
+
+    from cubam_b200.bgzf import _bgzf_compress, _deflate_spans
+
+    rng = np.random.default_rng(11)
+    noise = rng.integers(0, 256, 40_000, dtype=np.uint8).tobytes()
+    parts, at = [], 0
+    for d in (1, 2, 7, 31, 33, 600, 3000):  # a piece of noise of d bytes, then matches of it that it breaks off
+        for n in (4, 5, 19, 20, 21, 22, 147, 148, 149, 257, 258, 259, 600):
+            piece = noise[at % 30_000 : at % 30_000 + d]
+            at += d + 13
+            parts.append(piece + (piece * (n // d + 1))[:n] + noise[at % 30_000 : at % 30_000 + 3])
+    raw = b"".join(parts)
+    sizes = [m + k for m in (4, 32, 128, 512, 2048, 4096, 6144) for k in (-1, 0, 1, 5)] + [2, len(raw) // 2, len(raw)]
+    off = [int(rng.integers(0, len(raw) - n + 1)) for n in sizes]
+    (tmp_path / "in").write_bytes(raw)
+    np.stack([np.array(off, np.int64), np.array(sizes, np.int64)], 1).tofile(tmp_path / "spans")
+    subprocess.run([str(host_model), str(tmp_path / "in"), str(tmp_path / "spans"), str(level), str(tmp_path / "out")],
+                   check=True)
+    blob, p = (tmp_path / "out").read_bytes(), 0
+    out, oo, osz = _deflate_spans(dev(raw), off, sizes, level)
+    got = out.cpu().numpy().tobytes()
+    for i, (a, b) in enumerate(zip(oo.cpu().tolist(), osz.cpu().tolist(), strict=True)):
+        n = struct.unpack_from("<I", blob, p)[0]
+        assert got[a : a + b] == blob[p + 4 : p + 4 + n], (i, off[i], sizes[i])
+        p += 4 + n
+    assert p == len(blob)
+    blocks = _bgzf_compress(dev(raw), level, block_off=off, block_size=sizes).cpu().numpy().tobytes()
+    assert gzip.decompress(blocks) == b"".join(raw[a : a + n] for a, n in zip(off, sizes, strict=True))  # and the CRC32s
+
+
 def test_writer_flush_ends_blocks_and_failures_are_raised(tmp_path, monkeypatch):
     """flush() ends a block early (the oracle's block sizes); a write that fails in the writer thread is
     raised by the owner's next call."""
