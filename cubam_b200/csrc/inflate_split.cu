@@ -24,7 +24,7 @@
 // warps per SM by shared memory); with few, the chain of steps of one lane and of rounds of one member,
 // which is why a member takes more warps then.  Measured, in ms (one serial decoder per member, in one
 // kernel, before; a warp per member in between):
-//   39 GEX members (10,000 records)      decode 0.21 (0.46), copy 0.16 (0.43), CRC32 0.02; one kernel 4.2
+//   39 GEX members (10,000 records)      decode 0.17 (0.46), copy 0.16 (0.43), CRC32 0.02; one kernel 4.2
 //   about 70,000 (18 million records)    decode 12.6, copy 17.6, CRC32 2.5; all of it 47 with a member per lane
 //
 // Every loop is bounded: a decode step consumes input bits, bounded per member, a repair round
@@ -890,7 +890,7 @@ __device__ uint32_t decode_member(DecMember<W>& M, const cb_member_job& job, uin
 }
 
 template <int W>
-__global__ void __launch_bounds__(W == 1 ? 64 : W * 32, W == 1 ? 9 : 1)
+__global__ void __launch_bounds__(W == 1 ? 64 : W * 32, W == 1 ? 9 : 16 / W)
     k_decode(const cb_member_job* __restrict__ jobs, int64_t n_jobs, const int64_t* __restrict__ d_n_jobs,
              uint8_t* out_base, uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws, uint8_t* arena,
              unsigned long long arena_bytes, bool list_unfit, long long j0, long long j1, int qi) {
@@ -1455,41 +1455,49 @@ unsigned grid_for(const Call& c, Range r, int occ, int members) {
     return (unsigned)(grid < 1 ? 1 : grid);
 }
 
-// Warps per member: one member's serial work bounds a call of few, so each takes more warps while all of
-// them stay resident (28 warps per SM).
-int warps_per_member(const Call& c) {
-    const long long room = (long long)cb_device_sm_count() * 28;
-    return c.n_jobs * 8 <= room ? 8 : c.n_jobs * 4 <= room ? 4 : c.n_jobs * 2 <= room ? 2 : 1;
+// Each kernel takes as many warps per member as keep all members resident at once: one member's serial work
+// bounds a call of few, and a second round of members doubles it.  Decode and copy, in us, of 39 / 386 / 773 /
+// 1545 / 3090 GEX members: 8 warps 171 333 518 987 1835 and 161 339 531 1022 1893; 4 warps 193 218 393 607 1135
+// and 226 249 477 743 1266; 2 warps 255 283 306 536 837 and 343 367 394 760 1170; 1 warp 402 423 455 491 880
+// and 535 559 591 630 861.
+template <int W>
+int decode_occupancy() {
+    static int cache[MAX_DEVICES];
+    constexpr int MEMBERS = W == 1 ? 2 : 1;
+    return occupancy(cache, split::k_decode<W>, 32 * W * MEMBERS, MEMBERS * sizeof(split::DecMember<W>));
 }
+template <class C>
+int copy_occupancy() {
+    static int cache[MAX_DEVICES];
+    static_assert(sizeof(typename C::Smem) < 65536, "a source's offset has 16 bits");
+    return occupancy(cache, split::k_copy<C>, C::T, sizeof(typename C::Smem));
+}
+bool resident(const Call& c, int occ) { return c.n_jobs <= (long long)cb_device_sm_count() * occ; }
 
 template <int W>
 int launch_decode(const Call& c, Range r, cudaStream_t s) {
-    static int cache[MAX_DEVICES];
     constexpr int MEMBERS = W == 1 ? 2 : 1, NT = 32 * W * MEMBERS;
-    const size_t smem = MEMBERS * sizeof(split::DecMember<W>);
-    const int o = occupancy(cache, split::k_decode<W>, NT, smem);
+    const int o = decode_occupancy<W>();
     if (o <= 0) return fail_occ(o);
-    split::k_decode<W><<<grid_for(c, r, o, MEMBERS), NT, smem, s>>>(c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status,
-                                                                    c.summary, c.ws, c.arena, c.arena_bytes,
-                                                                    c.list_unfit, r.j0, r.j1, r.qd);
+    split::k_decode<W><<<grid_for(c, r, o, MEMBERS), NT, MEMBERS * sizeof(split::DecMember<W>), s>>>(
+        c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status, c.summary, c.ws, c.arena, c.arena_bytes, c.list_unfit,
+        r.j0, r.j1, r.qd);
     return CB_OK;
 }
 
 int decode_range(const Call& c, Range r, cudaStream_t s) {
-    const int w = warps_per_member(c);
-    return w == 8 ? launch_decode<8>(c, r, s) : w == 4 ? launch_decode<4>(c, r, s) : w == 2 ? launch_decode<2>(c, r, s)
-                                                                                          : launch_decode<1>(c, r, s);
+    return resident(c, decode_occupancy<8>())   ? launch_decode<8>(c, r, s)
+           : resident(c, decode_occupancy<4>()) ? launch_decode<4>(c, r, s)
+           : resident(c, decode_occupancy<2>()) ? launch_decode<2>(c, r, s)
+                                                : launch_decode<1>(c, r, s);
 }
 
 template <class C>
 int launch_copy(const Call& c, Range r, cudaStream_t s) {
-    static int cache[MAX_DEVICES];
-    static_assert(sizeof(typename C::Smem) < 65536, "a source's offset has 16 bits");
-    const size_t smem = sizeof(typename C::Smem);
-    const int o = occupancy(cache, split::k_copy<C>, C::T, smem);
+    const int o = copy_occupancy<C>();
     if (o <= 0) return fail_occ(o);
-    split::k_copy<C><<<grid_for(c, r, o, 1), C::T, smem, s>>>(c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status,
-                                                              c.summary, c.ws, c.arena, r.j0, r.j1, r.qd + 1);
+    split::k_copy<C><<<grid_for(c, r, o, 1), C::T, sizeof(typename C::Smem), s>>>(
+        c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status, c.summary, c.ws, c.arena, r.j0, r.j1, r.qd + 1);
     return CB_OK;
 }
 
@@ -1504,19 +1512,24 @@ int launch_crc(const Call& c, Range r, cudaStream_t s) {
 }
 
 int copy_range(const Call& c, Range r, cudaStream_t s) {
-    const int w = warps_per_member(c);
+    using C8 = split::CopyCfg<16384, 8>;
+    using C4 = split::CopyCfg<16384, 4>;
+    using C2 = split::CopyCfg<8192, 2>;
     const int cw = (int)cb_param(CB_PARAM_COPY_WARPS);
     int rc;
-    if (w == 8) rc = launch_copy<split::CopyCfg<16384, 8>>(c, r, s);
-    else if (w == 4) rc = launch_copy<split::CopyCfg<16384, 4>>(c, r, s);
-    else if (w == 2) rc = launch_copy<split::CopyCfg<8192, 2>>(c, r, s);
+    if (resident(c, copy_occupancy<C8>())) rc = launch_copy<C8>(c, r, s);
+    else if (resident(c, copy_occupancy<C4>())) rc = launch_copy<C4>(c, r, s);
+    else if (resident(c, copy_occupancy<C2>())) rc = launch_copy<C2>(c, r, s);
     // 4 KB: 28 warps per SM, 4.04 ms on 15,456 GEX members, 8 KB 16 warps and 4.39 ms
     else if (cw == 12) rc = launch_copy<split::CopyCfg<4096, 1>>(c, r, s);
     else if (cw == 24) rc = launch_copy<split::CopyCfg<8192, 1>>(c, r, s);
     else rc = launch_copy<split::CopyCfg<16384, 1>>(c, r, s);
     if (rc != CB_OK || !c.check_crc) return rc;
-    return w == 8 ? launch_crc<8>(c, r, s) : w == 4 ? launch_crc<4>(c, r, s) : w == 2 ? launch_crc<2>(c, r, s)
-                                                                                      : launch_crc<1>(c, r, s);
+    const long long room = (long long)cb_device_sm_count() * 28;  // warps
+    return c.n_jobs * 8 <= room   ? launch_crc<8>(c, r, s)
+           : c.n_jobs * 4 <= room ? launch_crc<4>(c, r, s)
+           : c.n_jobs * 2 <= room ? launch_crc<2>(c, r, s)
+                                  : launch_crc<1>(c, r, s);
 }
 
 // Two side streams per device for the pipelined form, and the events that join them to the caller's
