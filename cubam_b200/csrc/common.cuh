@@ -18,9 +18,15 @@ constexpr unsigned FULL = 0xffffffffu;
 __device__ __forceinline__ uint32_t ld_u16(const uint8_t* b, long long o) {
     return (uint32_t)b[o] | ((uint32_t)b[o + 1] << 8);
 }
-__device__ __forceinline__ uint32_t ld_u32(const uint8_t* b, long long o) {
-    return (uint32_t)b[o] | ((uint32_t)b[o + 1] << 8) | ((uint32_t)b[o + 2] << 16) | ((uint32_t)b[o + 3] << 24);
+// The first 4 bytes (or left, if fewer; the others are undefined) at p, from the aligned words that hold one of
+// them (two loads where bytes took four).
+__device__ __forceinline__ uint32_t ld_bytes4(const uint8_t* p, uint32_t left) {
+    const uint32_t k = (uint32_t)(uintptr_t)p & 3u;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(p - k);
+    const uint32_t lo = w[0], hi = k + left > 4 && k ? w[1] : 0u;
+    return __funnelshift_r(lo, hi, 8 * k);
 }
+__device__ __forceinline__ uint32_t ld_u32(const uint8_t* b, long long o) { return ld_bytes4(b + o, 4); }
 
 // Bytes of device data read straight from global memory (the accessor form of ld_u16 / ld_u32).
 struct GlobalBytes {

@@ -262,16 +262,27 @@ __global__ void __launch_bounds__(RW * 32) k_records(const uint8_t* __restrict__
     }
 }
 
+// The FNV-1a hash of l bytes at p (src/cubam/_kernels.py:391-403), eight bytes per round, the next round's loaded
+// ahead of the multiplications.
+__device__ __forceinline__ unsigned long long fnv1a(const uint8_t* p, uint32_t l) {
+    unsigned long long x = FNV_OFFSET;
+    uint32_t n0 = l ? ld_bytes4(p, l) : 0u, n1 = l > 4 ? ld_bytes4(p + 4, l - 4) : 0u;
+    for (uint32_t k = 0; k < l; k += 8) {
+        const uint32_t w0 = n0, w1 = n1;
+        n0 = l > k + 8 ? ld_bytes4(p + k + 8, l - k - 8) : 0u;
+        n1 = l > k + 12 ? ld_bytes4(p + k + 12, l - k - 12) : 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < 8; j++)
+            if (k + j < l) x = (x ^ ((j < 4 ? w0 : w1) >> (8 * (j & 3)) & 255u)) * FNV_PRIME;
+    }
+    return x;
+}
+
 __global__ void k_name_hash(const uint8_t* __restrict__ b, const int64_t* __restrict__ off, long long n, uint64_t* h) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const long long o = off[i];
         const uint32_t lrn = b[o + 12];
-        unsigned long long x = FNV_OFFSET;
-        for (uint32_t k = 0; k + 1 < lrn; k++) {
-            x ^= b[o + 36 + k];
-            x *= FNV_PRIME;
-        }
-        h[i] = x;
+        h[i] = fnv1a(b + o + 36, lrn ? lrn - 1 : 0u);
     }
 }
 
@@ -279,43 +290,43 @@ __global__ void k_hash_spans(const uint8_t* __restrict__ b, const int64_t* __res
                              const int32_t* __restrict__ vlen, long long n, uint64_t* out) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const int l = vlen[i];
-        if (l < 0) {
-            out[i] = 0;
-            continue;
-        }
-        unsigned long long x = FNV_OFFSET;
-        const long long o = voff[i];
-        for (int k = 0; k < l; k++) {
-            x ^= b[o + k];
-            x *= FNV_PRIME;
-        }
-        out[i] = x;
+        out[i] = l < 0 ? 0ull : fnv1a(b + voff[i], (uint32_t)l);
     }
 }
 
 __global__ void k_pack_acgt(const uint8_t* __restrict__ b, const int64_t* __restrict__ voff,
                             const int32_t* __restrict__ vlen, long long n, uint64_t* out, uint8_t* ok) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        long long k = voff[i];
-        const long long e = voff[i] + vlen[i];
+        // by words of the span: 1 million of 18 bytes 39 us, 59 by bytes
+        const uint8_t* p = b + voff[i];
+        const int l = vlen[i];
+        uint32_t w = 0;
+        auto at = [&](int q) {  // byte q, asked for in order
+            if ((q & 3) == 0) w = ld_bytes4(p + q, (uint32_t)(l - q));
+            return w >> (8 * (q & 3)) & 255u;
+        };
         unsigned long long code = 0, suffix = 0;
         uint32_t nb = 0;
-        bool good = vlen[i] > 0;
-        for (; good && k < e && b[k] != '-'; k++) {
-            const uint8_t c = b[k];
-            const uint32_t x = c == 'A' ? 0 : c == 'C' ? 1 : c == 'G' ? 2 : c == 'T' ? 3 : 4;
-            if (x == 4 || nb == 24) good = false;
+        bool good = l > 0;
+        int k = 0;
+        for (; good && k < l; k++) {
+            const uint32_t c = at(k);
+            if (c == '-') break;
+            const bool base = c - 'A' < 20u && (0x80045u >> (c - 'A') & 1u);  // A C G T
+            const uint32_t x = (c >> 1 & 3u) ^ (c >> 2 & 1u);                 // 0 1 2 3
+            if (!base || nb == 24) good = false;
             else code |= (unsigned long long)x << (2 * nb++);
         }
-        if (good && k < e) {
+        if (good && k < l) {
             k++;
             uint32_t nd = 0;
-            for (; k < e; k++, nd++) {
-                if (b[k] < '0' || b[k] > '9' || nd == 3) {
+            for (; k < l; k++, nd++) {
+                const uint32_t c = at(k);
+                if (c - '0' > 9u || nd == 3) {
                     good = false;
                     break;
                 }
-                suffix = suffix * 10 + (b[k] - '0');
+                suffix = suffix * 10 + (c - '0');
             }
             if (nd == 0) good = false;
             suffix += 1;
@@ -435,27 +446,53 @@ __global__ void k_base_at(const uint8_t* __restrict__ b, const int64_t* __restri
     }
 }
 
-// One warp per span; 16-byte copies when source and destination share their alignment.
-__global__ void k_copy_spans(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
-                             const int64_t* __restrict__ src_off, const int64_t* __restrict__ dst_off,
-                             const int64_t* __restrict__ size, long long n) {
-    const int lane = threadIdx.x & 31;
-    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n;
-         w += ((long long)gridDim.x * blockDim.x) >> 5) {
-        const uint8_t* s = src + src_off[w];
-        uint8_t* d = dst + dst_off[w];
-        const long long len = size[w];
-        long long i = 0;
-        if (((uintptr_t)s & 15) == ((uintptr_t)d & 15) && len >= 64) {
-            const long long head = (16 - ((uintptr_t)s & 15)) & 15;
-            for (long long k = lane; k < head; k += 32) d[k] = s[k];
-            const long long nv = (len - head) >> 4;
-            const uint4* sv = reinterpret_cast<const uint4*>(s + head);
-            uint4* dv = reinterpret_cast<uint4*>(d + head);
-            for (long long k = lane; k < nv; k += 32) dv[k] = sv[k];
-            i = head + nv * 16;
+// The 4-byte words of a destination span of len bytes at d (those that hold one of its bytes), from s, by
+// LANES lanes of which this is number l.  Source words are read when they hold a byte of the span.
+template <uint32_t LANES>
+__device__ __forceinline__ void copy_words(const uint8_t* s, uint8_t* d, long long len, uint32_t l) {
+    constexpr int U = 4;  // words in flight per lane
+    const uint32_t k = (uint32_t)(uintptr_t)d & 3u;
+    for (long long q0 = 4LL * l - k; q0 < len; q0 += 4 * LANES * U) {  // the word's place in the span
+        uint32_t x[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const long long q = q0 + 4LL * LANES * u;
+            x[u] = q >= len ? 0u : q >= 0 ? ld_bytes4(s + q, (uint32_t)min(len - q, 4LL)) : ld_bytes4(s, (uint32_t)min(len, 4LL)) << (8 * k);
         }
-        for (long long k = i + lane; k < len; k += 32) d[k] = s[k];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const long long q = q0 + 4LL * LANES * u;
+            if (q >= len) break;
+            if (q >= 0 && q + 4 <= len) {
+                *reinterpret_cast<uint32_t*>(d + q) = x[u];
+            } else {
+#pragma unroll
+                for (int t = 0; t < 4; t++)
+                    if (q + t >= 0 && q + t < len) d[q + t] = (uint8_t)(x[u] >> (8 * t));
+            }
+        }
+    }
+}
+
+// Spans by words of the destination, four lanes each; a warp takes its eight spans one by one when one of them
+// is longer than 512 bytes.  What bounds it is the
+// latency of the offsets and then the bytes: 1 million spans of 10 to 40 bytes, 300 apart: 50 us (81 with eight lanes
+// and one word in flight per lane, 145 with a warp per span and a byte per lane).
+__global__ void __launch_bounds__(256) k_copy_spans(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
+                                                    const int64_t* __restrict__ src_off,
+                                                    const int64_t* __restrict__ dst_off,
+                                                    const int64_t* __restrict__ size, long long n) {
+    const uint32_t lane = threadIdx.x & 31, l = lane & 3;
+    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; 8 * w < n;
+         w += ((long long)gridDim.x * blockDim.x) >> 5) {
+        const long long i = 8 * w + (lane >> 2);
+        const long long len = i < n ? size[i] : 0;
+        if (__any_sync(FULL, len > 512)) {
+            for (long long j = 8 * w; j < 8 * w + 8 && j < n; j++)
+                copy_words<32>(src + src_off[j], dst + dst_off[j], size[j], lane);
+        } else if (len > 0) {
+            copy_words<4>(src + src_off[i], dst + dst_off[i], len, l);
+        }
     }
 }
 
@@ -608,7 +645,7 @@ extern "C" int cb_copy_spans(const uint8_t* src, uint8_t* dst, const int64_t* sr
                              const int64_t* size, int64_t n, void* stream) {
     if (n < 0) return CB_ERR_ARG;
     if (n == 0) return CB_OK;
-    rec::k_copy_spans<<<grid_for(n * 32, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(src, dst, src_off,
+    rec::k_copy_spans<<<grid_for(n * 4, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(src, dst, src_off,
                                                                                                   dst_off, size, n);
     return cb_set_error(cudaGetLastError());
 }
