@@ -24,8 +24,8 @@
 // warps per SM by shared memory); with few, the chain of steps of one lane and of rounds of one member,
 // which is why a member takes more warps then.  Measured, in ms (one serial decoder per member, in one
 // kernel, before; a warp per member in between):
-//   39 GEX members (10,000 records)      decode 0.17 (0.46), copy 0.16 (0.43), CRC32 0.02; one kernel 4.2
-//   about 70,000 (18 million records)    decode 12.6, copy 17.6, CRC32 2.5; all of it 47 with a member per lane
+//   39 GEX members (10,000 records)      decode 0.17 (0.46), copy 0.15 (0.43), CRC32 0.01; one kernel 4.2
+//   about 70,000 (18 million records)    decode 12.6, copy 16.7, CRC32 2.1; all of it 47 with a member per lane
 //
 // Every loop is bounded: a decode step consumes input bits, bounded per member, a repair round
 // confirms at least one more segment; every shared-memory index is masked or checked; arena and
@@ -75,7 +75,8 @@ __constant__ uint8_t kClOrder[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12
 constexpr size_t WS_HEAD = 256;
 constexpr size_t PER_JOB = 32;
 constexpr int JW = PER_JOB / 4;           // words per job
-constexpr int Q_LISTED = 6;               // queue counter: members for the one-kernel form
+constexpr int PARTS = 2;                  // ranges of jobs of the pipelined form, each with two queue counters
+constexpr int Q_LISTED = 2 * PARTS;       // queue counter: members for the one-kernel form (and its queue)
 constexpr uint32_t ST_LISTED = 0x100;     // internal status: on that list
 __host__ __device__ __forceinline__ size_t arena_offset(long long n_jobs) {
     return (WS_HEAD + PER_JOB * (size_t)n_jobs + 255) & ~(size_t)255;
@@ -931,6 +932,16 @@ constexpr uint32_t LINE = 128;            // output bytes of a warp's round: a w
 constexpr uint32_t FAR_N = 32;            // sources fetched from HBM per warp and group, of up to FAR_LEN bytes each
 constexpr uint32_t FAR_WORDS = 8, FAR_LEN = 4 * FAR_WORDS - 3;
 
+// A group's tokens are the literal runs and matches of its sequences, numbered 4 t + 1 to 4 t + 4 for thread
+// t's two (so numbers rise along the output).  tok: above bit 16 what to add to a byte's place (from the
+// group's first line) to get its source's offset from the ring's start in shared memory; T_NEAR: a match
+// closer than a round, some of whose bytes may have their source in the same round, with its distance in
+// bits 0-11 (all ones in other tokens: far from any round).  The few tokens with T_WRAP (a source across the
+// ring's end) or T_DIRECT (one read from HBM: a literal with T_PLAIN) find it through aux: the distance above
+// bit 16 and the start, or for T_PLAIN what to add to get a literal's place in the slot.
+constexpr uint32_t T_WRAP = 1u << 12, T_DIRECT = 1u << 13, T_PLAIN = 1u << 14, T_NEAR = 1u << 15, T_FAR = 0xFFFu;
+constexpr uint32_t T_FLAGS = T_NEAR | T_WRAP | T_DIRECT;
+
 // RING_: bytes of output kept in shared memory: sources up to RING_ - GMAX - SPAN bytes back read it, older
 // ones the output already stored.
 template <uint32_t RING_, int W_>
@@ -942,7 +953,7 @@ struct CopyCfg {
     static constexpr uint32_t LITS = 256 * W_;    // literals of a group held in shared memory
     static_assert((RING_ & (RING_ - 1)) == 0 && RING_ >= GMAX + 2 * SPAN + 512 && RING_ <= 16384, "ring size");
     static_assert(GMAX >= 2 * (255 + 258), "two sequences fit a group");
-    static_assert(SPAN <= 1024 && 4 * T < 65536, "a token's number and a near distance have their bits");
+    static_assert(2 * SPAN < T_FAR && 4 * T < 65536, "a token's number and a near distance have their bits");
     using Id = typename std::conditional<W_ == 1, uint8_t, uint16_t>::type;
     struct alignas(16) Smem {
         uint8_t ring[RING_];
@@ -957,15 +968,6 @@ struct CopyCfg {
         uint32_t count[W_];
     };
 };
-
-// A group's tokens are the literal runs and matches of its sequences, numbered 4 t + 1 to 4 t + 4 for thread
-// t's two.  tok: in 16 bits what to add to a byte's place (from the group's first line) to get its source's
-// offset from the ring's start in shared memory; T_NEAR: a match closer than a round (its distance from bit
-// 20), some of whose bytes may have their source in the same round.  The few tokens with T_WRAP (a source
-// across the ring's end) or T_DIRECT (one read from HBM: a literal with T_PLAIN) find it through aux: the
-// distance above bit 16 and the start, or for T_PLAIN what to add to get a literal's place in the slot.
-constexpr uint32_t T_NEAR = 1u << 16, T_WRAP = 1u << 17, T_DIRECT = 1u << 18, T_PLAIN = 1u << 19;
-constexpr uint32_t T_FLAGS = T_NEAR | T_WRAP | T_DIRECT;
 
 // All ones, shifted left by n (0 from 32 on).
 __device__ __forceinline__ uint32_t shl_clamp(uint32_t n) { return __funnelshift_lc(0u, 0xFFFFFFFFu, n); }
@@ -1000,7 +1002,7 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
     };
     auto any = [&](bool x) { return W == 1 ? __any_sync(FULL, x) != 0 : __syncthreads_or(x) != 0; };
     for (uint32_t i = tid; i < C::GMAX + C::SPAN; i += T) M.map[i] = 0;
-    if (tid == 0) M.tok[0] = 0;  // bytes before the group's first
+    if (tid == 0) M.tok[0] = T_FAR;  // bytes before the group's first
 
     for (;;) {
         if (tid == 0) M.job = atomicAdd(queue, 1ull);
@@ -1136,15 +1138,15 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
                 auto literals = [&](uint32_t id, uint32_t start, uint32_t c, uint32_t l) {
                     place(id, start, c);
                     const bool held = l + c <= C::LITS;
-                    M.tok[id] = (((held ? LIT_AT + l : 0u) - start) & 0xFFFFu) | (held ? 0u : T_DIRECT | T_PLAIN);
+                    M.tok[id] = (((held ? LIT_AT + l : 0u) - start) << 16) | (held ? T_FAR : T_FAR | T_DIRECT | T_PLAIN);
                     M.aux[id] = lit0 + l - start;
                 };
                 auto match = [&](uint32_t id, uint32_t start, uint32_t len, uint32_t d, uint32_t x, bool is_old, uint32_t f) {
                     place(id, start, len);
                     const uint32_t at = x & C::RMASK;
                     const bool held = is_old ? f < FAR_N : at + len <= C::RING;
-                    M.tok[id] = (((!held ? 0u : is_old ? FAR_AT + 36 * f + (x & 3u) : at) - start) & 0xFFFFu) |
-                                (!held ? (is_old ? T_DIRECT : T_WRAP) : d < C::SPAN ? T_NEAR | (d << 20) : 0u);
+                    M.tok[id] = (((!held ? 0u : is_old ? FAR_AT + 36 * f + (x & 3u) : at) - start) << 16) |
+                                (!held ? (is_old ? T_FAR | T_DIRECT : T_FAR | T_WRAP) : d < C::SPAN ? T_NEAR | d : T_FAR);
                     M.aux[id] = start | (d << 16);
                 };
                 if (c0) literals(4 * tid + 1, b0, c0, l0);
@@ -1176,20 +1178,20 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
                 }
                 // the token of the byte before the word: the last one that starts in a lane below, else the
                 // line's first (W > 1) or the last of the line before
-                const uint32_t mlast = m[3] ? m[3] : m[2] ? m[2] : m[1] ? m[1] : m[0];
+                const uint32_t mlast = max(max(m[0], m[1]), max(m[2], m[3]));
                 const uint32_t below = __ballot_sync(FULL, mlast != 0) & lt;
                 uint32_t id = __shfl_sync(FULL, mlast, below ? 31 - __clz((int)below) : 0);
                 if (!below) id = carry;
                 uint32_t ids[4], tk[4], v[4];
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
-                    id = m[k] ? m[k] : id;
+                    id = max(id, m[k]);
                     ids[k] = id;
                     tk[k] = M.tok[id];
-                    v[k] = smem[(rel + k + tk[k]) & 0xFFFFu];
+                    v[k] = W == 1 ? smem[(int)(rel + k) + ((int)tk[k] >> 16)] : smem[(rel + k + (tk[k] >> 16)) & 0xFFFFu];
                 }
                 if (W == 1) carry = __shfl_sync(FULL, id, 31);
-                uint32_t word = v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24);
+                uint32_t word = __byte_perm(__byte_perm(v[0], v[1], 0x40), __byte_perm(v[2], v[3], 0x40), 0x5410);
                 if (rr == 0 && rel < p0) {  // bytes before the group's first are there already
                     const uint32_t mine = shl_clamp(8 * (p0 - rel));
                     word = (word & mine) | (ring4[(w & C::RMASK) >> 2] & ~mine);
@@ -1200,7 +1202,8 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
                 if (__any_sync(FULL, left > 0 && (fl & T_FLAGS))) {
 #pragma unroll
                     for (int k = 0; k < 4; k++)
-                        if ((tk[k] & T_NEAR) && k < left && (int)(rel + k - (tk[k] >> 20)) >= fresh) pend |= 1u << k;
+                        if ((int)(rel + k - (tk[k] & T_FAR)) >= fresh) pend |= 1u << k;
+                    pend &= ~shl_clamp((uint32_t)max(left, 0));
                     if (__any_sync(FULL, left > 0 && (fl & (T_WRAP | T_DIRECT)))) {
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
@@ -1225,7 +1228,10 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
                             const uint32_t ax = M.aux[ids[k]], d = ax >> 16;
                             const int start = (int)(ax & 0xFFFFu);
                             px[k] = (int)(rel + k - d);
-                            if (px[k] >= start) px[k] = start - (int)d + (int)((uint32_t)(px[k] - start) % d);
+                            if (px[k] >= start) {  // (the quotient of small numbers; half keeps it off the integers)
+                                const int n = px[k] - start;
+                                px[k] = start - (int)d + n - (int)d * (int)__fdividef((float)n + 0.5f, (float)d);
+                            }
                         }
                     }
                     if (W > 1) {
@@ -1281,20 +1287,32 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
 }
 
 // ---------------------------------------------------------------- k_crc: one member per W warps
-// The rows of crc.cuh, in registers.  (Tables for every byte took a shared-memory access with conflicts per byte.)
+// The rows of crc.cuh, in registers, eight at a time with the next eight being loaded.  What bounds it is the
+// latency of memory: 4.5 GB of output 2.06 ms (2.42 without the load ahead; 39 members 12.5 us, 20.8).  (Tables for
+// every byte took a shared-memory access with conflicts per byte.)
 
 constexpr int CRC_NT = 256;
 
-// The word of the message at byte position q (negative positions are zero bytes); with INV the first
-// four bytes are inverted (the CRC's initial value).
-__device__ __forceinline__ uint32_t crc_word_careful(const uint8_t* m, long long q, bool inv) {
-    uint32_t x = 0;
+// Eight rows (128 bytes each) of a message of len bytes, whose lane's first word is at byte q (negative
+// positions are zero bytes): as words of the message where the rows reach its first four bytes, which are
+// inverted (the CRC's initial value), else as the aligned words with x the one after the last row's (lane 0's).
+__device__ __forceinline__ void crc_load(const uint8_t* m, uint32_t len, long long q, bool head, uint32_t (&w)[8], uint32_t& x) {
+    if (head) {
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-        const long long r = q + t;
-        if (r >= 0) x |= ((uint32_t)m[r] ^ (inv && r < 4 ? 0xFFu : 0u)) << (8 * t);
+        for (int i = 0; i < 8; i++) {
+            const int p = (int)(q + 128 * i), at = max(p, 0);
+            uint32_t y = p > -4 ? ld_bytes4(m + at, len - (uint32_t)at) : 0u;
+            if (p < 0) y = p > -4 ? y << (-8 * p) : 0u;
+            if (len >= 4 && p < 4 && p > -4) y ^= p < 0 ? FULL << (-8 * p) : FULL >> (8 * p);
+            w[i] = y;
+        }
+    } else {
+        const uintptr_t ad = (uintptr_t)(m + q);
+        const uint32_t* wp = reinterpret_cast<const uint32_t*>(ad & ~(uintptr_t)3);
+#pragma unroll
+        for (int i = 0; i < 8; i++) w[i] = __ldg(wp + 32 * i);
+        x = (ad & 3) && (threadIdx.x & 31) == 0 ? __ldg(wp + 256) : 0u;
     }
-    return x;
 }
 
 // W warps per member, each a part of its 4,096-byte steps; parts are joined by x^(8 bytes after).
@@ -1323,41 +1341,35 @@ __global__ void __launch_bounds__(CRC_NT)
             const uint8_t* m = out_base + job.out_off;
             len = job.isize;
             want = job.crc;
-            const bool inv = len >= 4;
             const long long pad = (long long)((4096u - (len & 4095u)) & 4095u);
             const long long iters = ((long long)len + pad) >> 12;
             const long long i0 = iters * (warp % W) / W, i1 = iters * (warp % W + 1) / W;
             uint32_t v[32];
 #pragma unroll
             for (int i = 0; i < 32; i++) v[i] = 0;
+            const uint32_t sh = (uint32_t)((uintptr_t)(m - pad) & 3) * 8;
+            auto head = [&](long long row) { return row * 128 - pad < 4; };
+            uint32_t w[8], x = 0;
+            if (i0 < i1) crc_load(m, len, i0 * 4096 + 4 * lane - pad, head(i0 * 32), w, x);
             for (long long it = i0; it < i1; it++) {
                 const bool last = it + 1 == i1;
 #pragma unroll
                 for (int r0 = 0; r0 < 32; r0 += 8) {
-                    uint32_t w[8];
-                    const long long q0 = it * 4096 + r0 * 128 + 4 * lane - pad;
-                    if (it * 4096 - pad < 4) {  // rows with bytes before the member or its first four
+                    const long long row = it * 32 + r0, nr = row + 8;
+                    uint32_t nw[8], nx = 0;  // the next rows are loaded while these are folded
+                    if (r0 < 24 || !last) crc_load(m, len, nr * 128 + 4 * lane - pad, head(nr), nw, nx);
+                    if (sh && !head(row)) {
 #pragma unroll
-                        for (int i = 0; i < 8; i++) w[i] = crc_word_careful(m, q0 + 128 * i, inv);
-                    } else {
-                        const uintptr_t ad = (uintptr_t)(m + q0);
-                        const uint32_t* wp = reinterpret_cast<const uint32_t*>(ad & ~(uintptr_t)3);
-                        const uint32_t sh = (uint32_t)(ad & 3) * 8;
-                        if (sh) {
-                            uint32_t hi[8];
-#pragma unroll
-                            for (int i = 0; i < 8; i++) w[i] = __ldg(wp + 32 * i);
-#pragma unroll
-                            for (int i = 0; i < 8; i++) hi[i] = __ldg(wp + 32 * i + 1);
-#pragma unroll
-                            for (int i = 0; i < 8; i++) w[i] = __funnelshift_r(w[i], hi[i], sh);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 8; i++) w[i] = __ldg(wp + 32 * i);
+                        for (int i = 0; i < 8; i++) {
+                            const uint32_t hi = __shfl_sync(FULL, lane == 0 ? (i < 7 ? w[(i + 1) & 7] : x) : w[i], (lane + 1) & 31);
+                            w[i] = __funnelshift_r(w[i], hi, sh);
                         }
                     }
                     if (last) crc_rows<true>(v, w, r0);
                     else crc_rows<false>(v, w, r0);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) w[i] = nw[i];
+                    x = nx;
                 }
             }
             c = crc_fold_rows(fold, v);
@@ -1385,7 +1397,7 @@ __global__ void k_split_init(cb_inflate_summary* summary, unsigned long long* qu
     summary->reserved = 0;
     summary->n_bad = 0;
     summary->first_bad = INT64_MAX;
-    for (int q = 0; q < 8; q++) queue[q] = 0;  // decode and copy counters of up to two job ranges, the list's
+    for (int q = 0; q < Q_LISTED + 2; q++) queue[q] = 0;  // decode and copy counters of up to two job ranges, the list's
 }
 
 __global__ void k_split_finish(cb_inflate_summary* summary) {
@@ -1459,7 +1471,7 @@ unsigned grid_for(const Call& c, Range r, int occ, int members) {
 // bounds a call of few, and a second round of members doubles it.  Decode and copy, in us, of 39 / 386 / 773 /
 // 1545 / 3090 GEX members: 8 warps 171 333 518 987 1835 and 161 339 531 1022 1893; 4 warps 193 218 393 607 1135
 // and 226 249 477 743 1266; 2 warps 255 283 306 536 837 and 343 367 394 760 1170; 1 warp 402 423 455 491 880
-// and 535 559 591 630 861.
+// and 535 559 591 630 861.  (Before the copy's bytes were put together in fewer instructions: 4% less now.)
 template <int W>
 int decode_occupancy() {
     static int cache[MAX_DEVICES];
@@ -1469,7 +1481,7 @@ int decode_occupancy() {
 template <class C>
 int copy_occupancy() {
     static int cache[MAX_DEVICES];
-    static_assert(sizeof(typename C::Smem) < 65536, "a source's offset has 16 bits");
+    static_assert(sizeof(typename C::Smem) < (C::W == 1 ? 32768 : 65536), "a source's offset has 16 bits");
     return occupancy(cache, split::k_copy<C>, C::T, sizeof(typename C::Smem));
 }
 bool resident(const Call& c, int occ) { return c.n_jobs <= (long long)cb_device_sm_count() * occ; }
@@ -1587,9 +1599,11 @@ int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_
         split::k_slots<<<1, split::SLOT_NT, 0, s>>>(jobs, n_jobs, d_n_jobs, ws);
         // Pipelined: the jobs in two ranges, each decoded and then copied on its own stream, so that
         // the second range's decode and the first range's copy fill the warps that the other's end
-        // leaves idle.  Only with the job count known on the host.
+        // leaves idle: from 20 members per SM, where they take more than one round of resident warps
+        // (3,865 GEX members 2.45 ms -> 2.12, 15,457 6.95 -> 6.72; 2,320 1.358 -> 1.366; cut at three
+        // quarters 2.35 and 6.78; in four ranges 2.59 and 7.09).  Only with the job count known on the host.
         const long long pipe = cb_param(CB_PARAM_DECODE_PIPELINE);
-        const bool two = !d_n_jobs && n_jobs >= 2 && (pipe == 2 || (pipe == 1 && n_jobs >= 65536));
+        const bool two = !d_n_jobs && n_jobs >= 2 && (pipe == 2 || (pipe == 1 && n_jobs >= 20LL * cb_device_sm_count()));
         int rc = CB_OK;
         if (!two) {
             const Range all{0, n_jobs, 0};
@@ -1604,16 +1618,19 @@ int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_
             std::lock_guard<std::mutex> lock(g_side_mu);
             Side* sd = nullptr;
             if ((rc = side_for(dev, sd)) != CB_OK) return rc;
-            const long long cut = n_jobs - n_jobs / 4;  // three quarters first
-            const Range ra{0, cut, 0}, rb{cut, n_jobs, 2};
             e = cudaEventRecord(sd->start, s);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(sd->x, sd->start, 0);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(sd->y, sd->start, 0);
             if (e != cudaSuccess) return cb_set_error(e);
-            rc = decode_range(c, ra, sd->x);
-            if (rc == CB_OK) rc = decode_range(c, rb, sd->y);
-            if (rc == CB_OK) rc = copy_range(c, ra, sd->x);
-            if (rc == CB_OK) rc = copy_range(c, rb, sd->y);
+            constexpr int parts = split::PARTS;
+            for (int k = 0; k < parts && rc == CB_OK; k += 2) {
+                const Range ra{n_jobs * k / parts, n_jobs * (k + 1) / parts, 2 * k};
+                const Range rb{n_jobs * (k + 1) / parts, n_jobs * (k + 2) / parts, 2 * k + 2};
+                rc = decode_range(c, ra, sd->x);
+                if (rc == CB_OK) rc = decode_range(c, rb, sd->y);
+                if (rc == CB_OK) rc = copy_range(c, ra, sd->x);
+                if (rc == CB_OK) rc = copy_range(c, rb, sd->y);
+            }
             // join both side streams back to the caller's stream whatever happened above
             e = cudaEventRecord(sd->done_x, sd->x);
             if (e == cudaSuccess) e = cudaEventRecord(sd->done_y, sd->y);

@@ -104,7 +104,7 @@ int cb_device_sm_count(void);
  *   CB_PARAM_DECODE_PIPELINE  form 3 in two job ranges, each decoded and then copied on its own stream
  *                          (side streams joined back to the caller's by events), so that one range's
  *                          decode and the other's copy fill the lanes a decode leaves idle at its end:
- *                          0 never, 1 from 65,536 jobs, 2 always; only with the job count given on the
+ *                          0 never, 1 from 20 jobs per SM, 2 always; only with the job count given on the
  *                          host (d_n_jobs NULL).  The side streams and events are created by the first
  *                          pipelined call on a device, which should come before any stream capture (1)
  * cb_set_param(key, -1) restores the default; an unknown key or a value out of range is CB_ERR_ARG.

@@ -114,10 +114,11 @@ def test_split_matches_zlib(make, window):
         _lib.lib.cb_set_param(_lib.PARAM_COPY_WARPS, -1)
 
 
-@pytest.mark.parametrize("jobs,window", [(400, -1), (600, -1), (1100, -1), (2100, 6), (2100, 12), (2100, 24)])
+@pytest.mark.parametrize("jobs,window", [(400, -1), (600, -1), (1100, -1), (2100, 6), (2100, 12), (2100, 24), (3100, 12)])
 @pytest.mark.parametrize("make", [_edges, _distances, _blocks], ids=["edges", "distances", "blocks"])
 def test_split_matches_zlib_at_every_width(make, jobs, window):
-    """The same members many times over: members take 4, 2 and 1 warps as the calls hold more of them."""
+    """The same members many times over: members take 4, 2 and 1 warps as the calls hold more
+    of them, and then go in two ranges."""
     cases = make()
     times = -(-jobs // len(cases))
     buf, table, total = _table(cases, 3)
