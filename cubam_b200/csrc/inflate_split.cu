@@ -25,7 +25,7 @@
 // which is why a member takes more warps then.  Measured, in ms (one serial decoder per member, in one
 // kernel, before; a warp per member in between):
 //   39 GEX members (10,000 records)      decode 0.17 (0.46), copy 0.15 (0.43), CRC32 0.01; one kernel 4.2
-//   about 70,000 (18 million records)    decode 12.6, copy 16.7, CRC32 2.1; all of it 47 with a member per lane
+//   about 70,000 (18 million records)    decode 12.6, copy 13.6, CRC32 1.9; all of it 47 with a member per lane
 //
 // Every loop is bounded: a decode step consumes input bits, bounded per member, a repair round
 // confirms at least one more segment; every shared-memory index is masked or checked; arena and
@@ -929,8 +929,7 @@ __global__ void __launch_bounds__(W == 1 ? 64 : W * 32, W == 1 ? 9 : 16 / W)
 // ---------------------------------------------------------------- k_copy: one member per CTA of W warps
 
 constexpr uint32_t LINE = 128;            // output bytes of a warp's round: a word per lane
-constexpr uint32_t FAR_N = 32;            // sources fetched from HBM per warp and group, of up to FAR_LEN bytes each
-constexpr uint32_t FAR_WORDS = 8, FAR_LEN = 4 * FAR_WORDS - 3;
+constexpr uint32_t FAR_WORDS = 8, FAR_LEN = 4 * FAR_WORDS - 3;  // of a fetched source, at most
 
 // A group's tokens are the literal runs and matches of its sequences, numbered 4 t + 1 to 4 t + 4 for thread
 // t's two (so numbers rise along the output).  tok: above bit 16 what to add to a byte's place (from the
@@ -950,6 +949,7 @@ struct CopyCfg {
     static constexpr uint32_t T = 32 * W_, RING = RING_, RMASK = RING_ - 1;
     static constexpr uint32_t SPAN = LINE * W_;   // output bytes of a round of all warps
     static constexpr uint32_t GMAX = 1152 * W_;   // output bytes of a group of 64 sequences per warp, at most
+    static constexpr uint32_t FAR_N = W_ == 8 ? 32 : 40;  // sources fetched from HBM per warp and group
     static constexpr uint32_t LITS = 256 * W_;    // literals of a group held in shared memory
     static_assert((RING_ & (RING_ - 1)) == 0 && RING_ >= GMAX + 2 * SPAN + 512 && RING_ <= 16384, "ring size");
     static_assert(GMAX >= 2 * (255 + 258), "two sequences fit a group");
@@ -958,8 +958,7 @@ struct CopyCfg {
     struct alignas(16) Smem {
         uint8_t ring[RING_];
         uint32_t lit[LITS / 4];           // the group's first literals
-        uint32_t far[W_][FAR_N * 9];      // fetched sources (and one word more each: fewer conflicts)
-        uint2 want[W_][FAR_N];            // their slots and lengths
+        uint32_t far[W_][2][FAR_N * FAR_WORDS];  // fetched sources of this group and the next
         uint32_t tok[4 * T + 4], aux[4 * T + 4];
         alignas(8) Id map[GMAX + SPAN];   // per byte of the group's lines: the number of the token that starts there
         uint16_t head[(GMAX + SPAN) / LINE + 1];  // W > 1: per line, the token of its first byte
@@ -968,6 +967,20 @@ struct CopyCfg {
         uint32_t count[W_];
     };
 };
+
+// Copy the 4 bytes at src to dst in shared memory without waiting, and wait for this thread's copies.
+__device__ __forceinline__ void copy_async4(uint32_t* dst, const uint8_t* src) {
+#ifdef __CUDA_ARCH__
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+#else
+    *dst = *reinterpret_cast<const uint32_t*>(src);
+#endif
+}
+__device__ __forceinline__ void wait_async() {
+#ifdef __CUDA_ARCH__
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+#endif
+}
 
 // All ones, shifted left by n (0 from 32 on).
 __device__ __forceinline__ uint32_t shl_clamp(uint32_t n) { return __funnelshift_lc(0u, 0xFFFFFFFFu, n); }
@@ -991,6 +1004,7 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
     uint32_t* ring4 = reinterpret_cast<uint32_t*>(M.ring);
     const uint32_t LIT_AT = (uint32_t)(reinterpret_cast<const uint8_t*>(M.lit) - smem);
     const uint32_t FAR_AT = (uint32_t)(reinterpret_cast<const uint8_t*>(M.far[warp]) - smem);
+    constexpr uint32_t NOT_OLD = 255, FAR_N = C::FAR_N;
     unsigned long long* queue = reinterpret_cast<unsigned long long*>(ws) + qi;  // this launch's counter
     uint32_t* per_job = reinterpret_cast<uint32_t*>(ws + WS_HEAD);
     long long n = n_jobs;
@@ -1020,25 +1034,32 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
         const uint32_t Eend = a + job.isize;
         uint32_t P = a, st = CB_OK;
         uint32_t g = 0, lbase = 0;  // sequences (an even number) and literals done
-        uint2 seq;
         uint32_t lw0, lw1;
-        auto load = [&]() {  // the group's sequences and first literals
-            const uint32_t i = g + 2 * tid, l = (lbase & ~3u) + 4 * tid;
-            seq = i < ns ? __ldcg(sq - (i >> 1)) : make_uint2(0, 0);
-            if (i + 1 >= ns) seq.x = 0;
+        auto load_lits = [&]() {  // the group's first literals
+            const uint32_t l = (lbase & ~3u) + 4 * tid;
             lw0 = l < nl ? __ldcg(reinterpret_cast<const uint32_t*>(lits + l)) : 0u;
             lw1 = l + 4 * T < nl ? __ldcg(reinterpret_cast<const uint32_t*>(lits + l + 4 * T)) : 0u;
         };
-        load();
-        while (g < ns) {
-            // this thread's two sequences
-            const uint32_t s0 = seq.y, s1 = seq.x;
-            uint32_t c0 = s0 >> 24, m0 = s0 & SEQ_MATCH ? ((s0 >> 16) & 255u) + 3 : 0u;
-            uint32_t c1 = s1 >> 24, m1 = s1 & SEQ_MATCH ? ((s1 >> 16) & 255u) + 3 : 0u;
+        uint2 seq;
+        auto load_seqs = [&](uint32_t from) {  // this thread's two sequences of a group
+            const uint32_t i = from + 2 * tid;
+            seq = i < ns ? __ldcg(sq - (i >> 1)) : make_uint2(0, 0);
+            if (i + 1 >= ns) seq.x = 0;
+        };
+        // The plan of the group of seq that starts at P: this thread's literals and match lengths, output bytes and
+        // literals before them and of the group, its sequences, whether it is invalid, and where sources older
+        // than the ring come to `far` (f0, f1), of which those before `done` are on their way from here on.
+        uint32_t s0, s1, c0, m0, c1, m1, eb, el, glen, glit, cnt, f0, f1, half = 0;
+        bool bad;
+        auto plan = [&](uint32_t done) {
+            s0 = seq.y;
+            s1 = seq.x;
+            c0 = s0 >> 24;
+            m0 = s0 & SEQ_MATCH ? ((s0 >> 16) & 255u) + 3 : 0u;
+            c1 = s1 >> 24;
+            m1 = s1 & SEQ_MATCH ? ((s1 >> 16) & 255u) + 3 : 0u;
             const bool none0 = (s0 & 0xFFFFu) && !m0, none1 = (s1 & 0xFFFFu) && !m1;
-            // output bytes and literals before it, and of the group
             const uint32_t vb = c0 + m0 + c1 + m1, vl = c0 + c1;
-            uint32_t eb, el, glen, glit;
             if (W == 1) {
                 uint32_t gv;
                 const uint32_t ex = warp_exclusive_scan(vb | (vl << 16), gv);
@@ -1062,7 +1083,7 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
                 glen = (uint32_t)tot;
                 glit = (uint32_t)(tot >> 32);
             }
-            uint32_t cnt = min(2 * T, ns - g);
+            cnt = min(2 * T, ns - g);
             if (glen > C::GMAX) {  // the threads whose sequences end within GMAX bytes (at least one)
                 const uint32_t mine = __popc(__ballot_sync(FULL, eb + vb <= C::GMAX));
                 uint32_t keep = mine;
@@ -1089,46 +1110,52 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
                     el = glit;
                 }
             }
-            // places from the group's first line: its start, this thread's, and after each of its parts
             const uint32_t R0 = P & ~(LINE - 1), p0 = P - R0, pe = p0 + glen;
-            const uint32_t b0 = p0 + eb, b1 = b0 + c0, b2 = b1 + m0, b3 = b2 + c1;
-            const uint32_t d0 = (s0 & 0x7FFFu) + 1, d1 = (s1 & 0x7FFFu) + 1;
-            if (any(none0 || none1 || (m0 && d0 > R0 + b1 - a) || (m1 && d1 > R0 + b3 - a)) || glen > Eend - P) {
+            const uint32_t y0 = P + eb + c0, y1 = y0 + m0 + c1;  // the matches' slots
+            const uint32_t d0 = (s0 & 0x7FFFu) + 1, d1 = (s1 & 0x7FFFu) + 1, x0 = y0 - d0, x1 = y1 - d1;
+            bad = any(none0 || none1 || (m0 && d0 > y0 - a) || (m1 && d1 > y1 - a)) || glen > Eend - P;
+            const uint32_t old = R0 + (pe + C::SPAN - 1) / C::SPAN * C::SPAN;  // the ring will hold old - RING on
+            const bool old0 = m0 && x0 + C::RING < old, old1 = m1 && x1 + C::RING < old;
+            f0 = old0 ? FAR_N : NOT_OLD;
+            f1 = old1 ? FAR_N : NOT_OLD;
+            const bool get0 = !bad && old0 && m0 <= FAR_LEN && x0 + m0 <= done;
+            const bool get1 = !bad && old1 && m1 <= FAR_LEN && x1 + m1 <= done;
+            const uint32_t any0 = __ballot_sync(FULL, get0), any1 = __ballot_sync(FULL, get1);
+            if (any0 | any1) {
+                auto fetch = [&](uint32_t f, uint32_t x, uint32_t m) {
+                    const uint32_t nw = ((x & 3u) + m + 3) >> 2;
+                    const uint8_t* q = base + (x & ~3u);
+                    uint32_t* to = M.far[warp][half] + FAR_WORDS * f;
+#pragma unroll
+                    for (uint32_t k = 0; k < FAR_WORDS; k++)
+                        if (k < nw) copy_async4(to + k, q + 4 * k);
+                };
+                if (get0) f0 = min(FAR_N, (uint32_t)__popc(any0 & lt));
+                if (get1) f1 = min(FAR_N, (uint32_t)(__popc(any0) + __popc(any1 & lt)));
+                if (f0 < FAR_N) fetch(f0, x0, m0);
+                if (f1 < FAR_N) fetch(f1, x1, m1);
+            }
+        };
+        load_seqs(0);
+        load_lits();
+        if (ns) {
+            plan(a);
+            load_seqs(cnt);
+        }
+        while (g < ns) {
+            if (bad) {
                 st = CB_ERR_INFLATE;
                 break;
             }
             M.lit[tid] = lw0;
             M.lit[tid + T] = lw1;
+            // places from the group's first line: its start, this thread's, and after each of its parts
+            const uint32_t R0 = P & ~(LINE - 1), P0 = P, p0 = P - R0, pe = p0 + glen;
+            const uint32_t b0 = p0 + eb, b1 = b0 + c0, b2 = b1 + m0, b3 = b2 + c1;
+            const uint32_t d0 = (s0 & 0x7FFFu) + 1, d1 = (s1 & 0x7FFFu) + 1;
             const uint32_t l0 = (lbase & 3u) + el, l1 = l0 + c0, lit0 = lbase & ~3u;
-            // the next group's sequences and literals are loaded while this one is written
-            g += cnt;
-            lbase += glit;
-            load();
-            // sources older than the ring will hold come to `far`
             const uint32_t x0 = R0 + b1 - d0, x1 = R0 + b3 - d1;
-            const uint32_t old = R0 + (pe + C::SPAN - 1) / C::SPAN * C::SPAN;  // slots below old - RING
-            const bool old0 = m0 && x0 + C::RING < old, old1 = m1 && x1 + C::RING < old;
-            uint32_t f0 = FAR_N, f1 = FAR_N;  // their places there
-            const uint32_t any0 = __ballot_sync(FULL, old0 && m0 <= FAR_LEN);
-            const uint32_t any1 = __ballot_sync(FULL, old1 && m1 <= FAR_LEN);
-            if (any0 | any1) {
-                const uint32_t n0 = __popc(any0);
-                if (any0 >> lane & 1u) f0 = __popc(any0 & lt);
-                if (any1 >> lane & 1u) f1 = n0 + __popc(any1 & lt);
-                if (f0 < FAR_N) M.want[warp][f0] = make_uint2(x0, m0);
-                if (f1 < FAR_N) M.want[warp][f1] = make_uint2(x1, m1);
-                __syncwarp();
-                const uint2 t = lane < n0 + __popc(any1) ? M.want[warp][lane] : make_uint2(0, 0);
-                const uint32_t nw = t.y ? ((t.x & 3u) + t.y + 3) >> 2 : 0u;
-                const uint32_t* q = reinterpret_cast<const uint32_t*>(base + (t.x & ~3u));
-                uint32_t* f = M.far[warp] + 9 * lane;
-                uint32_t w[FAR_WORDS];
-#pragma unroll
-                for (uint32_t k = 0; k < FAR_WORDS; k++) w[k] = k < nw ? __ldcg(q + k) : 0u;
-#pragma unroll
-                for (uint32_t k = 0; k < FAR_WORDS; k++)
-                    if (k < nw) f[k] = w[k];
-            }
+            const uint32_t far_at = FAR_AT + half * (4 * FAR_WORDS * FAR_N);
             {
                 auto place = [&](uint32_t id, uint32_t start, uint32_t len) {
                     M.map[start] = (typename C::Id)id;
@@ -1141,19 +1168,32 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
                     M.tok[id] = (((held ? LIT_AT + l : 0u) - start) << 16) | (held ? T_FAR : T_FAR | T_DIRECT | T_PLAIN);
                     M.aux[id] = lit0 + l - start;
                 };
-                auto match = [&](uint32_t id, uint32_t start, uint32_t len, uint32_t d, uint32_t x, bool is_old, uint32_t f) {
+                auto match = [&](uint32_t id, uint32_t start, uint32_t len, uint32_t d, uint32_t x, uint32_t f) {
                     place(id, start, len);
                     const uint32_t at = x & C::RMASK;
-                    const bool held = is_old ? f < FAR_N : at + len <= C::RING;
-                    M.tok[id] = (((!held ? 0u : is_old ? FAR_AT + 36 * f + (x & 3u) : at) - start) << 16) |
+                    const bool is_old = f != NOT_OLD, held = is_old ? f < FAR_N : at + len <= C::RING;
+                    M.tok[id] = (((!held ? 0u : is_old ? far_at + 4 * FAR_WORDS * f + (x & 3u) : at) - start) << 16) |
                                 (!held ? (is_old ? T_FAR | T_DIRECT : T_FAR | T_WRAP) : d < C::SPAN ? T_NEAR | d : T_FAR);
                     M.aux[id] = start | (d << 16);
                 };
                 if (c0) literals(4 * tid + 1, b0, c0, l0);
-                if (m0) match(4 * tid + 2, b1, m0, d0, x0, old0, f0);
+                if (m0) match(4 * tid + 2, b1, m0, d0, x0, f0);
                 if (c1) literals(4 * tid + 3, b2, c1, l1);
-                if (m1) match(4 * tid + 4, b3, m1, d1, x1, old1, f1);
+                if (m1) match(4 * tid + 4, b3, m1, d1, x1, f1);
                 if (W > 1 && tid == 0 && p0) M.head[0] = 0;
+            }
+            // the next group is planned, and its old sources and the sequences after it loaded, while this one is
+            // written (with 32 old sources, fetched when their own group was planned, 61,825 members took 25.3 ms
+            // of decode, copy and CRC32, now 22.7: with 24 of them 26.9, 32 23.9, 48 23.1)
+            wait_async();
+            g += cnt;
+            lbase += glit;
+            P += glen;
+            half ^= 1;
+            load_lits();
+            if (g < ns) {
+                plan(P0);
+                load_seqs(g + cnt);
             }
             sync();
             uint32_t carry = 0;
@@ -1271,13 +1311,13 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
                         // bytes of the word after the group's end are overwritten by the next one
                         *reinterpret_cast<uint32_t*>(base + w) = word;
                     } else {  // the member's first or last word: its own bytes only
-                        for (uint32_t s = max(w, P); s < min(w + 4, R0 + pe); s++) base[s] = (uint8_t)(word >> (8 * (s - w)));
+                        for (uint32_t s = max(w, P0); s < min(w + 4, R0 + pe); s++) base[s] = (uint8_t)(word >> (8 * (s - w)));
                     }
                 }
                 sync();
             }
-            P += glen;
         }
+        wait_async();
         if (st == CB_OK && P != Eend) st = CB_ERR_INFLATE;
         if (tid == 0 && st != CB_OK) {
             per_job[JW * j + 1] = st;
@@ -1532,7 +1572,7 @@ int copy_range(const Call& c, Range r, cudaStream_t s) {
     if (resident(c, copy_occupancy<C8>())) rc = launch_copy<C8>(c, r, s);
     else if (resident(c, copy_occupancy<C4>())) rc = launch_copy<C4>(c, r, s);
     else if (resident(c, copy_occupancy<C2>())) rc = launch_copy<C2>(c, r, s);
-    // 4 KB: 28 warps per SM, 4.04 ms on 15,456 GEX members, 8 KB 16 warps and 4.39 ms
+    // 4 KB: 23 warps per SM; with 8 KB 16 (15,456 GEX members when it had 28: 4.04 ms, 8 KB 4.39)
     else if (cw == 12) rc = launch_copy<split::CopyCfg<4096, 1>>(c, r, s);
     else if (cw == 24) rc = launch_copy<split::CopyCfg<8192, 1>>(c, r, s);
     else rc = launch_copy<split::CopyCfg<16384, 1>>(c, r, s);
@@ -1603,7 +1643,14 @@ int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_
         // (3,865 GEX members 2.45 ms -> 2.12, 15,457 6.95 -> 6.72; 2,320 1.358 -> 1.366; cut at three
         // quarters 2.35 and 6.78; in four ranges 2.59 and 7.09).  Only with the job count known on the host.
         const long long pipe = cb_param(CB_PARAM_DECODE_PIPELINE);
-        const bool two = !d_n_jobs && n_jobs >= 2 && (pipe == 2 || (pipe == 1 && n_jobs >= 20LL * cb_device_sm_count()));
+        // (Below 65,536 jobs not under capture, where the side streams may be missing.)
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        bool many = n_jobs >= 65536;
+        if (!many && n_jobs >= 20LL * cb_device_sm_count()) {
+            if (cudaStreamIsCapturing(s, &cap) == cudaSuccess) many = cap == cudaStreamCaptureStatusNone;
+            else cudaGetLastError();
+        }
+        const bool two = !d_n_jobs && n_jobs >= 2 && (pipe == 2 || (pipe == 1 && many));
         int rc = CB_OK;
         if (!two) {
             const Range all{0, n_jobs, 0};
