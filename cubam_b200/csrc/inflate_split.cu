@@ -7,7 +7,7 @@
 //  1. k_decode: one member per CTA of W warps (W = 8, 4, 2 or 1, fewer the more members there are), its
 //     32 W lanes decoding as many segments of the member's bits at once.  A Huffman decoder that starts
 //     at a wrong bit falls in step with the true symbols soon (on BAM members after 64 bits in half of
-//     the cases, after 512 in 99.5%), so every lane starts OVERLAP bits before its segment and notes the
+//     the cases, after 512 in 99.5% and after 768 in 99.97%), so every lane starts OVERLAP bits before its segment and notes the
 //     first symbol that begins in it; that must be where the lane before stopped, and a lane for which
 //     it is not decodes its segment again from there.  The lanes share one set of code tables in shared
 //     memory.  Each lane writes its symbols, literal bytes and 4-byte sequences of a literal count and
@@ -170,7 +170,9 @@ constexpr uint32_t SLOW = F_BAD | 32;  // (as a second literal: none)
 constexpr int ROOT = 9, DROOT = 8;     // bits that index the root tables
 constexpr uint32_t LNG = 512;          // entries for the longer literal/length codes, after the root's
 constexpr uint32_t DST = (1u << ROOT) + LNG;
-constexpr uint32_t OVERLAP = 512;      // bits a lane decodes before its segment to fall in step
+// bits a lane decodes before its segment to fall in step (a lane that did not costs its warp a second pass: all
+// of form 3 on 2,320 members, in us, with 384 1226, 512 1210, 640 1180, 768 1190, 1024 1188)
+constexpr uint32_t OVERLAP = 640;
 constexpr uint32_t SEG_MIN = 128;      // bits of a segment, at least
 constexpr uint32_t WINDOW = 179200;    // bits of a window of segments: a zlib block of 16,383 BAM symbols
 constexpr uint32_t BITS = (1u << 30) - 1;  // of a position in the member's input (its segments' ends have two flags)
