@@ -52,11 +52,13 @@ sys.path.insert(0, str(ROOT))
 METRIC = "BAM decode GB/s (uncompressed) & records/s on 1 B200"
 UNIT = "GB/s"
 FALLBACK_HBM = 6650.0
-#: DRAM bytes (read + write) per inflated byte of each inflate form, from one ncu capture each on the
-#: 4M-record GEX file (1,008,824,685 inflated bytes); the bench scales them by its inflated bytes
+#: DRAM bytes (read + write) per inflated byte of each inflate form, from one ncu capture each of a GEX file
+#: (forms 1 and 2: 4M records, 1,008,824,685 inflated bytes; form 3: 2M records, 504,442,337); the bench scales
+#: them by its inflated bytes
 TRAFFIC_PER_BYTE = {"k_inflate_lanes": (6.916637e9 + 1.003612e9) / 1.008824685e9,
                     "k_inflate_warp": (1.593613e9 + 1.004537e9) / 1.008824685e9,
-                    "k_decode + k_copy": (0.414233344e9 + 0.754765312e9 + 1.45392e9 + 0.958392832e9) / 1.008824685e9}
+                    "k_decode + k_copy + k_crc": (539.836416e6 + 662.705408e6 + 535.985408e6 + 456.324352e6 + 505.957120e6
+                                                  + 3.871744e6) / 504.442337e6}
 
 
 def parse():
@@ -373,7 +375,7 @@ def run_ours(args):
     from cubam_b200.bgzf import inflate_form
 
     form = inflate_form(0, n_members)  # the form the batched decode runs
-    kernel = {1: "k_inflate_warp", 2: "k_inflate_lanes", 3: "k_decode + k_copy"}[form]
+    kernel = {1: "k_inflate_warp", 2: "k_inflate_lanes", 3: "k_decode + k_copy + k_crc"}[form]
 
     # the plain per-chunk form of the same kernels on device-resident chunks (cubam's structure)
     plain = None
@@ -709,7 +711,7 @@ def run_uneven(args):
     ms_per_file = s2.elapsed_time(e2)
     peak, peak_kind = peaks()
     achieved = inflated / (stage["inflated"] / 1e3) / 1e9
-    kernel = {1: "k_inflate_warp", 2: "k_inflate_lanes", 3: "k_decode + k_copy"}[plan.form]
+    kernel = {1: "k_inflate_warp", 2: "k_inflate_lanes", 3: "k_decode + k_copy + k_crc"}[plan.form]
     print(json.dumps({
         "metric": METRIC, "value": inflated / (ms / 1e3) / 1e9, "unit": UNIT, "n_gpus": 1, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,

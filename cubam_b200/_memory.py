@@ -3,8 +3,8 @@
 Mirrors ``src/cubam/_memory.py``: the chunk policy is the same rule (halved
 while 64 chunks do not fit in free GPU memory, never below 32 MB) from a
 ceiling of 1 GB instead of 256 MB: a B200's 180 GB hold 64 chunks of 1 GB, and
-a chunk of 1 GB holds about 39,000 BGZF members, enough for the two-kernel
-inflater (one member per lane) to run, while chunks stay small enough for the
+a chunk of 1 GB holds about 39,000 BGZF members, enough to fill the
+inflater's warps, while chunks stay small enough for the
 host reads of the next ones to overlap the GPU work (page cache to pinned
 memory ran at 29 GB/s with 1 GB chunks and 25 GB/s with 2 GB chunks, 16
 threads).  Below 32 GB of free memory the sizes are cubam's (64 MB on 8 GB,

@@ -20,8 +20,8 @@
 //  4. Members whose symbols do not fit their slot are inflated by the one-kernel form
 //     (cb_inflate_listed, inflate.cu).
 //
-// What bounds them: with many members the issue of instructions (decode 0.54 per cycle and scheduler, at 18
-// warps per SM by shared memory); with few, the chain of steps of one lane and of rounds of one member,
+// What bounds them: with many members the issue of instructions (decode 0.53 per cycle and scheduler at 18
+// warps per SM, copy 0.68 at 22, by shared memory); with few, the chain of steps of one lane and of rounds of one member,
 // which is why a member takes more warps then.  Measured, in ms (one serial decoder per member, in one
 // kernel, before; a warp per member in between):
 //   39 GEX members (10,000 records)      decode 0.17 (0.46), copy 0.15 (0.43), CRC32 0.01; one kernel 4.2
@@ -1574,7 +1574,7 @@ int copy_range(const Call& c, Range r, cudaStream_t s) {
     if (resident(c, copy_occupancy<C8>())) rc = launch_copy<C8>(c, r, s);
     else if (resident(c, copy_occupancy<C4>())) rc = launch_copy<C4>(c, r, s);
     else if (resident(c, copy_occupancy<C2>())) rc = launch_copy<C2>(c, r, s);
-    // 4 KB: 23 warps per SM; with 8 KB 16 (15,456 GEX members when it had 28: 4.04 ms, 8 KB 4.39)
+    // 4 KB: 22 warps per SM; with 8 KB 16 (15,456 GEX members when it had 28: 4.04 ms, 8 KB 4.39)
     else if (cw == 12) rc = launch_copy<split::CopyCfg<4096, 1>>(c, r, s);
     else if (cw == 24) rc = launch_copy<split::CopyCfg<8192, 1>>(c, r, s);
     else rc = launch_copy<split::CopyCfg<16384, 1>>(c, r, s);
