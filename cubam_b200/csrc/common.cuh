@@ -20,11 +20,15 @@ __device__ __forceinline__ uint32_t ld_u16(const uint8_t* b, long long o) {
 }
 // The first 4 bytes (or left, if fewer; the others are undefined) at p, from the aligned words that hold one of
 // them (two loads where bytes took four).
-__device__ __forceinline__ uint32_t ld_bytes4(const uint8_t* p, uint32_t left) {
+__host__ __device__ __forceinline__ uint32_t ld_bytes4(const uint8_t* p, uint32_t left) {
     const uint32_t k = (uint32_t)(uintptr_t)p & 3u;
     const uint32_t* w = reinterpret_cast<const uint32_t*>(p - k);
     const uint32_t lo = w[0], hi = k + left > 4 && k ? w[1] : 0u;
+#ifdef __CUDA_ARCH__
     return __funnelshift_r(lo, hi, 8 * k);
+#else
+    return (uint32_t)((lo | (uint64_t)hi << 32) >> (8 * k));
+#endif
 }
 __device__ __forceinline__ uint32_t ld_u32(const uint8_t* b, long long o) { return ld_bytes4(b + o, 4); }
 

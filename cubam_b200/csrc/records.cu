@@ -5,6 +5,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "spans.cuh"
 
 namespace cb {
 namespace rec {
@@ -446,34 +447,6 @@ __global__ void k_base_at(const uint8_t* __restrict__ b, const int64_t* __restri
     }
 }
 
-// The 4-byte words of a destination span of len bytes at d (those that hold one of its bytes), from s, by
-// LANES lanes of which this is number l.  Source words are read when they hold a byte of the span.
-template <uint32_t LANES>
-__device__ __forceinline__ void copy_words(const uint8_t* s, uint8_t* d, long long len, uint32_t l) {
-    constexpr int U = 4;  // words in flight per lane
-    const uint32_t k = (uint32_t)(uintptr_t)d & 3u;
-    for (long long q0 = 4LL * l - k; q0 < len; q0 += 4 * LANES * U) {  // the word's place in the span
-        uint32_t x[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const long long q = q0 + 4LL * LANES * u;
-            x[u] = q >= len ? 0u : q >= 0 ? ld_bytes4(s + q, (uint32_t)min(len - q, 4LL)) : ld_bytes4(s, (uint32_t)min(len, 4LL)) << (8 * k);
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const long long q = q0 + 4LL * LANES * u;
-            if (q >= len) break;
-            if (q >= 0 && q + 4 <= len) {
-                *reinterpret_cast<uint32_t*>(d + q) = x[u];
-            } else {
-#pragma unroll
-                for (int t = 0; t < 4; t++)
-                    if (q + t >= 0 && q + t < len) d[q + t] = (uint8_t)(x[u] >> (8 * t));
-            }
-        }
-    }
-}
-
 // Spans by words of the destination, four lanes each; a warp takes its eight spans one by one when one of them
 // is longer than 512 bytes.  What bounds it is the
 // latency of the offsets and then the bytes: 1 million spans of 10 to 40 bytes, 300 apart: 50 us (81 with eight lanes
@@ -490,7 +463,7 @@ __global__ void __launch_bounds__(256) k_copy_spans(const uint8_t* __restrict__ 
         if (__any_sync(FULL, len > 512)) {
             for (long long j = 8 * w; j < 8 * w + 8 && j < n; j++)
                 copy_words<32>(src + src_off[j], dst + dst_off[j], size[j], lane);
-        } else if (len > 0) {
+        } else if (i < n) {
             copy_words<4>(src + src_off[i], dst + dst_off[i], len, l);
         }
     }
