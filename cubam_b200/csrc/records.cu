@@ -447,11 +447,18 @@ __global__ void k_base_at(const uint8_t* __restrict__ b, const int64_t* __restri
     }
 }
 
-// Spans by words of the destination, four lanes each; a warp takes its eight spans one by one when one of them
-// is longer than 512 bytes.  What bounds it is the
-// latency of the offsets and then the bytes: 1 million spans of 10 to 40 bytes, 300 apart: 50 us (81 with eight lanes
-// and one word in flight per lane, 145 with a warp per span and a byte per lane).
-__global__ void __launch_bounds__(256) k_copy_spans(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
+// Many spans: four lanes each, by words of the destination; those of more than LONG bytes by the whole warp, one after
+// another.  What bounds it is the latency of the offsets and then the bytes, so the long ones' code may not take
+// registers from the short ones' (40; with 48 spans of 130 bytes took 66 us, not 61).  In us, before (eight spans of
+// which one is over 512 bytes one by one, in 4-byte words) and now: 1 million spans of 20 bytes 48, 48; 200,000 of 400
+// 70, 57; 100,000 of 600 78, 46; 50,000 of 3,000 148, 71.  LONG: spans of 300 bytes take 79 by lanes and 88 by the warp,
+// of 400 70 and 57.
+constexpr long long LONG = 384;
+template <int U> __device__ __forceinline__ void copy_by_warp(const uint8_t* s, uint8_t* d, long long len) {
+    for (; len > 0; s += MAX_SPAN, d += MAX_SPAN, len -= MAX_SPAN)
+        copy_long<32, U>(s, d, (int)min(len, (long long)MAX_SPAN), threadIdx.x & 31);
+}
+__global__ void __launch_bounds__(256, 6) k_copy_spans(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
                                                     const int64_t* __restrict__ src_off,
                                                     const int64_t* __restrict__ dst_off,
                                                     const int64_t* __restrict__ size, long long n) {
@@ -460,12 +467,28 @@ __global__ void __launch_bounds__(256) k_copy_spans(const uint8_t* __restrict__ 
          w += ((long long)gridDim.x * blockDim.x) >> 5) {
         const long long i = 8 * w + (lane >> 2);
         const long long len = i < n ? size[i] : 0;
-        if (__any_sync(FULL, len > 512)) {
-            for (long long j = 8 * w; j < 8 * w + 8 && j < n; j++)
-                copy_words<32>(src + src_off[j], dst + dst_off[j], size[j], lane);
-        } else if (i < n) {
-            copy_words<4>(src + src_off[i], dst + dst_off[i], len, l);
+        for (uint32_t big = __ballot_sync(FULL, len > LONG) & 0x11111111u; big; big &= big - 1) {
+            const long long j = 8 * w + (__ffs((int)big) - 1) / 4;
+            copy_by_warp<1>(src + src_off[j], dst + dst_off[j], size[j]);
         }
+        if (len > 0 && len <= LONG) copy_words<4>(src + src_off[i], dst + dst_off[i], (int)len, l);
+    }
+}
+
+// Few spans: `parts` warps each, every one a part of whole 16-byte blocks of the destination.  64 MB, in us, before and
+// now: 6,400 spans 360, 33 (39 where source and destination are aligned differently), 8 spans 216,000, 32 (37).
+__global__ void __launch_bounds__(256) k_copy_few_spans(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
+                                                        const int64_t* __restrict__ src_off,
+                                                        const int64_t* __restrict__ dst_off,
+                                                        const int64_t* __restrict__ size, long long n, long long parts) {
+    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n * parts;
+         w += ((long long)gridDim.x * blockDim.x) >> 5) {
+        const long long i = w / parts, p = w % parts, len = size[i];
+        uint8_t* d = dst + dst_off[i];
+        const long long k = (long long)((uintptr_t)d & 15);  // the first part is shorter by these
+        const long long step = ((len + k + parts - 1) / parts + 511) & ~511LL;
+        const long long from = max(p * step - k, 0LL), to = min((p + 1) * step - k, len);
+        copy_by_warp<2>(src + src_off[i] + from, d + from, to - from);
     }
 }
 
@@ -618,8 +641,14 @@ extern "C" int cb_copy_spans(const uint8_t* src, uint8_t* dst, const int64_t* sr
                              const int64_t* size, int64_t n, void* stream) {
     if (n < 0) return CB_ERR_ARG;
     if (n == 0) return CB_OK;
-    rec::k_copy_spans<<<grid_for(n * 4, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(src, dst, src_off,
-                                                                                                  dst_off, size, n);
+    const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    constexpr long long WARPS = 148 * 64;  // resident on the GPU
+    if (n >= 2 * WARPS) {  // (30,000 spans of 20 bytes: 18 us, 23 with a warp each)
+        rec::k_copy_spans<<<grid_for(n * 4, 256), 256, 0, s>>>(src, dst, src_off, dst_off, size, n);
+    } else {
+        const long long parts = n < WARPS ? WARPS / n : 1;
+        rec::k_copy_few_spans<<<grid_for(n * parts * 32, 256), 256, 0, s>>>(src, dst, src_off, dst_off, size, n, parts);
+    }
     return cb_set_error(cudaGetLastError());
 }
 

@@ -17,12 +17,13 @@ static uint8_t* page() {
     return m + 4096;
 }
 
-template <uint32_t LANES> static void copy_of(uint8_t* src, uint8_t* dst, int so, int d, int len) {
+template <uint32_t LANES, bool LONG> static void copy_of(uint8_t* src, uint8_t* dst, int so, int d, int len) {
     std::vector<uint8_t> want(4096, 0xA5);
     memset(dst, 0xA5, 4096);
     if (len > 0) memcpy(want.data() + d, src + so, len);
-    for (uint32_t l = 0; l < LANES; l++) cb::copy_words<LANES>(src + so, dst + d, len, l);
-    if (memcmp(dst, want.data(), 4096) && failures++ < 10) printf("FAIL lanes %u from %d to %d, %d bytes\n", LANES, so, d, len);
+    for (uint32_t l = 0; l < LANES; l++)
+        LONG ? cb::copy_long<LANES, 2>(src + so, dst + d, len, l) : cb::copy_words<LANES>(src + so, dst + d, len, l);
+    if (memcmp(dst, want.data(), 4096) && failures++ < 10) printf("FAIL lanes %u long %d from %d to %d, %d bytes\n", LANES, LONG, so, d, len);
 }
 
 int main() {
@@ -34,8 +35,9 @@ int main() {
             for (int b = 0; b < 20 && b + n <= 4096; b++)
                 for (int end = 0; end < 4; end++) {  // each at the page's start or its end
                     const int so = end & 1 ? 4096 - n - a : a, d = end & 2 ? 4096 - n - b : b;
-                    copy_of<4>(src, dst, so, d, len);
-                    copy_of<32>(src, dst, so, d, len);
+                    copy_of<4, false>(src, dst, so, d, len);
+                    copy_of<32, false>(src, dst, so, d, len);
+                    copy_of<32, true>(src, dst, so, d, len);
                 }
     }
     printf("%d failures\n", failures);
