@@ -263,18 +263,28 @@ __global__ void __launch_bounds__(RW * 32) k_records(const uint8_t* __restrict__
     }
 }
 
-// The FNV-1a hash of l bytes at p (src/cubam/_kernels.py:391-403), eight bytes per round, the next round's loaded
-// ahead of the multiplications.
+// The FNV-1a hash of l bytes at p (src/cubam/_kernels.py:391-403), eight bytes per round, from the aligned words that
+// hold one of them, each loaded once and a round ahead of the multiplications (1 million adjacent spans of 20 bytes 22 us,
+// 26 when each 4 bytes loaded their two words, 20 by bytes; 250 bytes apart 39, 43, 43; 4,000 of 20,000 bytes 530, 900, 1065).
 __device__ __forceinline__ unsigned long long fnv1a(const uint8_t* p, uint32_t l) {
     unsigned long long x = FNV_OFFSET;
-    uint32_t n0 = l ? ld_bytes4(p, l) : 0u, n1 = l > 4 ? ld_bytes4(p + 4, l - 4) : 0u;
+    if (l == 0) return x;
+    const uint32_t at = (uint32_t)(uintptr_t)p & 3u, sh = 8 * at;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(p - at);
+    const uint32_t last = (at + l - 1) >> 2;  // word
+    uint32_t a = w[0], b = last >= 1 ? w[1] : 0u, c = last >= 2 ? w[2] : 0u;
     for (uint32_t k = 0; k < l; k += 8) {
-        const uint32_t w0 = n0, w1 = n1;
-        n0 = l > k + 8 ? ld_bytes4(p + k + 8, l - k - 8) : 0u;
-        n1 = l > k + 12 ? ld_bytes4(p + k + 12, l - k - 12) : 0u;
+        const uint32_t w0 = __funnelshift_r(a, b, sh), w1 = __funnelshift_r(b, c, sh), i = (k >> 2) + 3;
+        a = c;
+        b = i <= last ? w[i] : 0u;
+        c = i < last ? w[i + 1] : 0u;
+        unsigned long long v = (unsigned long long)w1 << 32 | w0;
+        if (k + 8 <= l) {
 #pragma unroll
-        for (uint32_t j = 0; j < 8; j++)
-            if (k + j < l) x = (x ^ ((j < 4 ? w0 : w1) >> (8 * (j & 3)) & 255u)) * FNV_PRIME;
+            for (int j = 0; j < 8; j++) x = (x ^ (v >> (8 * j) & 255u)) * FNV_PRIME;
+        } else {
+            for (uint32_t j = k; j < l; j++, v >>= 8) x = (x ^ (v & 255u)) * FNV_PRIME;
+        }
     }
     return x;
 }

@@ -74,14 +74,14 @@ __host__ __device__ __forceinline__ void copy_long(const uint8_t* s, uint8_t* d,
     } else {
         for (int q = (int)l; q < nv; q += (int)LANES * U) {
             uint4 x[U], y[U];
-    #pragma unroll
+#pragma unroll
             for (int u = 0; u < U; u++) {
                 if (q + u * (int)LANES < nv) {
                     x[u] = sv[q + u * (int)LANES];
                     y[u] = sv[q + u * (int)LANES + 1];
                 }
             }
-    #pragma unroll
+#pragma unroll
             for (int u = 0; u < U; u++) {
                 if (q + u * (int)LANES < nv) {
                     const uint4 a = x[u], b = y[u];
