@@ -287,7 +287,8 @@ __device__ uint32_t tokenize(Smem& S, uint32_t a, uint32_t n, int level, uint32_
             if (__any_sync(FULL, cand[k] != 0)) {
                 const bool v4 = p + 4 <= n;
                 const uint32_t q = a + (v4 ? p : 0u), maxl = v4 ? min(MAX_MATCH, n - p) : 0u;
-                const uint32_t d1 = cand[k] >> 16, d2 = cand[k] & 0xFFFFu;
+                const uint32_t d1 = cand[k] >> 16;
+                uint32_t d2 = cand[k] & 0xFFFFu;
                 const uint32_t* pq = S.in + (q >> 2);
                 uint32_t x[5], lo = pq[0];
 #pragma unroll
@@ -299,6 +300,8 @@ __device__ uint32_t tokenize(Smem& S, uint32_t a, uint32_t n, int level, uint32_
                 if (__any_sync(FULL, d1 != 0)) {
                     const uint32_t L = match_lens(S.in, q, d1, x, maxl);
                     if (L >= MIN_MATCH) b = (L << 16) | d1;
+                    // cannot be beaten (64 MB of zeros 1.9 ms, 7.8 with d2 compared all the same; runs of 1,000 4.1, 6.7)
+                    if (L == maxl) d2 = 0;
                 }
                 const uint32_t L = match_lens(S.in, q, d2, x, maxl);
                 if (L >= MIN_MATCH && L > (b >> 16)) b = (L << 16) | d2;
