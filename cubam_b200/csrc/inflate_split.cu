@@ -36,6 +36,7 @@
 
 #include "common.cuh"
 #include "crc.cuh"
+#include "split_slots.cuh"
 
 namespace cb {
 namespace split {
@@ -81,16 +82,6 @@ constexpr uint32_t ST_LISTED = 0x100;     // internal status: on that list
 __host__ __device__ __forceinline__ size_t arena_offset(long long n_jobs) {
     return (WS_HEAD + PER_JOB * (size_t)n_jobs + 255) & ~(size_t)255;
 }
-// A member's slot holds its symbols: literal bytes from its start up, sequences (a word each) from its end
-// down: bits 24-31 literals before the match, 16-23 match length - 3, 15 set when there is a match, 0-14
-// distance - 1.  Symbols take at most 4 bytes per 3 output bytes (matches of length 3); the rest is room
-// for sequences without a match (one per 255 literals, and at the end of a segment or block).
-constexpr uint32_t SEQ_MATCH = 0x8000u;
-constexpr uint32_t SEQ_BAD = 1u;  // without SEQ_MATCH: the match has no valid distance
-__host__ __device__ __forceinline__ unsigned long long slot_bytes(uint32_t isize) {
-    return (2ull * isize + 64ull + 15ull) & ~15ull;
-}
-
 // The arena slot of every job: one CTA; thread t sums a contiguous run of jobs, a block scan joins
 // the runs, and each thread writes its run's offsets.
 constexpr int SLOT_NT = 1024;
@@ -175,7 +166,6 @@ constexpr uint32_t DST = (1u << ROOT) + LNG;
 constexpr uint32_t OVERLAP = 640;
 constexpr uint32_t SEG_MIN = 128;      // bits of a segment, at least
 constexpr uint32_t WINDOW = 179200;    // bits of a window of segments: a zlib block of 16,383 BAM symbols
-constexpr uint32_t BITS = (1u << 30) - 1;  // of a position in the member's input (its segments' ends have two flags)
 constexpr uint32_t RUN_MIN = 256;      // bytes of scratch per lane, at least (or one lane decodes alone)
 constexpr int ROWS = 16;               // words of input kept per lane
 constexpr int STEPS = 8;               // decode steps between refills
@@ -813,7 +803,7 @@ __device__ uint32_t decode_member(DecMember<W>& M, const cb_member_job& job, uin
     const uint32_t scratch_n = job.isize > skip ? (job.isize - skip) & ~15u : 0u;
     uint8_t* lens = reinterpret_cast<uint8_t*>(M.w[0].lst);
     nl = ns = 0;
-    if (job.in_len > BITS / 16) return ST_LISTED;
+    if (!in_reach(job.in_len, job.isize)) return ST_LISTED;
     for (;;) {
         if (p > E) return CB_ERR_INFLATE;
         if (warp == 0) {  // the block's header, and its code lengths
