@@ -20,8 +20,8 @@ OK, TRUNCATED, NO_CHAIN, CORRUPT_BLOCK, INFLATE, CRC, TOO_MANY, CAPACITY, CUDA, 
 #: launch parameters (cb_set_param / cb_get_param)
 (PARAM_CHAIN_TILE, PARAM_INFLATE_FORM, PARAM_DECODE_ROOT, PARAM_COPY_WARPS, PARAM_DECODE_STEPS, PARAM_DECODE_PREFETCH,
  PARAM_SPLIT_MIN_JOBS, PARAM_COPY_UNITS, PARAM_DECODE_PIPELINE) = range(1, 10)
-#: PARAM_SPLIT_MIN_JOBS by default: form 3 for any number of jobs
-SPLIT_MIN_JOBS_ANY = 8192
+#: a PARAM_SPLIT_MIN_JOBS: form 3 for any number of jobs (as when none is set)
+SPLIT_MIN_JOBS_ANY = 0
 
 
 class MemberJob(ctypes.Structure):
@@ -81,6 +81,7 @@ _SIGNATURES = {
     "cb_scan_members_noalloc": (c_int, [P, I64, c_int, I64, P, I64, P, P]),
     "cb_inflate_workspace_bytes": (c_size_t, []),
     "cb_inflate": (c_int, [P, I64, P, P, c_int, P, P, P, c_size_t, P]),
+    "cb_inflate_default_form": (c_int, [I64]),
     "cb_inflate_form": (c_int, [P, I64, P, P, c_int, P, P, P, c_size_t, c_int, P]),
     "cb_inflate_lane_slots": (I64, []),
     "cb_inflate_split_workspace_bytes": (c_size_t, [I64, I64]),

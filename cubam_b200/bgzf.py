@@ -279,11 +279,7 @@ def inflate_form(form: int = 0, n_jobs: int | None = None) -> int:
     ``CB_PARAM_SPLIT_MIN_JOBS`` jobs, when that was set)."""
     if form:
         return int(form)
-    f = int(_lib.lib.cb_get_param(_lib.PARAM_INFLATE_FORM))
-    least = int(_lib.lib.cb_get_param(_lib.PARAM_SPLIT_MIN_JOBS))
-    if f == 3 and n_jobs is not None and least != _lib.SPLIT_MIN_JOBS_ANY and n_jobs < least:
-        return 1
-    return f
+    return int(_lib.lib.cb_inflate_default_form(n_jobs if n_jobs is not None else 1 << 62))
 
 
 def inflate_workspace_bytes(n_jobs: int, out_bytes: int, form: int = 0) -> int:

@@ -36,7 +36,7 @@ constexpr Param kParams[] = {
     {CB_PARAM_COPY_WARPS, 2, 24, 12},
     {CB_PARAM_DECODE_STEPS, 1, 64, 16},
     {CB_PARAM_DECODE_PREFETCH, 0, 16, 4},
-    {CB_PARAM_SPLIT_MIN_JOBS, 0, 1LL << 40, CB_SPLIT_MIN_JOBS_ANY},
+    {CB_PARAM_SPLIT_MIN_JOBS, 0, 1LL << 40, 8192},
     {CB_PARAM_COPY_UNITS, 1, 4, 2},
     {CB_PARAM_DECODE_PIPELINE, 0, 2, 1},
 };
@@ -57,12 +57,12 @@ int64_t cb_param(int key) {
     return g_param_set[i].load(std::memory_order_acquire) ? g_param[i].load(std::memory_order_relaxed) : kParams[i].def;
 }
 
-// CB_PARAM_INFLATE_FORM; for form 3 the caller may have set a number of jobs below which form 1 runs (form
-// 3 itself is the faster at every size: 39 GEX members take it 0.4 ms and form 1 4.2 ms).
-int cb_default_form(int64_t n_jobs) {
+// CB_PARAM_INFLATE_FORM; for form 3 the caller may have set a number of jobs below which form 1 runs (39 GEX
+// members of 65 KB take form 3 0.4 ms and form 1 4.2 ms).
+extern "C" int cb_inflate_default_form(int64_t n_jobs) {
     const int form = (int)cb_param(CB_PARAM_INFLATE_FORM);
-    const int64_t min_jobs = cb_param(CB_PARAM_SPLIT_MIN_JOBS);
-    return form == 3 && min_jobs != CB_SPLIT_MIN_JOBS_ANY && n_jobs < min_jobs ? 1 : form;
+    const bool set = g_param_set[param_index(CB_PARAM_SPLIT_MIN_JOBS)].load(std::memory_order_acquire);
+    return form == 3 && set && n_jobs < cb_param(CB_PARAM_SPLIT_MIN_JOBS) ? 1 : form;
 }
 
 extern "C" int64_t cb_get_param(int key) { return param_index(key) < 0 ? -1 : cb_param(key); }

@@ -8,8 +8,6 @@
 
 // The current value of a launch parameter (abi.cu; cb_set_param / cb_get_param).
 int64_t cb_param(int key);
-// The inflate form of a call of n_jobs jobs that leaves it to the library (abi.cu).
-int cb_default_form(int64_t n_jobs);
 
 namespace cb {
 

@@ -1468,12 +1468,13 @@ extern "C" int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const 
                                int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
                                size_t workspace_bytes, int form, void* stream) {
     if (!summary || !workspace || workspace_bytes < cb_inflate_workspace_bytes() || n_jobs < 0) return CB_ERR_ARG;
-    // A call of few jobs that leaves the form to the library takes any workspace: what of it form 3's arena
-    // does not hold is inflated by the one-kernel form.
+    // A call of few jobs that leaves the form to the library takes any workspace (callers sized it for form 1, which
+    // such calls once ran): what form 3's arena does not hold is inflated by the one-kernel form.
+    constexpr int64_t ANY_WORKSPACE_JOBS = 8192;
     bool any_workspace = false;
     if (form == 0) {
-        form = cb_default_form(n_jobs);
-        any_workspace = form == 3 && n_jobs < CB_SPLIT_MIN_JOBS_ANY;
+        form = cb_inflate_default_form(n_jobs);
+        any_workspace = form == 3 && n_jobs < ANY_WORKSPACE_JOBS;
         if (any_workspace && workspace_bytes < cb_inflate_split_workspace_bytes(n_jobs, 0)) form = 1;
     }
     if (form == 3) {

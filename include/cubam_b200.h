@@ -98,8 +98,9 @@ int cb_device_sm_count(void);
  *                          memory: 16 KiB for 2, 3 or 6, 4 KiB for 12, 8 KiB for 24 (12)
  *   CB_PARAM_DECODE_STEPS  no effect (kept for callers that set it): 1-64 (16)
  *   CB_PARAM_DECODE_PREFETCH  no effect (kept for callers that set it): 0-16 (4)
- *   CB_PARAM_SPLIT_MIN_JOBS   with CB_PARAM_INFLATE_FORM 3, form 0 runs form 1 for calls of fewer jobs: 0
- *                          or more (CB_SPLIT_MIN_JOBS_ANY, the default: form 3 for any number of jobs)
+ *   CB_PARAM_SPLIT_MIN_JOBS   with CB_PARAM_INFLATE_FORM 3, form 0 runs form 1 for calls of fewer jobs than this: 0
+ *                          or more (CB_SPLIT_MIN_JOBS_ANY).  Until it is set there is no such number (it reads 8192
+ *                          then), nor after cb_set_param(key, -1)
  *   CB_PARAM_COPY_UNITS    no effect (kept for callers that set it): 1, 2 or 4 (2)
  *   CB_PARAM_DECODE_PIPELINE  form 3 in two job ranges, each decoded and then copied on its own stream
  *                          (side streams joined back to the caller's by events), so that one range's
@@ -120,7 +121,7 @@ enum {
     CB_PARAM_COPY_UNITS = 8,
     CB_PARAM_DECODE_PIPELINE = 9
 };
-#define CB_SPLIT_MIN_JOBS_ANY 8192
+#define CB_SPLIT_MIN_JOBS_ANY 0  /* form 3 for any number of jobs */
 int cb_set_param(int key, int64_t value);
 int64_t cb_get_param(int key);
 
@@ -182,6 +183,9 @@ int cb_inflate(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_job
 int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base,
                     int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
                     size_t workspace_bytes, int form, void* stream);
+
+/* The form that cb_inflate_form runs for n_jobs jobs with form 0 and a workspace for it. */
+int cb_inflate_default_form(int64_t n_jobs);
 
 /* Members the one-member-per-lane form keeps in flight on the current device (0 on error). */
 int64_t cb_inflate_lane_slots(void);
