@@ -397,9 +397,9 @@ class BatchPlan:
     # ------------------------------------------------------------------ tuning and graphs
     def autotune(self, reps: int = 2, cache_path=None, use_cache: bool = True) -> dict:
         """Choose the launch parameters for this batch by timing it (:func:`cubam_b200.tune.tune`: the
-        inflate form 1-3, form 3's decoder roots, copy warps, decode steps and prefetch, the chain tile),
-        apply them to the process and cache them by device and batch shape; returns the tuner's entry
-        (``params`` and the milliseconds of every candidate)."""
+        inflate form 1-3, form 3's copy window and two-range pipeline, the chain tile), apply them to the
+        process and cache them by device and batch shape; returns the tuner's entry (``params`` and the
+        milliseconds of every candidate)."""
         from cubam_b200 import tune
 
         entry = tune.tune(self, reps=reps, path=cache_path, use_cache=use_cache)

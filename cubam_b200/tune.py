@@ -53,12 +53,17 @@ def _pow2(x: float) -> int:
     return 1 << max(0, int(round(math.log2(max(x, 1.0)))))
 
 
+#: raised when a parameter's values change their meaning or a form its kernels: entries tuned before are not used
+#: (copy windows of 12 and 24 warps were exchanged, and form 1 was the fastest for few members, from 1 to 2)
+REVISION = 2
+
+
 def shape_key(n_members: int, total_out: int) -> str:
-    """Device name, SM count and the workload shape, rounded to powers of two."""
+    """Device name, SM count and the workload shape, rounded to powers of two, and what the values stand for."""
     dev = torch.cuda.get_device_name() if torch.cuda.is_available() else "cpu"
     sms = int(_lib.lib.cb_device_sm_count())
     mean = total_out / max(n_members, 1)
-    return f"{dev}|sm{sms}|members~{_pow2(n_members)}|isize~{_pow2(mean)}"
+    return f"{dev}|sm{sms}|members~{_pow2(n_members)}|isize~{_pow2(mean)}|rev{REVISION}"
 
 
 def load_cache(path: Path | None = None) -> dict:
