@@ -105,21 +105,30 @@ class _ChunkReader:
         self.path, self.chunk = Path(path), int(chunk_bytes)
         self.n_buffers, self.n_threads, self.piece = max(int(n_buffers), 1), max(int(n_threads), 1), max(int(piece), 1)
         self._cuda = torch.cuda.is_available()
+        self._failure: BaseException | None = None
+        self._fd, self._size = -1, 0
         try:
-            size = os.stat(self.path).st_size
-        except OSError:
-            size = 0  # the thread raises it
-        self._slot_bytes = max(min(self.chunk, size), 1)
-        self.n_buffers = max(min(self.n_buffers, -(-size // self._slot_bytes)), 1)
-        self._slots = [torch.empty(self._slot_bytes, dtype=torch.uint8, pin_memory=self._cuda) for _ in range(self.n_buffers)]
+            self._fd = os.open(self.path, os.O_RDONLY)
+            self._size = os.fstat(self._fd).st_size  # what is written after this is not read
+        except OSError as e:  # raised in the consumer
+            self._failure = e
+        self._slot_bytes = max(min(self.chunk, self._size), 1)
+        self.n_buffers = max(min(self.n_buffers, -(-self._size // self._slot_bytes)), 1)
+        try:
+            self._slots = [torch.empty(self._slot_bytes, dtype=torch.uint8, pin_memory=self._cuda)
+                           for _ in range(self.n_buffers)]
+        except BaseException:
+            if self._fd >= 0:
+                os.close(self._fd)
+            raise
         self._cv = threading.Condition()
         self._ready: dict[int, list] = {}          # chunk index -> [slot, nbytes, eof, bytes read so far]
         self._copied: list = [None] * self.n_buffers  # event of the last copy out of each slot
         self._taken = 0                              # chunks the consumer has taken from the thread
-        self._failure: BaseException | None = None
         self._closed = False
-        self._thread = threading.Thread(target=self._produce, name="cubam-reader", daemon=True)
-        self._thread.start()
+        if self._failure is None:
+            self._thread = threading.Thread(target=self._produce, name="cubam-reader", daemon=True)
+            self._thread.start()
 
     def close(self) -> None:
         with self._cv:
@@ -139,9 +148,8 @@ class _ChunkReader:
         from concurrent.futures import ThreadPoolExecutor
 
         try:
-            fd = os.open(self.path, os.O_RDONLY)
+            fd, size = self._fd, self._size
             try:
-                size = os.fstat(fd).st_size
                 with ThreadPoolExecutor(self.n_threads) as workers:
                     k = off = 0
                     while True:
