@@ -345,7 +345,7 @@ class BatchPlan:
             if self.graph is not None:
                 raise RuntimeError("the captured plan's inflate workspace is too small for this form")
             self.queue_ws = torch.empty(max(need, 512), dtype=torch.uint8, device="cuda")
-        ws = (self.queue_ws if inflate_form(form, self.job_base[-1]) == 3
+        ws = (self.queue_ws if inflate_form(form, self.job_base[-1], self.total_out) == 3
               else self.queue_ws[: int(_lib.lib.cb_inflate_workspace_bytes())])
         launch_inflate(self.jobs.data_ptr(), self.job_base[-1], self.out.data_ptr(), self.total_out, self.check_crc,
                        self.inflate_summ.data_ptr(), ws, form)

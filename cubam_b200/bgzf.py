@@ -281,18 +281,19 @@ def scan_members(buf: torch.Tensor, eof: bool, out_base: int = 0, jobs_cap: int 
         return jobs, s
 
 
-def inflate_form(form: int = 0, n_jobs: int | None = None) -> int:
-    """The inflate form a call of ``n_jobs`` jobs with ``form`` runs, as ``cb_inflate_form`` chooses it:
-    0 is the library's default (``CB_PARAM_INFLATE_FORM``; form 1 in place of form 3 below
-    ``CB_PARAM_SPLIT_MIN_JOBS`` jobs, when that was set)."""
+def inflate_form(form: int = 0, n_jobs: int | None = None, out_bytes: int | None = None) -> int:
+    """The inflate form a call of ``n_jobs`` jobs (``out_bytes`` inflated bytes together) with ``form`` runs:
+    0 is the library's default (``CB_PARAM_INFLATE_FORM``; form 1 in place of form 3 for members of few bytes,
+    or below ``CB_PARAM_SPLIT_MIN_JOBS`` jobs when that was set)."""
     if form:
         return int(form)
-    return int(_lib.lib.cb_inflate_default_form(n_jobs if n_jobs is not None else 1 << 62))
+    return int(_lib.lib.cb_inflate_default_form(n_jobs if n_jobs is not None else 1 << 62,
+                                                out_bytes if out_bytes is not None else -1))
 
 
 def inflate_workspace_bytes(n_jobs: int, out_bytes: int, form: int = 0) -> int:
     """Workspace bytes of an inflate of ``n_jobs`` jobs writing ``out_bytes`` bytes in total, in ``form``."""
-    if inflate_form(form, n_jobs) == 3:
+    if inflate_form(form, n_jobs, out_bytes) == 3:
         return max(int(_lib.lib.cb_inflate_split_workspace_bytes(n_jobs, out_bytes)), 512)
     return int(_lib.lib.cb_inflate_workspace_bytes())
 

@@ -127,7 +127,7 @@ int header_size(const uint8_t* dev, int64_t avail, cudaStream_t s, int64_t* size
 }
 
 int inflate_ws_for(cb_batch* b) {
-    const int form = cb_inflate_default_form(b->total_jobs);
+    const int form = cb_inflate_default_form(b->total_jobs, b->total_out);
     b->form = form;
     b->inflate_ws_bytes = form == 3 ? cb_inflate_split_workspace_bytes(b->total_jobs, b->total_out)
                                     : cb_inflate_workspace_bytes();

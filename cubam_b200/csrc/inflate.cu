@@ -1473,9 +1473,12 @@ extern "C" int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const 
     constexpr int64_t ANY_WORKSPACE_JOBS = 8192;
     bool any_workspace = false;
     if (form == 0) {
-        form = cb_inflate_default_form(n_jobs);
+        const size_t empty = cb_inflate_split_workspace_bytes(n_jobs, 0);
+        // the members' bytes, as far as the workspace tells
+        const int64_t out_bytes = n_jobs < ANY_WORKSPACE_JOBS && workspace_bytes >= empty ? (int64_t)(workspace_bytes - empty) / 2 : -1;
+        form = cb_inflate_default_form(n_jobs, out_bytes);
         any_workspace = form == 3 && n_jobs < ANY_WORKSPACE_JOBS;
-        if (any_workspace && workspace_bytes < cb_inflate_split_workspace_bytes(n_jobs, 0)) form = 1;
+        if (any_workspace && workspace_bytes < empty) form = 1;
     }
     if (form == 3) {
         // the split form needs its arena: a workspace of the forms-1/2 size runs form 1 instead

@@ -474,7 +474,8 @@ class Server:
             jobs = scratch.get("jobs", nb)
             jobs[:nb].copy_(host[:nb], non_blocking=True)
             out_bytes = int(sum(int((x[:, 2] >> 32).sum()) for x in rows))  # sum of ISIZE (high half of word 2)
-            qws = scratch.get("queue", inflate_workspace_bytes(n_jobs, out_bytes))
+            need = inflate_workspace_bytes(n_jobs, out_bytes)
+            qws = scratch.get("queue", need)[:need]
             launch_inflate(jobs.data_ptr(), n_jobs, self.pool.data_ptr(), out_bytes, self.check_crc, summ.data_ptr(),
                            qws)
         csz = ctypes_sizeof(_lib.ChainSummary)

@@ -100,7 +100,7 @@ int cb_device_sm_count(void);
  *   CB_PARAM_DECODE_PREFETCH  no effect (kept for callers that set it): 0-16 (4)
  *   CB_PARAM_SPLIT_MIN_JOBS   with CB_PARAM_INFLATE_FORM 3, form 0 runs form 1 for calls of fewer jobs than this: 0
  *                          or more (CB_SPLIT_MIN_JOBS_ANY).  Until it is set there is no such number (it reads 8192
- *                          then), nor after cb_set_param(key, -1)
+ *                          then), nor after cb_set_param(key, -1), but form 1 runs for small members
  *   CB_PARAM_COPY_UNITS    no effect (kept for callers that set it): 1, 2 or 4 (2)
  *   CB_PARAM_DECODE_PIPELINE  form 3 in two job ranges, each decoded and then copied on its own stream
  *                          (side streams joined back to the caller's by events), so that one range's
@@ -184,8 +184,9 @@ int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_
                     int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
                     size_t workspace_bytes, int form, void* stream);
 
-/* The form that cb_inflate_form runs for n_jobs jobs with form 0 and a workspace for it. */
-int cb_inflate_default_form(int64_t n_jobs);
+/* The form to size a workspace for: what cb_inflate_form runs for n_jobs jobs of out_bytes inflated bytes together (-1:
+ * not known) with form 0 and a workspace of that form's size.  1 in place of 3 for small members (1,000 bytes at most). */
+int cb_inflate_default_form(int64_t n_jobs, int64_t out_bytes);
 
 /* Members the one-member-per-lane form keeps in flight on the current device (0 on error). */
 int64_t cb_inflate_lane_slots(void);
