@@ -13,6 +13,7 @@
 //     memory.  Each lane writes its symbols, literal bytes and 4-byte sequences of a literal count and
 //     a match, to a run of its own in the member's output range, which is free until the copy; the
 //     warps then put the runs together in the member's slot of an arena in HBM.
+//     k_literals copies the members that have no match.
 //  2. k_copy: one member per CTA of W warps.  They take 64 W sequences at a time, place them by a prefix
 //     sum of their lengths and write the output in rounds of 128 bytes per warp, a 4-byte word per lane,
 //     to a ring in shared memory (the sources of matches) and to HBM.
@@ -36,6 +37,7 @@
 
 #include "common.cuh"
 #include "crc.cuh"
+#include "spans.cuh"
 #include "split_slots.cuh"
 
 namespace cb {
@@ -79,6 +81,7 @@ constexpr int JW = PER_JOB / 4;           // words per job
 constexpr int PARTS = 2;                  // ranges of jobs of the pipelined form, each with two queue counters
 constexpr int Q_LISTED = 2 * PARTS;       // queue counter: members for the one-kernel form (and its queue)
 constexpr uint32_t ST_LISTED = 0x100;     // internal status: on that list
+constexpr uint32_t ST_LITERALS = 0x200;   // internal status: its output written by k_literals
 __host__ __device__ __forceinline__ size_t arena_offset(long long n_jobs) {
     return (WS_HEAD + PER_JOB * (size_t)n_jobs + 255) & ~(size_t)255;
 }
@@ -918,6 +921,43 @@ __global__ void __launch_bounds__(W == 1 ? 64 : W * 32, W == 1 ? 9 : 16 / W)
     }
 }
 
+// ---------------------------------------------------------------- k_literals: members without a match
+// Members of literals alone (stored blocks, or codes without matches) from their slots to their places, before k_copy,
+// which takes literals in groups of a few sequences of at most 255 and most of them byte by byte: in us, all of form 3
+// without this kernel and with it, of members of 65 KB of stored blocks: 3,000 1448 739, 20,000 7808 2779.  (In k_copy or
+// k_decode itself the code for it cost all other members 1 to 16%.)  A CTA looks at 32 members at a time, 64 bytes each,
+// and its warps take those it finds.
+__global__ void __launch_bounds__(256) k_literals(const cb_member_job* __restrict__ jobs, int64_t n_jobs,
+                                                  const int64_t* __restrict__ d_n_jobs, uint8_t* out_base, uint8_t* ws,
+                                                  const uint8_t* arena, long long j0, long long j1) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t* per_job = reinterpret_cast<uint32_t*>(ws + WS_HEAD);
+    long long n = n_jobs;
+    if (d_n_jobs) n = min((long long)n, (long long)*d_n_jobs);
+    n = min(n, j1);
+    for (long long jb = j0 + 32LL * blockIdx.x; jb < n; jb += 32LL * gridDim.x) {
+        bool found = false;
+        if (jb + lane < n) {
+            const uint32_t st = *reinterpret_cast<volatile uint32_t*>(per_job + JW * (jb + lane) + 1);
+            // (another warp may have copied it)
+            found = (st == CB_OK || st == ST_LITERALS) && per_job[JW * (jb + lane) + 4] == jobs[jb + lane].isize;
+        }
+        const uint32_t all = __ballot_sync(FULL, found);
+        for (uint32_t left = all, k = 0; left; left &= left - 1, k++) {
+            if (k % 8 != warp) continue;
+            const long long j = jb + __ffs((int)left) - 1;
+            const uint32_t isize = jobs[j].isize, ns = per_job[JW * j + 5];
+            const uint8_t* lits = arena + reinterpret_cast<const unsigned long long*>(per_job)[(JW / 2) * j + 1];
+            const uint32_t* sq = reinterpret_cast<const uint32_t*>(lits + slot_bytes(isize)) - 1;
+            uint32_t more = 0;
+            for (uint32_t i = lane; i < ns; i += 32) more |= __ldcg(sq - i) & 0xFFFFFFu;
+            if (__any_sync(FULL, more != 0)) continue;  // a match, of no valid distance
+            copy_long<32, 4>(lits, out_base + jobs[j].out_off, (int)isize, lane);
+            if (lane == 0) per_job[JW * j + 1] = ST_LITERALS;
+        }
+    }
+}
+
 // ---------------------------------------------------------------- k_copy: one member per CTA of W warps
 
 constexpr uint32_t LINE = 128;            // output bytes of a warp's round: a word per lane
@@ -1016,7 +1056,7 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
         const long long j = j0 + (long long)M.job;
         sync();
         if (j >= n) break;
-        if (per_job[JW * j + 1] != CB_OK) continue;  // k_decode reported or listed it
+        if (per_job[JW * j + 1] != CB_OK) continue;  // k_decode reported or listed it, or k_literals copied it
         const cb_member_job job = jobs[j];
         const uint8_t* lits = arena + reinterpret_cast<const unsigned long long*>(per_job)[(JW / 2) * j + 1];
         const uint2* sq = reinterpret_cast<const uint2*>(lits + slot_bytes(job.isize)) - 1;  // sequences 1, 0
@@ -1366,7 +1406,8 @@ __global__ void __launch_bounds__(CRC_NT)
     for (long long jb = j0 + (long long)blockIdx.x * PER; jb < n; jb += (long long)gridDim.x * PER) {
         const long long j = jb + warp / W;
         uint32_t c = 0, want = 0;
-        const bool on = j < n && per_job[JW * j + 1] == CB_OK;
+        const uint32_t st = j < n ? per_job[JW * j + 1] : (uint32_t)CB_ERR_INFLATE;
+        const bool on = st == CB_OK || st == ST_LITERALS;
         uint32_t len = 0;
         if (on) {
             const cb_member_job job = jobs[j];
@@ -1560,6 +1601,10 @@ int copy_range(const Call& c, Range r, cudaStream_t s) {
     using C4 = split::CopyCfg<16384, 4>;
     using C2 = split::CopyCfg<8192, 2>;
     const int cw = (int)cb_param(CB_PARAM_COPY_WARPS);
+    // (where members have more warps, the copy takes those of literals in less than this launch and look, 8 us)
+    if (!resident(c, copy_occupancy<C4>()))
+        split::k_literals<<<(unsigned)((r.j1 - r.j0 + 31) / 32 < 4096 ? (r.j1 - r.j0 + 31) / 32 : 4096), 256, 0, s>>>(
+            c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.ws, c.arena, r.j0, r.j1);
     int rc;
     if (resident(c, copy_occupancy<C8>())) rc = launch_copy<C8>(c, r, s);
     else if (resident(c, copy_occupancy<C4>())) rc = launch_copy<C4>(c, r, s);

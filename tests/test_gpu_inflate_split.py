@@ -177,3 +177,26 @@ def test_split_workspace_too_small_is_an_error():
     assert set(codes.tolist()) == {_lib.OK, _lib.CAPACITY} and codes[0] == 0 and codes[-1] == _lib.CAPACITY
     assert summ.status == _lib.CAPACITY
     assert out[: len(cases[0][0])].tobytes() == cases[0][0]
+
+
+@pytest.mark.parametrize("jobs", [30, 400, 700, 1300, 3100])
+def test_stored_members(jobs):
+    """Members of one or several stored blocks, alone and before or after coded ones, at every width."""
+    rng = random.Random(8)
+    noise = rng.randbytes(BLOCK)
+    text = bytes(rng.choices(b"ACGT\n0123", k=9000))
+    cases = [(noise, {"level": 0}), (noise, {}), (noise[:40_000], {"mem": 1}), (noise[:20_000], {"level": 0, "flush_every": 700}),
+             (noise[:20_000] + text, {}), (text + noise[:20_000], {}), (noise[:1], {"level": 0}), (text, {})]
+    times = -(-jobs // len(cases))
+    buf, table, total = _table(cases, 3)
+    rows = table.cpu().numpy()
+    total -= 3
+    many = np.concatenate([rows + np.array([0, k * total, 0, 0]) for k in range(times)])
+    size = G.inflate_workspace_bytes(len(many), times * total, 3)
+    out, codes, summ = _run(torch.from_numpy(many).cuda(), 3 + times * total, size, 3)
+    assert summ.status == 0 and not codes.any()
+    want = np.frombuffer(b"".join(d for d, _ in cases), dtype=np.uint8)
+    assert (out[3 : 3 + times * total].reshape(times, total) == want).all()
+    many[:, 3] ^= np.arange(len(many)) % 3 == 1  # a wrong CRC32
+    _, codes, summ = _run(torch.from_numpy(many).cuda(), 3 + times * total, size, 3)
+    assert (codes == np.where(np.arange(len(many)) % 3 == 1, _lib.CRC, _lib.OK)).all()
