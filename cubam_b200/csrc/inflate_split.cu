@@ -1621,29 +1621,74 @@ int copy_range(const Call& c, Range r, cudaStream_t s) {
                                   : launch_crc<1>(c, r, s);
 }
 
-// Two side streams per device for the pipelined form, and the events that join them to the caller's
-// stream; the mutex keeps each call's records and waits together (a wait takes the event's state
-// when it is called), so calls from several host threads may share them.
+// A pair of side streams for the pipelined form, and the events that join them to the caller's stream.  A caller's
+// stream keeps its pair, so that calls on several streams do not wait for one another; a stream beyond SIDES takes the
+// pair that was used longest ago (calls then queue behind one another).  Side streams that joined a capture belong to
+// it until it ends: no other call may use them meanwhile, or the capture is lost.  The mutex keeps each call's records
+// and waits together (a wait takes the event's state when it is called).
 struct Side {
-    cudaStream_t x = nullptr, y = nullptr;
+    cudaStream_t x = nullptr, y = nullptr, owner = nullptr;
     cudaEvent_t start = nullptr, done_x = nullptr, done_y = nullptr;
-    bool ready = false;
+    unsigned long long used = 0;  // when, counted in calls; 0: the pair is not made yet
 };
-Side g_side[MAX_DEVICES];
+constexpr int SIDES = 8;
+Side g_side[MAX_DEVICES][SIDES];
+unsigned long long g_side_calls = 0;
 std::mutex g_side_mu;
 
-int side_for(int dev, Side*& out) {
-    Side& sd = g_side[dev];
-    if (!sd.ready) {
-        cudaError_t e = cudaStreamCreateWithFlags(&sd.x, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&sd.y, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sd.start, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sd.done_x, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sd.done_y, cudaEventDisableTiming);
-        if (e != cudaSuccess) return cb_set_error(e);
-        sd.ready = true;
+// The capture that stream s is part of, 0 for none; -1 (as an unsigned number) for one that was lost or cannot be told.
+unsigned long long capture_of(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(s, &st, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return ~0ull;
     }
-    out = &sd;
+    return st == cudaStreamCaptureStatusNone ? 0 : st == cudaStreamCaptureStatusActive ? id : ~0ull;
+}
+
+int make_side(Side& sd) {
+    // (another thread's capture does not forbid this thread to make streams in this mode)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return cb_set_error(e);
+    if (!sd.x) e = cudaStreamCreateWithFlags(&sd.x, cudaStreamNonBlocking);
+    if (e == cudaSuccess && !sd.y) e = cudaStreamCreateWithFlags(&sd.y, cudaStreamNonBlocking);
+    if (e == cudaSuccess && !sd.start) e = cudaEventCreateWithFlags(&sd.start, cudaEventDisableTiming);
+    if (e == cudaSuccess && !sd.done_x) e = cudaEventCreateWithFlags(&sd.done_x, cudaEventDisableTiming);
+    if (e == cudaSuccess && !sd.done_y) e = cudaEventCreateWithFlags(&sd.done_y, cudaEventDisableTiming);
+    const cudaError_t back = cudaThreadExchangeStreamCaptureMode(&mode);
+    return cb_set_error(e != cudaSuccess ? e : back);
+}
+
+// The pair for a call on s, under g_side_mu; none (out is null) when other captures hold them all.
+int side_for(int dev, cudaStream_t s, Side*& out) {
+    out = nullptr;
+    const unsigned long long capture = capture_of(s);
+    Side *oldest = nullptr, *fresh = nullptr;
+    for (Side& sd : g_side[dev]) {
+        if (!sd.used) {
+            if (!fresh) fresh = &sd;
+            continue;
+        }
+        const unsigned long long of = capture_of(sd.x);
+        if (of != 0 && of != capture) continue;
+        if (sd.owner == s) {
+            out = &sd;
+            break;
+        }
+        if (!oldest || sd.used < oldest->used) oldest = &sd;
+    }
+    if (!out && fresh) {
+        const int rc = make_side(*fresh);
+        if (rc != CB_OK) return rc;
+        out = fresh;
+    }
+    if (!out) out = oldest;
+    if (out) {
+        out->owner = s;
+        out->used = ++g_side_calls;
+    }
     return CB_OK;
 }
 
@@ -1689,20 +1734,23 @@ int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_
         }
         const bool two = !d_n_jobs && n_jobs >= 2 && (pipe == 2 || (pipe == 1 && many));
         int rc = CB_OK;
-        if (!two) {
+        std::unique_lock<std::mutex> lock(g_side_mu, std::defer_lock);
+        Side* sd = nullptr;
+        if (two) {
+            int dev = 0;
+            const cudaError_t e = cudaGetDevice(&dev);
+            if (e != cudaSuccess) return cb_set_error(e);
+            if (dev < 0 || dev >= MAX_DEVICES) return CB_ERR_ARG;
+            lock.lock();
+            if ((rc = side_for(dev, s, sd)) != CB_OK) return rc;
+        }
+        if (!sd) {
             const Range all{0, n_jobs, 0};
             rc = decode_range(c, all, s);
             if (rc == CB_OK) rc = copy_range(c, all, s);
             if (rc != CB_OK) return rc;
         } else {
-            int dev = 0;
-            cudaError_t e = cudaGetDevice(&dev);
-            if (e != cudaSuccess) return cb_set_error(e);
-            if (dev < 0 || dev >= MAX_DEVICES) return CB_ERR_ARG;
-            std::lock_guard<std::mutex> lock(g_side_mu);
-            Side* sd = nullptr;
-            if ((rc = side_for(dev, sd)) != CB_OK) return rc;
-            e = cudaEventRecord(sd->start, s);
+            cudaError_t e = cudaEventRecord(sd->start, s);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(sd->x, sd->start, 0);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(sd->y, sd->start, 0);
             if (e != cudaSuccess) return cb_set_error(e);
@@ -1723,6 +1771,7 @@ int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_
             if (rc != CB_OK) return rc;
             if (e != cudaSuccess) return cb_set_error(e);
         }
+        if (lock.owns_lock()) lock.unlock();
         rc = cb_inflate_listed(jobs, reinterpret_cast<const uint32_t*>(ws + split::WS_HEAD), split::JW,
                                queue + split::Q_LISTED,
                                out_base, check_crc, job_status, summary, queue + split::Q_LISTED + 1, s);

@@ -105,9 +105,10 @@ int cb_device_sm_count(void);
  *   CB_PARAM_DECODE_PIPELINE  form 3 in two job ranges, each decoded and then copied on its own stream
  *                          (side streams joined back to the caller's by events), so that one range's
  *                          decode and the other's copy fill the lanes a decode leaves idle at its end:
- *                          0 never, 1 from 20 jobs per SM, 2 always; only with the job count given on the
- *                          host (d_n_jobs NULL).  The side streams and events are created by the first
- *                          pipelined call on a device, which should come before any stream capture (1)
+ *                          0 never, 1 from 20 jobs per SM (from 65,536 jobs while the caller's stream is
+ *                          captured), 2 always; only with the job count given on the host (d_n_jobs NULL).
+ *                          Each of up to 8 caller's streams on a device has side streams of its own, made by its
+ *                          first pipelined call; while a capture holds all of them, calls run in one range (1)
  * cb_set_param(key, -1) restores the default; an unknown key or a value out of range is CB_ERR_ARG.
  * cb_get_param returns the current value, -1 for an unknown key. */
 enum {
