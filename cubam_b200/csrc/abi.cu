@@ -58,17 +58,16 @@ int64_t cb_param(int key) {
 }
 
 // CB_PARAM_INFLATE_FORM.  For form 3 the caller may have set a number of jobs below which form 1 runs; by itself form 1
-// runs for members so small that form 3's three kernels and its tables per member cost more than its segments give (39
-// GEX members of 65 KB take form 3 0.4 ms and form 1 4.2 ms).  In us, form 3 and 1, of GEX members: 100 of 400 bytes 105 90,
-// of 700 108 119; 2,000 of 700 bytes 146 133, of 1,000 151 156; 8,000 of 1,000 404 362, of 1,500 406 480; 200,000 of 700
-// 7660 6610, of 1,000 8000 7800.  (Members of nearly equal codes gain up to 1,500 bytes: 2,000 of base64 368 220.)
+// runs for members so small that form 3's kernels and its tables per member cost more than its segments give (39 GEX
+// members of 65 KB take form 3 0.4 ms and form 1 4.2 ms).  In us, form 3 and 1: 100 GEX members of 400 bytes 92 90, of 700
+// 93 117; 8,000 of 400 267 224, of 700 298 326; 200,000 of 400 5300 4640, of 700 6260 6610; text is even at 700 bytes.
 extern "C" int cb_inflate_default_form(int64_t n_jobs, int64_t out_bytes) {
     const int form = (int)cb_param(CB_PARAM_INFLATE_FORM);
     if (form != 3) return form;
     if (g_param_set[param_index(CB_PARAM_SPLIT_MIN_JOBS)].load(std::memory_order_acquire))
         return n_jobs < cb_param(CB_PARAM_SPLIT_MIN_JOBS) ? 1 : 3;
-    const int64_t small = n_jobs < 600 ? 600 : 1000;
-    return out_bytes >= 0 && n_jobs > 0 && out_bytes / n_jobs <= small ? 1 : 3;
+    constexpr int64_t SMALL = 600;
+    return out_bytes >= 0 && n_jobs > 0 && out_bytes / n_jobs <= SMALL ? 1 : 3;
 }
 
 extern "C" int64_t cb_get_param(int key) { return param_index(key) < 0 ? -1 : cb_param(key); }

@@ -11,8 +11,8 @@
 //     first symbol that begins in it; that must be where the lane before stopped, and a lane for which
 //     it is not decodes its segment again from there.  The lanes share one set of code tables in shared
 //     memory.  Each lane writes its symbols, literal bytes and 4-byte sequences of a literal count and
-//     a match, to a run of its own in the member's output range, which is free until the copy; the
-//     warps then put the runs together in the member's slot of an arena in HBM.
+//     a match, to a run of its own in the scratch of the members in flight; the warps
+//     then put the runs together in the member's slot of an arena in HBM.
 //     k_literals copies the members that have no match.
 //  2. k_copy: one member per CTA of W warps.  They take 64 W sequences at a time, place them by a prefix
 //     sum of their lengths and write the output in rounds of 128 bytes per warp, a 4-byte word per lane,
@@ -30,7 +30,7 @@
 //
 // Every loop is bounded: a decode step consumes input bits, bounded per member, a repair round
 // confirms at least one more segment; every shared-memory index is masked or checked; arena and
-// output writes stay within the member's slot and output range.
+// scratch writes stay within the member's, output writes within its output range.
 
 #include <mutex>
 #include <type_traits>
@@ -169,7 +169,9 @@ constexpr uint32_t DST = (1u << ROOT) + LNG;
 constexpr uint32_t OVERLAP = 640;
 constexpr uint32_t SEG_MIN = 128;      // bits of a segment, at least
 constexpr uint32_t WINDOW = 179200;    // bits of a window of segments: a zlib block of 16,383 BAM symbols
-constexpr uint32_t RUN_MIN = 256;      // bytes of scratch per lane, at least (or one lane decodes alone)
+// bytes of scratch per lane, at least (or one lane decodes alone): more lanes for small members, with the more overlap (in
+// us, with 128, 192 and 256: 4,000 GEX members of 700 bytes 187 187 192, 400 of text of 3,000 133 121 126)
+constexpr uint32_t RUN_MIN = 192;
 constexpr int ROWS = 16;               // words of input kept per lane
 constexpr int STEPS = 8;               // decode steps between refills
 constexpr uint32_t LSTAGE = 32, SSTAGE = 16;  // staged literals (bytes) and sequences per lane
@@ -788,11 +790,11 @@ __device__ uint32_t decode_block(DecMember<W>& M, LaneIn& in, uint32_t& p0, uint
     }
 }
 
-// One member's symbols into its slot, by the whole CTA (out: the member's output, scratch until it is
-// written).  CB_OK, CB_ERR_INFLATE or ST_LISTED, the same in every thread.
+// One member's symbols into its slot, by the whole CTA, with scratch_n bytes of scratch.  CB_OK, CB_ERR_INFLATE or
+// ST_LISTED, the same in every thread.
 template <int W>
-__device__ uint32_t decode_member(DecMember<W>& M, const cb_member_job& job, uint8_t* slot, uint8_t* out, uint32_t& nl,
-                                  uint32_t& ns) {
+__device__ uint32_t decode_member(DecMember<W>& M, const cb_member_job& job, uint8_t* slot, uint8_t* scratch,
+                                  uint32_t scratch_n, uint32_t& nl, uint32_t& ns) {
     const uint32_t tid = threadIdx.x % (32 * W), lane = tid & 31, warp = tid >> 5;
     LaneIn in;
     const uintptr_t src = (uintptr_t)job.in;
@@ -801,9 +803,6 @@ __device__ uint32_t decode_member(DecMember<W>& M, const cb_member_job& job, uin
     uint32_t p = (uint32_t)(src & 15) * 8;
     const uint32_t s0 = p, E = p + job.in_len * 8u;
     const uint32_t slot_n = (uint32_t)slot_bytes(job.isize);
-    const uint32_t skip = (uint32_t)(-(intptr_t)out & 15);
-    uint8_t* scratch = out + skip;
-    const uint32_t scratch_n = job.isize > skip ? (job.isize - skip) & ~15u : 0u;
     uint8_t* lens = reinterpret_cast<uint8_t*>(M.w[0].lst);
     nl = ns = 0;
     if (!in_reach(job.in_len, job.isize)) return ST_LISTED;
@@ -888,9 +887,12 @@ __device__ uint32_t decode_member(DecMember<W>& M, const cb_member_job& job, uin
 template <int W>
 __global__ void __launch_bounds__(W == 1 ? 64 : W * 32, W == 1 ? 9 : 16 / W)
     k_decode(const cb_member_job* __restrict__ jobs, int64_t n_jobs, const int64_t* __restrict__ d_n_jobs,
-             uint8_t* out_base, uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws, uint8_t* arena,
-             unsigned long long arena_bytes, bool list_unfit, long long j0, long long j1, int qi) {
+             uint32_t* job_status, cb_inflate_summary* summary, uint8_t* ws, uint8_t* arena,
+             unsigned long long arena_bytes, uint8_t* scratch, uint32_t scratch_n, bool list_unfit, long long j0, long long j1,
+             int qi) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
+    constexpr int MEMBERS = W == 1 ? 2 : 1;  // per CTA
+    scratch += (unsigned long long)(blockIdx.x * MEMBERS + threadIdx.x / (32 * W)) * scratch_n;
     DecMember<W>& M = reinterpret_cast<DecMember<W>*>(smem_raw)[threadIdx.x / (32 * W)];
     const bool first = threadIdx.x % (32 * W) == 0;
     unsigned long long* queue = reinterpret_cast<unsigned long long*>(ws);
@@ -907,7 +909,7 @@ __global__ void __launch_bounds__(W == 1 ? 64 : W * 32, W == 1 ? 9 : 16 / W)
         const unsigned long long so = reinterpret_cast<const unsigned long long*>(per_job)[(JW / 2) * j + 1];
         uint32_t nl = 0, ns = 0;
         const uint32_t st = so + slot_bytes(job.isize) <= arena_bytes
-                                ? decode_member<W>(M, job, arena + so, out_base + job.out_off, nl, ns)
+                                ? decode_member<W>(M, job, arena + so, scratch, scratch_n, nl, ns)
                             : list_unfit ? ST_LISTED
                                          : (uint32_t)CB_ERR_CAPACITY;
         sync_member<W>();
@@ -1224,7 +1226,7 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
             half ^= 1;
             load_lits();
             if (g < ns) {
-                plan(P0);
+                plan(P0 & ~3u);  // (the word that P0 lies in is stored by this group)
                 load_seqs(g + cnt);
             }
             sync();
@@ -1340,8 +1342,8 @@ __global__ void __launch_bounds__(C::T, C::W == 1 ? 28 : 1)
                 ring4[(w & C::RMASK) >> 2] = word;
                 if (rel < pe && rel + 4 > p0) {
                     if (rel >= full0 && rel + 4 <= full1) {
-                        // bytes of the word after the group's end are overwritten by the next one
-                        *reinterpret_cast<uint32_t*>(base + w) = word;
+                        // (a word that the group ends in is left to the next one: only final bytes are ever stored)
+                        if (rel + 4 <= pe) *reinterpret_cast<uint32_t*>(base + w) = word;
                     } else {  // the member's first or last word: its own bytes only
                         for (uint32_t s = max(w, P0); s < min(w + 4, R0 + pe); s++) base[s] = (uint8_t)(word >> (8 * (s - w)));
                     }
@@ -1523,6 +1525,8 @@ struct Call {
     cb_inflate_summary* summary;
     uint8_t *ws, *arena;
     unsigned long long arena_bytes;
+    uint8_t* scratch;  // decode's, scratch_n bytes per member in flight
+    uint32_t scratch_n;
     bool list_unfit;
 };
 
@@ -1530,6 +1534,7 @@ struct Call {
 struct Range {
     long long j0, j1;
     int qd;
+    long long s0, s1;  // its members in flight: [s0, s1) of the scratch
 };
 
 // CTAs for a persistent grid of `occ` per SM, `members` each at a time, no more than the range has work for.
@@ -1564,9 +1569,12 @@ int launch_decode(const Call& c, Range r, cudaStream_t s) {
     constexpr int MEMBERS = W == 1 ? 2 : 1, NT = 32 * W * MEMBERS;
     const int o = decode_occupancy<W>();
     if (o <= 0) return fail_occ(o);
-    split::k_decode<W><<<grid_for(c, r, o, MEMBERS), NT, MEMBERS * sizeof(split::DecMember<W>), s>>>(
-        c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.job_status, c.summary, c.ws, c.arena, c.arena_bytes, c.list_unfit,
-        r.j0, r.j1, r.qd);
+    const long long room = (r.s1 - r.s0) / MEMBERS;
+    if (room < 1) return CB_ERR_ARG;
+    const unsigned grid = grid_for(c, r, o, MEMBERS);
+    split::k_decode<W><<<grid < room ? grid : (unsigned)room, NT, MEMBERS * sizeof(split::DecMember<W>), s>>>(
+        c.jobs, c.n_jobs, c.d_n_jobs, c.job_status, c.summary, c.ws, c.arena, c.arena_bytes, c.scratch + r.s0 * c.scratch_n,
+        c.scratch_n, c.list_unfit, r.j0, r.j1, r.qd);
     return CB_OK;
 }
 
@@ -1696,7 +1704,7 @@ int side_for(int dev, cudaStream_t s, Side*& out) {
 
 extern "C" size_t cb_inflate_split_workspace_bytes(int64_t n_jobs, int64_t out_bytes) {
     if (n_jobs < 0 || out_bytes < 0) return 0;
-    return split::arena_offset(n_jobs) + 2 * (size_t)out_bytes + 80 * (size_t)n_jobs + 32;
+    return split::arena_offset(n_jobs) + 80 * (size_t)n_jobs + 32 + split::arena_and_scratch(n_jobs, out_bytes);
 }
 
 extern "C" int cb_inflate_split(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base,
@@ -1713,8 +1721,13 @@ int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
     uint8_t* arena = reinterpret_cast<uint8_t*>(((uintptr_t)(ws + split::arena_offset(n_jobs)) + 15) & ~(uintptr_t)15);
-    const Call c{jobs, n_jobs, d_n_jobs, out_base, check_crc, job_status, summary, ws, arena,
-                 (unsigned long long)(ws + workspace_bytes - arena), list_unfit};
+    // the scratch of the members in flight at the workspace's end, the arena before it
+    const unsigned long long rest = (unsigned long long)(ws + workspace_bytes - arena), fixed = 80ull * n_jobs + 16;
+    const long long flight = split::in_flight(n_jobs);
+    const uint32_t scratch_n = split::scratch_for(n_jobs, rest > fixed ? rest - fixed : 0);
+    const unsigned long long arena_bytes = (rest - (unsigned long long)flight * scratch_n) & ~15ull;
+    const Call c{jobs, n_jobs, d_n_jobs, out_base, check_crc, job_status, summary, ws, arena, arena_bytes,
+                 arena + arena_bytes, scratch_n, list_unfit};
     auto* queue = reinterpret_cast<unsigned long long*>(ws);
     split::k_split_init<<<1, 1, 0, s>>>(summary, queue);
     if (n_jobs > 0) {
@@ -1745,7 +1758,7 @@ int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_
             if ((rc = side_for(dev, s, sd)) != CB_OK) return rc;
         }
         if (!sd) {
-            const Range all{0, n_jobs, 0};
+            const Range all{0, n_jobs, 0, 0, flight};
             rc = decode_range(c, all, s);
             if (rc == CB_OK) rc = copy_range(c, all, s);
             if (rc != CB_OK) return rc;
@@ -1754,15 +1767,11 @@ int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_
             if (e == cudaSuccess) e = cudaStreamWaitEvent(sd->x, sd->start, 0);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(sd->y, sd->start, 0);
             if (e != cudaSuccess) return cb_set_error(e);
-            constexpr int parts = split::PARTS;
-            for (int k = 0; k < parts && rc == CB_OK; k += 2) {
-                const Range ra{n_jobs * k / parts, n_jobs * (k + 1) / parts, 2 * k};
-                const Range rb{n_jobs * (k + 1) / parts, n_jobs * (k + 2) / parts, 2 * k + 2};
-                rc = decode_range(c, ra, sd->x);
-                if (rc == CB_OK) rc = decode_range(c, rb, sd->y);
-                if (rc == CB_OK) rc = copy_range(c, ra, sd->x);
-                if (rc == CB_OK) rc = copy_range(c, rb, sd->y);
-            }
+            const Range ra{0, n_jobs / 2, 0, 0, flight / 2}, rb{n_jobs / 2, n_jobs, 2, flight / 2, flight};
+            rc = decode_range(c, ra, sd->x);
+            if (rc == CB_OK) rc = decode_range(c, rb, sd->y);
+            if (rc == CB_OK) rc = copy_range(c, ra, sd->x);
+            if (rc == CB_OK) rc = copy_range(c, rb, sd->y);
             // join both side streams back to the caller's stream whatever happened above
             e = cudaEventRecord(sd->done_x, sd->x);
             if (e == cudaSuccess) e = cudaEventRecord(sd->done_y, sd->y);

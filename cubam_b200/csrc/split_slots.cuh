@@ -25,5 +25,34 @@ __host__ __device__ constexpr bool in_reach(uint32_t in_len, uint32_t isize) {
 }
 static_assert(slot_bytes(MAX_ISIZE) < 1ull << 32, "a slot is counted in 32 bits");
 
+// The decode's scratch, apart from the members' output: jobs may share their output or have it read meanwhile, and a
+// member's lanes are not bounded by its size (with the output as scratch three took part in one of 1,000 bytes: 8,000 GEX
+// members of them 404 us, now 315; 65 KB members as before).  Every member in flight (at most FLIGHT: 18 warps on 148 SMs,
+// twice for two ranges) has scratch_bytes, four times the members' mean size (a lane's run holds its symbols with some
+// room, and 21 lanes take part from 4,096 bytes on) up to 64 KiB.
+constexpr long long FLIGHT = 2 * 18 * 148;
+constexpr uint32_t SCRATCH_MIN = 4096, SCRATCH_MAX = 65536;
+constexpr long long in_flight(long long n_jobs) { return n_jobs < FLIGHT ? n_jobs : FLIGHT; }
+constexpr uint32_t scratch_bytes(long long n_jobs, unsigned long long out_bytes) {
+    const unsigned long long s = n_jobs > 0 ? (out_bytes / (unsigned long long)n_jobs * 4 + 4095) & ~4095ull : 0;
+    return s < SCRATCH_MIN ? SCRATCH_MIN : s > SCRATCH_MAX ? SCRATCH_MAX : (uint32_t)s;
+}
+// What the arena (without 80 bytes a job) and the scratch take together for out_bytes of output.
+constexpr unsigned long long arena_and_scratch(long long n_jobs, unsigned long long out_bytes) {
+    return 2 * out_bytes + (unsigned long long)in_flight(n_jobs) * scratch_bytes(n_jobs, out_bytes);
+}
+// The scratch per member of a workspace that has `room` for the two: that of the most output it is large enough for
+// (so of out_bytes, where it was made for them), or none.
+inline uint32_t scratch_for(long long n_jobs, unsigned long long room) {
+    if (arena_and_scratch(n_jobs, 0) > room) return 0;
+    unsigned long long lo = 0, hi = room / 2 + 1;  // enough for lo, not for hi
+    while (hi - lo > 1) {
+        const unsigned long long mid = lo + (hi - lo) / 2;
+        if (arena_and_scratch(n_jobs, mid) <= room) lo = mid;
+        else hi = mid;
+    }
+    return scratch_bytes(n_jobs, lo);
+}
+
 }  // namespace split
 }  // namespace cb

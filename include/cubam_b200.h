@@ -186,7 +186,8 @@ int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_
                     size_t workspace_bytes, int form, void* stream);
 
 /* The form to size a workspace for: what cb_inflate_form runs for n_jobs jobs of out_bytes inflated bytes together (-1:
- * not known) with form 0 and a workspace of that form's size.  1 in place of 3 for small members (1,000 bytes at most). */
+ * not known) with form 0 and a workspace of that form's size.  1 in place of 3 for members of 600 bytes or
+ * less on average. */
 int cb_inflate_default_form(int64_t n_jobs, int64_t out_bytes);
 
 /* Members the one-member-per-lane form keeps in flight on the current device (0 on error). */
@@ -195,8 +196,8 @@ int64_t cb_inflate_lane_slots(void);
 /* ---- Inflate, form 3: the Huffman decode, the copy and the CRC32 as three kernels (same contract as
  *      cb_inflate, replacing the same nvCOMP call, src/cubam/bgzf.py:587-611) ------------------------
  * Each takes a member per 1 to 8 warps, more the fewer jobs there are.  The decode's lanes decode 32
- * segments per warp at once, with the member's output range as scratch, into an arena inside the workspace
- * (32 bytes and a slot of 2 isize + 64 bytes per job, rounded up to 16); the copy writes the member through
+ * segments per warp at once into an arena inside the workspace (32 bytes and a slot of 2 isize + 64 bytes per job,
+ * rounded up to 16, and scratch of 4 to 64 KiB for each of at most 5,328 members in flight); the copy writes the member through
  * a window in shared memory (CB_PARAM_COPY_WARPS, where a member has one warp).
  * out_bytes: the sum of isize over the jobs (or more); a job whose slot does not fit a smaller
  * workspace fails with CB_ERR_CAPACITY. */

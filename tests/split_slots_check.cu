@@ -23,6 +23,24 @@ int main() {
     }
     if (!in_reach(65535, 65536)) failures++;
     if (in_reach(3u << 20, 3u << 30)) failures++;  // 3 GB of zeros
+    // a workspace made for some output has the scratch for it and leaves the arena whole; a larger one no less of either
+    for (long long n : {1LL, 2LL, 39LL, 5327LL, 5328LL, 5329LL, 200'000LL, 10'000'000LL}) {
+        if (in_flight(n) > n || in_flight(n) > FLIGHT) failures++;
+        for (unsigned long long mean : {0ull, 1ull, 100ull, 1023ull, 1024ull, 1025ull, 4096ull, 16384ull, 16385ull, 65280ull, 1ull << 26}) {
+            for (unsigned long long more : {0ull, 1ull, 5ull}) {
+                const unsigned long long out = mean * n + more, need = arena_and_scratch(n, out);
+                for (unsigned long long k : {0ull, 1ull, 15ull, 16ull, 4095ull, 1ull << 20, 1ull << 40}) {
+                    const uint32_t s = scratch_for(n, need + k);
+                    const bool ok = s >= scratch_bytes(n, out) && (k > 16 || s == scratch_bytes(n, out)) &&
+                                    s % 4096 == 0 && s <= SCRATCH_MAX && need + k - (unsigned long long)in_flight(n) * s >= 2 * out;
+                    if (!ok && failures++ < 10) printf("FAIL %lld members, %llu bytes, %llu more: %u\n", n, out, k, s);
+                }
+                // a smaller one keeps room for what it holds
+                const unsigned long long less = need / 3;
+                if ((unsigned long long)in_flight(n) * scratch_for(n, less) > less && failures++ < 10) printf("FAIL %lld, %llu\n", n, less);
+            }
+        }
+    }
     printf("%d failures\n", failures);
     return failures != 0;
 }

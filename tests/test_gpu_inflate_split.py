@@ -200,3 +200,31 @@ def test_stored_members(jobs):
     many[:, 3] ^= np.arange(len(many)) % 3 == 1  # a wrong CRC32
     _, codes, summ = _run(torch.from_numpy(many).cuda(), 3 + times * total, size, 3)
     assert (codes == np.where(np.arange(len(many)) % 3 == 1, _lib.CRC, _lib.OK)).all()
+
+
+@pytest.mark.parametrize("jobs", [40, 400, 800, 3100])
+def test_jobs_may_share_their_output(jobs):
+    """Every member twice in a call, with one place for both; and places that are read while they are written again."""
+    rng = random.Random(9)
+    cases = [(bytes(rng.choices(b"ACGT\n0123", k=rng.choice([900, 9000, BLOCK]))), {"level": rng.choice([1, 6])}) for _ in range(20)]
+    buf, table, total = _table(cases)
+    rows = table.cpu().numpy()
+    half = jobs // 2
+    many = np.concatenate([rows + np.array([0, k * total, 0, 0]) for k in range(-(-half // len(cases)))])[:half]
+    both = torch.from_numpy(np.concatenate([many, many[::-1]])).cuda()
+    n = int(many[-1, 1] + (many[-1, 2] >> 32))
+    want = np.frombuffer(b"".join(d for d, _ in cases) * (len(many) // len(cases) + 1), dtype=np.uint8)[:n]
+    out = torch.full((n,), 0xA5, dtype=torch.uint8, device="cuda")
+    seen = torch.empty_like(out)
+    summ = torch.zeros(G.ctypes_sizeof(_lib.InflateSummary), dtype=torch.uint8, device="cuda")
+    ws = torch.empty(G.inflate_workspace_bytes(len(both), 2 * n, 3), dtype=torch.uint8, device="cuda")
+    reader = torch.cuda.Stream()
+    for k in range(3):
+        G.launch_inflate(both.data_ptr(), len(both), out.data_ptr(), 2 * n, True, summ.data_ptr(), ws, 3)
+        assert G.read_struct(summ, _lib.InflateSummary).status == 0
+        assert np.array_equal(out.cpu().numpy(), want)
+        G.launch_inflate(both.data_ptr(), len(both), out.data_ptr(), 2 * n, True, summ.data_ptr(), ws, 3)
+        with torch.cuda.stream(reader):
+            seen.copy_(out)
+        torch.cuda.synchronize()
+        assert np.array_equal(seen.cpu().numpy(), want)

@@ -20,7 +20,7 @@ def test_no_least_number_of_jobs_until_one_is_set():
 
 def test_small_members_take_form_1():
     """A rule on the mean size, and the workspace of the form that it names."""
-    for n, small in ((1, 600), (39, 600), (599, 600), (600, 1000), (8192, 1000), (1 << 20, 1000)):
+    for n, small in ((1, 600), (39, 600), (8192, 600), (1 << 20, 600)):
         assert bgzf.inflate_form(0, n, n * small) == 1 and bgzf.inflate_form(0, n, n * (small + 1)) == 3
         assert bgzf.inflate_workspace_bytes(n, n * small) == int(L.cb_inflate_workspace_bytes())
         assert bgzf.inflate_workspace_bytes(n, n * (small + 1)) >= int(L.cb_inflate_split_workspace_bytes(n, n * (small + 1)))
