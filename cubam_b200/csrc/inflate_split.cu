@@ -926,10 +926,11 @@ __global__ void __launch_bounds__(W == 1 ? 64 : W * 32, W == 1 ? 9 : 16 / W)
 // ---------------------------------------------------------------- k_literals: members without a match
 // Members of literals alone (stored blocks, or codes without matches) from their slots to their places, before k_copy,
 // which takes literals in groups of a few sequences of at most 255 and most of them byte by byte: in us, all of form 3
-// without this kernel and with it, of members of 65 KB of stored blocks: 3,000 1448 739, 20,000 7808 2779.  (In k_copy or
-// k_decode itself the code for it cost all other members 1 to 16%.)  A CTA looks at 32 members at a time, 64 bytes each,
-// and its warps take those it finds.
-__global__ void __launch_bounds__(256) k_literals(const cb_member_job* __restrict__ jobs, int64_t n_jobs,
+// without this kernel and with it, of members of 65 KB of stored blocks: 3,000 1448 769, 20,000 7808 2724.  (In k_copy or
+// k_decode itself the code for it cost all other members 1 to 16%, in k_crc 3%.)  A CTA looks at LOOK members at a time, 64
+// bytes each, and its two warps take those it finds; it is small, to find room beside the other range's kernels.
+constexpr int LOOK = 8;
+__global__ void __launch_bounds__(64) k_literals(const cb_member_job* __restrict__ jobs, int64_t n_jobs,
                                                   const int64_t* __restrict__ d_n_jobs, uint8_t* out_base, uint8_t* ws,
                                                   const uint8_t* arena, long long j0, long long j1) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -937,16 +938,16 @@ __global__ void __launch_bounds__(256) k_literals(const cb_member_job* __restric
     long long n = n_jobs;
     if (d_n_jobs) n = min((long long)n, (long long)*d_n_jobs);
     n = min(n, j1);
-    for (long long jb = j0 + 32LL * blockIdx.x; jb < n; jb += 32LL * gridDim.x) {
+    for (long long jb = j0 + (long long)LOOK * blockIdx.x; jb < n; jb += (long long)LOOK * gridDim.x) {
         bool found = false;
-        if (jb + lane < n) {
+        if (lane < LOOK && jb + lane < n) {
             const uint32_t st = *reinterpret_cast<volatile uint32_t*>(per_job + JW * (jb + lane) + 1);
             // (another warp may have copied it)
             found = (st == CB_OK || st == ST_LITERALS) && per_job[JW * (jb + lane) + 4] == jobs[jb + lane].isize;
         }
         const uint32_t all = __ballot_sync(FULL, found);
         for (uint32_t left = all, k = 0; left; left &= left - 1, k++) {
-            if (k % 8 != warp) continue;
+            if (k % 2 != warp) continue;
             const long long j = jb + __ffs((int)left) - 1;
             const uint32_t isize = jobs[j].isize, ns = per_job[JW * j + 5];
             const uint8_t* lits = arena + reinterpret_cast<const unsigned long long*>(per_job)[(JW / 2) * j + 1];
@@ -954,7 +955,7 @@ __global__ void __launch_bounds__(256) k_literals(const cb_member_job* __restric
             uint32_t more = 0;
             for (uint32_t i = lane; i < ns; i += 32) more |= __ldcg(sq - i) & 0xFFFFFFu;
             if (__any_sync(FULL, more != 0)) continue;  // a match, of no valid distance
-            copy_long<32, 4>(lits, out_base + jobs[j].out_off, (int)isize, lane);
+            copy_long<32, 2>(lits, out_base + jobs[j].out_off, (int)isize, lane);
             if (lane == 0) per_job[JW * j + 1] = ST_LITERALS;
         }
     }
@@ -1611,7 +1612,7 @@ int copy_range(const Call& c, Range r, cudaStream_t s) {
     const int cw = (int)cb_param(CB_PARAM_COPY_WARPS);
     // (where members have more warps, the copy takes those of literals in less than this launch and look, 8 us)
     if (!resident(c, copy_occupancy<C4>()))
-        split::k_literals<<<(unsigned)((r.j1 - r.j0 + 31) / 32 < 4096 ? (r.j1 - r.j0 + 31) / 32 : 4096), 256, 0, s>>>(
+        split::k_literals<<<(unsigned)min((r.j1 - r.j0 + split::LOOK - 1) / split::LOOK, 32768LL), 64, 0, s>>>(
             c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.ws, c.arena, r.j0, r.j1);
     int rc;
     if (resident(c, copy_occupancy<C8>())) rc = launch_copy<C8>(c, r, s);
