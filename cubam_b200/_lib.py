@@ -82,6 +82,7 @@ _SIGNATURES = {
     "cb_inflate_workspace_bytes": (c_size_t, []),
     "cb_inflate": (c_int, [P, I64, P, P, c_int, P, P, P, c_size_t, P]),
     "cb_inflate_default_form": (c_int, [I64, I64]),
+    "cb_inflate_launches": (c_int, [I64, c_int, c_int, c_int]),
     "cb_inflate_form": (c_int, [P, I64, P, P, c_int, P, P, P, c_size_t, c_int, P]),
     "cb_inflate_lane_slots": (I64, []),
     "cb_inflate_split_workspace_bytes": (c_size_t, [I64, I64]),

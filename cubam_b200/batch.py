@@ -38,7 +38,7 @@ from cubam_b200.bgzf import (
     stream_ptr,
 )
 
-#: kernels launched by each entry point (for the launch count of a step)
+#: kernels launched by each entry point (for the launch count of a step; inflate: forms 1 and 2)
 KERNELS = {"scan": 4, "inflate": 3, "chain": 9, "records": 1}
 
 
@@ -52,10 +52,11 @@ def _tag_arrays(k: int, nrec: int):
             torch.empty((k, nrec), dtype=torch.int64, device="cuda"))
 
 
-def inflate_launches(form: int = 0, n_jobs: int | None = None) -> int:
-    """Kernels of one inflate call: init, the persistent grid, finish; form 3 adds the slot scan, splits
-    the grid into decode, copy and CRC32, and launches the one-kernel form for members it leaves."""
-    return 7 if inflate_form(form, n_jobs) == 3 else KERNELS["inflate"]
+def inflate_launches(form: int = 0, n_jobs: int | None = None, out_bytes: int | None = None, check_crc: bool = True,
+                     captured: bool = False) -> int:
+    """Kernels of one inflate call of ``n_jobs`` jobs (many, if None), launched or captured."""
+    n = n_jobs if n_jobs is not None else 1 << 62
+    return int(_lib.lib.cb_inflate_launches(n, inflate_form(form, n_jobs, out_bytes), int(check_crc), int(captured)))
 
 
 @dataclass
@@ -167,7 +168,7 @@ def decode_many(files: list[tuple[torch.Tensor, BamHeader]], tags=("CB", "UB", "
         launch_inflate(all_jobs.data_ptr(), n_jobs, out.data_ptr(), total, check_crc, inflate_summ.data_ptr(), qws)
         del qws
         if counter is not None:
-            counter["launches"] = counter.get("launches", 0) + inflate_launches(0, n_jobs)
+            counter["launches"] = counter.get("launches", 0) + inflate_launches(0, n_jobs, total, check_crc)
     _trace.mark(events, "inflated")
     chains = []
     base = 0
@@ -372,11 +373,11 @@ class BatchPlan:
         _trace.mark(events, "decoded")
 
     def launches_per_run(self) -> int:
-        """Kernels of this library in one :meth:`launch` (the graph holds the same)."""
+        """Kernels of this library in one :meth:`replay` (the graph's, once captured, else those of :meth:`launch`)."""
         chains = sum(1 for d in self.data if int(d.numel()))
         decodes = sum(1 for n in self.n_records if n)
-        return (KERNELS["scan"] * self.n_files + inflate_launches(self.form or 0, self.job_base[-1]) + KERNELS["chain"] * chains
-                + KERNELS["records"] * decodes)
+        inflate = inflate_launches(self.form or 0, self.job_base[-1], self.total_out, self.check_crc, self.graph is not None)
+        return KERNELS["scan"] * self.n_files + inflate + KERNELS["chain"] * chains + KERNELS["records"] * decodes
 
     def check(self) -> None:
         """Raise on any device status of the last run, or counts that differ from the plan (one sync)."""

@@ -1510,6 +1510,14 @@ extern "C" int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const 
     return cb_set_error(cudaGetLastError());
 }
 
+int cb_split_launches(int64_t n_jobs, int check_crc, bool captured);  // inflate_split.cu
+
+extern "C" int cb_inflate_launches(int64_t n_jobs, int form, int check_crc, int captured) {
+    if (n_jobs < 0 || form < 1 || form > 3) return 0;
+    if (form == 3) return cb_split_launches(n_jobs, check_crc, captured != 0);
+    return n_jobs > 0 ? 3 : 2;  // init, the persistent grid, finish
+}
+
 extern "C" int cb_inflate(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_n_jobs, uint8_t* out_base,
                           int check_crc, uint32_t* job_status, cb_inflate_summary* summary, void* workspace,
                           size_t workspace_bytes, void* stream) {

@@ -1605,13 +1605,16 @@ int launch_crc(const Call& c, Range r, cudaStream_t s) {
     return CB_OK;
 }
 
+// Whether members without matches go through k_literals: not where a member has four warps or more, whose copy takes them
+// in less than that launch and look, 8 us.
+bool takes_literals(const Call& c) { return !resident(c, copy_occupancy<split::CopyCfg<16384, 4>>()); }
+
 int copy_range(const Call& c, Range r, cudaStream_t s) {
     using C8 = split::CopyCfg<16384, 8>;
     using C4 = split::CopyCfg<16384, 4>;
     using C2 = split::CopyCfg<8192, 2>;
     const int cw = (int)cb_param(CB_PARAM_COPY_WARPS);
-    // (where members have more warps, the copy takes those of literals in less than this launch and look, 8 us)
-    if (!resident(c, copy_occupancy<C4>()))
+    if (takes_literals(c))
         split::k_literals<<<(unsigned)min((r.j1 - r.j0 + split::LOOK - 1) / split::LOOK, 32768LL), 64, 0, s>>>(
             c.jobs, c.n_jobs, c.d_n_jobs, c.out_base, c.ws, c.arena, r.j0, r.j1);
     int rc;
@@ -1701,7 +1704,28 @@ int side_for(int dev, cudaStream_t s, Side*& out) {
     return CB_OK;
 }
 
+// Pipelined: the jobs in two ranges, each decoded and then copied on its own stream, so that the second range's decode and
+// the first range's copy fill the warps that the other's end leaves idle: from 20 members per SM, where they take more than
+// one round of resident warps (3,865 GEX members 2.45 ms -> 2.12, 15,457 6.95 -> 6.72; 2,320 1.358 -> 1.366; cut at three
+// quarters 2.35 and 6.78; in four ranges 2.59 and 7.09).  Only with the job count known on the host, and under capture only
+// from 65,536 jobs (or when it is always on).
+template <class Captured> bool two_ranges(int64_t n_jobs, Captured captured) {
+    const long long pipe = cb_param(CB_PARAM_DECODE_PIPELINE);
+    if (n_jobs < 2 || pipe == 0) return false;
+    if (pipe == 2 || n_jobs >= 65536) return true;
+    return n_jobs >= 20LL * cb_device_sm_count() && !captured();
+}
+
 }  // namespace
+
+// Kernels of one call of form 3.
+int cb_split_launches(int64_t n_jobs, int check_crc, bool captured) {
+    if (n_jobs <= 0) return 2;  // init and finish
+    Call c{};
+    c.n_jobs = n_jobs;
+    const int ranges = two_ranges(n_jobs, [&] { return captured; }) ? 2 : 1;
+    return 4 + ranges * (2 + (check_crc ? 1 : 0) + (takes_literals(c) ? 1 : 0));
+}
 
 extern "C" size_t cb_inflate_split_workspace_bytes(int64_t n_jobs, int64_t out_bytes) {
     if (n_jobs < 0 || out_bytes < 0) return 0;
@@ -1733,20 +1757,7 @@ int cb_inflate_split_any(const cb_member_job* jobs, int64_t n_jobs, const int64_
     split::k_split_init<<<1, 1, 0, s>>>(summary, queue);
     if (n_jobs > 0) {
         split::k_slots<<<1, split::SLOT_NT, 0, s>>>(jobs, n_jobs, d_n_jobs, ws);
-        // Pipelined: the jobs in two ranges, each decoded and then copied on its own stream, so that
-        // the second range's decode and the first range's copy fill the warps that the other's end
-        // leaves idle: from 20 members per SM, where they take more than one round of resident warps
-        // (3,865 GEX members 2.45 ms -> 2.12, 15,457 6.95 -> 6.72; 2,320 1.358 -> 1.366; cut at three
-        // quarters 2.35 and 6.78; in four ranges 2.59 and 7.09).  Only with the job count known on the host.
-        const long long pipe = cb_param(CB_PARAM_DECODE_PIPELINE);
-        // (Below 65,536 jobs not under capture, where the side streams may be missing.)
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        bool many = n_jobs >= 65536;
-        if (!many && n_jobs >= 20LL * cb_device_sm_count()) {
-            if (cudaStreamIsCapturing(s, &cap) == cudaSuccess) many = cap == cudaStreamCaptureStatusNone;
-            else cudaGetLastError();
-        }
-        const bool two = !d_n_jobs && n_jobs >= 2 && (pipe == 2 || (pipe == 1 && many));
+        const bool two = !d_n_jobs && two_ranges(n_jobs, [&] { return capture_of(s) != 0; });
         int rc = CB_OK;
         std::unique_lock<std::mutex> lock(g_side_mu, std::defer_lock);
         Side* sd = nullptr;

@@ -190,6 +190,10 @@ int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const int64_t* d_
  * less on average. */
 int cb_inflate_default_form(int64_t n_jobs, int64_t out_bytes);
 
+/* Kernels that a call of n_jobs jobs (their number given on the host) launches in form 1, 2 or 3, on a stream that is
+ * being captured or not; 0 for other forms. */
+int cb_inflate_launches(int64_t n_jobs, int form, int check_crc, int captured);
+
 /* Members the one-member-per-lane form keeps in flight on the current device (0 on error). */
 int64_t cb_inflate_lane_slots(void);
 
