@@ -228,3 +228,64 @@ def test_jobs_may_share_their_output(jobs):
             seen.copy_(out)
         torch.cuda.synchronize()
         assert np.array_equal(seen.cpu().numpy(), want)
+
+
+def _damaged():
+    """Members of up to 65 KB with bits flipped in their headers, code lengths and symbols, cut short, or of another size or
+    CRC32 than said: (raw stream, size said, CRC32 said)."""
+    rng = random.Random(12)
+    text = b"".join(bytes(rng.choices(b"ACGTN\tchr12345:,;\n", k=40)) * rng.choice([1, 1, 2]) for _ in range(1200))[:BLOCK]
+    skew = bytes(rng.choices(range(64), weights=[1.0 / (1 << min(i, 20)) for i in range(64)], k=BLOCK))
+    bases = [(text, {}), (text, {"level": 1, "mem": 1}), (text, {"strategy": zlib.Z_FIXED}), (skew, {"strategy": zlib.Z_HUFFMAN_ONLY}),
+             (rng.randbytes(BLOCK), {}), (text[:30_000], {"flush_every": 3000})]
+    out = []
+    for data, kw in bases:
+        raw = _raw(data, **kw)
+        for region in ((0, 4), (4, 90), (90, len(raw) // 2), (len(raw) // 2, len(raw)), (len(raw) - 6, len(raw))):
+            for _ in range(3):
+                bad = bytearray(raw)
+                for _ in range(rng.randint(1, 3)):
+                    bad[rng.randrange(*region)] ^= 1 << rng.randrange(8)
+                out.append((bytes(bad), len(data), zlib.crc32(data)))
+        out.append((raw[: len(raw) * 2 // 3], len(data), zlib.crc32(data)))
+        out.append((raw[:40], len(data), zlib.crc32(data)))
+        out.append((raw, len(data) - 1, zlib.crc32(data)))
+        out.append((raw, len(data) // 2, zlib.crc32(data)))
+        out.append((raw, len(data) + 1, zlib.crc32(data)))
+        out.append((raw, len(data), zlib.crc32(data) ^ 1))
+    return out, [(_raw(d, **kw), len(d), zlib.crc32(d)) for d, kw in bases], [d for d, _ in bases]
+
+
+@pytest.mark.parametrize("jobs", [60, 400, 800, 1500, 3200])
+def test_damaged_members_at_every_width(jobs):
+    """Damaged members among good ones, at 8, 4, 2 and 1 warps per member and in two ranges: the codes of the one-kernel form,
+    the good members' bytes, and nothing written between the members' outputs."""
+    bad, good, data = _damaged()
+    gap, rng = 5, np.random.default_rng(jobs)
+    blob, at, rows, off = bytearray(), {}, [], 3
+    kinds = np.where(rng.random(jobs) < 0.5, rng.integers(0, len(bad), jobs), -1 - rng.integers(0, len(good), jobs))
+    for k in kinds.tolist():
+        raw, size, crc = bad[k] if k >= 0 else good[-1 - k]
+        if k not in at:
+            blob += bytes(18)
+            at[k] = len(blob)
+            blob += raw + bytes(8)
+        rows.append([at[k], off, len(raw) | (size << 32), crc])
+        off += size + gap
+    buf = torch.frombuffer(blob, dtype=torch.uint8).cuda()
+    table = np.array(rows, dtype=np.int64)
+    table[:, 0] += buf.data_ptr()
+    table = torch.from_numpy(table).cuda()
+    results = {}
+    for form in (1, 3):
+        out, codes, summ = _run(table, off, G.inflate_workspace_bytes(jobs, off, form), form)
+        assert summ.n_bad == int((codes != 0).sum()) and summ.first_bad == int(np.flatnonzero(codes)[0])
+        results[form] = codes, int(summ.status)
+        between = np.ones(len(out), dtype=bool)
+        for k, (_, o, w, _), code in zip(kinds.tolist(), rows, codes.tolist(), strict=True):
+            between[o : o + (w >> 32)] = False
+            if k < 0:
+                assert code == 0 and out[o : o + (w >> 32)].tobytes() == data[-1 - k]
+        assert (out[between] == 0xA5).all()
+    assert (results[1][0] == results[3][0]).all() and results[1][1] == results[3][1]
+    assert set(results[3][0].tolist()) == {_lib.OK, _lib.INFLATE, _lib.CRC}
