@@ -43,15 +43,12 @@ constexpr unsigned long long arena_and_scratch(long long n_jobs, unsigned long l
 }
 // The scratch per member of a workspace that has `room` for the two: that of the most output it is large enough for
 // (so of out_bytes, where it was made for them), or none.
-inline uint32_t scratch_for(long long n_jobs, unsigned long long room) {
-    if (arena_and_scratch(n_jobs, 0) > room) return 0;
-    unsigned long long lo = 0, hi = room / 2 + 1;  // enough for lo, not for hi
-    while (hi - lo > 1) {
-        const unsigned long long mid = lo + (hi - lo) / 2;
-        if (arena_and_scratch(n_jobs, mid) <= room) lo = mid;
-        else hi = mid;
+constexpr uint32_t scratch_for(long long n_jobs, unsigned long long room) {
+    for (uint32_t s = SCRATCH_MAX; s; s -= 4096) {
+        const unsigned long long all = (unsigned long long)in_flight(n_jobs) * s;
+        if (all <= room && scratch_bytes(n_jobs, (room - all) / 2) >= s) return s;
     }
-    return scratch_bytes(n_jobs, lo);
+    return 0;
 }
 
 }  // namespace split
