@@ -1605,9 +1605,9 @@ int launch_crc(const Call& c, Range r, cudaStream_t s) {
     return CB_OK;
 }
 
-// Whether members without matches go through k_literals: not where a member has four warps or more, whose copy takes them
-// in less than that launch and look, 8 us.
-bool takes_literals(const Call& c) { return !resident(c, copy_occupancy<split::CopyCfg<16384, 4>>()); }
+// Whether members without matches go through k_literals: not where a member has two warps or more, whose copy takes them
+// well enough (1,000 of 65 KB 583 us) and the launch and look cost the others 6 us.
+bool takes_literals(const Call& c) { return !resident(c, copy_occupancy<split::CopyCfg<8192, 2>>()); }
 
 int copy_range(const Call& c, Range r, cudaStream_t s) {
     using C8 = split::CopyCfg<16384, 8>;
