@@ -10,7 +10,7 @@ fixed columns and the CB/UB/GN tags.  The metric is GB/s of decompressed
 (uncompressed) BAM bytes, whole job over all ranks; records/s rides along.
 
 - ``value``: the batched decoder (``cubam_b200.batch``) with the compressed file
-  resident in HBM (one persistent inflate launch for all members), timed with
+  resident in HBM (one inflate call for all members), timed with
   CUDA events between barriers, max over ranks.  Inputs (4-5 GB compressed,
   12.6 GB inflated) are far larger than the 126 MB L2, so no flush is needed.
 - ``e2e``: the public API, ``cubam_b200.read_bam(path)`` from the page cache with
@@ -53,12 +53,12 @@ METRIC = "BAM decode GB/s (uncompressed) & records/s on 1 B200"
 UNIT = "GB/s"
 FALLBACK_HBM = 6650.0
 #: DRAM bytes (read + write) per inflated byte of each inflate form, from one ncu capture each of a GEX file
-#: (forms 1 and 2: 4M records, 1,008,824,685 inflated bytes; form 3: 2M records, 504,442,337); the bench scales
+#: (forms 1 and 2: 4M records, 1,008,824,685 inflated bytes; form 3: 2M records, 504,425,865); the bench scales
 #: them by its inflated bytes
 TRAFFIC_PER_BYTE = {"k_inflate_lanes": (6.916637e9 + 1.003612e9) / 1.008824685e9,
                     "k_inflate_warp": (1.593613e9 + 1.004537e9) / 1.008824685e9,
-                    "k_decode + k_copy + k_crc": (539.836416e6 + 662.705408e6 + 535.985408e6 + 456.324352e6 + 505.957120e6
-                                                  + 3.871744e6) / 504.442337e6}
+                    "k_decode + k_copy + k_crc": (517.089536e6 + 617.955072e6 + 530.711552e6 + 455.931392e6 + 505.952256e6
+                                                  + 3.588352e6 + 0.513280e6) / 504.425865e6}
 
 
 def parse():
@@ -421,7 +421,7 @@ def run_ours(args):
             "members": n_members,
             "records": n_rec,
             "tags": list(tags),
-            "form": "batched: whole file resident, one persistent inflate launch",
+            "form": "batched: whole file resident, one inflate call",
             "l2": "inputs larger than L2 (no flush)",
             "parallelism": f"replicas x{world}",
             "generate_s": round(gen_s, 1),

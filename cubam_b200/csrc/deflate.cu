@@ -27,8 +27,8 @@
 // k_offsets (one CTA) sums the stream sizes into output offsets; k_pack copies each slot to its
 // offset, with the BGZF header and trailer when framing.
 //
-// What bounds k_deflate is the issue of instructions between barriers (0.5 per cycle and scheduler; two
-// CTAs per SM by shared memory, 64 registers): per span about 170,000 cycles for the hash heads, 145,000 for
+// What bounds k_deflate is the issue of instructions between barriers (0.58 per cycle and scheduler; two
+// CTAs per SM by shared memory, 64 registers): per span about 185,000 cycles for the hash heads, 145,000 for
 // the matches, 310,000 for the parse and its tokens, 55,000 for the codes, 85,000 for the bits.  Measured on 64 MB of
 // GEX records in 1,024 spans: 1.88 ms (2.39 with a parse of twelve barriers per tile, each position
 // comparing for itself, a serial merge that waited for each load, an atomic per token and tables for the

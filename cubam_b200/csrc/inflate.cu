@@ -1475,7 +1475,8 @@ extern "C" int cb_inflate_form(const cb_member_job* jobs, int64_t n_jobs, const 
     if (form == 0) {
         const size_t empty = cb_inflate_split_workspace_bytes(n_jobs, 0);
         // the members' bytes, as far as the workspace tells
-        const int64_t out_bytes = n_jobs < ANY_WORKSPACE_JOBS && workspace_bytes >= empty ? (int64_t)(workspace_bytes - empty) / 2 : -1;
+        const bool tells = n_jobs < ANY_WORKSPACE_JOBS && workspace_bytes >= empty;
+        const int64_t out_bytes = tells ? (int64_t)(workspace_bytes - empty) / 2 : -1;
         form = cb_inflate_default_form(n_jobs, out_bytes);
         any_workspace = form == 3 && n_jobs < ANY_WORKSPACE_JOBS;
         if (any_workspace && workspace_bytes < empty) form = 1;

@@ -1,4 +1,4 @@
-// Raw-DEFLATE inflater for BGZF members, form 3: the Huffman decode and the copy in two kernels.
+// Raw-DEFLATE inflater for BGZF members, form 3: the Huffman decode, the copy and the CRC32 as kernels of their own.
 //
 // Replaces cubam's nvcompBatchedDeflateDecompressAsync call and its status/size check
 // (src/cubam/bgzf.py:587-611) with the CRC32 check added (cubam's reader does not check it,
@@ -7,12 +7,14 @@
 //  1. k_decode: one member per CTA of W warps (W = 8, 4, 2 or 1, fewer the more members there are), its
 //     32 W lanes decoding as many segments of the member's bits at once.  A Huffman decoder that starts
 //     at a wrong bit falls in step with the true symbols soon (on BAM members after 64 bits in half of
-//     the cases, after 512 in 99.5% and after 768 in 99.97%), so every lane starts OVERLAP bits before its segment and notes the
-//     first symbol that begins in it; that must be where the lane before stopped, and a lane for which
-//     it is not decodes its segment again from there.  The lanes share one set of code tables in shared
-//     memory.  Each lane writes its symbols, literal bytes and 4-byte sequences of a literal count and
-//     a match, to a run of its own in the scratch of the members in flight; the warps
-//     then put the runs together in the member's slot of an arena in HBM.
+//     the cases, after 512 in 99.5% and after 768 in 99.97%), so every lane starts OVERLAP bits before its
+//     segment and notes the first symbol that begins in it; that must be where the lane before stopped, and
+//     a lane for which it is not decodes its segment again from there.  (Codes of nearly one length do not
+//     fall in step: uniform 7-bit bytes need up to 12 such passes at one warp and 92 at eight, and 20,000
+//     members of 65 KB of them take 40 ms, 26 with a member per lane; as many of BAM records 7.4.)  The lanes
+//     share one set of code tables in shared memory.  Each lane writes its symbols, literal bytes and 4-byte
+//     sequences of a literal count and a match, to a run of its own in the scratch of the members in flight;
+//     the warps then put the runs together in the member's slot of an arena in HBM.
 //     k_literals copies the members that have no match.
 //  2. k_copy: one member per CTA of W warps.  They take 64 W sequences at a time, place them by a prefix
 //     sum of their lengths and write the output in rounds of 128 bytes per warp, a 4-byte word per lane,
@@ -21,10 +23,10 @@
 //  4. Members whose symbols do not fit their slot are inflated by the one-kernel form
 //     (cb_inflate_listed, inflate.cu).
 //
-// What bounds them: with many members the issue of instructions (decode 0.53 per cycle and scheduler at 18
-// warps per SM, copy 0.68 at 22, by shared memory); with few, the chain of steps of one lane and of rounds of one member,
-// which is why a member takes more warps then.  Measured, in ms (one serial decoder per member, in one
-// kernel, before; a warp per member in between):
+// What bounds them: with many members the issue of instructions (decode 0.53 per cycle and scheduler, copy
+// 0.68, at the 18 and 22 warps per SM that fit, of which 16.4 and 18.9 were active); with few, the chain of
+// steps of one lane and of rounds of one member, which is why a member takes more warps then.  Measured, in
+// ms (one serial decoder per member, in one kernel, before; a warp per member in between):
 //   39 GEX members (10,000 records)      decode 0.17 (0.46), copy 0.15 (0.43), CRC32 0.01; one kernel 4.2
 //   about 70,000 (18 million records)    decode 12.6, copy 13.6, CRC32 1.9; all of it 47 with a member per lane
 //

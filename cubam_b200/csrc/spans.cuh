@@ -1,5 +1,5 @@
-// Copies of byte spans (at most MAX_SPAN bytes at a time) at any alignment by words, each lane's share a host function too (checked there against
-// pages that may not be touched).
+// Copies of byte spans (at most MAX_SPAN bytes at a time) at any alignment, each lane's share a host function too
+// (checked there against pages that may not be touched).
 #pragma once
 
 #include "common.cuh"

@@ -343,7 +343,9 @@ class Server:
     """Continuous batching of decode requests (see the module docstring).
 
     ``budget_bytes`` is the HBM the in-flight requests may hold: the pool for their inflated bytes
-    is ``pool_frac`` of it, the rest bounds their offsets, columns and tags.  A step holds up to
+    is ``pool_frac`` of it, the rest bounds their offsets, columns and tags.  Beside it two steps' scratch
+    is held: for each the inflater's workspace (twice the step's inflated bytes and up to 350 MB; about
+    14 GB for the two at the default step size) and the record chain's.  A step holds up to
     ``step_bytes`` compressed bytes, or ``short_step_bytes`` while a request of at most
     ``small_bytes`` waits to start: shorter steps for a small request's latency, longer ones for
     throughput.
@@ -462,6 +464,8 @@ class Server:
             r, rf = sl.req, self.files[sl.req.file]
             ix = rf.index
             if sl.mb > sl.ma:
+                # the member that a slice's last record ends in is inflated again by the next step, to the same
+                # place and bytes, on the one stream of all steps
                 last = sl.mb if (sl.mb < rf.n_members and int(ix.first_rec[sl.mb]) > 0) else sl.mb - 1
                 rows.append(_job_rows(rf, sl.ma, last, r._region, r.m0))
         n_jobs = sum(len(x) for x in rows)

@@ -199,10 +199,11 @@ int64_t cb_inflate_lane_slots(void);
 
 /* ---- Inflate, form 3: the Huffman decode, the copy and the CRC32 as three kernels (same contract as
  *      cb_inflate, replacing the same nvCOMP call, src/cubam/bgzf.py:587-611) ------------------------
- * Each takes a member per 1 to 8 warps, more the fewer jobs there are.  The decode's lanes decode 32
- * segments per warp at once into an arena inside the workspace (32 bytes and a slot of 2 isize + 64 bytes per job,
- * rounded up to 16, and scratch of 4 to 64 KiB for each of at most 5,328 members in flight); the copy writes the member through
- * a window in shared memory (CB_PARAM_COPY_WARPS, where a member has one warp).
+ * Each takes a member per 1 to 8 warps, more the fewer jobs there are.  The decode's lanes decode 32 segments
+ * per warp at once into an arena inside the workspace (32 bytes and a slot of 2 isize + 64 bytes per job, rounded
+ * up to 16, and scratch of 4 to 64 KiB for each of at most 5,328 members in flight); the copy writes the member
+ * through a window in shared memory (CB_PARAM_COPY_WARPS, where a member has one warp), and of a valid member
+ * nothing but its final bytes, so jobs of the same bytes may share their output.
  * out_bytes: the sum of isize over the jobs (or more); a job whose slot does not fit a smaller
  * workspace fails with CB_ERR_CAPACITY. */
 size_t cb_inflate_split_workspace_bytes(int64_t n_jobs, int64_t out_bytes);
